@@ -245,6 +245,30 @@ __device__ __forceinline__ float sqdist_exact_src(const Src &src, int64_t i, con
     return acc;
 }
 
+// The exact float32 distance of one row pair by a whole warp: lanes load and
+// square 32 features at a time (coalesced), and the 32 squares go to every
+// lane in feature order by shuffles, so each lane adds them in the oracle's
+// sequence: the result is sqdist_exact's, bit for bit, in every lane.  One
+// thread walking the row waits on memory for every group of loads; here the
+// wait is shared by 32 lanes.
+template <class Src>
+__device__ __forceinline__ float warp_sqdist_exact(const Src &src, int64_t i, const float *__restrict__ c, int d,
+                                                   int lane) {
+    float acc = 0.0f;
+    for (int f0 = 0; f0 < d; f0 += 32) {
+        const int f = f0 + lane;
+        const float q = f < d ? sq_term(src.get(i, f), __ldg(c + f)) : 0.0f;
+        const int fw = min(32, d - f0);
+        if (fw == 32) {
+#pragma unroll
+            for (int l = 0; l < 32; ++l) acc = __fadd_rn(acc, __shfl_sync(0xffffffffu, q, l));
+        } else {
+            for (int l = 0; l < fw; ++l) acc = __fadd_rn(acc, __shfl_sync(0xffffffffu, q, l));
+        }
+    }
+    return acc;
+}
+
 // Neumaier-compensated float32 sum: value() is within a few u of the exact
 // sum of the added terms (plus an O(n u^2) remainder).
 struct CSum {
