@@ -14,11 +14,19 @@
 // Layout: frames and centers are centered once into float copies with their
 // traces G (double).  The centered centers are also stored transposed
 // (feature-major, k padded to 32) so that the lanes of a warp, one center
-// each, read them coalesced.  The assignment kernel gives one warp to one
-// frame: the frame's coordinates are the same for every lane (broadcast
-// loads), each lane accumulates the nine correlation sums of its center in
-// atom order, solves the QCP quartic in double, and the warp keeps the
-// lowest-index minimum.
+// each, read them coalesced.
+//
+// Assignment: the double QCP solve is the expensive part of a pair (about 180
+// float64 operations, and this part runs two of them per SM and clock), and
+// almost every center is far from being the nearest.  So a warp takes several
+// frames, every lane the nine float correlation sums of its center with each
+// of them, and a float32 bracket of the largest root (qcp_bracket) gives a
+// lower and an upper bound of every msd.  Only the centers whose lower bound
+// does not exceed the frame's smallest upper bound are solved in double, with
+// the same sums and operations as before, so labels and distances are the
+// same bit for bit.
+#include <algorithm>
+
 #include "km_common.cuh"
 #include "km_internal.h"
 #include "km_rmsd.cuh"
@@ -29,7 +37,8 @@ namespace {
 
 constexpr int kRmsdWarps = 8;  // warps per CTA
 
-// Every row of an (n, d) array centered into Xc, traces into G.
+// Every row of an (n, d) array centered into Xc, traces into G: a warp per
+// row.  For rows too long for rmsd_center_tile_kernel.
 __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_center_kernel(const float *__restrict__ X, int64_t n, int d,
                                                                       float *__restrict__ Xc, double *__restrict__ G) {
     const int lane = threadIdx.x & 31;
@@ -37,6 +46,107 @@ __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_center_kernel(const floa
     for (int64_t r = (int64_t)blockIdx.x * kRmsdWarps + (threadIdx.x >> 5); r < n; r += nw) {
         const double g = rmsd_center_row_warp(X + r * d, d / 3, Xc + r * d);
         if (lane == 0) G[r] = g;
+    }
+}
+
+// The same with one thread per row: a warp stages its 32 rows in shared
+// memory (coalesced; odd row stride), and each thread adds its row in the
+// order of rmsd_center_row_warp (32 partial sums, then the butterfly's tree),
+// so the results are the same bit for bit.  The warp-per-row form repeats the
+// divisions and the tree in all 32 lanes, at 64 cycles per float64
+// instruction: 5.9 ms for 1,000,000 rows of 58 atoms; this one kCenterMs.
+constexpr int kCenterMaxSmem = 200 * 1024;
+
+int center_stride(int d) { return d | 1; }
+int center_warps(int d) {  // warps per CTA; 0: the rows do not fit
+    const int64_t per = (int64_t)32 * center_stride(d) * 4;
+    const int64_t w = kCenterMaxSmem / per;
+    return w >= 4 ? 2 : (int)std::min<int64_t>(w, 1);
+}
+
+// The tree of rmsd_center_row_warp over 32 partial sums part(l).
+template <class Part>
+__device__ __forceinline__ double rmsd_tree32(const Part &part) {
+    double r[8];
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+        r[l] = __dadd_rn(__dadd_rn(part(l), part(l + 16)), __dadd_rn(part(l + 8), part(l + 24)));
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int l = 0; l < h; ++l) r[l] = __dadd_rn(r[l], r[l + h]);
+    return r[0];
+}
+
+__global__ void rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, int d, int stride,
+                                        float *__restrict__ Xc, double *__restrict__ G) {
+    extern __shared__ float center_smem[];
+    const int lane = threadIdx.x & 31;
+    const int warps = blockDim.x >> 5;
+    float *rows = center_smem + (size_t)(threadIdx.x >> 5) * 32 * stride;
+    const int n_atoms = d / 3;
+    const int64_t tiles = (n + 31) / 32;
+    for (int64_t t = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); t < tiles; t += (int64_t)gridDim.x * warps) {
+        const int64_t r0 = t * 32;
+        const int m = (int)(n - r0 < 32 ? n - r0 : 32);
+        // the tile's rows are consecutive floats; eight loads in flight per lane
+        const float *src = X + r0 * d;
+        const int total = m * d;
+        int f = lane % d, r = lane / d;
+        for (int e0 = lane; e0 < total; e0 += 256) {
+            float v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = e0 + 32 * q < total ? __ldg(src + e0 + 32 * q) : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (e0 + 32 * q < total) rows[r * stride + f] = v[q];
+                f += 32;
+                while (f >= d) {
+                    f -= d;
+                    ++r;
+                }
+            }
+        }
+        __syncwarp();
+        if (lane < m) {
+            float *x = rows + lane * stride;
+            double mean[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double sum = rmsd_tree32([&](int l) {
+                    double acc = 0.0;
+                    for (int i = l; i < n_atoms; i += 32) acc = __dadd_rn(acc, (double)x[3 * i + c]);
+                    return acc;
+                });
+                mean[c] = __ddiv_rn(sum, (double)n_atoms);
+            }
+            const double g = rmsd_tree32([&](int l) {
+                double acc = 0.0;
+                for (int i = l; i < n_atoms; i += 32) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float v = __double2float_rn(__dsub_rn((double)x[3 * i + c], mean[c]));
+                        x[3 * i + c] = v;
+                        // the square of a float is exact in double: one rounding, as product then sum
+                        acc = __fma_rn((double)v, (double)v, acc);
+                    }
+                }
+                return acc;
+            });
+            G[r0 + lane] = g;
+        }
+        __syncwarp();
+        f = lane % d;
+        r = lane / d;
+        for (int e = lane; e < total; e += 32) {
+            Xc[r0 * d + e] = rows[r * stride + f];
+            f += 32;
+            while (f >= d) {
+                f -= d;
+                ++r;
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -57,58 +167,369 @@ __device__ __forceinline__ bool rmsd_better(double m, int j, double bm, int bj) 
     return m < bm || (m == bm && j < bj);
 }
 
-__global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_assign_kernel(
+// The nearest center of one frame with every pair solved in double, by one
+// warp (lanes own centers); (msd, index) in every lane.
+__device__ __forceinline__ void rmsd_full_frame(const float *__restrict__ a, double ga, int n_atoms,
+                                                const float *__restrict__ Ct, const double *__restrict__ H, int k,
+                                                int kp, int lane, double &bm, int &bj) {
+    bm = 0.0;
+    bj = -1;
+    for (int j0 = 0; j0 < k; j0 += 32) {
+        const int j = j0 + lane;  // j < kp: the padding centers are zero rows
+        float S[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) S[e] = 0.0f;
+        const float *b = Ct + j;
+        for (int i = 0; i < n_atoms; ++i) {
+            const float a0 = a[3 * i], a1 = a[3 * i + 1], a2 = a[3 * i + 2];
+            const float b0 = b[(int64_t)(3 * i) * kp], b1 = b[(int64_t)(3 * i + 1) * kp],
+                        b2 = b[(int64_t)(3 * i + 2) * kp];
+            S[0] = __fmaf_rn(a0, b0, S[0]);
+            S[1] = __fmaf_rn(a0, b1, S[1]);
+            S[2] = __fmaf_rn(a0, b2, S[2]);
+            S[3] = __fmaf_rn(a1, b0, S[3]);
+            S[4] = __fmaf_rn(a1, b1, S[4]);
+            S[5] = __fmaf_rn(a1, b2, S[5]);
+            S[6] = __fmaf_rn(a2, b0, S[6]);
+            S[7] = __fmaf_rn(a2, b1, S[7]);
+            S[8] = __fmaf_rn(a2, b2, S[8]);
+        }
+        if (j < k) {
+            const double m = qcp_msd(S, ga, H[j], n_atoms);
+            if (rmsd_better(m, j, bm, bj)) {
+                bm = m;
+                bj = j;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double om = __shfl_xor_sync(0xffffffffu, bm, off);
+        const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
+        if (rmsd_better(om, oj, bm, bj)) {
+            bm = om;
+            bj = oj;
+        }
+    }
+}
+
+__device__ __forceinline__ void rmsd_store(int64_t r, double bm, int bj, int32_t *__restrict__ labels,
+                                           float *__restrict__ rmsd) {
+    labels[r] = bj < 0 ? 0 : bj;
+    if (rmsd) rmsd[r] = bj < 0 ? __int_as_float(0x7fc00000) : __double2float_rn(sqrt(bm));
+}
+
+// One warp per frame, every pair solved in double.  For one or two atoms,
+// whose correlation matrices have rank at most one: the largest root is then
+// a double root, and qcp_bracket never holds.
+__global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_assign_full_kernel(
     const float *__restrict__ Xc, const double *__restrict__ G, int64_t n, int d, const float *__restrict__ Ct,
     const double *__restrict__ H, int k, int kp, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
     const int lane = threadIdx.x & 31;
-    const int n_atoms = d / 3;
     const int64_t nw = (int64_t)gridDim.x * kRmsdWarps;
     for (int64_t r = (int64_t)blockIdx.x * kRmsdWarps + (threadIdx.x >> 5); r < n; r += nw) {
-        const float *a = Xc + r * d;
-        const double ga = G[r];
-        double bm = 0.0;
-        int bj = -1;
+        double bm;
+        int bj;
+        rmsd_full_frame(Xc + r * d, G[r], d / 3, Ct, H, k, kp, lane, bm, bj);
+        if (lane == 0) rmsd_store(r, bm, bj, labels, rmsd);
+    }
+}
+
+// A bracket of E = Ga + Gb - 2 lambda (n_atoms times the msd before it is
+// clipped at 0) from the correlation sums S in float32: lb <= E_qcp <= ub for
+// the lambda that qcp_msd finds.  tot: Ga + Gb rounded to float (within 3 u).
+//
+// With s = ||S||_F and T = S / s the quartic of the key matrix is
+//   P(x) = x^4 - 2 x^2 - 8 det(T) x + (2 ||T T^t||_F^2 - 1),
+// lambda = s x for its largest root x <= sqrt(3).  (Its constant term is the
+// product of the key matrix's eigenvalues.)  u = 2^-24.  ||T||^2 = 1 within
+// 20 u; the float values of the coefficients are off by at most 40 u, 64 u
+// and 75 u, and P at 0 < x <= 1.75 by at most 120 + 110 + 75 + 45 = 350 u: e
+// below allows 512 u.  All roots are real, so
+//   P(x) > 0, P'(x) > 0, P''(x) > 0 (x > 0.6)  =>  x is above every root;
+//   P(x) < 0                                   =>  x is below the largest.
+// Both tests are made on the float value with the margin e, at points found
+// by five Newton steps from above.  P' is required to be 0.05 at least: there
+// the double Newton of qcp_msd converges to the root within 1e-10 of s.  The
+// roundings of s, T and the final sum are below 64 u tot.
+// Where a test fails (an ill-conditioned root, sums outside the range in
+// which qcp_msd's float reciprocal is normal, a value that is not finite) the
+// bound is 0 or infinity and the pair is solved in double.
+__device__ __forceinline__ void qcp_bracket(const float (&S)[9], float tot, float &lb, float &ub) {
+    constexpr float kErr = 512.0f * 5.9604645e-8f;
+    lb = 0.0f;
+    ub = __int_as_float(0x7f800000);
+    float ss = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) ss = fmaf(S[e], S[e], ss);
+    const float rs = rsqrtf(ss);
+    const float s = ss * rs;
+    float T[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) T[e] = S[e] * rs;
+    const float m0 = fmaf(T[4], T[8], -T[5] * T[7]);
+    const float m1 = fmaf(T[3], T[8], -T[5] * T[6]);
+    const float m2 = fmaf(T[3], T[7], -T[4] * T[6]);
+    const float C1 = -8.0f * fmaf(T[0], m0, fmaf(T[2], m2, -T[1] * m1));
+    const float b00 = fmaf(T[0], T[0], fmaf(T[1], T[1], T[2] * T[2]));
+    const float b11 = fmaf(T[3], T[3], fmaf(T[4], T[4], T[5] * T[5]));
+    const float b22 = fmaf(T[6], T[6], fmaf(T[7], T[7], T[8] * T[8]));
+    const float b01 = fmaf(T[0], T[3], fmaf(T[1], T[4], T[2] * T[5]));
+    const float b02 = fmaf(T[0], T[6], fmaf(T[1], T[7], T[2] * T[8]));
+    const float b12 = fmaf(T[3], T[6], fmaf(T[4], T[7], T[5] * T[8]));
+    const float diag = fmaf(b00, b00, fmaf(b11, b11, b22 * b22));
+    const float offd = fmaf(b01, b01, fmaf(b02, b02, b12 * b12));
+    const float C0 = fmaf(2.0f, fmaf(2.0f, offd, diag), -1.0f);
+    float x = fminf(1.7320509f, __fdividef(0.500001f * tot, s));
+    float P, D;
+    auto eval = [&](float y) {
+        const float l2 = y * y;
+        const float a2 = l2 - 2.0f;
+        P = fmaf(a2, l2, fmaf(C1, y, C0));
+        D = fmaf(2.0f * y, l2 + a2, C1);
+    };
+#pragma unroll
+    for (int it = 0; it < 5; ++it) {
+        eval(x);
+        x -= __fdividef(P, D);
+    }
+    eval(x);
+    const float inv = __fdividef(1.0f, D);
+    const float xu = x + fmaf(fmaxf(-P, 0.0f), 1.01f * inv, 2.5f * kErr * inv);
+    const float xl = x - fmaf(fmaxf(P, 0.0f), 1.01f * inv, 2.5f * kErr * inv);
+    const bool fine = ss >= 1e-22f && ss <= 1e30f && D >= 0.05f && x > 0.6f && xu < 1.75f && tot <= 1e37f;
+    eval(xu);
+    const bool above = P > kErr && D >= 0.04f;
+    eval(xl);
+    const bool below = P < -kErr && xl > 0.0f;
+    const float slack = 64.0f * 5.9604645e-8f * tot;
+    if (fine && above) lb = fmaxf(fmaf(-2.0f * xu, s, tot) - slack, 0.0f);
+    if (fine && below) ub = fmaxf(fmaf(-2.0f * xl, s, tot) + slack, 0.0f);
+}
+
+// Two float32 fused multiply-adds in one instruction.
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// The assignment: a warp takes F frames at a time and walks the centers in
+// groups of 32, one per lane.  The frames' coordinates lie in shared memory
+// atom by atom with the F frames side by side, so that one broadcast load
+// serves two frames' packed multiply-adds; each center coordinate, read once
+// from L1/L2, serves all F frames (9 F multiply-adds per 3 loads).
+// Per frame a list of the centers whose lower bound does not exceed the
+// smallest upper bound so far, with their correlation sums; at the end the
+// lists of all F frames are solved in double, one entry per lane.  A frame
+// whose list runs over (near-ties, or pairs without a bracket) has all its
+// pairs solved in double.
+// Bound by the FP32 pipe: 9 n_atoms multiply-adds and about 140 operations of
+// the bracket per pair.  1,000,000 frames of 58 atoms, k = 100: kAssignMs,
+// where solving every pair in double took 68.6 ms.
+constexpr int kRmsdAtoms = 96;  // atoms staged at a time
+constexpr int kRmsdList = 8;    // candidates kept per frame
+
+template <int F>
+struct RmsdWarpSmem {
+    // [atom][axis][frame]; the row of 3 F floats is padded by 4 (fewer store conflicts)
+    float a[kRmsdAtoms][3 * F + 4];
+    float S[F][kRmsdList][9];
+    float lb[F][kRmsdList];
+    int32_t j[F][kRmsdList];
+    double ga[F];
+    int32_t cnt[F];   // entries listed
+    int32_t full[F];  // the list ran over
+};
+
+template <int F>
+__global__ void __launch_bounds__(kRmsdWarps * 32, 2) rmsd_assign_kernel(
+    const float *__restrict__ Xc, const double *__restrict__ G, int64_t n, int d, const float *__restrict__ Ct,
+    const double *__restrict__ H, int k, int kp, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
+    static_assert(F % 4 == 0, "frames go in fours (16-byte shared loads)");
+    extern __shared__ __align__(16) unsigned char rmsd_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    RmsdWarpSmem<F> &sm = reinterpret_cast<RmsdWarpSmem<F> *>(rmsd_smem)[warp];
+    const int n_atoms = d / 3;
+    const int64_t tiles = (n + F - 1) / F;
+    const float kInf = __int_as_float(0x7f800000);
+    auto stage = [&](int64_t r0, int i0, int cnt) {
+        __syncwarp();
+        for (int i = lane; i < cnt; i += 32)
+#pragma unroll
+            for (int f = 0; f < F; ++f) {
+                const bool in = r0 + f < n;
+                const float *src = Xc + (in ? r0 + f : r0) * d + 3 * (i0 + i);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sm.a[i][c * F + f] = __ldg(src + c);
+            }
+        __syncwarp();
+    };
+    for (int64_t t = (int64_t)blockIdx.x * kRmsdWarps + warp; t < tiles; t += (int64_t)gridDim.x * kRmsdWarps) {
+        const int64_t r0 = t * F;
+        if (n_atoms <= kRmsdAtoms) stage(r0, 0, n_atoms);
+        if (lane < F) {
+            sm.ga[lane] = G[r0 + lane < n ? r0 + lane : r0];
+            sm.cnt[lane] = 0;
+            sm.full[lane] = 0;
+        }
+        __syncwarp();
+        float best[F];  // smallest upper bound so far
+#pragma unroll
+        for (int f = 0; f < F; ++f) best[f] = kInf;
         for (int j0 = 0; j0 < k; j0 += 32) {
             const int j = j0 + lane;  // j < kp: the padding centers are zero rows
-            float S[9];
+            unsigned long long S2[F / 2][9];
 #pragma unroll
-            for (int e = 0; e < 9; ++e) S[e] = 0.0f;
-            const float *b = Ct + j;
-            for (int i = 0; i < n_atoms; ++i) {
-                const float a0 = a[3 * i], a1 = a[3 * i + 1], a2 = a[3 * i + 2];
-                const float b0 = b[(int64_t)(3 * i) * kp], b1 = b[(int64_t)(3 * i + 1) * kp],
-                            b2 = b[(int64_t)(3 * i + 2) * kp];
-                S[0] = __fmaf_rn(a0, b0, S[0]);
-                S[1] = __fmaf_rn(a0, b1, S[1]);
-                S[2] = __fmaf_rn(a0, b2, S[2]);
-                S[3] = __fmaf_rn(a1, b0, S[3]);
-                S[4] = __fmaf_rn(a1, b1, S[4]);
-                S[5] = __fmaf_rn(a1, b2, S[5]);
-                S[6] = __fmaf_rn(a2, b0, S[6]);
-                S[7] = __fmaf_rn(a2, b1, S[7]);
-                S[8] = __fmaf_rn(a2, b2, S[8]);
+            for (int q = 0; q < F / 2; ++q)
+#pragma unroll
+                for (int e = 0; e < 9; ++e) S2[q][e] = 0ull;
+            for (int i0 = 0; i0 < n_atoms; i0 += kRmsdAtoms) {
+                const int cnt = min(kRmsdAtoms, n_atoms - i0);
+                if (n_atoms > kRmsdAtoms) stage(r0, i0, cnt);
+                const float *b = Ct + (int64_t)(3 * i0) * kp + j;
+#pragma unroll 2
+                for (int i = 0; i < cnt; ++i) {
+                    unsigned long long bb[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float v = __ldg(b + (int64_t)(3 * i + c) * kp);
+                        bb[c] = pack2(v, v);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int q = 0; q < F / 4; ++q) {
+                            const ulonglong2 av = *reinterpret_cast<const ulonglong2 *>(&sm.a[i][c * F + 4 * q]);
+#pragma unroll
+                            for (int e = 0; e < 3; ++e) {
+                                fma2(S2[2 * q][3 * c + e], av.x, bb[e]);
+                                fma2(S2[2 * q + 1][3 * c + e], av.y, bb[e]);
+                            }
+                        }
+                }
             }
-            if (j < k) {
-                const double m = qcp_msd(S, ga, H[j], n_atoms);
-                if (rmsd_better(m, j, bm, bj)) {
-                    bm = m;
-                    bj = j;
+            const float hj = j < k ? (float)H[j] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < F / 2; ++q) {
+                float Sp[2][9];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) unpack2(S2[q][e], Sp[0][e], Sp[1][e]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int f = 2 * q + h;
+                    float lb, ub;
+                    qcp_bracket(Sp[h], (float)sm.ga[f] + hj, lb, ub);
+                    if (j >= k) ub = kInf;
+                    // non-negative floats order as their bits
+                    best[f] = fminf(best[f], __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(ub))));
+                    const unsigned cand = __ballot_sync(0xffffffffu, j < k && lb <= best[f]);
+                    if (cand == 0u) continue;
+                    // Append; when the list would run over, first drop the
+                    // entries that the bound rules out by now.
+                    int cnt = sm.cnt[f];
+                    if (cnt + __popc(cand) > kRmsdList && cnt <= kRmsdList) {
+                        float l = kInf, Sl[9];
+                        int jl = -1;
+                        if (lane < cnt) {
+                            l = sm.lb[f][lane];
+                            jl = sm.j[f][lane];
+#pragma unroll
+                            for (int e = 0; e < 9; ++e) Sl[e] = sm.S[f][lane][e];
+                        }
+                        const unsigned keep = __ballot_sync(0xffffffffu, lane < cnt && l <= best[f]);
+                        __syncwarp();
+                        if ((keep >> lane) & 1u) {
+                            const int to = __popc(keep & ((1u << lane) - 1u));
+                            sm.lb[f][to] = l;
+                            sm.j[f][to] = jl;
+#pragma unroll
+                            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = Sl[e];
+                        }
+                        cnt = __popc(keep);
+                    }
+                    if ((cand >> lane) & 1u) {
+                        const int to = cnt + __popc(cand & ((1u << lane) - 1u));
+                        if (to < kRmsdList) {
+                            sm.lb[f][to] = lb;
+                            sm.j[f][to] = j;
+#pragma unroll
+                            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = Sp[h][e];
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        sm.cnt[f] = min(cnt + __popc(cand), kRmsdList);
+                        if (cnt + __popc(cand) > kRmsdList) sm.full[f] = 1;
+                    }
+                    __syncwarp();
                 }
             }
         }
+        // Lane f < F keeps frame f's best; lane e solves entry e of the
+        // frames' lists laid end to end.
+        float my_best = kInf;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double om = __shfl_xor_sync(0xffffffffu, bm, off);
-            const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
-            if (rmsd_better(om, oj, bm, bj)) {
-                bm = om;
-                bj = oj;
+        for (int f = 0; f < F; ++f)
+            if (lane == f) my_best = best[f];
+        const bool mine = lane < F && r0 + lane < n && !sm.full[lane < F ? lane : 0];
+        const int my_cnt = mine ? sm.cnt[lane] : 0;
+        int end = my_cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, end, off);
+            if (lane >= off) end += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        double bm = 0.0;
+        int bj = -1;
+        for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = e0 + lane;
+            // the frame whose range holds e
+            int f = 0;
+#pragma unroll
+            for (int q = 0; q < F; ++q) f += e >= __shfl_sync(0xffffffffu, end, q) ? 1 : 0;
+            const int first = __shfl_sync(0xffffffffu, end - my_cnt, f < F ? f : 0);
+            const float ubf = __shfl_sync(0xffffffffu, my_best, f < F ? f : 0);
+            double m = 0.0;
+            int j = -1;
+            if (e < total) {
+                const int slot = e - first;
+                if (sm.lb[f][slot] <= ubf) {
+                    j = sm.j[f][slot];
+                    float S[9];
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) S[q] = sm.S[f][slot][q];
+                    m = qcp_msd(S, sm.ga[f], H[j], n_atoms);
+                }
+            }
+            // every frame's lane collects its entries of this round
+            for (int q = 0; q < 32; ++q) {
+                const double om = __shfl_sync(0xffffffffu, m, q);
+                const int oj = __shfl_sync(0xffffffffu, j, q);
+                const int x = e0 + q;
+                if (x >= total) break;
+                if (x >= end - my_cnt && x < end && rmsd_better(om, oj, bm, bj)) {
+                    bm = om;
+                    bj = oj;
+                }
             }
         }
-        if (lane == 0) {
-            labels[r] = bj < 0 ? 0 : bj;
-            if (rmsd) rmsd[r] = bj < 0 ? __int_as_float(0x7fc00000) : __double2float_rn(sqrt(bm));
+        if (mine) rmsd_store(r0 + lane, bm, bj, labels, rmsd);
+        for (int f = 0; f < F; ++f) {
+            if (!sm.full[f] || r0 + f >= n) continue;
+            double fm;
+            int fj;
+            rmsd_full_frame(Xc + (r0 + f) * d, sm.ga[f], n_atoms, Ct, H, k, kp, lane, fm, fj);
+            if (lane == 0) rmsd_store(r0 + f, fm, fj, labels, rmsd);
         }
+        __syncwarp();
     }
 }
 
@@ -175,7 +596,23 @@ int check_rmsd_shape(int64_t n, int d, int k) {
 
 int center_rows(const float *X, int64_t n, int d, float *Xc, double *G, cudaStream_t s) {
     if (n == 0) return KM_OK;
-    rmsd_center_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(X, n, d, Xc, G);
+    const int warps = center_warps(d);
+    if (warps > 0) {
+        static bool attr_done[kDeviceSlots] = {};
+        const int dev = current_device();
+        if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
+            KM_CUDA(cudaFuncSetAttribute(rmsd_center_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kCenterMaxSmem));
+            if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
+        }
+        const size_t smem = (size_t)warps * 32 * center_stride(d) * sizeof(float);
+        int64_t g = ((n + 31) / 32 + warps - 1) / warps;
+        const int64_t cap = (int64_t)num_sms() * 16;
+        if (g > cap) g = cap;
+        rmsd_center_tile_kernel<<<(unsigned)g, warps * 32, smem, s>>>(X, n, d, center_stride(d), Xc, G);
+    } else {
+        rmsd_center_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(X, n, d, Xc, G);
+    }
     KM_CUDA(cudaGetLastError());
     return KM_OK;
 }
@@ -191,13 +628,37 @@ int prepare_centers(const float *C, int d, int k, const RmsdCenters &rc, cudaStr
     return KM_OK;
 }
 
+template <int F>
+int launch_rmsd_assign_f(const float *Xc, const double *G, int64_t n, int d, const RmsdCenters &rc, int k,
+                         int32_t *labels, float *rmsd, cudaStream_t s) {
+    const size_t smem = sizeof(RmsdWarpSmem<F>) * kRmsdWarps;
+    static bool attr_done[kDeviceSlots] = {};
+    const int dev = current_device();
+    if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
+        KM_CUDA(cudaFuncSetAttribute(rmsd_assign_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
+    }
+    int64_t g = ((n + F - 1) / F + kRmsdWarps - 1) / kRmsdWarps;
+    const int64_t cap = (int64_t)num_sms() * 2;
+    if (g > cap) g = cap;
+    rmsd_assign_kernel<F><<<(unsigned)g, kRmsdWarps * 32, smem, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, kp_of_k(k), labels,
+                                                                    rmsd);
+    KM_CUDA(cudaGetLastError());
+    return KM_OK;
+}
+
 int launch_rmsd_assign(const float *Xc, const double *G, int64_t n, int d, const RmsdCenters &rc, int k,
                        int32_t *labels, float *rmsd, cudaStream_t s) {
     if (n == 0) return KM_OK;
-    rmsd_assign_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, kp_of_k(k), labels,
-                                                               rmsd);
-    KM_CUDA(cudaGetLastError());
-    return KM_OK;
+    if (d < 9) {
+        rmsd_assign_full_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, kp_of_k(k),
+                                                                        labels, rmsd);
+        KM_CUDA(cudaGetLastError());
+        return KM_OK;
+    }
+    // Eight frames per warp once that fills every SM's warps; four below.
+    if (n >= (int64_t)num_sms() * 2 * kRmsdWarps * 8) return launch_rmsd_assign_f<8>(Xc, G, n, d, rc, k, labels, rmsd, s);
+    return launch_rmsd_assign_f<4>(Xc, G, n, d, rc, k, labels, rmsd, s);
 }
 
 }  // namespace
