@@ -50,12 +50,25 @@ __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_center_kernel(const floa
 }
 
 // The same with one thread per row: a warp stages its 32 rows in shared
-// memory (coalesced; odd row stride), and each thread adds its row in the
-// order of rmsd_center_row_warp (32 partial sums, then the butterfly's tree),
-// so the results are the same bit for bit.  The warp-per-row form repeats the
-// divisions and the tree in all 32 lanes, at 64 cycles per float64
-// instruction: 5.9 ms for 1,000,000 rows of 58 atoms; this one kCenterMs.
+// memory (coalesced; odd row stride).  The results are those of
+// rmsd_center_row_warp bit for bit, with as little float64 work as that
+// allows (two float64 lanes per SM and clock here, conversions at the same
+// rate):
+//   * the sum over an axis: every float64 partial sum is exact while the
+//     values span at most 53 - ceil(log2 n_atoms) bits, and then any exact
+//     summation gives the same value: each value is cut into three slices
+//     whose float32 sums are exact;
+//   * a = (float)(x - mean): x - mean to 2^-47 in float pairs; its float
+//     rounding is final unless the value lies that close to the middle of two
+//     floats, where the float64 form decides;
+//   * G: the square of a float is exact in float64, so a fused multiply-add
+//     rounds as product and sum; the tree over the 32 partial sums is walked
+//     in bit-reversed order with a five-entry stack.
+// Rows outside these conditions take the float64 form.  1,000,000 rows of 58
+// atoms: 1.5 ms (FP64 pipe 40% busy); 5.9 ms with a warp per row, which
+// repeats the divisions and the tree in every lane.
 constexpr int kCenterMaxSmem = 200 * 1024;
+constexpr int kCenterSlicedAtoms = 128;  // a slice's sum of this many values is exact
 
 int center_stride(int d) { return d | 1; }
 int center_warps(int d) {  // warps per CTA; 0: the rows do not fit
@@ -64,30 +77,100 @@ int center_warps(int d) {  // warps per CTA; 0: the rows do not fit
     return w >= 4 ? 2 : (int)std::min<int64_t>(w, 1);
 }
 
-// The tree of rmsd_center_row_warp over 32 partial sums part(l).
-template <class Part>
-__device__ __forceinline__ double rmsd_tree32(const Part &part) {
-    double r[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l)
-        r[l] = __dadd_rn(__dadd_rn(part(l), part(l + 16)), __dadd_rn(part(l + 8), part(l + 24)));
-#pragma unroll
-    for (int h = 4; h > 0; h >>= 1)
-#pragma unroll
-        for (int l = 0; l < h; ++l) r[l] = __dadd_rn(r[l], r[l + h]);
-    return r[0];
+// The tree of rmsd_center_row_warp (offsets 16, 8, 4, 2, 1) over the 32
+// partial sums leaf(l): leaves in bit-reversed order, equal subtrees added as
+// soon as both are complete.
+template <class Leaf>
+__device__ __forceinline__ double rmsd_tree32(const Leaf &leaf) {
+    double st[6];  // in local memory: a loop of its own, or every level's addition is made and selected
+    double v = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < 32; ++q) {
+        v = leaf((int)(__brev((unsigned)q) >> 27));
+        int b = 0;
+#pragma unroll 1
+        for (; (q >> b) & 1; ++b) v = __dadd_rn(st[b], v);
+        st[b] = v;
+    }
+    return v;
 }
 
-__global__ void rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, int d, int stride,
-                                        float *__restrict__ Xc, double *__restrict__ G) {
+// The exact sum of n_atoms values x[0], x[3], ... as a double; false when the
+// values span too many bits for the slices (or are not finite).
+__device__ __forceinline__ bool rmsd_sliced_sum(const float *x, int n_atoms, double &sum) {
+    unsigned hi = 0u, lo = 0xffffffffu;  // bits of the largest, of the smallest non-zero magnitude less one
+    for (int i = 0; i < n_atoms; ++i) {
+        const unsigned b = __float_as_uint(x[3 * i]) & 0x7fffffffu;
+        hi = max(hi, b);
+        lo = min(lo, b - 1u);
+    }
+    sum = 0.0;
+    if (hi == 0u) return true;
+    const int e = (int)(hi >> 23), el = (int)((lo + 1u) >> 23);
+    // |x| < 2^(E + 1), E = e - 127; every x a multiple of 2^(E - 46)
+    if (e > 200 || el < 60 || e - el > 23) return false;
+    const float m1 = __uint_as_float((unsigned)(e + 8) << 23 | 0x400000u);  // 1.5 2^(E + 8): slice of 2^(E - 15)
+    const float m2 = __uint_as_float((unsigned)(e - 9) << 23 | 0x400000u);  // 1.5 2^(E - 9): slice of 2^(E - 32)
+    float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+    for (int i = 0; i < n_atoms; ++i) {
+        const float v = x[3 * i];
+        const float h1 = __fsub_rn(__fadd_rn(v, m1), m1);
+        const float r1 = __fsub_rn(v, h1);
+        const float h2 = __fsub_rn(__fadd_rn(r1, m2), m2);
+        const float r2 = __fsub_rn(r1, h2);
+        s1 = __fadd_rn(s1, h1);
+        s2 = __fadd_rn(s2, h2);
+        s3 = __fadd_rn(s3, r2);
+    }
+    sum = __dadd_rn(__dadd_rn((double)s1, (double)s2), (double)s3);
+    return true;
+}
+
+// The float64 forms, out of line: inlined, the compiler computes them for
+// every value and selects.
+__device__ __noinline__ float rmsd_center_value_d(float x, double mean) {
+    return __double2float_rn(__dsub_rn((double)x, mean));
+}
+__device__ __noinline__ double rmsd_widen_d(float v) { return (double)v; }
+
+// (float)(x - mean) as double subtraction and conversion give it; mh + ml is
+// mean to 2^-49.
+__device__ __forceinline__ float rmsd_center_value(float x, double mean, float mh, float ml) {
+    // x - mh = s + e exactly, t = e - ml, s + t = v + r exactly
+    const float s = __fsub_rn(x, mh);
+    const float bb = __fsub_rn(s, x);
+    const float e = __fsub_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fadd_rn(mh, bb));
+    const float t = __fsub_rn(e, ml);
+    const float v = __fadd_rn(s, t);
+    const float tv = __fsub_rn(v, s);
+    const float r = __fadd_rn(__fsub_rn(s, __fsub_rn(v, tv)), __fsub_rn(t, tv));
+    const unsigned b = __float_as_uint(v);
+    const float half = __uint_as_float((b & 0x7f800000u) - (24u << 23));  // half a unit in the last place
+    const float tol = 1.42e-14f * (fabsf(s) + fabsf(mh));                 // 2^-46
+    const bool sure = (b & 0x7f800000u) > (60u << 23) && (b & 0x7fffffu) != 0u && half - fabsf(r) > tol;
+    if (!sure) return rmsd_center_value_d(x, mean);
+    return v;
+}
+
+// (double)v without the conversion unit.
+__device__ __forceinline__ double rmsd_widen(float v) {
+    const unsigned b = __float_as_uint(v), a = b & 0x7fffffffu;
+    if (a - 0x800000u >= 0x7f000000u) return rmsd_widen_d(v);  // zero, subnormal, infinite, NaN
+    return __hiloint2double((int)((b & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+__global__ void __launch_bounds__(64) rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, int d,
+                                                              int stride, float *__restrict__ Xc,
+                                                              double *__restrict__ G) {
     extern __shared__ float center_smem[];
     const int lane = threadIdx.x & 31;
     const int warps = blockDim.x >> 5;
     float *rows = center_smem + (size_t)(threadIdx.x >> 5) * 32 * stride;
     const int n_atoms = d / 3;
     const int64_t tiles = (n + 31) / 32;
-    for (int64_t t = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); t < tiles; t += (int64_t)gridDim.x * warps) {
-        const int64_t r0 = t * 32;
+    for (int64_t tile = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); tile < tiles;
+         tile += (int64_t)gridDim.x * warps) {
+        const int64_t r0 = tile * 32;
         const int m = (int)(n - r0 < 32 ? n - r0 : 32);
         // the tile's rows are consecutive floats; eight loads in flight per lane
         const float *src = X + r0 * d;
@@ -111,29 +194,33 @@ __global__ void rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, 
         if (lane < m) {
             float *x = rows + lane * stride;
             double mean[3];
+            float mh[3], ml[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double sum = rmsd_tree32([&](int l) {
-                    double acc = 0.0;
-                    for (int i = l; i < n_atoms; i += 32) acc = __dadd_rn(acc, (double)x[3 * i + c]);
-                    return acc;
-                });
+                double sum;
+                if (n_atoms > kCenterSlicedAtoms || !rmsd_sliced_sum(x + c, n_atoms, sum))
+                    sum = rmsd_tree32([&](int l) {
+                        double acc = 0.0;
+                        for (int i = l; i < n_atoms; i += 32) acc = __dadd_rn(acc, (double)x[3 * i + c]);
+                        return acc;
+                    });
                 mean[c] = __ddiv_rn(sum, (double)n_atoms);
+                mh[c] = __double2float_rn(mean[c]);
+                ml[c] = __double2float_rn(__dsub_rn(mean[c], (double)mh[c]));
             }
-            const double g = rmsd_tree32([&](int l) {
+            G[r0 + lane] = rmsd_tree32([&](int l) {
                 double acc = 0.0;
                 for (int i = l; i < n_atoms; i += 32) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        const float v = __double2float_rn(__dsub_rn((double)x[3 * i + c], mean[c]));
+                        const float v = rmsd_center_value(x[3 * i + c], mean[c], mh[c], ml[c]);
                         x[3 * i + c] = v;
-                        // the square of a float is exact in double: one rounding, as product then sum
-                        acc = __fma_rn((double)v, (double)v, acc);
+                        const double w = rmsd_widen(v);
+                        acc = __fma_rn(w, w, acc);
                     }
                 }
                 return acc;
             });
-            G[r0 + lane] = g;
         }
         __syncwarp();
         f = lane % d;
@@ -150,11 +237,13 @@ __global__ void rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, 
     }
 }
 
-// Ct[f * kp + j] = Cc[j * d + f]; zero for the padding centers.
+// The centers by groups of 32 lanes: Ct[(g * n_atoms + i) * 96 + 32 c + l] =
+// coordinate c of atom i of center 32 g + l; zero for the padding centers.
 __global__ void rmsd_transpose_kernel(const float *__restrict__ Cc, int k, int kp, int d, float *__restrict__ Ct) {
     const int64_t total = (int64_t)kp * d;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int f = (int)(e / kp), j = (int)(e - (int64_t)f * kp);
+        const int f = (int)((e >> 5) % d);  // feature 3 i + c
+        const int j = (int)((e >> 5) / d) * 32 + (int)(e & 31);
         Ct[e] = j < k ? Cc[(int64_t)j * d + f] : 0.0f;
     }
 }
@@ -169,9 +258,9 @@ __device__ __forceinline__ bool rmsd_better(double m, int j, double bm, int bj) 
 
 // The nearest center of one frame with every pair solved in double, by one
 // warp (lanes own centers); (msd, index) in every lane.
-__device__ __forceinline__ void rmsd_full_frame(const float *__restrict__ a, double ga, int n_atoms,
-                                                const float *__restrict__ Ct, const double *__restrict__ H, int k,
-                                                int kp, int lane, double &bm, int &bj) {
+__device__ __noinline__ void rmsd_full_frame(const float *__restrict__ a, double ga, int n_atoms,
+                                             const float *__restrict__ Ct, const double *__restrict__ H, int k,
+                                             int lane, double &bm, int &bj) {
     bm = 0.0;
     bj = -1;
     for (int j0 = 0; j0 < k; j0 += 32) {
@@ -179,11 +268,10 @@ __device__ __forceinline__ void rmsd_full_frame(const float *__restrict__ a, dou
         float S[9];
 #pragma unroll
         for (int e = 0; e < 9; ++e) S[e] = 0.0f;
-        const float *b = Ct + j;
-        for (int i = 0; i < n_atoms; ++i) {
+        const float *b = Ct + (int64_t)j0 * 3 * n_atoms + lane;
+        for (int i = 0; i < n_atoms; ++i, b += 96) {
             const float a0 = a[3 * i], a1 = a[3 * i + 1], a2 = a[3 * i + 2];
-            const float b0 = b[(int64_t)(3 * i) * kp], b1 = b[(int64_t)(3 * i + 1) * kp],
-                        b2 = b[(int64_t)(3 * i + 2) * kp];
+            const float b0 = b[0], b1 = b[32], b2 = b[64];
             S[0] = __fmaf_rn(a0, b0, S[0]);
             S[1] = __fmaf_rn(a0, b1, S[1]);
             S[2] = __fmaf_rn(a0, b2, S[2]);
@@ -224,13 +312,13 @@ __device__ __forceinline__ void rmsd_store(int64_t r, double bm, int bj, int32_t
 // a double root, and qcp_bracket never holds.
 __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_assign_full_kernel(
     const float *__restrict__ Xc, const double *__restrict__ G, int64_t n, int d, const float *__restrict__ Ct,
-    const double *__restrict__ H, int k, int kp, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
+    const double *__restrict__ H, int k, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
     const int lane = threadIdx.x & 31;
     const int64_t nw = (int64_t)gridDim.x * kRmsdWarps;
     for (int64_t r = (int64_t)blockIdx.x * kRmsdWarps + (threadIdx.x >> 5); r < n; r += nw) {
         double bm;
         int bj;
-        rmsd_full_frame(Xc + r * d, G[r], d / 3, Ct, H, k, kp, lane, bm, bj);
+        rmsd_full_frame(Xc + r * d, G[r], d / 3, Ct, H, k, lane, bm, bj);
         if (lane == 0) rmsd_store(r, bm, bj, labels, rmsd);
     }
 }
@@ -244,33 +332,49 @@ __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_assign_full_kernel(
 // lambda = s x for its largest root x <= sqrt(3).  (Its constant term is the
 // product of the key matrix's eigenvalues.)  u = 2^-24.  ||T||^2 = 1 within
 // 20 u; the float values of the coefficients are off by at most 40 u, 64 u
-// and 75 u, and P at 0 < x <= 1.75 by at most 120 + 110 + 75 + 45 = 350 u: e
-// below allows 512 u.  All roots are real, so
+// and 75 u, and P at 0 < x <= 1.75 by at most 120 + 110 + 75 + 45 = 350 u:
+// kQcpErr allows 512 u.  All roots are real, so
 //   P(x) > 0, P'(x) > 0, P''(x) > 0 (x > 0.6)  =>  x is above every root;
 //   P(x) < 0                                   =>  x is below the largest.
-// Both tests are made on the float value with the margin e, at points found
-// by five Newton steps from above.  P' is required to be 0.05 at least: there
-// the double Newton of qcp_msd converges to the root within 1e-10 of s.  The
-// roundings of s, T and the final sum are below 64 u tot.
+// Both tests are made on the float value with the margin kQcpErr.  The
+// roundings of s, T and of E itself are below kQcpSlack tot = 64 u tot.
+//
+// qcp_msd's double Newton ends at the largest root (within 1e-9 of s) when
+// that root is well separated: P' there is 8 (a + b)(a + c)(b + c) for the
+// singular values a >= b >= |c| of T, c with the sign of det(T).  well says
+// that it is 1e-5 at least, from
+//   a^2 (b + c)^2 >= ||cof T||^2 - det^2 / a^2 - 2 a |det|   (det < 0)
+// with ||T T^t||_F^2 <= a^2 <= ||T T^t||_F and ||cof T||^2 = (1 - ||T
+// T^t||_F^2) / 2 (for det >= 0 the first term alone bounds b + c).  Measured
+// on random-walk chains: 99% of the pairs.
 // Where a test fails (an ill-conditioned root, sums outside the range in
 // which qcp_msd's float reciprocal is normal, a value that is not finite) the
 // bound is 0 or infinity and the pair is solved in double.
-__device__ __forceinline__ void qcp_bracket(const float (&S)[9], float tot, float &lb, float &ub) {
-    constexpr float kErr = 512.0f * 5.9604645e-8f;
-    lb = 0.0f;
-    ub = __int_as_float(0x7f800000);
+struct QcpQuartic {
+    float s, C1, C0;
+    bool well;  // the double solve ends at the largest root
+    __device__ __forceinline__ void eval(float x, float &P, float &D) const {
+        const float l2 = x * x;
+        const float a2 = l2 - 2.0f;
+        P = fmaf(a2, l2, fmaf(C1, x, C0));
+        D = fmaf(2.0f * x, l2 + a2, C1);
+    }
+};
+
+constexpr float kQcpErr = 512.0f * 5.9604645e-8f;
+constexpr float kQcpSlack = 64.0f * 5.9604645e-8f;
+
+__device__ __forceinline__ QcpQuartic qcp_quartic(const float (&S)[9], float tot) {
     float ss = 0.0f;
 #pragma unroll
     for (int e = 0; e < 9; ++e) ss = fmaf(S[e], S[e], ss);
     const float rs = rsqrtf(ss);
-    const float s = ss * rs;
     float T[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) T[e] = S[e] * rs;
     const float m0 = fmaf(T[4], T[8], -T[5] * T[7]);
     const float m1 = fmaf(T[3], T[8], -T[5] * T[6]);
     const float m2 = fmaf(T[3], T[7], -T[4] * T[6]);
-    const float C1 = -8.0f * fmaf(T[0], m0, fmaf(T[2], m2, -T[1] * m1));
     const float b00 = fmaf(T[0], T[0], fmaf(T[1], T[1], T[2] * T[2]));
     const float b11 = fmaf(T[3], T[3], fmaf(T[4], T[4], T[5] * T[5]));
     const float b22 = fmaf(T[6], T[6], fmaf(T[7], T[7], T[8] * T[8]));
@@ -279,32 +383,47 @@ __device__ __forceinline__ void qcp_bracket(const float (&S)[9], float tot, floa
     const float b12 = fmaf(T[3], T[6], fmaf(T[4], T[7], T[5] * T[8]));
     const float diag = fmaf(b00, b00, fmaf(b11, b11, b22 * b22));
     const float offd = fmaf(b01, b01, fmaf(b02, b02, b12 * b12));
-    const float C0 = fmaf(2.0f, fmaf(2.0f, offd, diag), -1.0f);
-    float x = fminf(1.7320509f, __fdividef(0.500001f * tot, s));
+    QcpQuartic q;
+    q.s = ss * rs;
+    q.C1 = -8.0f * fmaf(T[0], m0, fmaf(T[2], m2, -T[1] * m1));
+    q.C0 = fmaf(2.0f, fmaf(2.0f, offd, diag), -1.0f);
+    const float nb = 0.5f * (q.C0 + 1.0f);
+    const float det = fmaxf(0.125f * q.C1, 0.0f) + 2e-6f;  // of a negative determinant, its size
+    const float sep = fmaf(0.25f, 1.0f - q.C0, -__fdividef(det * det, nb)) - 2.0f * det * sqrtf(sqrtf(nb));
+    q.well = sep >= 2e-5f && ss >= 1e-22f && ss <= 1e30f && tot <= 1e37f;
+    return q;
+}
+
+// True when E_qcp > best is certain: the point x at which E would be best
+// (less the slack) is above every root (sqrt(3) always is).
+__device__ __forceinline__ bool qcp_beyond(const QcpQuartic &q, float tot, float best) {
+    const float x = fminf(__fdividef(0.5f * (tot - best - 2.0f * kQcpSlack * tot), q.s), 1.74f);
     float P, D;
-    auto eval = [&](float y) {
-        const float l2 = y * y;
-        const float a2 = l2 - 2.0f;
-        P = fmaf(a2, l2, fmaf(C1, y, C0));
-        D = fmaf(2.0f * y, l2 + a2, C1);
-    };
+    q.eval(x, P, D);
+    return q.well && x > 0.6f && (x == 1.74f || (P > kQcpErr && D >= 1e-3f));
+}
+
+// The bracket at the point that eight Newton steps from above reach.
+__device__ __forceinline__ void qcp_bracket(const QcpQuartic &q, float tot, float &lb, float &ub) {
+    lb = 0.0f;
+    ub = __int_as_float(0x7f800000);
+    float x = fminf(1.7320509f, __fdividef(0.500001f * tot, q.s));
+    float P, D;
 #pragma unroll
-    for (int it = 0; it < 5; ++it) {
-        eval(x);
+    for (int it = 0; it < 8; ++it) {
+        q.eval(x, P, D);
         x -= __fdividef(P, D);
     }
-    eval(x);
+    q.eval(x, P, D);
     const float inv = __fdividef(1.0f, D);
-    const float xu = x + fmaf(fmaxf(-P, 0.0f), 1.01f * inv, 2.5f * kErr * inv);
-    const float xl = x - fmaf(fmaxf(P, 0.0f), 1.01f * inv, 2.5f * kErr * inv);
-    const bool fine = ss >= 1e-22f && ss <= 1e30f && D >= 0.05f && x > 0.6f && xu < 1.75f && tot <= 1e37f;
-    eval(xu);
-    const bool above = P > kErr && D >= 0.04f;
-    eval(xl);
-    const bool below = P < -kErr && xl > 0.0f;
-    const float slack = 64.0f * 5.9604645e-8f * tot;
-    if (fine && above) lb = fmaxf(fmaf(-2.0f * xu, s, tot) - slack, 0.0f);
-    if (fine && below) ub = fmaxf(fmaf(-2.0f * xl, s, tot) + slack, 0.0f);
+    const float xu = x + fmaf(fmaxf(-P, 0.0f), 1.01f * inv, 2.5f * kQcpErr * inv);
+    const float xl = x - fmaf(fmaxf(P, 0.0f), 1.01f * inv, 2.5f * kQcpErr * inv);
+    q.eval(xu, P, D);
+    if (q.well && xu > 0.6f && xu < 1.75f && P > kQcpErr && D >= 1e-3f)
+        lb = fmaxf(fmaf(-2.0f * xu, q.s, tot) - kQcpSlack * tot, 0.0f);
+    q.eval(xl, P, D);
+    if (q.well && xl > 0.0f && xl < 1.75f && P < -kQcpErr)
+        ub = fmaxf(fmaf(-2.0f * xl, q.s, tot) + kQcpSlack * tot, 0.0f);
 }
 
 // Two float32 fused multiply-adds in one instruction.
@@ -331,8 +450,13 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &
 // whose list runs over (near-ties, or pairs without a bracket) has all its
 // pairs solved in double.
 // Bound by the FP32 pipe: 9 n_atoms multiply-adds and about 140 operations of
-// the bracket per pair.  1,000,000 frames of 58 atoms, k = 100: kAssignMs,
-// where solving every pair in double took 68.6 ms.
+// the bracket per pair, with three warps in four waiting (ncu, 200,000 frames:
+// issue slots 40% busy, FP32 pipe 34%, FP64 pipe 33%).  1,000,000 frames of
+// 58 atoms, k = 100: 5.9 ms; solving every pair in double took 68.6 ms.
+// Four frames per warp, 24 warps per SM: 7.7 ms the whole call; eight frames reuse each
+// center coordinate twice as often but leave 16 warps per SM (126 registers)
+// and twice the code after the sums: 9.3 ms.
+constexpr int kRmsdFrames = 4;
 constexpr int kRmsdAtoms = 96;  // atoms staged at a time
 constexpr int kRmsdList = 8;    // candidates kept per frame
 
@@ -348,10 +472,68 @@ struct RmsdWarpSmem {
     int32_t full[F];  // the list ran over
 };
 
+// Brackets one frame's pairs with the warp's 32 centers, lists the ones that
+// the smallest upper bound (returned) does not rule out.  Out of line: few
+// groups of centers need it, and eight copies of it would not stay in the
+// instruction cache.
 template <int F>
-__global__ void __launch_bounds__(kRmsdWarps * 32, 2) rmsd_assign_kernel(
+__device__ __noinline__ float rmsd_candidates(RmsdWarpSmem<F> &sm, int f, const float (&S)[9], QcpQuartic qu,
+                                              float tot, float best, int j, int k) {
+    const int lane = threadIdx.x & 31;
+    const float kInf = __int_as_float(0x7f800000);
+    float lb, ub;
+    qcp_bracket(qu, tot, lb, ub);
+    if (j >= k) ub = kInf;
+    // non-negative floats order as their bits
+    best = fminf(best, __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(ub))));
+    const unsigned cand = __ballot_sync(0xffffffffu, j < k && lb <= best);
+    if (cand == 0u) return best;
+    // When the list would run over, first drop the entries that the bound
+    // rules out by now.
+    int cnt = sm.cnt[f];
+    if (cnt + __popc(cand) > kRmsdList) {
+        float l = kInf, Sl[9];
+        int jl = -1;
+        if (lane < cnt) {
+            l = sm.lb[f][lane];
+            jl = sm.j[f][lane];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) Sl[e] = sm.S[f][lane][e];
+        }
+        const unsigned keep = __ballot_sync(0xffffffffu, lane < cnt && l <= best);
+        __syncwarp();
+        if ((keep >> lane) & 1u) {
+            const int to = __popc(keep & ((1u << lane) - 1u));
+            sm.lb[f][to] = l;
+            sm.j[f][to] = jl;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = Sl[e];
+        }
+        cnt = __popc(keep);
+        __syncwarp();
+    }
+    if ((cand >> lane) & 1u) {
+        const int to = cnt + __popc(cand & ((1u << lane) - 1u));
+        if (to < kRmsdList) {
+            sm.lb[f][to] = lb;
+            sm.j[f][to] = j;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = S[e];
+        }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        sm.cnt[f] = min(cnt + __popc(cand), kRmsdList);
+        if (cnt + __popc(cand) > kRmsdList) sm.full[f] = 1;
+    }
+    __syncwarp();
+    return best;
+}
+
+template <int F>
+__global__ void __launch_bounds__(kRmsdWarps * 32, 3) rmsd_assign_kernel(
     const float *__restrict__ Xc, const double *__restrict__ G, int64_t n, int d, const float *__restrict__ Ct,
-    const double *__restrict__ H, int k, int kp, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
+    const double *__restrict__ H, int k, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
     static_assert(F % 4 == 0, "frames go in fours (16-byte shared loads)");
     extern __shared__ __align__(16) unsigned char rmsd_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -393,15 +575,17 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 2) rmsd_assign_kernel(
             for (int i0 = 0; i0 < n_atoms; i0 += kRmsdAtoms) {
                 const int cnt = min(kRmsdAtoms, n_atoms - i0);
                 if (n_atoms > kRmsdAtoms) stage(r0, i0, cnt);
-                const float *b = Ct + (int64_t)(3 * i0) * kp + j;
+                // the next atom's center coordinates are loaded one step ahead
+                const float *b = Ct + ((int64_t)(j0 >> 5) * n_atoms + i0) * 96 + lane;
+                float nb[3] = {__ldg(b), __ldg(b + 32), __ldg(b + 64)};
 #pragma unroll 2
                 for (int i = 0; i < cnt; ++i) {
                     unsigned long long bb[3];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const float v = __ldg(b + (int64_t)(3 * i + c) * kp);
-                        bb[c] = pack2(v, v);
-                    }
+                    for (int c = 0; c < 3; ++c) bb[c] = pack2(nb[c], nb[c]);
+                    if (i + 1 < cnt) b += 96;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) nb[c] = __ldg(b + 32 * c);
 #pragma unroll
                     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -424,51 +608,12 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 2) rmsd_assign_kernel(
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int f = 2 * q + h;
-                    float lb, ub;
-                    qcp_bracket(Sp[h], (float)sm.ga[f] + hj, lb, ub);
-                    if (j >= k) ub = kInf;
-                    // non-negative floats order as their bits
-                    best[f] = fminf(best[f], __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(ub))));
-                    const unsigned cand = __ballot_sync(0xffffffffu, j < k && lb <= best[f]);
-                    if (cand == 0u) continue;
-                    // Append; when the list would run over, first drop the
-                    // entries that the bound rules out by now.
-                    int cnt = sm.cnt[f];
-                    if (cnt + __popc(cand) > kRmsdList && cnt <= kRmsdList) {
-                        float l = kInf, Sl[9];
-                        int jl = -1;
-                        if (lane < cnt) {
-                            l = sm.lb[f][lane];
-                            jl = sm.j[f][lane];
-#pragma unroll
-                            for (int e = 0; e < 9; ++e) Sl[e] = sm.S[f][lane][e];
-                        }
-                        const unsigned keep = __ballot_sync(0xffffffffu, lane < cnt && l <= best[f]);
-                        __syncwarp();
-                        if ((keep >> lane) & 1u) {
-                            const int to = __popc(keep & ((1u << lane) - 1u));
-                            sm.lb[f][to] = l;
-                            sm.j[f][to] = jl;
-#pragma unroll
-                            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = Sl[e];
-                        }
-                        cnt = __popc(keep);
-                    }
-                    if ((cand >> lane) & 1u) {
-                        const int to = cnt + __popc(cand & ((1u << lane) - 1u));
-                        if (to < kRmsdList) {
-                            sm.lb[f][to] = lb;
-                            sm.j[f][to] = j;
-#pragma unroll
-                            for (int e = 0; e < 9; ++e) sm.S[f][to][e] = Sp[h][e];
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) {
-                        sm.cnt[f] = min(cnt + __popc(cand), kRmsdList);
-                        if (cnt + __popc(cand) > kRmsdList) sm.full[f] = 1;
-                    }
-                    __syncwarp();
+                    const float tot = (float)sm.ga[f] + hj;
+                    const QcpQuartic qu = qcp_quartic(Sp[h], tot);
+                    // one evaluation of the quartic rules out most centers
+                    // once the frame has a bound
+                    if (__all_sync(0xffffffffu, j >= k || qcp_beyond(qu, tot, best[f]))) continue;
+                    best[f] = rmsd_candidates<F>(sm, f, Sp[h], qu, tot, best[f], j, k);
                 }
             }
         }
@@ -526,7 +671,7 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 2) rmsd_assign_kernel(
             if (!sm.full[f] || r0 + f >= n) continue;
             double fm;
             int fj;
-            rmsd_full_frame(Xc + (r0 + f) * d, sm.ga[f], n_atoms, Ct, H, k, kp, lane, fm, fj);
+            rmsd_full_frame(Xc + (r0 + f) * d, sm.ga[f], n_atoms, Ct, H, k, lane, fm, fj);
             if (lane == 0) rmsd_store(r0 + f, fm, fj, labels, rmsd);
         }
         __syncwarp();
@@ -597,7 +742,9 @@ int check_rmsd_shape(int64_t n, int d, int k) {
 int center_rows(const float *X, int64_t n, int d, float *Xc, double *G, cudaStream_t s) {
     if (n == 0) return KM_OK;
     const int warps = center_warps(d);
-    if (warps > 0) {
+    // a warp per row while the rows (centers, short calls) give every SM no
+    // more than a few tiles: the thread-per-row form takes 0.18 ms for one tile
+    if (warps > 0 && n >= (int64_t)num_sms() * 128) {
         static bool attr_done[kDeviceSlots] = {};
         const int dev = current_device();
         if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
@@ -639,10 +786,9 @@ int launch_rmsd_assign_f(const float *Xc, const double *G, int64_t n, int d, con
         if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
     }
     int64_t g = ((n + F - 1) / F + kRmsdWarps - 1) / kRmsdWarps;
-    const int64_t cap = (int64_t)num_sms() * 2;
+    const int64_t cap = (int64_t)num_sms() * 3;
     if (g > cap) g = cap;
-    rmsd_assign_kernel<F><<<(unsigned)g, kRmsdWarps * 32, smem, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, kp_of_k(k), labels,
-                                                                    rmsd);
+    rmsd_assign_kernel<F><<<(unsigned)g, kRmsdWarps * 32, smem, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, labels, rmsd);
     KM_CUDA(cudaGetLastError());
     return KM_OK;
 }
@@ -651,14 +797,12 @@ int launch_rmsd_assign(const float *Xc, const double *G, int64_t n, int d, const
                        int32_t *labels, float *rmsd, cudaStream_t s) {
     if (n == 0) return KM_OK;
     if (d < 9) {
-        rmsd_assign_full_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, kp_of_k(k),
-                                                                        labels, rmsd);
+        rmsd_assign_full_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, labels,
+                                                                        rmsd);
         KM_CUDA(cudaGetLastError());
         return KM_OK;
     }
-    // Eight frames per warp once that fills every SM's warps; four below.
-    if (n >= (int64_t)num_sms() * 2 * kRmsdWarps * 8) return launch_rmsd_assign_f<8>(Xc, G, n, d, rc, k, labels, rmsd, s);
-    return launch_rmsd_assign_f<4>(Xc, G, n, d, rc, k, labels, rmsd, s);
+    return launch_rmsd_assign_f<kRmsdFrames>(Xc, G, n, d, rc, k, labels, rmsd, s);
 }
 
 }  // namespace
