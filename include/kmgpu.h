@@ -63,7 +63,13 @@ typedef enum {
  *                 one; the center norms are applied in the epilogue.  A
  *                 3-bit mantissa makes the bound wide, so most frames are
  *                 re-checked; same labels.
- *   KM_PREC_AUTO: the library picks by (d, k) (km_tune can measure it). */
+ *   KM_PREC_AUTO: the library picks by (d, k) (km_tune can measure it).
+ * Frames of at most 31 features take a tensor-core kernel of their own under
+ * KM_PREC_FP16, and under KM_PREC_AUTO where it resolves to KM_PREC_FP32 and
+ * the call is large: operands split into two FP16 parts single out eight
+ * centers per frame, whose exact float32 distances give the label; frames it
+ * cannot settle (counted in n_full) are evaluated over all centers.  Same
+ * labels; the reported precision is the one AUTO resolved to. */
 typedef enum {
     KM_PREC_FP32 = 0,
     KM_PREC_FP16 = 1,

@@ -125,12 +125,44 @@ int resolve_precision(int precision, int d, int k, bool check_device) {
     return KM_PREC_FP32;
 }
 
-struct AssignWs {
-    TcBuffers tc;
-};
+// Whether an assignment that resolves to `prec` takes the narrow-frame kernel
+// (assign_small.cu): FP16 at every size, and KM_PREC_AUTO where it resolves
+// to FP32 by the rule (not by km_tune) and there is enough work; in both
+// cases without a tile shape set for (d, k).
+// n < 0: whatever n is.
+//
+// The lines, measured on AR(1) frames about 8 means (us per resident
+// assignment, 28 of them host work):
+//   * FP16, d <= 15: always (1M x 10: k = 50 565 -> 117, k = 2000 1230 -> 387);
+//     d = 16..31, whose centers take more launches, up to k = 2048 (1M x 24: k
+//     = 1000 881 -> 545, k = 2000 1169 -> 945, and the gap closes by 300 per
+//     1,000 centers).
+//   * AUTO where the rule says FP32: from n k (3 d + 2) = 3.5e8, the exact
+//     kernel's instructions, on.  Above: 200k x 2, k = 250 72 -> 67; 200k x 5, k
+//     = 100 76 -> 68; 2M x 4, k = 500 964 -> 230.  Below: 200k x 2, k = 100 58
+//     -> 61; 60k x 5, k = 250 53 -> 59.  Not for d = 1: there the centers lie
+//     so densely that 5-89% of the frames are re-checked over all of them (1M,
+//     k = 1000 506 -> 1024).
+constexpr double kSmallMinWork = 3.5e8;
+bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_device) {
+    if (!small_shape_ok(d, k) || (d > 15 && k > 2048) || !small_allowed() || (check_device && !tc_supported(d, k)) || tc_plan_set(d, k)) return false;
+    if (prec == KM_PREC_FP16) return true;
+    if (precision != KM_PREC_AUTO || prec != KM_PREC_FP32) return false;
+    {
+        std::lock_guard<std::mutex> lk(g_tune.m);
+        if (g_tune.choice.count(std::make_pair(d, k))) return false;
+    }
+    return small_forced() || (d >= 2 && (n < 0 || (double)n * k * (3 * d + 2) >= kSmallMinWork));
+}
 
-size_t assign_ws_bytes(int64_t n, int d, int k, int prec) {
-    if (!is_tc(prec)) return 0;
+// The workspace of an assignment; small: the narrow-frame kernel may run
+// (its center half and lists; the FP16 form's workspace holds both).
+size_t small_ws_bytes(int64_t n, int d, int k) {
+    return tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k) + 2 * 256;
+}
+
+size_t assign_ws_bytes(int64_t n, int d, int k, int prec, bool small = false) {
+    if (!is_tc(prec)) return small ? small_ws_bytes(n, d, k) : 0;
     return tc_frames_ws_size(n, d) + tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k) + 3 * 256;
 }
 
@@ -138,6 +170,13 @@ void carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
     char *p = static_cast<char *>(ws);
     tc_carve_frames(p, n, d, b);
     p += (tc_frames_ws_size(n, d) + 255) / 256 * 256;
+    tc_carve_centers(p, d, k, b);
+    p += (tc_centers_ws_size(d, k) + 255) / 256 * 256;
+    tc_carve_assign(p, n, d, k, b);
+}
+
+void carve_small(void *ws, int64_t n, int d, int k, TcBuffers &b) {
+    char *p = static_cast<char *>(ws);
     tc_carve_centers(p, d, k, b);
     p += (tc_centers_ws_size(d, k) + 255) / 256 * 256;
     tc_carve_assign(p, n, d, k, b);
@@ -159,8 +198,8 @@ int check_device_errors(uint32_t e) {
 // For the tensor-core precisions, b holds the carved buffers (operand type set);
 // centers_ready means the
 // center half (FP16 copy, norms, shift, scale) is already prepared.
-int assign_core(const float *X, int64_t n, int32_t d, const float *C, int32_t k, int prec, int32_t *labels,
-                TcBuffers &b, bool centers_ready, km_assign_stats *stats, cudaStream_t s,
+int assign_core(const float *X, int64_t n, int32_t d, const float *C, int32_t k, int prec, bool small,
+                int32_t *labels, TcBuffers &b, bool centers_ready, km_assign_stats *stats, cudaStream_t s,
                 const PairSrc *ps = nullptr) {
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
@@ -174,7 +213,7 @@ int assign_core(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
         ProfEvents &p;
         ~Closer() { p.close(); }
     } closer{prof};
-    if (prec == KM_PREC_FP32) {
+    if (prec == KM_PREC_FP32 && !small) {
         prof.begin(kProfFp32, s);
         KM_TRY(launch_assign_fp32(X, nullptr, nullptr, n, d, C, k, labels, nullptr, nullptr, s, ps));
         prof.end(kProfFp32, s);
@@ -184,27 +223,27 @@ int assign_core(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
     }
     if (!centers_ready) {
         KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
-        KM_TRY(tc_prepare_centers(C, d, k, b, s));
+        KM_TRY(small ? small_prepare_centers(C, d, k, b, s) : tc_prepare_centers(C, d, k, b, s));
     }
-    KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
-    KM_TRY(tc_assign(X, n, d, C, k, labels, b, s, &prof, nullptr, nullptr, ps));
+    if (small) {
+        KM_TRY(small_assign(X, n, d, k, labels, b, s, &prof));
+    } else {
+        KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
+        KM_TRY(tc_assign(X, n, d, C, k, labels, b, s, &prof, nullptr, nullptr, ps));
+    }
     if (prof.active) {
         KM_CUDA(cudaStreamSynchronize(s));
         prof.collect();
     }
     if (stats) {
-        int32_t cnt[3];
-        unsigned long long flips = 0;
-        uint32_t err = 0;
-        KM_CUDA(cudaMemcpyAsync(cnt, b.counters, sizeof(cnt), cudaMemcpyDeviceToHost, s));
-        KM_CUDA(cudaMemcpyAsync(&flips, b.flipped, sizeof(flips), cudaMemcpyDeviceToHost, s));
-        KM_CUDA(cudaMemcpyAsync(&err, b.err, sizeof(err), cudaMemcpyDeviceToHost, s));
+        TcStatus st;
+        KM_CUDA(cudaMemcpyAsync(&st, b.counters, sizeof(st), cudaMemcpyDeviceToHost, s));
         KM_CUDA(cudaStreamSynchronize(s));
-        stats->n_recheck = cnt[0];
-        stats->n_full = cnt[1];
-        stats->n_pairs = cnt[2];
-        stats->n_flipped = (int64_t)flips;
-        KM_TRY(check_device_errors(err));
+        stats->n_recheck = st.counters[0];
+        stats->n_full = st.counters[1];
+        stats->n_pairs = st.counters[2];
+        stats->n_flipped = (int64_t)st.flipped;
+        KM_TRY(check_device_errors(st.err));
     }
     return KM_OK;
 }
@@ -226,22 +265,25 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
-    KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec)));
+    const bool small = !ps && small_route(precision, prec, n, d, k, true);
+    KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec, small)));
     TcBuffers b;
     if (is_tc(prec) && n > 0) {
         carve_assign(ws, n, d, k, b);
         tc_set_operand(b, d, prec);
+    } else if (small && n > 0) {
+        carve_small(ws, n, d, k, b);
     }
     if (ps && prec == KM_PREC_FP8) {
         set_error("FP8 operands are not built for coordinate frames");
         return KM_ERR_UNSUPPORTED;
     }
-    return assign_core(X, n, d, C, k, prec, labels, b, false, stats, s, ps);
+    return assign_core(X, n, d, C, k, prec, small, labels, b, false, stats, s, ps);
 }
 
 // Workspace of an assignment whose centers are prepared: frames + lists.
-size_t resident_ws_bytes(int64_t n, int d, int k, int prec) {
-    if (!is_tc(prec)) return 0;
+size_t resident_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
+    if (!is_tc(prec)) return small ? tc_assign_ws_size(n, d, k) + 256 : 0;
     return tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k) + 2 * 256;
 }
 
@@ -346,7 +388,7 @@ __global__ void lloyd_loop_step_kernel(LoopState *st, const double *cost, const 
     cudaGraphSetConditional(h, (conv || e != 0u || it + 1 >= st->max_it) ? 0u : 1u);
 }
 
-size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec) {
+size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
     Carver c(nullptr);
     c.take<unsigned long long>(2);  // host copy counter pair
     c.take<LoopState>(1);
@@ -355,8 +397,8 @@ size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec) {
     c.take<float>((size_t)k * d);  // C_new
     c.take<double>(1);             // cost
     c.take<uint32_t>(1);           // error word
-    c.take<char>(assign_ws_bytes(n, d, k, prec));
-    if (is_tc(prec)) {
+    c.take<char>(assign_ws_bytes(n, d, k, prec, small));
+    if (is_tc(prec) || small) {
         c.take<int32_t>(3 * (size_t)n);  // flip list
         c.take<int32_t>(1);              // its count
     }
@@ -376,6 +418,10 @@ struct km_centers {
     size_t bytes = 0;
     float *C = nullptr;
     TcBuffers tc;  // center half: ch, cnorm, shift, scal (tensor-core precisions)
+    bool small = false;       // the narrow-frame form of the center half is prepared too
+    int asked = KM_PREC_FP32; // the precision km_centers_create was given
+    // Whether n frames take the narrow-frame kernel.
+    bool small_for(int64_t n) const { return small && small_route(asked, prec, n, d, k, true); }
 };
 
 namespace km {
@@ -385,12 +431,19 @@ namespace km {
 int assign_centers_enqueue(const float *X, int64_t n, const km_centers *h, int32_t *labels, void *ws,
                            size_t ws_bytes, uint32_t *err_host, cudaStream_t s) {
     *err_host = 0;
-    KM_TRY(check_ws(ws, ws_bytes, resident_ws_bytes(n, h->d, h->k, h->prec)));
+    const bool small = h->small_for(n);
+    KM_TRY(check_ws(ws, ws_bytes, resident_ws_bytes(n, h->d, h->k, h->prec, small)));
     if (n == 0) return KM_OK;
-    if (h->prec == KM_PREC_FP32)
-        return launch_assign_fp32(X, nullptr, nullptr, n, h->d, h->C, h->k, labels, nullptr, nullptr, s);
     TcBuffers b = h->tc;
     char *p = static_cast<char *>(ws);
+    if (small) {
+        tc_carve_assign(p, n, h->d, h->k, b);
+        KM_TRY(small_assign(X, n, h->d, h->k, labels, b, s));
+        KM_CUDA(cudaMemcpyAsync(err_host, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        return KM_OK;
+    }
+    if (h->prec == KM_PREC_FP32)
+        return launch_assign_fp32(X, nullptr, nullptr, n, h->d, h->C, h->k, labels, nullptr, nullptr, s);
     tc_carve_frames(p, n, h->d, b);
     p += (tc_frames_ws_size(n, h->d) + 255) / 256 * 256;
     tc_carve_assign(p, n, h->d, h->k, b);
@@ -401,7 +454,10 @@ int assign_centers_enqueue(const float *X, int64_t n, const km_centers *h, int32
     return KM_OK;
 }
 
-size_t assign_centers_ws_bytes(int64_t n, const km_centers *h) { return resident_ws_bytes(n, h->d, h->k, h->prec); }
+// (enough for any number of frames up to n: the slots of the serving loop)
+size_t assign_centers_ws_bytes(int64_t n, const km_centers *h) {
+    return resident_ws_bytes(n, h->d, h->k, h->prec, h->small);
+}
 int centers_d(const km_centers *h) { return h->d; }
 int centers_device(const km_centers *h) { return h->device; }
 int device_error_status(uint32_t e) { return check_device_errors(e); }
@@ -462,7 +518,8 @@ int km_profile_read(int32_t kind, double *ms_total, int64_t *launches) {
 
 size_t km_assign_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
     if (check_shape(n, d, k) != KM_OK) return 0;
-    return assign_ws_bytes(n, d, k, resolve_precision(precision, d, k, false));
+    const int prec = resolve_precision(precision, d, k, false);
+    return assign_ws_bytes(n, d, k, prec, small_route(precision, prec, n, d, k, false));
 }
 
 int km_assign(const float *X, int64_t n, int32_t d, const float *C, int32_t k, int32_t precision,
@@ -522,7 +579,7 @@ int km_debug_tc_distances(const float *X, int64_t n, int32_t d, const float *C, 
     // The 8 wait counters live in the unused tail of the candidate counters block.
     unsigned long long *dev_wait = nullptr;
     if (wait_cycles) {
-        dev_wait = reinterpret_cast<unsigned long long *>(b.counters + 4);
+        dev_wait = reinterpret_cast<unsigned long long *>(b.counters + kTcDiagWords);
         KM_CUDA(cudaMemsetAsync(dev_wait, 0, 8 * sizeof(unsigned long long), s));
     }
     KM_TRY(tc_assign(X, n, d, C, k, labels, b, s, nullptr, V, dev_wait));
@@ -579,7 +636,8 @@ int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, floa
 
 size_t km_lloyd_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
     if (check_shape(n, d, k) != KM_OK) return 0;
-    return lloyd_ws_bytes(n, d, k, resolve_precision(precision, d, k, false));
+    const int prec = resolve_precision(precision, d, k, false);
+    return lloyd_ws_bytes(n, d, k, prec, small_route(precision, prec, n, d, k, false));
 }
 
 }  // extern "C"
@@ -838,7 +896,9 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
-    const size_t need = lloyd_ws_bytes(n, d, k, prec);
+    const bool small = !ps && small_route(precision, prec, n, d, k, true);
+    const bool tc = is_tc(prec) || small;
+    const size_t need = lloyd_ws_bytes(n, d, k, prec, small);
     KM_TRY(check_ws(workspace, workspace_bytes, need));
     if (max_iter == 0 && !hf) return KM_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -852,7 +912,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     float *C_new = cv.take<float>((size_t)k * d);
     double *cost = cv.take<double>(1);
     uint32_t *err = cv.take<uint32_t>(1);
-    void *ws_assign = cv.take<char>(assign_ws_bytes(n, d, k, prec));
+    void *ws_assign = cv.take<char>(assign_ws_bytes(n, d, k, prec, small));
 
     // Host frames: one chunked copy on a side stream, an event per chunk.
     struct Streamed {
@@ -964,7 +1024,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             if (st) cudaStreamDestroy(st);
         }
     } side;
-    if (is_tc(prec)) {
+    if (tc) {
         fl.rows = cv.take<int32_t>(3 * (size_t)n);
         fl.count = cv.take<int32_t>(1);
         fl.cap = n;
@@ -974,13 +1034,17 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     }
 
     TcBuffers b;
-    if (is_tc(prec)) {
+    if (tc) {
         // The shift and scale stay fixed for the whole run so that the 16-bit
-        // frame copy is made once.
-        carve_assign(ws_assign, n, d, k, b);
-        tc_set_operand(b, d, prec);
+        // frame copy is made once (narrow frames have none).
+        if (is_tc(prec)) {
+            carve_assign(ws_assign, n, d, k, b);
+            tc_set_operand(b, d, prec);
+        } else {
+            carve_small(ws_assign, n, d, k, b);
+        }
         KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
-        if (!hf) KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
+        if (!hf && !small) KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
     }
     KM_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
 
@@ -1003,14 +1067,17 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         return KM_OK;
     };
     auto enqueue = [&](cudaStream_t st) -> int {
-        if (is_tc(prec)) {
-            KM_TRY(tc_prepare_centers(C, d, k, b, st));
+        if (tc) {
+            KM_TRY(small ? small_prepare_centers(C, d, k, b, st) : tc_prepare_centers(C, d, k, b, st));
             KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
             // the tensor-core pass counts the members as it writes the labels
             int32_t *counts = update_counts_from_labels(d, k, ps) ? update_counts(ws_update, n, d, k) : nullptr;
             if (counts) KM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * k, st));
-            KM_TRY(tc_assign_deferred(X, n, d, C, k, labels, b, st, side.st, side.fork, kTcMaxChunks, fl, &prof, ps,
-                                      counts));
+            if (small)
+                KM_TRY(small_assign(X, n, d, k, labels, b, st, &prof, side.st, side.fork[0], &fl, counts));
+            else
+                KM_TRY(tc_assign_deferred(X, n, d, C, k, labels, b, st, side.st, side.fork, kTcMaxChunks, fl, &prof,
+                                          ps, counts));
             prof.begin(kProfUpdate, st);
             // one segment-sum CTA per SM: room for the re-check beside it
             KM_TRY(launch_update_accumulate(X, n, d, labels, k, C, err, ws_update, st, 1, ps, counts != nullptr));
@@ -1029,8 +1096,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         return enqueue_update(st);
     };
     auto enqueue_streamed = [&](cudaStream_t st) -> int {
-        if (is_tc(prec)) {
-            KM_TRY(tc_prepare_centers(C, d, k, b, st));
+        if (tc) {
+            KM_TRY(small ? small_prepare_centers(C, d, k, b, st) : tc_prepare_centers(C, d, k, b, st));
             KM_CUDA(cudaMemsetAsync(b.err, 0, sizeof(uint32_t), st));
         }
         // Each chunk's members join the update's sums as soon as the chunk
@@ -1043,7 +1110,11 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
                 KM_TRY(stager->wait_chunk(st, c));
             else
                 KM_CUDA(cudaStreamWaitEvent(st, sm.ev[c + 1], 0));
-            if (is_tc(prec)) {
+            if (small) {
+                TcBuffers v = b;
+                v.keep_err = 1;
+                KM_TRY(small_assign(X + a * d, rows, d, k, labels + a, v, st, &prof));
+            } else if (is_tc(prec)) {
                 TcBuffers v = tc_rows_from(b, a);
                 v.keep_err = 1;
                 KM_TRY(tc_prepare_frames(X + a * d, rows, d, v, st));
@@ -1091,7 +1162,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
                  cudaSuccess;
             if (ok) {
                 const int st = enqueue(cs);
-                lloyd_loop_step_kernel<<<1, 1, 0, cs>>>(loop_st, cost, err, is_tc(prec) ? b.err : nullptr,
+                lloyd_loop_step_kernel<<<1, 1, 0, cs>>>(loop_st, cost, err, tc ? b.err : nullptr,
                                                         loop_inertias, h);
                 cudaGraph_t out = nullptr;
                 const cudaError_t e2 = cudaStreamEndCapture(cs, &out);
@@ -1181,7 +1252,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         uint32_t h_err = 0, tc_err = 0;
         cudaError_t e = cudaMemcpyAsync(&h_cost, cost, sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && is_tc(prec))
+        if (e == cudaSuccess && tc)
             e = cudaMemcpyAsync(&tc_err, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
@@ -1340,7 +1411,10 @@ int km_centers_create(const float *C, int32_t k, int32_t d, int32_t precision, v
     h->prec = prec;
     cudaGetDevice(&h->device);
     const size_t c_bytes = ((size_t)k * d * sizeof(float) + 255) / 256 * 256;
-    h->bytes = c_bytes + (is_tc(prec) ? tc_centers_ws_size(d, k) : 0);
+    h->asked = precision;
+    h->small = small_route(precision, prec, -1, d, k, true);
+    const bool center_half = is_tc(prec) || h->small;
+    h->bytes = c_bytes + (center_half ? tc_centers_ws_size(d, k) : 0);
     cudaError_t e = cudaMalloc(&h->mem, h->bytes);
     if (e != cudaSuccess) {
         delete h;
@@ -1350,11 +1424,12 @@ int km_centers_create(const float *C, int32_t k, int32_t d, int32_t precision, v
     int st = KM_OK;
     e = cudaMemcpyAsync(h->C, C, (size_t)k * d * sizeof(float), cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) st = cuda_fail(e, "cudaMemcpyAsync (resident centers)");
-    if (st == KM_OK && is_tc(prec)) {
+    if (st == KM_OK && center_half) {
         tc_carve_centers(static_cast<char *>(h->mem) + c_bytes, d, k, h->tc);
-        tc_set_operand(h->tc, d, prec);
+        if (is_tc(prec)) tc_set_operand(h->tc, d, prec);
         st = tc_prepare_shift_from_centers(h->C, d, k, h->tc, s);
-        if (st == KM_OK) st = tc_prepare_centers(h->C, d, k, h->tc, s);
+        if (st == KM_OK && is_tc(prec)) st = tc_prepare_centers(h->C, d, k, h->tc, s);
+        if (st == KM_OK && h->small) st = small_prepare_centers(h->C, d, k, h->tc, s);
     }
     if (st == KM_OK) {
         e = cudaStreamSynchronize(s);
@@ -1395,7 +1470,7 @@ int km_centers_info(const km_centers *h, int32_t *k, int32_t *d, int32_t *precis
 
 size_t km_assign_centers_workspace_size(int64_t n, const km_centers *h) {
     if (!h || check_shape(n, h->d, h->k) != KM_OK) return 0;
-    return resident_ws_bytes(n, h->d, h->k, h->prec);
+    return resident_ws_bytes(n, h->d, h->k, h->prec, h->small_for(n));
 }
 
 int km_assign_centers(const float *X, int64_t n, int32_t d, const km_centers *h, int32_t *labels, void *workspace,
@@ -1413,9 +1488,13 @@ int km_assign_centers(const float *X, int64_t n, int32_t d, const km_centers *h,
         set_error("X and labels must be non-NULL");
         return KM_ERR_BAD_SHAPE;
     }
-    KM_TRY(check_ws(workspace, workspace_bytes, resident_ws_bytes(n, d, h->k, h->prec)));
+    const bool small = h->small_for(n);
+    KM_TRY(check_ws(workspace, workspace_bytes, resident_ws_bytes(n, d, h->k, h->prec, small)));
     TcBuffers b;
-    if (is_tc(h->prec) && n > 0) {
+    if (small && n > 0) {
+        b = h->tc;  // no frame copy: the lists only
+        tc_carve_assign(workspace, n, d, h->k, b);
+    } else if (is_tc(h->prec) && n > 0) {
         b = h->tc;  // prepared center half; the carves below fill the frame and list fields
         char *p = static_cast<char *>(workspace);
         tc_carve_frames(p, n, d, b);
@@ -1423,7 +1502,7 @@ int km_assign_centers(const float *X, int64_t n, int32_t d, const km_centers *h,
         tc_carve_assign(p, n, d, h->k, b);
         tc_set_operand(b, d, h->prec);
     }
-    return assign_core(X, n, d, h->C, h->k, h->prec, labels, b, true, stats, static_cast<cudaStream_t>(stream));
+    return assign_core(X, n, d, h->C, h->k, h->prec, small, labels, b, true, stats, static_cast<cudaStream_t>(stream));
 }
 
 // ---- precision autotuning ----------------------------------------------------

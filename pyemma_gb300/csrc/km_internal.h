@@ -161,9 +161,14 @@ void tc_store_plan(int d, int k, const TilePlan &plan);
 void tc_clear_plans();
 // The shape a call for (d, k) uses now; *tuned: it comes from the table.
 bool tc_current_plan(int d, int k, TilePlan *out, bool *tuned);
+// A shape is forced on this thread or stored for (d, k).
+bool tc_plan_set(int d, int k);
 size_t tc_frames_ws_size(int64_t n, int d);     // fp16 frame copy + norms
 size_t tc_centers_ws_size(int d, int k);        // fp16 centers + norms + shift + scalars
 size_t tc_assign_ws_size(int64_t n, int d, int k);  // candidate lists + counters
+
+// Word of counters at which the eight 64-bit diagnostic counters start.
+constexpr int kTcDiagWords = 8;
 
 #define TC_CANDIDATES 16  // candidate centers kept per frame by the tensor-core pass
 
@@ -187,9 +192,13 @@ struct TcBuffers {
     int32_t *amb_mask = nullptr;            // their candidates (bit t: pair first + t) for the exact pass
     int32_t *full_frames = nullptr;
     unsigned long long *full_keys = nullptr;
+    // The words of a call's status lie side by side, so that one memset clears
+    // and one copy reads them (TcStatus).
     int32_t *counters = nullptr;  // [0] recheck entries, [1] full entries, [2] pairs, [3] unsettled entries
     unsigned long long *flipped = nullptr;
     uint32_t *err = nullptr;
+    void *sch = nullptr;         // narrow frames (assign_small.cu): split FP16 operand rows of the centers
+    float *scg = nullptr;        // narrow frames: the centers by groups of eight, [group][feature][8]
     float *chn = nullptr;        // FP8 only: -||c~_j||^2 / 2 per center (the norm is not folded into the GEMM)
     int kp = 0;        // operand row length in elements
     int esize = 2;     // operand bytes per element: 2 (FP16, BF16) or 1 (FP8 e4m3)
@@ -197,6 +206,15 @@ struct TcBuffers {
     int fp8 = 0;       // 1: e4m3 operands (frames scaled per row), norms applied in the epilogue
     int keep_err = 0;  // 1: tc_assign leaves err as it is (the caller clears it once for several calls)
 };
+
+// The status words as one copy from counters gives them.
+struct TcStatus {
+    int32_t counters[4];
+    unsigned long long flipped;
+    uint32_t err, pad;
+};
+// counters[0..4), flipped and (unless keep_err) err cleared on s.
+int tc_clear_status(const TcBuffers &b, cudaStream_t s);
 
 // The same buffers for frames [a, ...): the per-frame arrays start at row a.
 inline TcBuffers tc_rows_from(const TcBuffers &b, int64_t a) {
@@ -238,6 +256,25 @@ int tc_assign_deferred(const float *X, int64_t n, int d, const float *C, int k, 
                        cudaStream_t s, cudaStream_t side, const cudaEvent_t *ev_fork, int n_fork,
                        const FlipList &fl, ProfEvents *prof = nullptr, const PairSrc *ps = nullptr,
                        int32_t *label_counts = nullptr);
+
+// ---- assign_small.cu ---------------------------------------------------------
+// Assignment of narrow frames by split FP16 operands, converted in the kernel
+// (no frame copy), with the exact distances of the best eight centers in the
+// epilogue.  Uses shift, scal, sch, scg and the candidate-list half of
+// TcBuffers.  KM_TC_SMALL=0 or 1 in the environment keeps it off or forces it
+// (the labels are the same).
+bool small_shape_ok(int d, int k);
+bool small_allowed();
+bool small_forced();
+size_t small_centers_elems(int d, int k);  // FP16 elements of sch
+size_t small_groups_floats(int d, int k);  // floats of scg
+int small_prepare_centers(const float *C, int d, int k, TcBuffers &b, cudaStream_t s);
+// The pass on s, then the exact re-check over all centers of the frames it
+// could not settle: on s, or with `side` on that stream (after `fork`,
+// recorded on s) with the changed labels in fl, as in tc_assign_deferred.
+int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuffers &b, cudaStream_t s,
+                 ProfEvents *prof = nullptr, cudaStream_t side = nullptr, cudaEvent_t fork = nullptr,
+                 const FlipList *fl = nullptr, int32_t *label_counts = nullptr);
 
 // Resident center sets (capi.cu), used by the serving loop (serve.cu).
 int assign_centers_enqueue(const float *X, int64_t n, const km_centers *h, int32_t *labels, void *ws,
