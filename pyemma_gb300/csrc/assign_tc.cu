@@ -256,6 +256,35 @@ __global__ void scale_finalize_kernel(uint32_t *__restrict__ scal) {
     scal[kInvScale2] = __float_as_uint(ldexpf(1.0f, -2 * sigma));
 }
 
+// The three sums of a frame row over a warp's lanes: ||x_hat||^2 enters the
+// distance itself: a Kahan sum per lane (within about 2u of the lane's terms;
+// the distance bound allows 8u for this norm).  The other two are bounds
+// inflated by norm_inflate (far above the few units of rounding of a plain
+// per-lane sum): plain float32.
+struct PrepSums {
+    float hs = 0.0f, hc = 0.0f, s2 = 0.0f, e2 = 0.0f;
+    // the operand h of the scaled value ia = a * scale
+    __device__ __forceinline__ void add(float h, float ia, float a) {
+        const float ee = h - ia;
+        const float y = __fsub_rn(__fmul_rn(h, h), hc);
+        const float t = __fadd_rn(hs, y);
+        hc = __fsub_rn(__fsub_rn(t, hs), y);
+        hs = t;
+        s2 = __fmaf_rn(a, a, s2);
+        e2 = __fmaf_rn(ee, ee, e2);
+    }
+    __device__ __forceinline__ void store(float4 *xnorm, float inv_sc, float norm_inflate, int lane) const {
+        const float th = warp_sum_ff(hs, -hc);
+        const float ts = warp_sum_ff(s2, 0.0f);
+        const float te = warp_sum_ff(e2, 0.0f);
+        if (lane == 0) {
+            const float sx = __fsqrt_ru(__fmul_ru(ts, norm_inflate));
+            const float hx = __fmul_ru(__fadd_ru(__fsqrt_ru(__fmul_ru(te, norm_inflate)), 1e-30f), inv_sc);
+            *xnorm = make_float4(th, sx, hx, 0.0f);
+        }
+    }
+};
+
 // Frames: one warp per row.  xnorm = (||x_hat||^2 in scaled units, upper
 // bound of ||x'||, upper bound of ||x_hat/s - x'||, 0) in unscaled units.
 // get(f) gives feature f of row i.
@@ -266,7 +295,7 @@ __device__ __forceinline__ void prep_one_row(const Get &get, int64_t i, int d, i
                                              int lane) {
     using O = Op16<T>;
     typename O::T2 *dst = reinterpret_cast<typename O::T2 *>(xh + i * kp);
-    CSum h2, s2, e2;
+    PrepSums sums;
     for (int f = 2 * lane; f < kp; f += 64) {
         // Columns < d: centered, scaled frame values; d and d+1: 1 (they
         // meet the hi/lo norm columns of the centers); the rest: 0.
@@ -285,29 +314,10 @@ __device__ __forceinline__ void prep_one_row(const Get &get, int64_t i, int d, i
         }
         const typename O::T2 h = O::pack(ia, ib);
         dst[f >> 1] = h;
-        if (f < d) {
-            const float ha = O::lo(h);
-            const float ea = ha - ia;
-            h2.add(ha * ha);
-            s2.add(a * a);
-            e2.add(ea * ea);
-        }
-        if (f + 1 < d) {
-            const float hb = O::hi(h);
-            const float eb = hb - ib;
-            h2.add(hb * hb);
-            s2.add(b * b);
-            e2.add(eb * eb);
-        }
+        if (f < d) sums.add(O::lo(h), ia, a);
+        if (f + 1 < d) sums.add(O::hi(h), ib, b);
     }
-    const float th = warp_sum_ff(h2.s, h2.c);
-    const float ts = warp_sum_ff(s2.s, s2.c);
-    const float te = warp_sum_ff(e2.s, e2.c);
-    if (lane == 0) {
-        const float sx = __fsqrt_ru(__fmul_ru(ts, norm_inflate));
-        const float hx = __fmul_ru(__fadd_ru(__fsqrt_ru(__fmul_ru(te, norm_inflate)), 1e-30f), inv_sc);
-        xnorm[i] = make_float4(th, sx, hx, 0.0f);
-    }
+    sums.store(xnorm + i, inv_sc, norm_inflate, lane);
 }
 
 template <typename T, class Src>
@@ -415,12 +425,7 @@ __global__ void __launch_bounds__(256, 2) prep_frames_v4_kernel(const float *__r
         // The next row's loads are in flight while this row is converted.
         float4 nx[IT];
         load_row(i + nw, nx);
-        // ||x_hat||^2 enters the distance itself: a Kahan sum per lane (within
-        // about 2u of the lane's terms; the distance bound allows 8u for this
-        // norm).  The other two are bounds inflated by norm_inflate (far above
-        // the few units of rounding of a plain per-lane sum): plain float32.
-        float hs = 0.0f, hc = 0.0f;
-        float s2 = 0.0f, e2 = 0.0f;
+        PrepSums sums;
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int f = 4 * lane + 128 * it;
@@ -445,28 +450,58 @@ __global__ void __launch_bounds__(256, 2) prep_frames_v4_kernel(const float *__r
             *reinterpret_cast<uint2 *>(xh + i * kp + f) = packed;
             const float hv[4] = {O::lo(h01), O::hi(h01), O::lo(h23), O::hi(h23)};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (f + e < d) {
-                    const float ee = hv[e] - ia[e];
-                    const float y = __fsub_rn(__fmul_rn(hv[e], hv[e]), hc);
-                    const float t = __fadd_rn(hs, y);
-                    hc = __fsub_rn(__fsub_rn(t, hs), y);
-                    hs = t;
-                    s2 = __fmaf_rn(a[e], a[e], s2);
-                    e2 = __fmaf_rn(ee, ee, e2);
-                }
-            }
+            for (int e = 0; e < 4; ++e)
+                if (f + e < d) sums.add(hv[e], ia[e], a[e]);
         }
-        const float th = warp_sum_ff(hs, -hc);
-        const float ts = warp_sum_ff(s2, 0.0f);
-        const float te = warp_sum_ff(e2, 0.0f);
-        if (lane == 0) {
-            const float sx = __fsqrt_ru(__fmul_ru(ts, norm_inflate));
-            const float hx = __fmul_ru(__fadd_ru(__fsqrt_ru(__fmul_ru(te, norm_inflate)), 1e-30f), inv_sc);
-            xnorm[i] = make_float4(th, sx, hx, 0.0f);
-        }
+        sums.store(xnorm + i, inv_sc, norm_inflate, lane);
 #pragma unroll
         for (int it = 0; it < IT; ++it) xv[it] = nx[it];
+    }
+}
+
+// The same for rows of any length and alignment: lanes own consecutive
+// columns (coalesced 4-byte loads, 2-byte stores), kPrepSlices 32-column slices of
+// the row in flight per warp.  250,007 x 1,023 frames: 343 us (4.7 TB/s), 588 with two
+// columns per lane, one slice at a time and three compensated sums per value.
+constexpr int kPrepSlices = 8;
+template <typename T>
+__global__ void __launch_bounds__(256, 6) prep_frames_dense_kernel(const float *__restrict__ X, int64_t n, int d,
+                                                                   int kp, const float *__restrict__ shift,
+                                                                   const uint32_t *__restrict__ scal,
+                                                                   T *__restrict__ xh, float4 *__restrict__ xnorm,
+                                                                   float norm_inflate) {
+    using O = Op16<T>;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const float sc = __uint_as_float(scal[kScale]);
+    const float inv_sc = 1.0f / sc;  // exact: a power of two
+    for (int64_t i = w; i < n; i += nw) {
+        const float *src = X + i * d;
+        T *dst = xh + i * kp;
+        PrepSums sums;
+        for (int f0 = lane; f0 < kp; f0 += 32 * kPrepSlices) {
+            float v[kPrepSlices], m[kPrepSlices];
+#pragma unroll
+            for (int q = 0; q < kPrepSlices; ++q) {
+                const int f = f0 + 32 * q;
+                v[q] = f < d ? __ldg(src + f) : 0.0f;
+                m[q] = f < d ? __ldg(shift + f) : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < kPrepSlices; ++q) {
+                // Columns < d: centered, scaled frame values; d and d+1: 1
+                // (they meet the hi/lo norm columns of the centers); the rest: 0.
+                const int f = f0 + 32 * q;
+                if (f >= kp) break;
+                const float a = __fsub_rn(v[q], m[q]);
+                const float ia = f < d ? a * sc : (f == d || f == d + 1) ? 1.0f : 0.0f;
+                const T h = O::one(ia);
+                dst[f] = h;
+                if (f < d) sums.add(O::to_float(h), ia, a);
+            }
+        }
+        sums.store(xnorm + i, inv_sc, norm_inflate, lane);
     }
 }
 
@@ -1682,9 +1717,8 @@ void prepare_frames_t(const float *X, int64_t n, int d, TcBuffers &b, cudaStream
             default: launch_prep_v4<T, 9>(X, n, d, b, s); break;
         }
     } else {
-        prep_frames_kernel<T><<<(unsigned)prep_blocks(n), 256, 0, s>>>(DenseRows{X, d}, n, d, b.kp, b.shift, b.scal,
-                                                                     reinterpret_cast<T *>(b.xh), b.xnorm,
-                                                                     norm_inflate_of(d));
+        prep_frames_dense_kernel<T><<<(unsigned)prep_blocks(n), 256, 0, s>>>(
+            X, n, d, b.kp, b.shift, b.scal, reinterpret_cast<T *>(b.xh), b.xnorm, norm_inflate_of(d));
     }
 }
 
