@@ -361,15 +361,8 @@ cudaError_t instantiate_with_priorities(cudaGraphExec_t *gx, cudaGraph_t g) {
 // inertia, applies the stopping rule on the device and sets the loop's
 // condition, so a run of iterations costs one launch and one read-back.
 // A launch runs at most kLoopBatch iterations (the size of the inertia
-// buffer in the workspace).
-struct LoopState {
-    double prev;
-    double tol;
-    int32_t it;      // iterations run by this launch
-    int32_t max_it;  // bound for this launch
-    int32_t converged;
-    uint32_t err;
-};
+// buffer in the workspace).  Few, narrow centers under FP32 take one
+// cooperative launch instead (lloyd_small.cu).
 constexpr int kLoopBatch = 64;
 
 __global__ void lloyd_loop_step_kernel(LoopState *st, const double *cost, const uint32_t *err_update,
@@ -402,6 +395,8 @@ size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
         c.take<int32_t>(3 * (size_t)n);  // flip list
         c.take<int32_t>(1);              // its count
     }
+    // at every n, so that the size of the largest n serves the smaller ones
+    if (!is_tc(prec) && small_lloyd_shape_ok(d, k)) c.take<char>(small_lloyd_ws_size(d, k));
     return c.bytes();
 }
 
@@ -896,9 +891,13 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
-    const bool small = !ps && small_route(precision, prec, n, d, k, true);
+    const bool narrow = !ps && small_route(precision, prec, n, d, k, true);
+    // Few, narrow centers: whole iterations in one launch (lloyd_small.cu).
+    const bool fits = !ps && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
+                      (!narrow || (!small_forced() && small_lloyd_beats_narrow(n, d, k)));
+    const bool small = narrow && !fits;
     const bool tc = is_tc(prec) || small;
-    const size_t need = lloyd_ws_bytes(n, d, k, prec, small);
+    const size_t need = lloyd_ws_bytes(n, d, k, prec, narrow);
     KM_TRY(check_ws(workspace, workspace_bytes, need));
     if (max_iter == 0 && !hf) return KM_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1209,10 +1208,42 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         return status;
     };
 
+    // The iterations it0, it0+1, ..., one launch per kLoopBatch of them (one
+    // per iteration with a callback).
+    const bool fused = fits && !prof.active;
+    void *ws_fused = fused ? cv.take<char>(small_lloyd_ws_size(d, k)) : nullptr;
+    auto fused_loop = [&](int32_t it0, double prev0) -> int {
+        int32_t it = it0;
+        double prev = prev0;
+        while (it < max_iter) {
+            LoopState hs{prev, tolerance, 0, cb ? 1 : std::min(kLoopBatch, max_iter - it), 0, 0u};
+            double hin[kLoopBatch];
+            KM_CUDA(cudaMemcpyAsync(loop_st, &hs, sizeof(hs), cudaMemcpyHostToDevice, s));
+            KM_TRY(launch_small_lloyd(X, n, d, k, C, labels, ws_fused, loop_st, loop_inertias, s));
+            KM_CUDA(cudaMemcpyAsync(&hs, loop_st, sizeof(hs), cudaMemcpyDeviceToHost, s));
+            KM_CUDA(cudaMemcpyAsync(hin, loop_inertias, sizeof(double) * hs.max_it, cudaMemcpyDeviceToHost, s));
+            KM_CUDA(cudaStreamSynchronize(s));
+            KM_TRY(check_device_errors(hs.err));
+            for (int32_t j = 0; j < hs.it; ++j)
+                if (inertias) inertias[it + j] = hin[j];
+            it += hs.it;
+            *n_iter = it;
+            if (hs.it > 0) prev = hin[hs.it - 1];
+            if (cb) cb(cb_user);
+            if (hs.converged) *converged = 1;
+            if (hs.converged || hs.it == 0) break;
+        }
+        return KM_OK;
+    };
+
     cudaGraphExec_t exec = nullptr;
     int status = KM_OK;
     double prev = 0.0;
     for (int32_t it = 0; it < max_iter; ++it) {
+        if (fused && (it == 1 || !hf)) {
+            status = fused_loop(it, prev);
+            break;
+        }
         if (it == 1 && !cb && !prof.active) {
             int handled = 0;
             status = device_loop(it, prev, handled);

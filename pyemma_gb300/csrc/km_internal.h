@@ -126,6 +126,26 @@ int launch_update_parts_finish(int64_t n, int d, int k, const float *C_old, floa
 int launch_apply_flips(const float *X, int64_t n, int d, int k, const float *C_old, const FlipList &fl,
                        int32_t *labels, void *ws, cudaStream_t s, const PairSrc *ps = nullptr);
 
+// ---- lloyd_small.cu ----------------------------------------------------------
+// State of a run of Lloyd iterations on the device.
+struct LoopState {
+    double prev;     // inertia before the first iteration
+    double tol;
+    int32_t it;      // iterations run by this launch
+    int32_t max_it;  // bound for this launch
+    int32_t converged;
+    uint32_t err;
+};
+// Up to st->max_it exact float32 Lloyd iterations of few, narrow centers in
+// one cooperative launch: C and labels as km_lloyd leaves them, inertias[0..it)
+// (device) and st updated.  st->err takes the bit of a wait that ran out.
+bool small_lloyd_shape_ok(int d, int k);
+bool small_lloyd_ok(int64_t n, int d, int k);            // fits, and beats the separate FP32 kernels
+bool small_lloyd_beats_narrow(int64_t n, int d, int k);  // beats iterations on the narrow-frame kernel
+size_t small_lloyd_ws_size(int d, int k);
+int launch_small_lloyd(const float *X, int64_t n, int d, int k, float *C, int32_t *labels, void *ws, LoopState *st,
+                       double *inertias, cudaStream_t s);
+
 // ---- kmpp.cu -----------------------------------------------------------------
 size_t kmpp_ws_size(int64_t n, int d, int k);
 // D^2 of kmeans++ under the minRMSD metric: the centered frames Xc with
