@@ -336,4 +336,36 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// Barrier over the CTAs of a cooperative launch: one count per CTA, target =
+// gridDim.x times the barriers so far.  False when the others did not arrive
+// in time or another CTA gave up (*err != 0).
+__device__ __forceinline__ bool grid_barrier(unsigned int *count, unsigned int target, uint32_t *err) {
+    __shared__ bool ok_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(count, 1u);
+        bool ok = true;
+        const uint64_t t0 = globaltimer_ns();
+        for (uint32_t spin = 1;; ++spin) {
+            unsigned int c;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+            if (c >= target) break;
+            if ((spin & 255u) == 0) {
+                uint32_t e;
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
+                if (e != 0u || globaltimer_ns() - t0 > kWaitLimitNs) {
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        if (!ok) atomicOr(err, (uint32_t)kDevTimeoutEpi);
+        __threadfence();
+        ok_s = ok;
+    }
+    __syncthreads();
+    return ok_s;
+}
+
 }  // namespace km

@@ -15,27 +15,26 @@
 // t = floor(u * W / 2^64) for the weight total W and picks the first frame
 // whose inclusive prefix weight exceeds t.
 //
-// Per round one launch: a pass over X (distance to the newest center,
-// running minimum, per-tile weight sums; HBM-bound), after which the CTA that
-// finishes last (a fenced atomic count, no waiting) draws the round's frame
-// and copies it into the centers.
+// Euclidean rounds run in cooperative launches of up to kRoundBatch rounds
+// (kmpp_rounds_kernel): every warp keeps the same frames in every round,
+// lowers their minima by the newest center and adds the change of their
+// integer weights to the tile sums; after a grid barrier every CTA makes the
+// same draw from the same sums, so the new center needs no second exchange.
 //
-// Pruning (Euclidean metric, large n d): each frame keeps, besides
-// D^2 = mind, the index a of a center whose exact distance is mind.  Round r
-// (r >= 2) runs three launches:
-//   1. cc_j = ||c_new - c_j||^2 for every earlier center j (float32);
-//   2. a pass over (mind, a) only: by the triangle inequality
-//      ||x - c_new|| >= ||c_new - c_a|| - ||x - c_a||, so when cc_a >= 4 mind
-//      (times a factor covering the float32 rounding of mind, of the new
-//      distance and of cc) the exact new distance cannot fall below mind;
-//      the other frames go into a list;
-//   3. the listed frames' exact distances, spread over every SM; a frame
-//      whose minimum drops updates mind and a, and adds the change of its
-//      integer weight to its tile's sum; the CTA that finishes last draws.
-// The running minima, and so the draws, are the same as without pruning, bit
-// for bit.  A skipped frame costs 8 bytes (mind, a) instead of 4d + 4, and
-// the tile sums are kept exact by the integer deltas (the first round stores
-// them in full).
+// Pruning (large n d): each frame keeps, besides D^2 = mind, the index a of a
+// center whose exact distance is mind.  Each round starts with
+//   cc_j = ||c_new - c_j||^2 for every earlier center j (float32), a warp per
+//   center over the whole grid, and a second barrier.
+// By the triangle inequality ||x - c_new|| >= ||c_new - c_a|| - ||x - c_a||,
+// so when cc_a >= 4 mind (times a factor covering the float32 rounding of
+// mind, of the new distance and of cc) the exact new distance cannot fall
+// below mind and the frame's row is not read.  The running minima, and so the
+// draws, are the same as without pruning, bit for bit.  A skipped frame costs
+// 8 bytes (mind, a) instead of 4d + 4.
+//
+// Under the minRMSD metric a round is one launch per center: a pass over the
+// frames, after which the CTA that finishes last (a fenced atomic count, no
+// waiting) draws the round's frame and copies it into the centers.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -50,34 +49,49 @@ namespace km {
 
 namespace {
 
-constexpr int kTile = 2048;  // frames per weight tile
+constexpr int kTile = 2048;  // frames per weight tile (minRMSD)
 constexpr int kTileThreads = 256;
+constexpr int kRoundThreads = 1024;
+constexpr int kRoundBatch = 64;   // rounds per launch
+constexpr int kWide = 32;         // features from which a warp forms the distances together
+
+// Tiles of the Euclidean rounds: 128 to 16,384 frames, about 2,048 tiles in
+// between (the draw scans the tiles, then one tile: two or three values per
+// thread each up to 4 million frames).
+int tile_shift(int64_t n) {
+    int sh = 7;
+    while (sh < 14 && (n >> sh) > 2048) ++sh;
+    return sh;
+}
+
+int64_t tile_slots(int64_t n) {
+    const int sh = tile_shift(n);
+    return std::max<int64_t>((n + (int64_t(1) << sh) - 1) >> sh, 1);
+}
 
 struct KmppWs {
     float *mind;
-    int32_t *near;  // a center whose exact distance is mind (pruned Euclidean pass)
+    int32_t *near;  // a center whose exact distance is mind (pruned rounds), or mind of the other parity
     float *cc;      // bounds of ||c_new - c_j||^2 for the current round
-    unsigned long long *tile_sum;
+    unsigned long long *tile_sum;  // three sets (Euclidean) of tile_slots, or one of n / kTile
     uint32_t *maxbits;
     int *qexp;      // e of the weights floor(D^2 2^e); INT_MIN: every weight is 0
-    unsigned int *done;  // CTAs of the current round that have finished
-    int32_t *list;       // frames of the round that the bound does not rule out
-    int32_t *list_n;
+    unsigned int *done;  // CTAs of the current round that have finished; barrier count
+    uint32_t *err;
 };
 
 KmppWs carve(void *ws, int64_t n, int k, size_t *bytes) {
     Carver c(ws);
     KmppWs w;
-    const int64_t ntiles = (n + kTile - 1) / kTile;
+    const int64_t tiles = std::max<int64_t>(3 * tile_slots(n), (n + kTile - 1) / kTile);
     w.mind = c.take<float>(n > 0 ? n : 1);
     w.near = c.take<int32_t>(n > 0 ? n : 1);
     w.cc = c.take<float>(k > 0 ? k : 1);
-    w.tile_sum = c.take<unsigned long long>(ntiles > 0 ? ntiles : 1);
+    w.tile_sum = c.take<unsigned long long>(tiles);
     w.maxbits = c.take<uint32_t>(1);
     w.qexp = c.take<int>(1);
     w.done = c.take<unsigned int>(1);
-    w.list = c.take<int32_t>(n > 0 ? n : 1);
-    w.list_n = c.take<int32_t>(1);
+    w.err = c.take<uint32_t>(1);
     if (bytes) *bytes = c.bytes();
     return w;
 }
@@ -107,41 +121,22 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
     return s;  // valid in thread 0
 }
 
-// D^2 of frame i to center c (round r's newest center, frame idx[r] under
-// the minRMSD metric).
-__device__ __forceinline__ float kmpp_d2(const float *__restrict__ X, int64_t i, int d, const float *__restrict__ c,
-                                         const KmppMetric &m, int r) {
-    if (!m.Xc) return sqdist_exact(X + i * d, c, d);
+// D^2 of frame i to the center drawn in round r under the minRMSD metric.
+__device__ __forceinline__ float kmpp_rmsd_d2(int64_t i, int d, const KmppMetric &m, int r) {
     const int64_t p = m.idx[r];
     return __double2float_rn(rmsd_msd_rows(m.Xc + i * d, m.Xc + p * d, m.G[i], m.G[p], d / 3));
 }
 
-// The exact float32 D^2 of frame i of a row source to the center c.
-template <class Src>
-__device__ __forceinline__ float src_d2(const Src &src, int64_t i, const float *__restrict__ c, int d) {
-    if constexpr (std::is_same<Src, DenseRows>::value)
-        return sqdist_exact(src.X + i * d, c, d);
-    else
-        return sqdist_exact_src(src, i, c, d);
-}
-
-// Round 1 pass: mind = D^2 to center 0 (near = 0); max of the finite values.
-template <class Src>
-__global__ void __launch_bounds__(kTileThreads) kmpp_first_kernel(
-    const Src src, int64_t n, int d, const float *__restrict__ c0,
-    float *__restrict__ mind, int32_t *__restrict__ near, uint32_t *__restrict__ maxbits, KmppMetric m) {
+// minRMSD, round 1: mind = D^2 to center 0; max of the finite values.
+__global__ void __launch_bounds__(kTileThreads) kmpp_first_kernel(int64_t n, int d, float *__restrict__ mind,
+                                                                  uint32_t *__restrict__ maxbits, KmppMetric m) {
     float mx = 0.0f;
     const int64_t t0 = (int64_t)blockIdx.x * kTile;
     for (int u = 0; u < kTile / kTileThreads; ++u) {
         const int64_t i = t0 + u * kTileThreads + threadIdx.x;
         if (i < n) {
-            float dd;
-            if constexpr (std::is_same<Src, DenseRows>::value)
-                dd = kmpp_d2(src.X, i, d, c0, m, 0);
-            else
-                dd = src_d2(src, i, c0, d);
+            const float dd = kmpp_rmsd_d2(i, d, m, 0);
             mind[i] = dd;
-            near[i] = 0;
             if (dd < __int_as_float(0x7f800000) && dd > mx) mx = dd;
         }
     }
@@ -151,13 +146,9 @@ __global__ void __launch_bounds__(kTileThreads) kmpp_first_kernel(
 
 // e = 62 - ceil(log2 n) - E(max) with 2^(E-1) <= max < 2^E (weights
 // floor(D^2 2^e)); INT_MIN when no distance is finite and positive.
-__global__ void kmpp_scale_kernel(const uint32_t *__restrict__ maxbits, int64_t n, int *__restrict__ qexp) {
-    const uint32_t b = *maxbits;
+__device__ __forceinline__ int weight_exponent(uint32_t b, int64_t n) {
     const float m = __uint_as_float(b);
-    if (!(m > 0.0f) || m == __int_as_float(0x7f800000)) {
-        *qexp = INT_MIN;
-        return;
-    }
+    if (!(m > 0.0f) || m == __int_as_float(0x7f800000)) return INT_MIN;
     int L = 0;
     while ((int64_t(1) << L) < n) ++L;
     const int be = (int)((b >> 23) & 0xFFu);
@@ -168,28 +159,11 @@ __global__ void kmpp_scale_kernel(const uint32_t *__restrict__ maxbits, int64_t 
         const int p = 31 - __clz(b & 0x7FFFFFu);
         E = p - 148;
     }
-    *qexp = 62 - L - E;
+    return 62 - L - E;
 }
 
-// Round r's bounds: cc[j] = the float32 value of ||C0[rc] - C0[j]||^2 for
-// j < rc, one warp per center (lanes stride over the features with fused
-// multiply-adds, then a shuffle tree).  Its rounding is covered by the prune
-// factor (prune_factor()).
-__global__ void __launch_bounds__(256) kmpp_cc_kernel(const float *__restrict__ C0, int d, int rc,
-                                                      float *__restrict__ cc) {
-    const int j = (int)(blockIdx.x * 8 + (threadIdx.x >> 5));
-    const int lane = threadIdx.x & 31;
-    if (j >= rc) return;
-    const float *a = C0 + (int64_t)rc * d;
-    const float *b = C0 + (int64_t)j * d;
-    float acc = 0.0f;
-    for (int f = lane; f < d; f += 32) {
-        const float t = __fsub_rn(__ldg(a + f), __ldg(b + f));
-        acc = __fmaf_rn(t, t, acc);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-    if (lane == 0) cc[j] = acc;
+__global__ void kmpp_scale_kernel(const uint32_t *__restrict__ maxbits, int64_t n, int *__restrict__ qexp) {
+    *qexp = weight_exponent(*maxbits, n);
 }
 
 // Exclusive prefix sum of v over the CTA (THREADS threads, warp shuffles
@@ -223,20 +197,19 @@ __device__ __forceinline__ unsigned long long cta_exclusive_scan_u64(unsigned lo
     return (warp > 0 ? warp_tot[warp - 1] : 0ull) + x - v;
 }
 
-// The draw of round r by the CTA that finished last (the tile sums and the
-// minima of the other CTAs are read past L1): t = floor(u W / 2^64) for the
-// weight total W over the ntiles tiles, the first frame whose inclusive
-// prefix weight exceeds t (a uniform frame when W = 0), copied into C0[r].
-template <int THREADS, class Src>
-__device__ __forceinline__ void kmpp_draw_round(int64_t ntiles, const Src &src, int64_t n, int d,
-                                                float *__restrict__ C0, int64_t *__restrict__ idx_out,
-                                                const float *__restrict__ mind, int qexp,
-                                                const unsigned long long *__restrict__ tile_sum,
-                                                unsigned int *__restrict__ done, int r, uint32_t seed) {
-    constexpr int kPer = kTile / THREADS;  // frames per thread in the draw's tile
+// The draw of round r by a whole CTA (the tile sums and the minima of other
+// CTAs are read past L1): t = floor(u W / 2^64) for the weight total W over
+// the tiles of 2^shift frames, the first frame whose inclusive prefix weight
+// exceeds t (a uniform frame when W = 0).  The frame, in every thread.
+template <int THREADS>
+__device__ __forceinline__ int64_t kmpp_draw_round(int64_t ntiles, int shift, int64_t n,
+                                                   const float *__restrict__ mind, int qexp,
+                                                   const unsigned long long *__restrict__ tile_sum, int r,
+                                                   uint32_t seed) {
     __shared__ unsigned long long red[THREADS / 32];
     __shared__ long long tile_hit, pick;
     __shared__ unsigned long long target;
+    __syncthreads();  // the last draw's values have been read
     if (threadIdx.x == 0) {
         tile_hit = -1;
         pick = -1;
@@ -266,37 +239,28 @@ __device__ __forceinline__ void kmpp_draw_round(int64_t ntiles, const Src &src, 
     }
     __syncthreads();
     if (tile_hit >= 0) {
-        // Inside the tile: kPer consecutive frames per thread.
-        const int64_t f0 = tile_hit * kTile + (int64_t)threadIdx.x * kPer;
-        unsigned long long w[kPer], ws = 0;
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            w[q] = f0 + q < n ? quant_weight(__ldcg(mind + f0 + q), qexp) : 0ull;
-            ws += w[q];
-        }
+        // Inside the tile: consecutive frames per thread.
+        const int tper = max(1, (1 << shift) / THREADS);
+        const int64_t first = (int64_t)tile_hit << shift, end = min(n, first + (int64_t(1) << shift));
+        const int64_t f0 = min(first + (int64_t)threadIdx.x * tper, end), f1 = min(f0 + tper, end);
+        unsigned long long ws = 0;
+        for (int64_t f = f0; f < f1; ++f) ws += quant_weight(__ldcg(mind + f), qexp);
         unsigned long long tile_total;
         unsigned long long run = cta_exclusive_scan_u64<THREADS>(ws, red, &tile_total);
         const unsigned long long tt = target;
         if (run <= tt && tt < run + ws) {
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                if (tt < run + w[q]) {
-                    pick = f0 + q;
+            for (int64_t f = f0; f < f1; ++f) {
+                const unsigned long long w = quant_weight(__ldcg(mind + f), qexp);
+                if (tt < run + w) {
+                    pick = f;
                     break;
                 }
-                run += w[q];
+                run += w;
             }
         }
     }
     __syncthreads();
-    if (pick < 0 && threadIdx.x == 0) pick = (long long)__umul64hi(u, (unsigned long long)n);
-    __syncthreads();
-    const int64_t p = pick;
-    for (int f = threadIdx.x; f < d; f += THREADS) C0[(int64_t)r * d + f] = src.get(p, f);
-    if (threadIdx.x == 0) {
-        if (idx_out) idx_out[r] = p;
-        *done = 0u;  // for the next round's launch
-    }
+    return pick >= 0 ? (int64_t)pick : (int64_t)__umul64hi(u, (unsigned long long)n);
 }
 
 // True in every thread of the CTA that counts itself last among gridDim.x
@@ -312,35 +276,25 @@ __device__ __forceinline__ bool kmpp_last_cta(unsigned int *__restrict__ done) {
     return last;
 }
 
-// Round r >= 1, one CTA per tile of kTile frames, one thread per frame (at
-// a time).  With r_center >= 0 the running minimum first takes the distance
-// to center r_center (rounds >= 2; round 1 uses the minimum of
+// minRMSD, round r >= 1, one CTA per tile of kTile frames, one thread per
+// frame (at a time).  With r_center >= 0 the running minimum first takes the
+// distance to center r_center (rounds >= 2; round 1 uses the minimum of
 // kmpp_first_kernel as it is).  Then the tile's weight sum is stored and the
-// CTA that finishes last draws.  THREADS = 1024 for the Euclidean metric
-// (two frames per thread: the pass is latency-bound at small n), 256 for
-// minRMSD (the QCP solve needs the registers).  The pruned rounds' first
-// round runs here too (r_center = -1), which stores every tile sum.
-template <int THREADS, bool RMSD, class Src>
-__global__ void __launch_bounds__(THREADS) kmpp_round_kernel(
-    const Src src, int64_t n, int d, float *__restrict__ C0, int64_t *__restrict__ idx_out,
+// CTA that finishes last draws.
+__global__ void __launch_bounds__(kTileThreads) kmpp_round_kernel(
+    const DenseRows src, int64_t n, int d, float *__restrict__ C0, int64_t *__restrict__ idx_out,
     float *__restrict__ mind, const int *__restrict__ qexp_p, unsigned long long *__restrict__ tile_sum,
     unsigned int *__restrict__ done, KmppMetric m, int r_center, int r, uint32_t seed) {
-    constexpr int kPer = kTile / THREADS;
-    __shared__ unsigned long long red[THREADS / 32];
+    __shared__ unsigned long long red[kTileThreads / 32];
     const int qexp = *qexp_p;
     const int64_t t0 = (int64_t)blockIdx.x * kTile;
     unsigned long long s = 0;
-    for (int u = 0; u < kPer; ++u) {
-        const int64_t i = t0 + u * THREADS + threadIdx.x;
+    for (int u = 0; u < kTile / kTileThreads; ++u) {
+        const int64_t i = t0 + u * kTileThreads + threadIdx.x;
         if (i < n) {
             float mi = mind[i];
             if (r_center >= 0) {
-                const float *c = C0 + (int64_t)r_center * d;
-                float dd;
-                if constexpr (RMSD)
-                    dd = kmpp_d2(src.X, i, d, c, m, r_center);
-                else
-                    dd = src_d2(src, i, c, d);
+                const float dd = kmpp_rmsd_d2(i, d, m, r_center);
                 if (dd < mi) {
                     mi = dd;
                     mind[i] = mi;
@@ -352,148 +306,416 @@ __global__ void __launch_bounds__(THREADS) kmpp_round_kernel(
     s = block_sum_u64(s, red);
     if (threadIdx.x == 0) tile_sum[blockIdx.x] = s;
     if (!kmpp_last_cta(done)) return;
-    kmpp_draw_round<THREADS>(gridDim.x, src, n, d, C0, idx_out, mind, qexp, tile_sum, done, r, seed);
-}
-
-// Pruned round, launch 2: four frames per thread (vector loads of mind and
-// a); the frames that the bound does not rule out are appended to the list,
-// one atomic per warp.  The skip needs a finite mind; a NaN bound never
-// skips.
-__global__ void __launch_bounds__(256) kmpp_prune_kernel(int64_t n, const float *__restrict__ mind,
-                                                         const int32_t *__restrict__ near,
-                                                         const float *__restrict__ cc, float prune_factor,
-                                                         int32_t *__restrict__ list, int32_t *__restrict__ list_n) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nq = (n + 3) / 4;
-    for (int64_t q0 = (int64_t)blockIdx.x * blockDim.x; q0 < nq; q0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t q = q0 + threadIdx.x;
-        float mi[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        int32_t a[4] = {0, 0, 0, 0};
-        const int64_t i0 = 4 * q;
-        if (i0 + 3 < n) {
-            const float4 m4 = __ldg(reinterpret_cast<const float4 *>(mind) + q);
-            const int4 a4 = __ldg(reinterpret_cast<const int4 *>(near) + q);
-            mi[0] = m4.x, mi[1] = m4.y, mi[2] = m4.z, mi[3] = m4.w;
-            a[0] = a4.x, a[1] = a4.y, a[2] = a4.z, a[3] = a4.w;
-        } else {
-            for (int v = 0; v < 4; ++v)
-                if (i0 + v < n) {
-                    mi[v] = mind[i0 + v];
-                    a[v] = near[i0 + v];
-                }
-        }
-        unsigned keep = 0u;
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-            if (i0 + v < n && !(mi[v] <= 3.4028234663852886e38f && __ldg(cc + a[v]) >= __fmul_ru(mi[v], prune_factor)))
-                keep |= 1u << v;
-        const int cnt = __popc(keep);
-        int excl = cnt;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, excl, off);
-            if (lane >= off) excl += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, excl, 31);
-        int base = 0;
-        if (lane == 31 && total > 0) base = atomicAdd(list_n, total);
-        base = __shfl_sync(0xffffffffu, base, 31) + excl - cnt;
-        for (int v = 0; v < 4; ++v)
-            if ((keep >> v) & 1u) list[base++] = (int32_t)(i0 + v);
+    const int64_t p = kmpp_draw_round<kTileThreads>(gridDim.x, 11, n, mind, qexp, tile_sum, r, seed);
+    for (int f = threadIdx.x; f < d; f += kTileThreads) C0[(int64_t)r * d + f] = src.get(p, f);
+    if (threadIdx.x == 0) {
+        if (idx_out) idx_out[r] = p;
+        *done = 0u;  // for the next round's launch
     }
 }
+static_assert(kTile == 1 << 11, "the draw's tiles");
 
-// Pruned round, launch 3: the listed frames' exact distances, 32 frames per
-// warp at a time (grid-stride over the groups of 32 list entries; rows of
-// fewer than 32 features take one frame per thread instead).  For
-// each run of 32 features, lane f holds feature f0 + f of one listed frame
-// at a time (stored rows: one coalesced 128-byte load per frame, where a
-// thread per frame makes every load touch 32 rows), squares its difference
-// to the center and stores it transposed in shared memory; lane j then adds
-// frame j's 32 squares in feature order.  So each distance is the same
-// sequence of float32 operations as sqdist_exact (every subtraction, square
-// and addition rounded once, features in order), bit for bit.  A smaller
-// distance replaces mind and a and moves the frame's integer weight in its
-// tile's sum (modular 64-bit deltas, exact).  The CTA that finishes last
-// clears the list and draws.
-constexpr int kEvalWarps = 8;
-
-template <class Src>
-__global__ void __launch_bounds__(kEvalWarps * 32) kmpp_eval_kernel(
-    const Src src, int64_t n, int d, float *__restrict__ C0, int64_t *__restrict__ idx_out,
-    float *__restrict__ mind, int32_t *__restrict__ near, const int *__restrict__ qexp_p,
-    unsigned long long *__restrict__ tile_sum, unsigned int *__restrict__ done, const int32_t *__restrict__ list,
-    int32_t *__restrict__ list_n, int64_t ntiles, int r_center, int r, uint32_t seed) {
-    __shared__ float sq_s[kEvalWarps][32][33];  // [feature][frame], padded: conflict-free both ways
-    __shared__ int32_t frame_s[kEvalWarps][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float(*sq)[33] = sq_s[warp];
-    int32_t *frames = frame_s[warp];
-    const int qexp = *qexp_p;
-    const int64_t cnt = *list_n;
-    const float *c = C0 + (int64_t)r_center * d;
-    // A smaller distance dd of frame i replaces mind and a, and moves the
-    // frame's integer weight in its tile's sum.
-    auto lower = [&](int64_t i, float dd) {
-        const float mi = mind[i];
-        if (dd < mi) {
-            mind[i] = dd;
-            near[i] = r_center;
-            const unsigned long long delta = quant_weight(dd, qexp) - quant_weight(mi, qexp);
-            if (delta) atomicAdd(&tile_sum[i / kTile], delta);
-        }
-    };
-    if (d < 32) {
-        // Rows shorter than a warp: one frame per thread.
-        for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt;
-             e += (int64_t)gridDim.x * blockDim.x) {
-            const int64_t i = list[e];
-            lower(i, src_d2(src, i, c, d));
-        }
-    } else {
-        const int64_t groups = (cnt + 31) / 32;
-        for (int64_t g = (int64_t)blockIdx.x * kEvalWarps + warp; g < groups;
-             g += (int64_t)gridDim.x * kEvalWarps) {
-            const int m = (int)(cnt - g * 32 < 32 ? cnt - g * 32 : 32);  // frames in this group
-            const int32_t mine = lane < m ? list[g * 32 + lane] : 0;
-            frames[lane] = mine;
-            __syncwarp();
-            float acc = 0.0f;
-            for (int f0 = 0; f0 < d; f0 += 32) {
-                const int f = f0 + lane;
-                const bool in = f < d;
-                const float cf = in ? __ldg(c + f) : 0.0f;
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = (j < m && in) ? src.get(frames[j], f) : 0.0f;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) sq[lane][j] = sq_term(v[j], cf);
-                __syncwarp();
-                if (f0 + 32 <= d) {
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) acc = __fadd_rn(acc, sq[q][lane]);
-                } else {
-                    for (int q = 0; q < d - f0; ++q) acc = __fadd_rn(acc, sq[q][lane]);
-                }
-                __syncwarp();  // sq is overwritten by the next run of features
-            }
-            if (lane < m) lower(mine, acc);
-            __syncwarp();  // frames is overwritten by the next group
-        }
-    }
-    if (!kmpp_last_cta(done)) return;
-    if (threadIdx.x == 0) *list_n = 0;  // for the next round
-    kmpp_draw_round<kEvalWarps * 32>(ntiles, src, n, d, C0, idx_out, mind, qexp, tile_sum, done, r, seed);
-}
-
-// Round 0: a uniformly drawn frame, copied into C0[0].
-template <class Src>
-__global__ void __launch_bounds__(kTileThreads) kmpp_uniform_kernel(const Src src, int64_t n, int d,
+// Round 0 under the minRMSD metric: a uniformly drawn frame, copied into C0[0].
+__global__ void __launch_bounds__(kTileThreads) kmpp_uniform_kernel(const DenseRows src, int64_t n, int d,
                                                                     float *__restrict__ C0,
                                                                     int64_t *__restrict__ idx_out, uint32_t seed) {
     const int64_t p = (int64_t)__umul64hi(kmpp_draw(seed, 0u), (unsigned long long)n);
     for (int f = threadIdx.x; f < d; f += blockDim.x) C0[f] = src.get(p, f);
     if (idx_out && threadIdx.x == 0) idx_out[0] = p;
+}
+
+// ---- Euclidean rounds ----------------------------------------------------------
+
+// A warp's scratch for the distances of wide rows.  With more (5 KB squares,
+// lists of 160 frames and their minima) the shared memory of 32 warps left the
+// L1 cache so little that rows in flight were evicted: 500,000 x 528, every
+// row, 290 us instead of 194.
+struct WarpScratch {
+    float sq[128 * 9];  // [feature][frame], row stride frames + 1 (odd: no bank conflicts either way)
+    int32_t id[96];     // the frames that the bound left, compacted
+};
+
+// Exact distances of the m <= J rows ids[0..m) to c, row j's in lane j.  Each
+// run of 32 * (32 / J) features of J rows is loaded at once (32 coalesced
+// loads in flight, beside the sums of the run before), squared and stored transposed; lane j then adds row j's
+// squares in feature order, so each distance is the same sequence of float32
+// operations as sqdist_exact, bit for bit.
+template <int J, class Src>
+__device__ __forceinline__ float warp_rows_sqdist(const Src &src, const int32_t *ids, int m, const float *c, int d,
+                                                  float *sq) {
+    constexpr int kRuns = 32 / J;
+    const int lane = threadIdx.x & 31, j0 = lane & (J - 1);
+    float v[32];
+    auto load = [&](int f0) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int q = 0; q < kRuns; ++q) {
+                const int f = f0 + q * 32 + lane;
+                v[j * kRuns + q] = (j < m && f < d) ? src.get(ids[j], f) : 0.0f;
+            }
+    };
+    load(0);
+    float acc = 0.0f;
+    for (int f0 = 0; f0 < d; f0 += 32 * kRuns) {
+#pragma unroll
+        for (int q = 0; q < kRuns; ++q) {
+            const int f = f0 + q * 32 + lane;
+            const float cf = f < d ? c[f] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < J; ++j) sq[(q * 32 + lane) * (J + 1) + j] = sq_term(v[j * kRuns + q], cf);
+        }
+        __syncwarp();
+        if (f0 + 32 * kRuns < d) load(f0 + 32 * kRuns);  // on its way during the sums
+        const int run = min(32 * kRuns, d - f0);
+        if (run == 32 * kRuns) {
+#pragma unroll 8
+            for (int f = 0; f < 32 * kRuns; ++f) acc = __fadd_rn(acc, sq[f * (J + 1) + j0]);
+        } else {
+#pragma unroll 8
+            for (int f = 0; f < run; ++f) acc = __fadd_rn(acc, sq[f * (J + 1) + j0]);
+        }
+        __syncwarp();  // sq is overwritten by the next run of features
+    }
+    return acc;
+}
+
+template <class Src>
+__device__ __forceinline__ float warp_rows_sqdist(const Src &src, const int32_t *ids, int m, const float *c, int d,
+                                                  float *sq) {
+    if (m > 16) return warp_rows_sqdist<32>(src, ids, m, c, d, sq);
+    if (m > 8) return warp_rows_sqdist<16>(src, ids, m, c, d, sq);
+    return warp_rows_sqdist<8>(src, ids, m, c, d, sq);
+}
+
+// Row i, zero beyond its d <= DP features.
+template <int DP, class Src>
+__device__ __forceinline__ void load_row(const Src &src, int64_t i, int d, float (&v)[DP]) {
+    if constexpr (std::is_same<Src, DenseRows>::value && DP >= 4) {
+        if ((d & 3) == 0 && (reinterpret_cast<uintptr_t>(src.X) & 15) == 0) {
+            const float4 *x = reinterpret_cast<const float4 *>(src.X + i * d);
+#pragma unroll
+            for (int f = 0; f < DP; f += 4) {
+                const float4 t = f < d ? __ldg(x + (f >> 2)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                v[f] = t.x, v[f + 1] = t.y, v[f + 2] = t.z, v[f + 3] = t.w;
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < DP; ++f) v[f] = f < d ? src.get(i, f) : 0.0f;
+}
+
+// The operations of sqdist_exact on a loaded row; c is zero beyond d, where
+// the added squares are zero.
+template <int DP>
+__device__ __forceinline__ float row_sqdist(const float (&v)[DP], const float *c) {
+    float acc = 0.0f;
+#pragma unroll
+    for (int f = 0; f < DP; ++f) acc = __fadd_rn(acc, sq_term(v[f], c[f]));
+    return acc;
+}
+
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+struct RoundParams {
+    int64_t n, ntiles;
+    int d, shift;
+    int r0, r1;  // the rounds of this launch
+    float *C0;
+    int64_t *idx;
+    KmppWs w;
+    float prune;  // prune_factor(d)
+    uint32_t seed;
+    int cc_s;  // bounds that fit in shared memory
+};
+
+// Rounds r0..r1-1: round r lowers the minima by center r - 1 and draws center
+// r (round 0 draws uniformly).  DP = 0: wide rows, whose distances a warp forms
+// together; else rows of d <= DP features, a thread per frame.  PRUNE: see the
+// head of this file; without it every round rewrites the minima into the
+// buffer of the other parity and the tile sums from zero, so a CTA that is
+// still drawing round r is not disturbed by one that works on round r + 1,
+// and one barrier per round is enough.
+//
+// A warp's frames lie in runs of 8 (wide) or 32 spread evenly over the
+// frames: the frames of a trajectory near the newest center are neighbours,
+// and their rows are the work of a round.
+//
+// What bounds it: early rounds read nearly every row (HBM), later rounds are
+// a chain of barrier, scans and row latency (about 6 us unpruned, 9 us
+// pruned).  us per round, launches per round -> here: 100,000 x 2 10 -> 7;
+// 500,000 x 10 15 -> 11; 100,000 x 67 21 -> 14; 20,000 x 528 33 -> 17;
+// 500,000 x 528, k = 300 56 -> 44, its first 50 rounds 120 -> 120.
+template <class Src, int DP, bool PRUNE>
+__global__ void __launch_bounds__(kRoundThreads, 1) kmpp_rounds_kernel(const Src src, const RoundParams p) {
+    extern __shared__ float4 kmpp_sm[];
+    constexpr bool WIDE = DP == 0;
+    constexpr int kRun = WIDE ? 8 : 32;                        // consecutive frames of a warp
+    constexpr int kSlots = WIDE ? 2 : 4;                        // loads of 32 minima in flight,
+    constexpr int kAll = WIDE || DP > 8 ? 1 : DP == 8 ? 2 : 4;  // and of 32 narrow rows
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    WarpScratch *scr = reinterpret_cast<WarpScratch *>(kmpp_sm) + warp;
+    float *c_s = reinterpret_cast<float *>(reinterpret_cast<WarpScratch *>(kmpp_sm) + (WIDE ? kRoundThreads / 32 : 0));
+    const int64_t n = p.n;
+    const int d = p.d;
+    const int64_t W = (int64_t)gridDim.x * (kRoundThreads / 32);
+    const int64_t gw = (int64_t)warp * gridDim.x + blockIdx.x;  // neighbours in different CTAs
+    const int64_t runs = (n + kRun - 1) / kRun;
+    float *cc_s = c_s + (WIDE ? d : DP);
+    unsigned int bars = 0;
+    bool ok = *p.w.err == 0u;
+    int qexp = INT_MIN;
+    // frame of this lane in slot s (32 frames from 32 / kRun runs); >= n: none
+    auto frame = [&](int64_t g0, int s) -> int64_t {
+        const int64_t run = g0 + (int64_t)(s * (32 / kRun) + lane / kRun) * W;
+        return run < runs ? run * kRun + lane % kRun : n;
+    };
+    auto barrier = [&]() { return grid_barrier(p.w.done, ++bars * gridDim.x, p.w.err); };
+    if (!WIDE && threadIdx.x < DP) c_s[threadIdx.x] = 0.0f;  // stays zero beyond d
+    __syncthreads();
+    int r = p.r0;
+    if (r > 0 && ok) {
+        const float *row = p.C0 + (int64_t)(r - 1) * d;
+        for (int f = threadIdx.x; f < d; f += kRoundThreads) c_s[f] = __ldcg(row + f);
+        __syncthreads();
+        if (r > 1) qexp = weight_exponent(__ldcg(p.w.maxbits), n);
+    }
+    for (; ok && r < p.r1; ++r) {
+        int64_t pick;
+        if (r == 0) {
+            pick = (int64_t)__umul64hi(kmpp_draw(p.seed, 0u), (unsigned long long)n);
+        } else {
+            const float *m_in = PRUNE || ((r - 1) & 1) == 0 ? p.w.mind : reinterpret_cast<float *>(p.w.near);
+            float *m_out = PRUNE || (r & 1) == 0 ? p.w.mind : reinterpret_cast<float *>(p.w.near);
+            unsigned long long *tiles = p.w.tile_sum + (PRUNE ? 0 : (r % 3) * p.ntiles);
+            if constexpr (PRUNE) {
+                if (r > 1) {  // cc
+                    for (int64_t j = gw; j < r - 1; j += W) {
+                        const float *b = p.C0 + j * d;
+                        float acc = 0.0f;
+                        for (int f = lane; f < d; f += 32) {
+                            const float t = __fsub_rn(c_s[f], __ldcg(b + f));
+                            acc = __fmaf_rn(t, t, acc);
+                        }
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1)
+                            acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+                        if (lane == 0) p.w.cc[j] = acc;
+                    }
+                    ok = barrier();
+                    if (!ok) break;
+                    // Read past L1 by every frame they would queue up at the
+                    // few L2 lines that hold them (2M x 32, k = 300: 61 us a
+                    // round, 46 from shared memory).
+                    for (int j = threadIdx.x; j < min(r - 1, p.cc_s); j += kRoundThreads) cc_s[j] = __ldcg(p.w.cc + j);
+                    __syncthreads();
+                }
+            }
+            // Every frame's distance, 32 frames at a time (round 1, and every unpruned round).
+            if (!PRUNE || r == 1) {
+                float mx = 0.0f;
+                for (int64_t g0 = gw; g0 < runs; g0 += W * (32 / kRun) * kAll) {
+                    float dd[kAll], mi[kAll];
+                    int64_t i[kAll];
+#pragma unroll
+                    for (int s = 0; s < kAll; ++s) {
+                        i[s] = frame(g0, s);
+                        mi[s] = r > 1 && i[s] < n ? __ldcg(m_in + i[s]) : 0.0f;
+                    }
+                    if constexpr (WIDE) {
+                        scr->id[lane] = i[0] < n ? (int32_t)i[0] : 0;
+                        const int m = __popc(__ballot_sync(0xffffffffu, i[0] < n));  // the first m lanes
+                        __syncwarp();
+                        dd[0] = warp_rows_sqdist(src, scr->id, m, c_s, d, scr->sq);
+                    } else {
+                        float v[kAll][DP];
+#pragma unroll
+                        for (int s = 0; s < kAll; ++s)
+                            if (i[s] < n) load_row<DP>(src, i[s], d, v[s]);
+#pragma unroll
+                        for (int s = 0; s < kAll; ++s) dd[s] = i[s] < n ? row_sqdist<DP>(v[s], c_s) : 0.0f;
+                    }
+#pragma unroll
+                    for (int s = 0; s < kAll; ++s) {
+                        unsigned long long w = 0ull;
+                        if (i[s] < n) {
+                            if (r == 1) {
+                                if (dd[s] < __int_as_float(0x7f800000) && dd[s] > mx) mx = dd[s];
+                                if constexpr (PRUNE) p.w.near[i[s]] = 0;
+                            } else {
+                                dd[s] = dd[s] < mi[s] ? dd[s] : mi[s];
+                                w = quant_weight(dd[s], qexp);
+                            }
+                            m_out[i[s]] = dd[s];
+                        }
+                        if (r > 1) {  // a run lies in one tile
+#pragma unroll
+                            for (int off = kRun / 2; off > 0; off >>= 1) w += __shfl_xor_sync(0xffffffffu, w, off);
+                            if (lane % kRun == 0 && w) atomicAdd(tiles + (i[s] >> p.shift), w);
+                        }
+                    }
+                }
+                if (r == 1) {
+                    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+                    if (lane == 0 && mx > 0.0f) atomicMax(p.w.maxbits, __float_as_uint(mx));
+                    ok = barrier();
+                    if (!ok) break;
+                    qexp = weight_exponent(__ldcg(p.w.maxbits), n);
+                    for (int64_t g0 = gw; g0 < runs; g0 += W * (32 / kRun)) {
+                        const int64_t i = frame(g0, 0);
+                        unsigned long long w = i < n ? quant_weight(__ldcg(m_out + i), qexp) : 0ull;
+#pragma unroll
+                        for (int off = kRun / 2; off > 0; off >>= 1) w += __shfl_xor_sync(0xffffffffu, w, off);
+                        if (lane % kRun == 0 && w) atomicAdd(tiles + (i >> p.shift), w);
+                    }
+                }
+            } else {
+                const int rc = r - 1;
+                // A smaller distance dd of frame i replaces its minimum mi and
+                // a, and moves its integer weight in its tile's sum (modular
+                // 64-bit deltas, exact).
+                auto lower = [&](bool in, int64_t i, float mi, float dd) {
+                    const bool less = in && dd < mi;
+                    unsigned long long delta = 0ull;
+                    if (less) {
+                        p.w.mind[i] = dd;
+                        p.w.near[i] = rc;
+                        delta = quant_weight(dd, qexp) - quant_weight(mi, qexp);
+                    }
+                    const unsigned any = __ballot_sync(0xffffffffu, delta != 0ull);
+                    if (!any) return;
+                    const int t = (int)(i >> p.shift), first = __shfl_sync(0xffffffffu, t, __ffs(any) - 1);
+                    if (__all_sync(0xffffffffu, delta == 0ull || t == first)) {
+                        delta = warp_sum_u64(delta);
+                        if (lane == 0 && delta) atomicAdd(tiles + first, delta);
+                    } else if (delta) {
+                        atomicAdd(tiles + t, delta);
+                    }
+                };
+                int cnt = 0;  // wide: listed frames
+                for (int64_t g0 = gw; g0 < runs; g0 += W * (32 / kRun) * kSlots) {
+                    float mi[kSlots];
+                    int32_t a[kSlots];
+#pragma unroll
+                    for (int s = 0; s < kSlots; ++s) {
+                        const int64_t i = frame(g0, s);
+                        mi[s] = i < n ? __ldcg(p.w.mind + i) : 0.0f;
+                        a[s] = i < n ? __ldcg(p.w.near + i) : 0;
+                    }
+                    bool keep[kSlots];
+#pragma unroll
+                    for (int s = 0; s < kSlots; ++s) {  // the skip needs a finite minimum; a NaN bound never skips
+                        const float cc = a[s] < p.cc_s ? cc_s[a[s]] : __ldcg(p.w.cc + a[s]);
+                        keep[s] = frame(g0, s) < n &&
+                                  !(mi[s] <= 3.4028234663852886e38f && cc >= __fmul_ru(mi[s], p.prune));
+                    }
+                    if constexpr (WIDE) {
+                        // Full groups of 32 rows; the rest waits for the next
+                        // frames' or the end.
+#pragma unroll
+                        for (int s = 0; s < kSlots; ++s) {
+                            const unsigned b = __ballot_sync(0xffffffffu, keep[s]);
+                            if (keep[s]) {
+                                const int q = cnt + __popc(b & ((1u << lane) - 1u));
+                                scr->id[q] = (int32_t)frame(g0, s);
+                            }
+                            cnt += __popc(b);
+                        }
+                        __syncwarp();
+                        const bool last = g0 + W * (32 / kRun) * kSlots >= runs;
+                        int b0 = 0;
+                        for (; cnt - b0 >= 32 || (last && b0 < cnt); b0 += 32) {
+                            const int m = min(32, cnt - b0);
+                            const int32_t id = lane < m ? scr->id[b0 + lane] : 0;
+                            const float old = __ldcg(p.w.mind + id);
+                            lower(lane < m, id, old, warp_rows_sqdist(src, scr->id + b0, m, c_s, d, scr->sq));
+                        }
+                        cnt -= min(b0, cnt);
+                        const int32_t id = lane < cnt ? scr->id[b0 + lane] : 0;
+                        __syncwarp();
+                        scr->id[lane] = id;
+                        __syncwarp();
+                    } else {
+#pragma unroll
+                        for (int s0 = 0; s0 < kSlots; s0 += kAll) {
+                            float v[kAll][DP];
+#pragma unroll
+                            for (int s = 0; s < kAll; ++s)
+                                if (keep[s0 + s]) load_row<DP>(src, frame(g0, s0 + s), d, v[s]);
+#pragma unroll
+                            for (int s = 0; s < kAll; ++s) {
+                                const bool in = keep[s0 + s];
+                                if (!__any_sync(0xffffffffu, in)) continue;
+                                lower(in, frame(g0, s0 + s), mi[s0 + s], in ? row_sqdist<DP>(v[s], c_s) : 0.0f);
+                            }
+                        }
+                    }
+                }
+            }
+            if (!PRUNE && blockIdx.x == 0) {  // the next round's tile sums
+                unsigned long long *z = p.w.tile_sum + ((r + 1) % 3) * p.ntiles;
+                for (int64_t t = threadIdx.x; t < p.ntiles; t += kRoundThreads) z[t] = 0ull;
+            }
+            ok = barrier();
+            if (!ok) break;
+            pick = kmpp_draw_round<kRoundThreads>(p.ntiles, p.shift, n, m_out, qexp, tiles, r, p.seed);
+        }
+        // Center r: in every CTA's shared memory, and in C0.
+        for (int f = threadIdx.x; f < d; f += kRoundThreads) {
+            const float x = src.get(pick, f);
+            c_s[f] = x;
+            if (blockIdx.x == 0) p.C0[(int64_t)r * d + f] = x;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0 && p.idx) p.idx[r] = pick;
+        __syncthreads();
+    }
+    if (!ok && blockIdx.x == 0) {  // a wait ran out: no centers from here on
+        for (; r < p.r1; ++r) {
+            for (int f = threadIdx.x; f < d; f += kRoundThreads) p.C0[(int64_t)r * d + f] = __int_as_float(0x7fc00000);
+            if (threadIdx.x == 0 && p.idx) p.idx[r] = -1;
+        }
+    }
+}
+
+template <class Src, int DP, bool PRUNE>
+int launch_rounds_dp(const Src &src, RoundParams &p, int k, cudaStream_t s) {
+    constexpr size_t kMax = 226 * 1024;
+    const size_t fixed = (DP == 0 ? sizeof(WarpScratch) * (kRoundThreads / 32) : 0) +
+                         sizeof(float) * (DP == 0 ? p.d : DP);
+    p.cc_s = PRUNE ? (int)std::min<size_t>(k, (kMax - fixed) / sizeof(float)) : 0;
+    const size_t smem = fixed + sizeof(float) * p.cc_s;
+    static bool set[kDeviceSlots] = {};
+    const int dev = current_device();
+    if (!(dev >= 0 && dev < kDeviceSlots && set[dev])) {
+        KM_CUDA(cudaFuncSetAttribute(kmpp_rounds_kernel<Src, DP, PRUNE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kMax));
+        if (dev >= 0 && dev < kDeviceSlots) set[dev] = true;
+    }
+    KM_CUDA(cudaMemsetAsync(p.w.done, 0, sizeof(unsigned int), s));
+    // one CTA per SM, all resident at once (they wait for each other)
+    constexpr int kRun = DP == 0 ? 8 : 32;
+    const unsigned grid = (unsigned)std::min<int64_t>(num_sms(), (p.n + kRun - 1) / kRun);
+    void *args[] = {(void *)&src, (void *)&p};
+    KM_CUDA(cudaLaunchCooperativeKernel((const void *)kmpp_rounds_kernel<Src, DP, PRUNE>, dim3(grid),
+                                        dim3(kRoundThreads), args, smem, s));
+    return KM_OK;
+}
+
+template <class Src, bool PRUNE>
+int launch_rounds(const Src &src, RoundParams &p, int k, cudaStream_t s) {
+    if (p.d >= kWide) return launch_rounds_dp<Src, 0, PRUNE>(src, p, k, s);
+    if constexpr (std::is_same<Src, DenseRows>::value) {
+        if (p.d <= 2) return launch_rounds_dp<Src, 2, PRUNE>(src, p, k, s);
+        if (p.d <= 4) return launch_rounds_dp<Src, 4, PRUNE>(src, p, k, s);
+        if (p.d <= 8) return launch_rounds_dp<Src, 8, PRUNE>(src, p, k, s);
+        if (p.d <= 16) return launch_rounds_dp<Src, 16, PRUNE>(src, p, k, s);
+    }
+    return launch_rounds_dp<Src, 32, PRUNE>(src, p, k, s);
 }
 
 }  // namespace
@@ -529,47 +751,57 @@ namespace {
 
 template <class Src>
 int run_kmpp_src(const Src &src, int64_t n, int d, int k, uint32_t seed, float *C0, int64_t *idx,
-                 void (*cb)(void *), void *cb_user, void *ws, cudaStream_t s, const KmppMetric &m) {
+                 void (*cb)(void *), void *cb_user, void *ws, cudaStream_t s) {
+    RoundParams p;
+    p.w = carve(ws, n, k, nullptr);
+    p.n = n;
+    p.ntiles = tile_slots(n);
+    p.d = d;
+    p.shift = tile_shift(n);
+    p.C0 = C0;
+    p.idx = idx;
+    p.prune = prune_factor(d);
+    p.seed = seed;
+    KM_CUDA(cudaMemsetAsync(p.w.tile_sum, 0, 3 * p.ntiles * sizeof(unsigned long long), s));
+    KM_CUDA(cudaMemsetAsync(p.w.maxbits, 0, sizeof(uint32_t), s));
+    KM_CUDA(cudaMemsetAsync(p.w.err, 0, sizeof(uint32_t), s));
+    // A pruned round pays a second barrier and the bounds, and saves rows of
+    // d words less two.  us per round (unpruned, pruned), k = 300:
+    //   d = 2:    n = 500,000 8.6, 10.5;  2M 16.2, 15.1;  10M 67, 39
+    //   d = 10:   n = 100,000 6.6, 9.1;   500,000 11.4, 11.1;  2M 25, 17
+    //   d = 67:   n = 20,000 9.0, 11.2;   100,000 15.0, 14.2;  500,000 46, 25
+    //   d = 528:  n = 1,000 12, 15;       20,000 19, 17.5;     100,000 53, 21
+    // KM_KMPP_PRUNE=0 or 1 in the environment forces the choice (both give
+    // the same draws).
+    bool prune = n * (int64_t)(d + 4) >= (int64_t(1) << 23);
+    if (const char *e = std::getenv("KM_KMPP_PRUNE")) prune = e[0] == '1';
+    const int batch = cb ? 1 : kRoundBatch;
+    for (int r = 0; r < k; r += batch) {
+        p.r0 = r;
+        p.r1 = std::min(k, r + batch);
+        KM_TRY(prune ? (launch_rounds<Src, true>(src, p, k, s)) : (launch_rounds<Src, false>(src, p, k, s)));
+        if (cb) cb(cb_user);
+    }
+    return KM_OK;
+}
+
+int run_kmpp_rmsd(const DenseRows &src, int64_t n, int d, int k, uint32_t seed, float *C0, int64_t *idx,
+                  void (*cb)(void *), void *cb_user, void *ws, cudaStream_t s, const KmppMetric &m) {
     KmppWs w = carve(ws, n, k, nullptr);
-    const int64_t ntiles = (n + kTile - 1) / kTile;
+    const unsigned ntiles = (unsigned)((n + kTile - 1) / kTile);
     kmpp_uniform_kernel<<<1, kTileThreads, 0, s>>>(src, n, d, C0, idx, seed);
     KM_CUDA(cudaGetLastError());
     if (cb) cb(cb_user);
     if (k == 1) return KM_OK;
     KM_CUDA(cudaMemsetAsync(w.maxbits, 0, sizeof(uint32_t), s));
     KM_CUDA(cudaMemsetAsync(w.done, 0, sizeof(unsigned int), s));
-    kmpp_first_kernel<<<(unsigned)ntiles, kTileThreads, 0, s>>>(src, n, d, C0, w.mind, w.near, w.maxbits, m);
+    kmpp_first_kernel<<<ntiles, kTileThreads, 0, s>>>(n, d, w.mind, w.maxbits, m);
     KM_CUDA(cudaGetLastError());
     kmpp_scale_kernel<<<1, 1, 0, s>>>(w.maxbits, n, w.qexp);
     KM_CUDA(cudaGetLastError());
-    const float pf = prune_factor(d);
-    // Pruned rounds pay three launches per round; below this size the
-    // unpruned pass is about as short as a launch.  KM_KMPP_PRUNE=0 or 1 in
-    // the environment forces the choice (both give the same draws).
-    bool prune = !m.Xc && n * (int64_t)d >= (int64_t(1) << 22);
-    if (const char *e = std::getenv("KM_KMPP_PRUNE")) prune = !m.Xc && e[0] == '1';
-    if (prune) KM_CUDA(cudaMemsetAsync(w.list_n, 0, sizeof(int32_t), s));
-    const int64_t nq = (n + 3) / 4;
-    const unsigned prune_grid = (unsigned)std::min<int64_t>((nq + 255) / 256, (int64_t)num_sms() * 8);
-    const unsigned eval_grid = (unsigned)num_sms() * 4;
     for (int r = 1; r < k; ++r) {
-        const int rc = r >= 2 ? r - 1 : -1;
-        if (m.Xc) {
-            if constexpr (std::is_same<Src, DenseRows>::value)
-                kmpp_round_kernel<256, true><<<(unsigned)ntiles, 256, 0, s>>>(src, n, d, C0, idx, w.mind, w.qexp,
-                                                                              w.tile_sum, w.done, m, rc, r, seed);
-        } else if (!prune || rc < 0) {
-            kmpp_round_kernel<1024, false><<<(unsigned)ntiles, 1024, 0, s>>>(src, n, d, C0, idx, w.mind, w.qexp,
-                                                                             w.tile_sum, w.done, m, rc, r, seed);
-        } else {
-            kmpp_cc_kernel<<<(unsigned)((rc + 7) / 8), 256, 0, s>>>(C0, d, rc, w.cc);
-            KM_CUDA(cudaGetLastError());
-            kmpp_prune_kernel<<<prune_grid, 256, 0, s>>>(n, w.mind, w.near, w.cc, pf, w.list, w.list_n);
-            KM_CUDA(cudaGetLastError());
-            kmpp_eval_kernel<<<eval_grid, kEvalWarps * 32, 0, s>>>(src, n, d, C0, idx, w.mind, w.near, w.qexp,
-                                                                   w.tile_sum, w.done, w.list, w.list_n, ntiles, rc, r,
-                                                                   seed);
-        }
+        kmpp_round_kernel<<<ntiles, kTileThreads, 0, s>>>(src, n, d, C0, idx, w.mind, w.qexp, w.tile_sum, w.done, m,
+                                                          r >= 2 ? r - 1 : -1, r, seed);
         KM_CUDA(cudaGetLastError());
         if (cb) cb(cb_user);
     }
@@ -592,9 +824,10 @@ int run_kmpp(const float *X, int64_t n, int d, int k, uint32_t seed, float *C0, 
             return KM_ERR_UNSUPPORTED;
         }
         const PairRows pr{ps->xyz, reinterpret_cast<const int2 *>(ps->pairs), ps->n_atoms, d};
-        return run_kmpp_src(pr, n, d, k, seed, C0, idx, cb, cb_user, ws, s, m);
+        return run_kmpp_src(pr, n, d, k, seed, C0, idx, cb, cb_user, ws, s);
     }
-    return run_kmpp_src(DenseRows{X, d}, n, d, k, seed, C0, idx, cb, cb_user, ws, s, m);
+    if (m.Xc) return run_kmpp_rmsd(DenseRows{X, d}, n, d, k, seed, C0, idx, cb, cb_user, ws, s, m);
+    return run_kmpp_src(DenseRows{X, d}, n, d, k, seed, C0, idx, cb, cb_user, ws, s);
 }
 
 }  // namespace km

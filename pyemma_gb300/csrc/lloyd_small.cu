@@ -66,37 +66,6 @@ size_t fu_smem(int d, int k) {
 // Doubles of one buffer of global sums: S (k x d), Q (k), and the counts.
 __host__ __device__ inline size_t fu_buf_doubles(int d, int k) { return (size_t)k * d + k + (k + 1) / 2; }
 
-// One count per CTA and iteration; false when the others did not arrive in
-// time or another CTA gave up.
-__device__ __forceinline__ bool fu_barrier(unsigned int *count, unsigned int target, uint32_t *err) {
-    __shared__ bool ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-        bool ok = true;
-        const uint64_t t0 = globaltimer_ns();
-        for (uint32_t spin = 1;; ++spin) {
-            unsigned int c;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-            if (c >= target) break;
-            if ((spin & 255u) == 0) {
-                uint32_t e;
-                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
-                if (e != 0u || globaltimer_ns() - t0 > kWaitLimitNs) {
-                    ok = false;
-                    break;
-                }
-            }
-        }
-        if (!ok) atomicOr(err, (uint32_t)kDevTimeoutEpi);
-        __threadfence();
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s;
-}
-
 // Sum over the CTA in a fixed order (warp shuffles, then warp 0), in every thread.
 __device__ __forceinline__ double fu_block_sum(double v, double *red) {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -282,7 +251,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) small_lloyd_kernel(
             double *z = bufs + (size_t)((it + 1) % 3) * bd;
             for (size_t e = tid; e < bd; e += kFuThreads) z[e] = 0.0;
         }
-        ok = fu_barrier(bar, (unsigned int)(it + 1) * gridDim.x, &st->err);
+        ok = grid_barrier(bar, (unsigned int)(it + 1) * gridDim.x, &st->err);
         if (!ok) break;
         // New centers, a thread per center:
         //   mu_j = c_j + S_j / n_j, inertia_j = Q_j - 2 delta_j.S_j + n_j ||delta_j||^2
