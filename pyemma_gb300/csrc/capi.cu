@@ -117,11 +117,11 @@ int resolve_precision(int precision, int d, int k, bool check_device) {
         auto it = g_tune.choice.find(std::make_pair(d, k));
         if (it != g_tune.choice.end()) return it->second;
     }
-    const bool tc_ok = check_device ? tc_supported(d, k) : tc_plan_exists(d, k);
     // Measured on GB300 (1-4.3M frames): FP16 + re-check wins from d = 64 at
     // every k, and from d = 8 once k >= 1000 (d = 10, k = 1000: 2.5 against
     // 7.2 ms per Lloyd iteration; d = 16, k = 1000: 1.4 against 2.7 ms).
-    if (tc_ok && (d >= 64 || (d >= 8 && k >= 1000))) return KM_PREC_FP16;
+    if (d >= 64 || (d >= 8 && k >= 1000))
+        if (check_device ? tc_supported(d, k) : tc_plan_exists(d, k)) return KM_PREC_FP16;
     return KM_PREC_FP32;
 }
 
@@ -145,14 +145,19 @@ int resolve_precision(int precision, int d, int k, bool check_device) {
 //     k = 1000 506 -> 1024).
 constexpr double kSmallMinWork = 3.5e8;
 bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_device) {
-    if (!small_shape_ok(d, k) || (d > 15 && k > 2048) || !small_allowed() || (check_device && !tc_supported(d, k)) || tc_plan_set(d, k)) return false;
-    if (prec == KM_PREC_FP16) return true;
-    if (precision != KM_PREC_AUTO || prec != KM_PREC_FP32) return false;
-    {
-        std::lock_guard<std::mutex> lk(g_tune.m);
-        if (g_tune.choice.count(std::make_pair(d, k))) return false;
+    // The cheap tests first: small calls are host-bound, and the plan lookups
+    // took 2 of their 37 us.
+    if (!small_shape_ok(d, k) || (d > 15 && k > 2048)) return false;
+    const bool fp16 = prec == KM_PREC_FP16;
+    if (!fp16) {
+        if (precision != KM_PREC_AUTO || prec != KM_PREC_FP32) return false;
+        const bool enough = d >= 2 && (n < 0 || (double)n * k * (3 * d + 2) >= kSmallMinWork);
+        if (!enough && !small_forced()) return false;
     }
-    return small_forced() || (d >= 2 && (n < 0 || (double)n * k * (3 * d + 2) >= kSmallMinWork));
+    if (!small_allowed() || (check_device && !tc_supported(d, k)) || tc_plan_set(d, k)) return false;
+    if (fp16) return true;
+    std::lock_guard<std::mutex> lk(g_tune.m);
+    return g_tune.choice.count(std::make_pair(d, k)) == 0;
 }
 
 // The workspace of an assignment; small: the narrow-frame kernel may run
