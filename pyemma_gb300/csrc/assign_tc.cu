@@ -119,6 +119,16 @@ struct TcParams {
     const void *seed_xh;
     const void *seed_ch;
     float seed_coef;
+    // Center bounds (all nullable).  perm: operand row -> center, inv its
+    // inverse; unit_mask: the center tiles that can hold the argmin of a
+    // frame unit; ub: an upper bound of each frame's distance to its center,
+    // written by the pass; tile_lo: instead of labels, a lower bound of the
+    // distance of each row to the centers of each tile (n x n_ctiles).
+    const int32_t *perm;
+    const int32_t *inv;
+    const uint32_t *unit_mask;
+    float *ub;
+    float *tile_lo;
 };
 
 // Diagnostic counters: SM cycles each role spent waiting (summed over CTAs).
@@ -512,7 +522,8 @@ __global__ void __launch_bounds__(256, 6) prep_frames_dense_kernel(const float *
 template <typename T>
 __global__ void prep_centers_kernel(const float *__restrict__ C, int k, int k_pad, int d, int kp,
                                     const float *__restrict__ shift, uint32_t *__restrict__ scal,
-                                    T *__restrict__ ch, float2 *__restrict__ cnorm, float norm_inflate) {
+                                    T *__restrict__ ch, float2 *__restrict__ cnorm, float norm_inflate,
+                                    const int32_t *__restrict__ perm) {
     using O = Op16<T>;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -520,7 +531,7 @@ __global__ void prep_centers_kernel(const float *__restrict__ C, int k, int k_pa
     const float sc = __uint_as_float(scal[kScale]);
     const float inv_sc = 1.0f / sc;
     for (int64_t j = w; j < k; j += nw) {
-        const float *src = C + j * d;
+        const float *src = C + (perm ? (int64_t)perm[j] : j) * d;
         typename O::T2 *dst = reinterpret_cast<typename O::T2 *>(ch + j * kp);
         double h2 = 0.0;
         CSum s2, e2;
@@ -829,6 +840,8 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     const int64_t n_units = (p.n - p.frame0 + unit - 1) / unit;
     const int64_t unit0 = PAIR ? blockIdx.x / 2 : blockIdx.x;
     const int64_t unit_stride = PAIR ? gridDim.x / 2 : gridDim.x;
+    // The center tiles of a unit: all of them, or the set bits of its mask.
+    const uint32_t *masks = p.unit_mask ? p.unit_mask + p.frame0 / unit : nullptr;
 
     if (threadIdx.x == 0) {
         for (int c = 0; c < nab; ++c) {
@@ -881,9 +894,12 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         uint32_t s = 0, sph = 0;
         for (int64_t ft = unit0; ft < n_units && ok; ft += unit_stride, ++t_local) {
             const int frame_row = (int)(p.frame0 + ft * unit + rank * kBM);
-            for (int ct = 0; ct < p.n_ctiles && ok; ++ct) {
+            uint32_t todo = masks ? masks[ft] : 0u;
+            const int n_ct = masks ? __popc(todo) : p.n_ctiles;
+            for (int q = 0; q < n_ct && ok; ++q, todo &= todo - 1u) {
+                const int ct = masks ? __ffs(todo) - 1 : q;
                 for (int t = 0; t < p.nbst; ++t) {
-                    if (!stream && ct == 0) {
+                    if (!stream && q == 0) {
                         if (ok) ok = mbar_wait_timed(&a_empty[t], (t_local & 1u) ^ 1u, pw_a);
                         if (elect_one() && ok) {
                             if (PAIR) {
@@ -917,7 +933,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         sph ^= 1u;
                     }
                 }
-                if (ct == 0) a_issued_tiles += 1;
+                if (q == 0) a_issued_tiles += 1;
                 ok = __all_sync(0xffffffffu, ok) && !__any_sync(0xffffffffu, *abort_flag != 0);
             }
         }
@@ -972,14 +988,15 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         uint32_t s = 0, sph = 0;  // B stage and its phase
         uint64_t sdesc = sdesc0;  // descriptor of stage s
         for (int64_t ft = unit0; (!PAIR || leader) && ft < n_units && ok; ft += unit_stride, ++t_local) {
-            for (int ct = 0; ct < p.n_ctiles && ok; ++ct) {
+            const int n_ct = masks ? __popc(masks[ft]) : p.n_ctiles;
+            for (int q = 0; q < n_ct && ok; ++q) {
                 const uint32_t buf = accq & 1u;
                 // The peer CTA's epilogue warps arrive here too (cluster scope).
                 ok = PAIR ? mbar_wait_cluster_timed(&acc_empty[buf], ((accq >> 1) & 1u) ^ 1u, pw_acc)
                           : mbar_wait_timed(&acc_empty[buf], ((accq >> 1) & 1u) ^ 1u, pw_acc);
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * (uint32_t)p.bn;
-                const bool first = ct == 0, last = ct == p.n_ctiles - 1;
+                const bool first = q == 0, last = q == n_ct - 1;
                 uint64_t ad = adesc0;
                 for (int t = 0; t < p.nbst; ++t) {
                     if (!stream && first && ok) ok = mbar_wait_timed(&a_full[t], t_local & 1u, pw_a);
@@ -1083,8 +1100,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 // is one; any center in range is valid).  The true maximum is
                 // at least as large, so the threshold only starts higher and
                 // no candidate is lost; the frame's lists stay short.
-                const int pl = p.labels[i];
-                if (pl >= 0 && pl < p.k) {
+                const int named = p.labels[i];
+                if (named >= 0 && named < p.k) {
+                    const int pl = p.inv ? p.inv[named] : named;
                     const float2 cn = p.cnorm[pl];
                     const float sj = xn.y + cn.x;
                     const float Ej = __fmul_ru(p.e_coef, __fmul_ru(sj, sj));
@@ -1111,7 +1129,12 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 la[m] = kNegInf;
                 lid[m] = -1;
             }
-            for (int ct = 0; ct < p.n_ctiles; ++ct) {
+            if (p.tile_lo) thr = kInf;  // no candidates
+            uint32_t todo = masks ? masks[ft] : 0u;
+            const int n_ct = masks ? __popc(todo) : p.n_ctiles;
+            for (int q = 0; q < n_ct; ++q, todo &= todo - 1u) {
+                const int ct = masks ? __ffs(todo) - 1 : q;
+                float top = kNegInf;  // the largest accumulator of the tile
                 const uint32_t buf = accq & 1u;
                 const bool got = __all_sync(0xffffffffu, mbar_wait_timed(&acc_full[buf], (accq >> 1) & 1u, pw_acc));
                 if (!got) {
@@ -1163,6 +1186,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     const float m4c = max3f(m12[6], m12[7], m12[8]);
                     const float m4d = max3f(m12[9], m12[10], m12[11]);
                     const float mx = fmaxf(max3f(m4a, m4b, m4c), m4d);
+                    top = fmaxf(top, mx);
                     if (mx >= thr && mx > kNegInf) {
                         if (mx > best) {
                             best = mx;
@@ -1216,8 +1240,18 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         mbar_arrive(&acc_empty[buf]);
                 }
                 ++accq;
+                if (p.tile_lo && i < p.n) {
+                    // sqrt(v - E) - R of the nearest one; 0 (no bound) unless finite
+                    const float v = fmaf(-2.0f, top, xn.x) * inv_s2;
+                    const float lo = __fsub_rd(__fsqrt_rd(fmaxf(__fsub_rd(v, Emax), 0.0f)), Rmax);
+                    p.tile_lo[i * p.n_ctiles + ct] = lo > 0.0f && lo < kInf ? lo : 0.0f;
+                }
             }
             if (!ok) break;
+            if (p.tile_lo) {
+                if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
+                continue;
+            }
 
             // ---- decision ----
             bool need_rc = false, need_full = false;
@@ -1265,7 +1299,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         jb = lid[m];
                     }
                 }
+                if (p.perm) jb = cmask ? p.perm[jb] : 0;  // no candidate: center 0, until the re-check
                 p.labels[i] = jb;
+                // The exact label's float32 distance is at most H (also where
+                // the re-checks decide): its true distance, rounded up.
+                if (p.ub) p.ub[i] = finite ? __fmul_ru(__fsqrt_ru(H), p.g_ratio) : kInf;
             }
             // member counts for the centroid update: one reduction per frame
             // (its value unused, so the warp does not wait for it; gathering
@@ -1305,7 +1343,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     for (int m = 0; m < L; ++m) {
                         if ((cmask >> m) & 1u) {
                             const int q = pbase + excl + __popc(cmask & ((1u << m) - 1u));
-                            p.pair_center[q] = lid[m];
+                            p.pair_center[q] = p.perm ? p.perm[lid[m]] : lid[m];
                             p.pair_lo[q] = lo[m];
                         }
                     }
@@ -1773,10 +1811,11 @@ int tc_prepare_centers(const float *C, int d, int k, TcBuffers &b, cudaStream_t 
     else if (b.bf16)
         prep_centers_kernel<__nv_bfloat16><<<(unsigned)prep_blocks(kpad), 256, 0, s>>>(
             C, k, kpad, d, b.kp, b.shift, b.scal, reinterpret_cast<__nv_bfloat16 *>(b.ch), b.cnorm,
-            norm_inflate_of(d));
+            norm_inflate_of(d), b.perm);
     else
         prep_centers_kernel<__half><<<(unsigned)prep_blocks(kpad), 256, 0, s>>>(
-            C, k, kpad, d, b.kp, b.shift, b.scal, reinterpret_cast<__half *>(b.ch), b.cnorm, norm_inflate_of(d));
+            C, k, kpad, d, b.kp, b.shift, b.scal, reinterpret_cast<__half *>(b.ch), b.cnorm, norm_inflate_of(d),
+            b.perm);
     KM_CUDA(cudaGetLastError());
     return KM_OK;
 }
@@ -1849,7 +1888,7 @@ cudaError_t launch_tc_variant(const cudaLaunchConfig_t &cfg, int list_len, bool 
 int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int32_t *labels, TcBuffers &b,
                    cudaStream_t s, ProfEvents *prof, float *dump, unsigned long long *wait_cycles, cudaStream_t side,
                    const cudaEvent_t *ev_fork, int n_fork, const FlipList *fl, const PairSrc *ps,
-                   int32_t *label_counts) {
+                   int32_t *label_counts, float *tile_lo = nullptr) {
     if (n == 0) return KM_OK;
     Plan pl;
     if (!make_plan(d, k, pl, b.fp8 != 0, b.bf16 != 0) || !device_is_sm10x()) {
@@ -1943,6 +1982,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     // operands (both give the same labels).
     bool seed = !b.fp8 && b.kp <= 128 && k >= 2048;
     if (const char *e = std::getenv("KM_TC_SEED")) seed = !b.fp8 && e[0] == '1';
+    seed = seed && !tile_lo;
     p.seed_xh = seed ? b.xh : nullptr;
     p.seed_ch = seed ? b.ch : nullptr;
     {
@@ -1950,6 +1990,11 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         const double kk = (double)b.kp + 2.0;
         p.seed_coef = std::nextafter((float)(kk * uu / (1.0 - kk * uu) * 1.01), INFINITY);
     }
+    p.perm = b.perm;
+    p.inv = b.inv;
+    p.unit_mask = b.unit_mask;
+    p.ub = b.ub;
+    p.tile_lo = tile_lo;
     set_lists(p, b);
     p.err = b.err;
     p.dump = dump;
@@ -2038,6 +2083,8 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         return KM_OK;
     };
 
+    if (tile_lo) return launch_pass(p);
+
     // Each chunk: the tensor-core launch on s, then its exact re-checks on s,
     // or on `side` beside the next chunk (and, after the last chunk, beside
     // the caller's next work).  Beside the centroid update the re-check keeps
@@ -2064,7 +2111,9 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
             KM_CUDA(cudaStreamWaitEvent(side, ev_fork[c], 0));
         }
         if (prof && c == 0) prof->begin(kProfRecheck, r);
-        const int per_sm = !side ? 8 : c + 1 < n_chunks ? 1 : kRecheckBesidePerSm;
+        // (a masked launch is shorter than its re-check at one CTA per SM:
+        // 2M x 528, k = 2000, 2.67 ms per iteration with one, 2.19 with four)
+        const int per_sm = !side ? 8 : c + 1 < n_chunks && !b.unit_mask ? 1 : kRecheckBesidePerSm;
         KM_TRY(launch_recheck_pairs(X, d, C, v.rc_frames, v.rc_best, v.rc_pairs, v.pair_center, v.pair_lo,
                                     v.rc_keys, v.amb_entries, v.amb_mask, v.counters, f1 - f0, labels, b.flipped, r,
                                     fl, per_sm, ps));
@@ -2082,6 +2131,252 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     return KM_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Center bounds of Lloyd iterations.
+//
+// The pass compares every frame with every center, but after an iteration a
+// frame's distance to its own center is known from above (ub, plus what the
+// center has moved since).  By the triangle inequality a center farther from
+// the frame's center than twice that distance cannot be nearer.  The centers
+// are ordered once per run so that near ones share a tile of the pass; per
+// iteration the pass itself, with the centers as its frames, gives a lower
+// bound of the distance of each center to each tile, and a tile is left out
+// of a frame unit (128 or 256 consecutive frames) when the bound rules it out
+// for every frame.  The margins cover the float32 rounding of the distances
+// that define the labels, so the labels are the same, ties included.
+//
+// Frames of a trajectory stay near a few centers, and most units need one or
+// two tiles (2M x 528 pair distances, k = 2000: 1.5 of 8).  What bounds the
+// pass then is L2: a unit loads its 147 KB and 147 KB per tile and CTA.  Per
+// iteration there: the pass 2.6 -> 1.04 ms, bounds and masks 0.07 ms, the
+// iteration 3.69 -> 2.19 ms.
+// ---------------------------------------------------------------------------
+constexpr int kMaxMaskTiles = 32;  // bits of a unit's mask
+constexpr int kLeaders = 64;       // centers that the others are grouped by
+
+// The nearest of kl evenly spread centers of every center (a warp each), and
+// the distances between those.
+__global__ void __launch_bounds__(256) center_group_kernel(const float *__restrict__ C, int k, int d, int kl,
+                                                           int32_t *__restrict__ group, float *__restrict__ lead) {
+    const int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (j >= k) return;
+    const float *c = C + (int64_t)j * d;
+    float best = __int_as_float(0x7f800000);
+    int g = 0;
+    int own = -1;  // j is this leader
+    for (int l = 0; l < kl; ++l) {
+        const int jl = (int)((int64_t)l * k / kl);
+        if (jl == j) own = l;
+    }
+    for (int l0 = 0; l0 < kl; l0 += 8) {  // eight rows in flight
+        const float *r[8];
+        float acc[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            r[q] = C + (int64_t)((int64_t)min(l0 + q, kl - 1) * k / kl) * d;
+            acc[q] = 0.0f;
+        }
+        for (int f = lane; f < d; f += 32) {
+            const float x = __ldg(c + f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float t = x - __ldg(r[q] + f);
+                acc[q] = fmaf(t, t, acc[q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
+            if (l0 + q < kl) {
+                if (own >= 0 && lane == 0) lead[own * kl + l0 + q] = acc[q];
+                if (acc[q] < best) {
+                    best = acc[q];
+                    g = l0 + q;
+                }
+            }
+        }
+    }
+    if (lane == 0) group[j] = g;
+}
+
+// The leaders in a chain of nearest neighbours, the centers sorted by the
+// place of their leader: perm[operand row] = center, inv its inverse.
+__global__ void __launch_bounds__(1024) center_order_kernel(int k, int kl, const int32_t *__restrict__ group,
+                                                            const float *__restrict__ lead,
+                                                            int32_t *__restrict__ perm, int32_t *__restrict__ inv) {
+    __shared__ int place[kLeaders], start[kLeaders + 1];
+    __shared__ float lead_s[kLeaders * kLeaders];
+    for (int e = threadIdx.x; e < kl * kl; e += blockDim.x) lead_s[e] = lead[e];
+    const int lane = threadIdx.x & 31;
+    for (int l = threadIdx.x; l <= kl; l += blockDim.x) start[l] = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        unsigned long long left = 0ull;  // leaders not yet placed
+        for (int l = 0; l < kl; ++l) left |= 1ull << l;
+        int at = 0;
+        for (int q = 0; q < kl; ++q) {
+            if (lane == 0) place[at] = q;
+            left &= ~(1ull << at);
+            float bd = __int_as_float(0x7f800000);
+            int bl = kLeaders;
+            for (int l = lane; l < kl; l += 32)
+                if ((left >> l) & 1ull) {
+                    const float v = lead_s[at * kl + l];
+                    const float w = v == v ? fminf(v, 3.4028234663852886e38f) : 3.4028234663852886e38f;
+                    if (w < bd) {
+                        bd = w;
+                        bl = l;
+                    }
+                }
+            warp_argmin(bd, bl);
+            if (bl < kl) at = bl;
+        }
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < k; j += blockDim.x) atomicAdd(&start[place[group[j]] + 1], 1);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int l = 0; l < kl; ++l) start[l + 1] += start[l];
+    __syncthreads();
+    for (int j = threadIdx.x; j < k; j += blockDim.x) {
+        const int r = atomicAdd(&start[place[group[j]]], 1);
+        perm[r] = j;
+        inv[j] = r;
+    }
+}
+
+// Upper bound of what each center has moved (a warp each).
+__global__ void __launch_bounds__(256) center_drift_kernel(const float *__restrict__ C, const float *__restrict__ C_new,
+                                                           int k, int d, float inflate, float *__restrict__ drift) {
+    const int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (j >= k) return;
+    float acc = 0.0f;
+    for (int f = lane; f < d; f += 32) {
+        const float t = __fsub_rn(__ldg(C_new + (int64_t)j * d + f), __ldg(C + (int64_t)j * d + f));
+        acc = __fmaf_ru(t, t, acc);
+    }
+    for (int off = 16; off > 0; off >>= 1) acc = __fadd_ru(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+    if (lane == 0) drift[j] = __fadd_ru(__fsqrt_ru(__fmul_ru(acc, inflate)), 1e-30f);
+}
+
+// One CTA per frame unit, a thread per frame.
+__global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int n_ct, int bn,
+                                                        const int32_t *__restrict__ labels,
+                                                        const float *__restrict__ ub,
+                                                        const float *__restrict__ drift,
+                                                        const int32_t *__restrict__ inv,
+                                                        const float *__restrict__ tile_lo, float factor,
+                                                        uint32_t *__restrict__ mask,
+                                                        unsigned long long *__restrict__ bits) {
+    __shared__ uint32_t any;
+    if (threadIdx.x == 0) any = 0u;
+    __syncthreads();
+    const int64_t i = (int64_t)blockIdx.x * unit + threadIdx.x;
+    uint32_t m = 0u;
+    if (i < n) {
+        const int a = labels[i];
+        const float far = __fmul_ru(__fadd_ru(ub[i], drift[a]), factor);
+        const float *lo = tile_lo + (int64_t)a * n_ct;
+        m = 1u << (inv[a] / bn);
+        for (int t = 0; t < n_ct; ++t)
+            if (!(__ldg(lo + t) > far)) m |= 1u << t;  // also where either is not a number
+    }
+    m = __reduce_or_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicOr(&any, m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mask[blockIdx.x] = any;
+        if (bits) atomicAdd(bits, (unsigned long long)__popc(any));
+    }
+}
+
+}  // namespace
+
+// Worth asking for from 4e11 flop per pass on (0.3 ms; the order and the first
+// masks cost about 0.15 ms once, and the masks are used only where they leave
+// out a quarter of the tiles).  KM_TC_BOUNDS=0 or 1 in the environment forces
+// the choice (the labels are the same).
+bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b) {
+    Plan pl;
+    if (b.fp8 || !make_plan(d, k, pl, false, b.bf16 != 0)) return false;
+    const int n_ct = (k + pl.bn - 1) / pl.bn;
+    if (n_ct < 2 || n_ct > kMaxMaskTiles || max_iter < 2) return false;
+    if (const char *e = std::getenv("KM_TC_BOUNDS")) return e[0] == '1';
+    return max_iter >= 4 && 2.0 * (double)n * k * d >= 4e11;
+}
+
+bool tc_bounds_forced() {
+    const char *e = std::getenv("KM_TC_BOUNDS");
+    return e && e[0] == '1';
+}
+
+size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t) {
+    Carver c(ws);
+    t.perm = c.take<int32_t>(k);
+    t.inv = c.take<int32_t>(k);
+    t.group = c.take<int32_t>(k);
+    t.lead = c.take<float>(kLeaders * kLeaders);
+    t.drift = c.take<float>(k);
+    t.ub = c.take<float>(n > 0 ? n : 1);
+    t.mask = c.take<uint32_t>((n > 0 ? n : 1) / kBM + 2);
+    t.bits = c.take<unsigned long long>(1);
+    t.tile_lo = c.take<float>((size_t)k * kMaxMaskTiles);
+    t.cxh = c.take<uint16_t>((size_t)k * kp_of(d));
+    t.cxnorm = c.take<float4>(k);
+    return c.bytes();
+}
+
+int tc_bounds_order(const float *C, int d, int k, TcBuffers &b, const TcBounds &t, cudaStream_t s) {
+    const int kl = std::min(kLeaders, k);
+    center_group_kernel<<<(unsigned)((k + 7) / 8), 256, 0, s>>>(C, k, d, kl, t.group, t.lead);
+    KM_CUDA(cudaGetLastError());
+    center_order_kernel<<<1, 1024, 0, s>>>(k, kl, t.group, t.lead, t.perm, t.inv);
+    KM_CUDA(cudaGetLastError());
+    b.perm = t.perm;
+    b.inv = t.inv;
+    b.ub = t.ub;
+    return KM_OK;
+}
+
+int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBounds &t, cudaStream_t s) {
+    center_drift_kernel<<<(unsigned)((k + 7) / 8), 256, 0, s>>>(C, C_new, k, d, norm_inflate_of(d), t.drift);
+    KM_CUDA(cudaGetLastError());
+    return KM_OK;
+}
+
+// The units' masks for centers C (whose operands are prepared), from the
+// labels, ub and drift of the last iteration; *bits (nullable, cleared here)
+// counts the tiles they hold.
+int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
+                    unsigned long long *bits, int64_t *units, int *tiles, cudaStream_t s) {
+    Plan pl;
+    if (!make_plan(d, k, pl, false, b.bf16 != 0)) return KM_ERR_UNSUPPORTED;
+    TcBuffers v = b;
+    v.xh = t.cxh;
+    v.xnorm = t.cxnorm;
+    v.unit_mask = nullptr;
+    v.ub = nullptr;
+    v.keep_err = 0;
+    KM_TRY(tc_prepare_frames(C, k, d, v, s, nullptr));
+    KM_TRY(tc_assign_impl(C, k, d, C, k, nullptr, v, s, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr,
+                          nullptr, nullptr, t.tile_lo));
+    const int unit = pl.pair ? 2 * kBM : kBM;
+    const int n_ct = (k + pl.bn - 1) / pl.bn;
+    const int64_t n_units = (n + unit - 1) / unit;
+    // 1 + sqrt((1 + g) / (1 - g)): twice the distance, and the rounding of both
+    const double u = std::ldexp(1.0, -24), g = (d + 2) * u / (1.0 - (d + 2) * u) * 1.01;
+    const float factor =
+        std::nextafter((float)((1.0 + std::sqrt((1.0 + g) / (1.0 - g))) * (1.0 + std::ldexp(1.0, -19))), INFINITY);
+    if (bits) KM_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned long long), s));
+    unit_mask_kernel<<<(unsigned)n_units, unit, 0, s>>>(n, unit, n_ct, pl.bn, labels, t.ub, t.drift, t.inv, t.tile_lo,
+                                                        factor, t.mask, bits);
+    KM_CUDA(cudaGetLastError());
+    if (units) *units = n_units;
+    if (tiles) *tiles = n_ct;
+    return KM_OK;
+}
+
+namespace {
 }  // namespace
 
 int tc_assign(const float *X, int64_t n, int d, const float *C, int k, int32_t *labels, TcBuffers &b,

@@ -400,6 +400,10 @@ size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
         c.take<int32_t>(3 * (size_t)n);  // flip list
         c.take<int32_t>(1);              // its count
     }
+    if (is_tc(prec)) {
+        TcBounds t;
+        c.take<char>(tc_bounds_carve(nullptr, n, d, k, t));
+    }
     // at every n, so that the size of the largest n serves the smaller ones
     if (!is_tc(prec) && small_lloyd_shape_ok(d, k)) c.take<char>(small_lloyd_ws_size(d, k));
     return c.bytes();
@@ -1038,6 +1042,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     }
 
     TcBuffers b;
+    TcBounds bounds;
+    bool with_bounds = false;  // the pass keeps the bounds; masked below once they are worth it
     if (tc) {
         // The shift and scale stay fixed for the whole run so that the 16-bit
         // frame copy is made once (narrow frames have none).
@@ -1048,6 +1054,11 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             carve_small(ws_assign, n, d, k, b);
         }
         KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
+        if (is_tc(prec)) {
+            tc_bounds_carve(cv.take<char>(tc_bounds_carve(nullptr, n, d, k, bounds)), n, d, k, bounds);
+            with_bounds = tc_bounds_wanted(n, d, k, max_iter, b);
+            if (with_bounds) KM_TRY(tc_bounds_order(C, d, k, b, bounds, s));
+        }
         if (!hf && !small) KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
     }
     KM_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
@@ -1073,6 +1084,10 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     auto enqueue = [&](cudaStream_t st) -> int {
         if (tc) {
             KM_TRY(small ? small_prepare_centers(C, d, k, b, st) : tc_prepare_centers(C, d, k, b, st));
+            if (b.unit_mask) {
+                KM_TRY(tc_bounds_masks(C, n, d, k, labels, b, bounds, nullptr, nullptr, nullptr, st));
+                b.keep_err = 1;  // cleared by the masks' pass
+            }
             KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
             // the tensor-core pass counts the members as it writes the labels
             int32_t *counts = update_counts_from_labels(d, k, ps) ? update_counts(ws_update, n, d, k) : nullptr;
@@ -1089,6 +1104,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             KM_CUDA(cudaStreamWaitEvent(st, side.join, 0));
             KM_TRY(launch_apply_flips(X, n, d, k, C, fl, labels, ws_update, st, ps));
             KM_TRY(launch_update_finish(n, d, k, C, C_new, nullptr, cost, ws_update, st));
+            if (with_bounds) KM_TRY(tc_bounds_drift(C, C_new, d, k, bounds, st));
             prof.end(kProfUpdate, st);
             KM_CUDA(cudaMemcpyAsync(C, C_new, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, st));
             return KM_OK;
@@ -1132,6 +1148,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             KM_TRY(launch_update_part(X + a * d, n, d, labels + a, rows, k, C, err, ws_update, st));
         }
         KM_TRY(launch_update_parts_finish(n, d, k, C, C_new, cost, ws_update, st));
+        if (with_bounds) KM_TRY(tc_bounds_drift(C, C_new, d, k, bounds, st));
         prof.end(kProfUpdate, st);
         KM_CUDA(cudaMemcpyAsync(C, C_new, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, st));
         return KM_OK;
@@ -1248,6 +1265,28 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         if (fused && (it == 1 || !hf)) {
             status = fused_loop(it, prev);
             break;
+        }
+        if (it == 1 && with_bounds) {
+            // Masks on trial: kept where they leave out a quarter of the tiles.
+            unsigned long long set = 0;
+            int64_t units = 0;
+            int tiles = 0;
+            status = tc_prepare_centers(C, d, k, b, s);
+            if (status == KM_OK)
+                status = tc_bounds_masks(C, n, d, k, labels, b, bounds, bounds.bits, &units, &tiles, s);
+            if (status != KM_OK) break;
+            cudaError_t e = cudaMemcpyAsync(&set, bounds.bits, sizeof(set), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) {
+                status = cuda_fail(e, "center bounds");
+                break;
+            }
+            if (tc_bounds_forced() || (double)set <= 0.75 * (double)units * tiles)
+                b.unit_mask = bounds.mask;
+            else {
+                with_bounds = false;
+                b.ub = nullptr;
+            }
         }
         if (it == 1 && !cb && !prof.active) {
             int handled = 0;

@@ -220,6 +220,12 @@ struct TcBuffers {
     void *sch = nullptr;         // narrow frames (assign_small.cu): split FP16 operand rows of the centers
     float *scg = nullptr;        // narrow frames: the centers by groups of eight, [group][feature][8]
     float *chn = nullptr;        // FP8 only: -||c~_j||^2 / 2 per center (the norm is not folded into the GEMM)
+    // Center bounds (nullable, tc_bounds_*): the order of the operand rows,
+    // the frames' distance bounds, the tiles of each frame unit.
+    const int32_t *perm = nullptr;
+    const int32_t *inv = nullptr;
+    float *ub = nullptr;
+    const uint32_t *unit_mask = nullptr;
     int kp = 0;        // operand row length in elements
     int esize = 2;     // operand bytes per element: 2 (FP16, BF16) or 1 (FP8 e4m3)
     int bf16 = 0;      // operand type of xh / ch: 0 FP16, 1 BF16
@@ -241,8 +247,26 @@ inline TcBuffers tc_rows_from(const TcBuffers &b, int64_t a) {
     TcBuffers v = b;
     v.xh = static_cast<char *>(b.xh) + (size_t)a * b.kp * b.esize;
     v.xnorm = b.xnorm + a;
+    if (b.ub) v.ub = b.ub + a;
     return v;
 }
+
+// Buffers and steps of the center bounds of Lloyd iterations (assign_tc.cu).
+struct TcBounds {
+    int32_t *perm, *inv, *group;
+    float *lead, *drift, *ub, *tile_lo;
+    uint32_t *mask;
+    unsigned long long *bits;
+    void *cxh;  // the centers as frames
+    float4 *cxnorm;
+};
+bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b);
+bool tc_bounds_forced();
+size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t);  // its size with ws = nullptr
+int tc_bounds_order(const float *C, int d, int k, TcBuffers &b, const TcBounds &t, cudaStream_t s);
+int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBounds &t, cudaStream_t s);
+int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
+                    unsigned long long *bits, int64_t *units, int *tiles, cudaStream_t s);
 
 // Sets the operand type of carved buffers from the precision (KM_PREC_FP16,
 // KM_PREC_BF16 or KM_PREC_FP8): element size and row length.
