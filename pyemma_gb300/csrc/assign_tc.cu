@@ -129,6 +129,15 @@ struct TcParams {
     const uint32_t *unit_mask;
     float *ub;
     float *tile_lo;
+    // Frames whose lists overflowed, a second time: *n_dev of them, the
+    // threshold each ended with, and instead of labels a bit per operand row
+    // that reaches it (bit_words words per frame).  full_thr = 1: the pass
+    // leaves those thresholds (NaN: not finite) in full_keys.
+    const int32_t *n_dev;
+    const float *row_thr;
+    uint32_t *bits;
+    int bit_words;
+    int full_thr;
 };
 
 // Diagnostic counters: SM cycles each role spent waiting (summed over CTAs).
@@ -837,9 +846,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     // Frame units: 128 frames per CTA; a pair takes 256 consecutive frames,
     // its rank-r CTA the r-th half.
     const int64_t unit = PAIR ? 2 * kBM : kBM;
-    const int64_t n_units = (p.n - p.frame0 + unit - 1) / unit;
+    const int64_t n_end = p.n_dev ? min((int64_t)*p.n_dev, p.n) : p.n;
+    const int64_t n_units = (n_end - p.frame0 + unit - 1) / unit;
     const int64_t unit0 = PAIR ? blockIdx.x / 2 : blockIdx.x;
     const int64_t unit_stride = PAIR ? gridDim.x / 2 : gridDim.x;
+    if (unit0 >= n_units) return;  // both CTAs of a pair; only where the count is the device's
     // The center tiles of a unit: all of them, or the set bits of its mask.
     const uint32_t *masks = p.unit_mask ? p.unit_mask + p.frame0 / unit : nullptr;
 
@@ -1079,6 +1090,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         const float hc_max = __uint_as_float(p.scal[kHcMax]);
         const float kNegInf = __int_as_float(0xff800000);
         const float kInf = __int_as_float(0x7f800000);
+        const float kNaN = __int_as_float(0x7fc00000);
         uint32_t accq = 0;
         bool ok = true;
         unsigned long long w_acc = 0;
@@ -1086,7 +1098,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         unsigned long long *pw_acc = (p.wait_cycles && warp == 2 && lane == 0) ? &w_acc : nullptr;
         for (int64_t ft = unit0; ft < n_units && ok; ft += unit_stride) {
             const int64_t i = p.frame0 + ft * unit + (int64_t)rank * kBM + row;
-            const float4 xn = i < p.n ? p.xnorm[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 xn = i < n_end ? p.xnorm[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             // Worst-case bound terms over all centers: the acceptance window
             // and the overflow decision use them.
             const float smax = xn.y + sc_max;
@@ -1094,7 +1106,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             const float Emax = __fmul_ru(p.e_coef, __fmul_ru(smax, smax));
             const float Rpad = __fadd_ru(Rmax, 1e-18f);
             float best = kNegInf, thr = kNegInf;
-            if (!F8 && p.seed_xh && i < p.n) {
+            if (!F8 && p.seed_xh && i < n_end) {
                 // Seed: a lower bound of the accumulator of the center the
                 // frame's label names (the previous iteration's, where there
                 // is one; any center in range is valid).  The true maximum is
@@ -1130,6 +1142,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 lid[m] = -1;
             }
             if (p.tile_lo) thr = kInf;  // no candidates
+            if (p.bits) {
+                best = kInf;  // the threshold stays
+                thr = i < n_end ? p.row_thr[i] : kInf;
+            }
             uint32_t todo = masks ? masks[ft] : 0u;
             const int n_ct = masks ? __popc(todo) : p.n_ctiles;
             for (int q = 0; q < n_ct; ++q, todo &= todo - 1u) {
@@ -1169,7 +1185,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         for (int c = 0; c < 32; ++c)
                             if (j0 + c >= p.k) v[c] = kNegInf;
                     }
-                    if (p.dump && i < p.n) {
+                    if (p.dump && i < n_end) {
 #pragma unroll
                         for (int c = 0; c < 32; ++c)
                             if (j0 + c < p.k) p.dump[i * p.k + j0 + c] = fmaf(-2.0f, v[c], xn.x) * inv_s2;
@@ -1187,6 +1203,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     const float m4d = max3f(m12[9], m12[10], m12[11]);
                     const float mx = fmaxf(max3f(m4a, m4b, m4c), m4d);
                     top = fmaxf(top, mx);
+                    uint32_t reach = 0u;
                     if (mx >= thr && mx > kNegInf) {
                         if (mx > best) {
                             best = mx;
@@ -1203,6 +1220,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         unsigned msk = (mk[0] | mk[1]) | (mk[2] | mk[3]);
                         const int nv = p.k - j0;
                         if (nv < 32) msk &= nv > 0 ? (1u << nv) - 1u : 0u;
+                        if (p.bits) {
+                            reach = msk;
+                            msk = 0u;
+                        }
                         const bool lone = (msk & (msk - 1u)) == 0u;
                         while (msk) {
                             const int c = __ffs(msk) - 1;
@@ -1230,6 +1251,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                             lid[0] = j0 + c;
                         }
                     }
+                    if (p.bits && i < n_end) p.bits[i * p.bit_words + (j0 >> 5)] = reach;
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -1240,7 +1262,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         mbar_arrive(&acc_empty[buf]);
                 }
                 ++accq;
-                if (p.tile_lo && i < p.n) {
+                if (p.tile_lo && i < n_end) {
                     // sqrt(v - E) - R of the nearest one; 0 (no bound) unless finite
                     const float v = fmaf(-2.0f, top, xn.x) * inv_s2;
                     const float lo = __fsub_rd(__fsqrt_rd(fmaxf(__fsub_rd(v, Emax), 0.0f)), Rmax);
@@ -1248,17 +1270,17 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 }
             }
             if (!ok) break;
-            if (p.tile_lo) {
+            if (p.tile_lo || p.bits) {
                 if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
                 continue;
             }
 
             // ---- decision ----
-            bool need_rc = false, need_full = false;
+            bool need_rc = false, need_full = false, settled = false;  // settled: its threshold holds
             unsigned cmask = 0;  // bit m: list entry m is a candidate
             int jb = 0;          // candidate with the largest accumulator
             float lo[L];        // lower bounds of the candidates' exact distances
-            if (i < p.n) {
+            if (i < n_end) {
                 float vv[L], RR[L], EE[L];
                 float H = kInf;
 #pragma unroll
@@ -1278,6 +1300,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 const bool finite = best > kNegInf && H < kInf && Rmax < kInf && Emax < kInf;
                 if (!finite || ovf) {
                     need_full = true;
+                    settled = finite;
                 } else {
 #pragma unroll
                     for (int m = 0; m < L; ++m) {
@@ -1308,7 +1331,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             // member counts for the centroid update: one reduction per frame
             // (its value unused, so the warp does not wait for it; gathering
             // equal labels of a warp first cost the kernel more than it saved)
-            if (p.label_counts && i < p.n) atomicAdd(&p.label_counts[jb], 1);
+            if (p.label_counts && i < n_end) atomicAdd(&p.label_counts[jb], 1);
             const unsigned m_rc = __ballot_sync(0xffffffffu, need_rc);
             if (m_rc) {
                 // One entry per re-checked frame and one pair per candidate,
@@ -1358,7 +1381,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 if (need_full) {
                     const int e = base + __popc(m_full & ((1u << lane) - 1u));
                     p.full_frames[e] = (int32_t)i;
-                    p.full_keys[e] = ~0ull;
+                    p.full_keys[e] = p.full_thr ? (unsigned long long)__float_as_uint(settled ? thr : kNaN) : ~0ull;
                 }
             }
             if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
@@ -1671,7 +1694,10 @@ constexpr int kMaxTcChunks = kTcMaxChunks;
 constexpr int kChunkCounters0 = kTcDiagWords + 16;
 
 // One carving sequence for sizing (ws == nullptr) and for carving.
-size_t carve_assign(void *ws, int64_t n, TcBuffers &b) {
+// Frames that a pass takes a second time at most (0: none).
+int64_t wide_cap(int64_t n, int d) { return d >= 32 && n >= 4096 ? (n / 16 + 255) / 256 * 256 : 0; }
+
+size_t carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
     Carver c(ws);
     const size_t nn = n > 0 ? n : 1;
     b.rc_frames = c.take<int32_t>(nn);
@@ -1685,31 +1711,38 @@ size_t carve_assign(void *ws, int64_t n, TcBuffers &b) {
     b.full_frames = c.take<int32_t>(nn);
     b.full_keys = c.take<unsigned long long>(nn);
     // [0] recheck entries, [1] full entries, [2] pairs, [3] entries left to the exact pass, then flipped (two words),
-    // err and a spare word; [kTcDiagWords..kChunkCounters0) diagnostics; then the first four again for chunks 1.. of
+    // err and a spare word; [kTcDiagWords..kChunkCounters0) diagnostics, or the second pass's two counts; then the first four again for chunks 1.. of
     // a chunked pass
     b.counters = c.take<int32_t>(kChunkCounters0 + 4 * (kMaxTcChunks - 1));
     b.flipped = reinterpret_cast<unsigned long long *>(b.counters + 4);
     b.err = reinterpret_cast<uint32_t *>(b.counters + 6);
+    b.wide_cap = wide_cap(n, d);
+    if (b.wide_cap > 0) {
+        b.wide_xh = c.take<uint16_t>((size_t)b.wide_cap * kp_of(d));
+        b.wide_xnorm = c.take<float4>(b.wide_cap);
+        b.wide_thr = c.take<float>(b.wide_cap);
+        b.wide_frames = c.take<int32_t>(b.wide_cap);
+        b.wide_bits = c.take<uint32_t>((size_t)b.wide_cap * (k_pad_of(k) / 32 + 8));
+        b.wide_counts = b.counters + kTcDiagWords;
+    }
     return c.bytes();
 }
 }  // namespace
 
 size_t tc_assign_ws_size(int64_t n, int d, int k) {
-    (void)d;
-    (void)k;
     TcBuffers b;
-    return carve_assign(nullptr, n, b);
+    return carve_assign(nullptr, n, d, k, b);
 }
 
 void tc_carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
-    (void)d;
-    (void)k;
-    carve_assign(ws, n, b);
+    carve_assign(ws, n, d, k, b);
 }
 
 int tc_clear_status(const TcBuffers &b, cudaStream_t s) {
     // err is the last of the words
-    KM_CUDA(cudaMemsetAsync(b.counters, 0, (b.keep_err ? 6 : 8) * sizeof(int32_t), s));
+    // err is the last of the words before the second pass's counts
+    KM_CUDA(cudaMemsetAsync(b.counters, 0, (b.keep_err ? 6 : kTcDiagWords + 2) * sizeof(int32_t), s));
+    if (b.keep_err) KM_CUDA(cudaMemsetAsync(b.counters + kTcDiagWords, 0, 2 * sizeof(int32_t), s));
     return KM_OK;
 }
 
@@ -1885,6 +1918,184 @@ cudaError_t launch_tc_variant(const cudaLaunchConfig_t &cfg, int list_len, bool 
     return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 16, false>, tmA, tmB, p);
 }
 
+// ---------------------------------------------------------------------------
+// Frames whose candidate lists overflowed (more than L centers within the
+// rounding bound of the best).  Comparing them with every center in float32
+// was most of some assignments: 4% of 2M x 528 frames, k = 2000, took 17 of
+// 22 ms.  Their operand rows are gathered and go through the same kernel
+// again, with the threshold that the first pass ended with, which now writes
+// a bit per center that reaches it; each frame's exact distances to those
+// centers follow, 32 at a time.  There 21.96 -> 6.06 ms; 500,000 x 528 with 6%
+// such frames 8.26 -> 1.95 ms; 1M x 528, k = 1000, 1,772 frames 2.23 -> 2.02.
+// Lists of at most kWideFew frames, frames beyond the room for the copies
+// (n / 16) and frames that are not finite go to the full re-check.
+// ---------------------------------------------------------------------------
+constexpr int64_t kWideFew = 256;
+
+struct FullCounts {
+    int chunks;
+    const int32_t *count[kMaxTcChunks];  // frames listed by each chunk,
+    int64_t first[kMaxTcChunks];         // whose list starts here
+};
+
+// A warp per listed frame: its operand row into the gathered rows, or its
+// number into the list of the full re-check.
+__global__ void __launch_bounds__(256) wide_gather_kernel(
+    const FullCounts fc, int64_t n, const int32_t *__restrict__ frames, const unsigned long long *__restrict__ thr_keys,
+    const uint4 *__restrict__ xh, const float4 *__restrict__ xnorm, int row16, int64_t cap, uint4 *__restrict__ wxh,
+    float4 *__restrict__ wxnorm, float *__restrict__ wthr, int32_t *__restrict__ wframes,
+    int32_t *__restrict__ rest, unsigned long long *__restrict__ rest_keys, int32_t *__restrict__ counts) {
+    int64_t total = 0, cnt[kMaxTcChunks];
+    for (int c = 0; c < fc.chunks; ++c) {
+        cnt[c] = *fc.count[c];
+        total += cnt[c];
+    }
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
+        int64_t e = w;
+        int c = 0;
+        while (c + 1 < fc.chunks && e >= cnt[c]) e -= cnt[c++];
+        e += fc.first[c];
+        const int32_t i = frames[e];
+        const float thr = __uint_as_float((uint32_t)thr_keys[e]);
+        int slot = -1;
+        if (lane == 0 && total > kWideFew && thr == thr) slot = atomicAdd(&counts[0], 1);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (slot >= 0 && slot < cap) {
+            for (int t = lane; t < row16; t += 32) wxh[(int64_t)slot * row16 + t] = xh[(int64_t)i * row16 + t];
+            if (lane == 0) {
+                wxnorm[slot] = xnorm[i];
+                wthr[slot] = thr;
+                wframes[slot] = i;
+            }
+        } else if (lane == 0) {
+            const int q = atomicAdd(&counts[1], 1);
+            rest[q] = i;
+            rest_keys[q] = ~0ull;
+        }
+    }
+}
+
+// A warp per gathered frame: the exact distances to the centers of its bits,
+// 32 at a time (coalesced rows, squares transposed in shared memory, lane j
+// adds center j's in feature order: sqdist_exact, bit for bit), the smallest
+// (distance, center) and the label from it as in recheck_finalize_kernel.
+constexpr int kSettleWarps = 8;
+template <class Src>
+__global__ void __launch_bounds__(kSettleWarps * 32) wide_settle_kernel(
+    const Src src, int d, const float *__restrict__ C, int k, const int32_t *__restrict__ perm,
+    const int32_t *__restrict__ count, int64_t cap, const int32_t *__restrict__ frames,
+    const uint32_t *__restrict__ bits, int words, int32_t *__restrict__ labels, unsigned long long *flipped,
+    int32_t *__restrict__ flips, int32_t *__restrict__ n_flips, int64_t max_flips) {
+    __shared__ float sq_s[kSettleWarps][32][33];
+    __shared__ int32_t id_s[kSettleWarps][32 + 4 * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float(*sq)[33] = sq_s[warp];
+    int32_t *ids = id_s[warp];
+    const int64_t n = min((int64_t)*count, cap);
+    for (int64_t r = (int64_t)blockIdx.x * kSettleWarps + warp; r < n; r += (int64_t)gridDim.x * kSettleWarps) {
+        const int64_t i = frames[r];
+        const uint32_t *row = bits + r * words;
+        unsigned long long key = ~0ull;
+        auto eval = [&](int m) {
+            float acc = 0.0f;
+            for (int f0 = 0; f0 < d; f0 += 32) {
+                const int f = f0 + lane;
+                float v[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = (j < m && f < d) ? __ldg(C + (int64_t)ids[j] * d + f) : 0.0f;
+                const float x = f < d ? src.get(i, f) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sq[lane][j] = sq_term(x, v[j]);
+                __syncwarp();
+                const int run = min(32, d - f0);
+                if (run == 32) {
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) acc = __fadd_rn(acc, sq[q][lane]);
+                } else {
+                    for (int q = 0; q < run; ++q) acc = __fadd_rn(acc, sq[q][lane]);
+                }
+                __syncwarp();
+            }
+            if (lane < m) {
+                const unsigned long long kk = ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)ids[lane];
+                key = kk < key ? kk : key;
+            }
+            __syncwarp();
+        };
+        bool any = false;  // some center reached the threshold (the best one does; else all are compared)
+        for (int w0 = lane; w0 < words; w0 += 32) any |= row[w0] != 0u;
+        any = __any_sync(0xffffffffu, any);
+        int cnt = 0;
+        for (int w0 = 0; w0 < words; w0 += 4) {
+            uint32_t b = lane < 4 && w0 + lane < words ? (any ? row[w0 + lane] : ~0u) : 0u;
+            const int c = __popc(b);
+            int ex = c;
+#pragma unroll
+            for (int off = 1; off < 4; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, ex, off);
+                if (lane >= off) ex += y;
+            }
+            const int add = __shfl_sync(0xffffffffu, ex, 3);
+            if (add == 0) continue;
+            int at = cnt + ex - c;
+            while (b) {
+                const int j = (w0 + lane) * 32 + __ffs(b) - 1;
+                b &= b - 1u;
+                ids[at++] = j < k ? (perm ? perm[j] : j) : 0;  // (rows beyond k never reach it)
+            }
+            cnt += add;
+            __syncwarp();
+            while (cnt >= 32) {
+                eval(32);
+                cnt -= 32;
+                int32_t keep[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) keep[q] = 32 * q + lane < cnt ? ids[32 + 32 * q + lane] : 0;
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ids[32 * q + lane] = keep[q];
+                __syncwarp();
+            }
+        }
+        if (cnt > 0) eval(cnt);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, off);
+            key = o < key ? o : key;
+        }
+        if (lane == 0) {
+            const int lbl = (uint32_t)(key >> 32) < 0x7f800000u ? (int)(uint32_t)key : 0;
+            const int before = labels[i];
+            if (before != lbl) {
+                atomicAdd(flipped, 1ull);
+                if (flips) {
+                    const int slot = atomicAdd(n_flips, 1);
+                    if (slot < max_flips) {
+                        flips[3 * (int64_t)slot] = (int32_t)i;
+                        flips[3 * (int64_t)slot + 1] = before;
+                        flips[3 * (int64_t)slot + 2] = lbl;
+                    }
+                } else {
+                    labels[i] = lbl;
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <class Src>
+int launch_wide_settle(const Src &src, int d, const float *C, int k, const TcBuffers &b, int words, int32_t *labels,
+                       cudaStream_t s, const FlipList *fl) {
+    wide_settle_kernel<Src><<<(unsigned)num_sms() * 4, kSettleWarps * 32, 0, s>>>(
+        src, d, C, k, b.perm, b.wide_counts, b.wide_cap, b.wide_frames, b.wide_bits, words, labels,
+        b.flipped, fl ? fl->rows : nullptr, fl ? fl->count : nullptr, fl ? fl->cap : 0);
+    KM_CUDA(cudaGetLastError());
+    return KM_OK;
+}
+
 int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int32_t *labels, TcBuffers &b,
                    cudaStream_t s, ProfEvents *prof, float *dump, unsigned long long *wait_cycles, cudaStream_t side,
                    const cudaEvent_t *ev_fork, int n_fork, const FlipList *fl, const PairSrc *ps,
@@ -1995,6 +2206,18 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     p.unit_mask = b.unit_mask;
     p.ub = b.ub;
     p.tile_lo = tile_lo;
+    p.n_dev = nullptr;
+    p.row_thr = nullptr;
+    p.bits = nullptr;
+    p.bit_words = p.n_ctiles * p.bn / 32;
+    // The launches of the second pass cost about 10 us when no list overflows
+    // (250,007 x 1,023, k = 777 922 -> 933 us; 50,000 x 128, k = 500 168 ->
+    // 178, which keeps the full re-check).  KM_TC_WIDE=0 or 1 in the environment forces the choice (the
+    // labels are the same).
+    bool wide = 2.0 * (double)n * k * d >= 2e11;
+    if (const char *e = std::getenv("KM_TC_WIDE")) wide = e[0] == '1';
+    wide = wide && b.wide_cap > 0 && !b.fp8 && !dump && !wait_cycles && !tile_lo;
+    p.full_thr = wide;
     set_lists(p, b);
     p.err = b.err;
     p.dump = dump;
@@ -2046,14 +2269,14 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     }
     // Frames one launch takes in one round of units over all its CTAs.
     const int64_t wave = pl.pair ? 2 * kBM * (int64_t)clusters_fit : kBM * (int64_t)num_sms();
-    auto launch_pass = [&](const TcParams &q) -> int {
+    auto launch_pass = [&](const TcParams &q, const CUtensorMap &tmF, cudaStream_t st) -> int {
         const int64_t rows = q.n - q.frame0;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
         int na = 0;
         cfg.blockDim = dim3(kThreadsTC, 1, 1);
         cfg.dynamicSmemBytes = (size_t)pl.smem;
-        cfg.stream = s;
+        cfg.stream = st;
         cfg.attrs = attr;
         if (pl.pair) {
             attr[na].id = cudaLaunchAttributeClusterDimension;
@@ -2077,13 +2300,13 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
             ++na;
         }
         cfg.numAttrs = na;
-        KM_CUDA(pl.pair ? launch_tc_variant<true>(cfg, pl.list_len, b.fp8 != 0, tmA, tmB, q)
-                        : launch_tc_variant<false>(cfg, pl.list_len, b.fp8 != 0, tmA, tmB, q));
+        KM_CUDA(pl.pair ? launch_tc_variant<true>(cfg, pl.list_len, b.fp8 != 0, tmF, tmB, q)
+                        : launch_tc_variant<false>(cfg, pl.list_len, b.fp8 != 0, tmF, tmB, q));
         KM_CUDA(cudaGetLastError());
         return KM_OK;
     };
 
-    if (tile_lo) return launch_pass(p);
+    if (tile_lo) return launch_pass(p, tmA, s);
 
     // Each chunk: the tensor-core launch on s, then its exact re-checks on s,
     // or on `side` beside the next chunk (and, after the last chunk, beside
@@ -2104,7 +2327,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         const int64_t f1 = q.n;
         f_next = f1;
         set_lists(q, v);
-        KM_TRY(launch_pass(q));
+        KM_TRY(launch_pass(q, tmA, s));
         if (prof && c + 1 == n_chunks) prof->end(kProfTc, s);
         if (side) {
             KM_CUDA(cudaEventRecord(ev_fork[c], s));
@@ -2117,12 +2340,53 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         KM_TRY(launch_recheck_pairs(X, d, C, v.rc_frames, v.rc_best, v.rc_pairs, v.pair_center, v.pair_lo,
                                     v.rc_keys, v.amb_entries, v.amb_mask, v.counters, f1 - f0, labels, b.flipped, r,
                                     fl, per_sm, ps));
-        if (n_chunks > 1)
+        if (n_chunks > 1 && !wide)
             KM_TRY(launch_full_recheck(X, v.full_frames, v.counters + 1, f1 - f0, d, C, k, v.full_keys, labels,
                                        b.flipped, r, fl, ps));
     }
     if (prof) prof->end(kProfRecheck, r);
-    if (n_chunks == 1) {
+    if (wide) {
+        if (prof) prof->begin(kProfFull, r);
+        FullCounts fc = {};
+        fc.chunks = n_chunks;
+        int64_t f0 = 0;
+        for (int c = 0; c < n_chunks; ++c) {
+            TcBuffers v;
+            chunk_lists(b, f0, c, v);
+            fc.count[c] = v.counters + 1;
+            fc.first[c] = f0;
+            if (c + 1 < n_chunks) f0 = std::min(n, std::max(f0 + 256, chunk_first(n, n_chunks, c + 1, wave)));
+        }
+        // (the candidate lists' frames and keys are free again)
+        wide_gather_kernel<<<(unsigned)num_sms() * 2, 256, 0, r>>>(
+            fc, n, b.full_frames, b.full_keys, static_cast<const uint4 *>(b.xh), b.xnorm, b.kp / 8, b.wide_cap,
+            static_cast<uint4 *>(b.wide_xh), b.wide_xnorm, b.wide_thr, b.wide_frames, b.rc_frames, b.rc_keys,
+            b.wide_counts);
+        KM_CUDA(cudaGetLastError());
+        CUtensorMap tmW;
+        KM_TRY(make_map(&tmW, b.wide_xh, b.wide_cap, b.kp, kBM, b, CU_TENSOR_MAP_SWIZZLE_128B));
+        TcParams q = p;
+        q.frame0 = 0;
+        q.n = b.wide_cap;
+        q.n_dev = b.wide_counts;
+        q.xnorm = b.wide_xnorm;
+        q.row_thr = b.wide_thr;
+        q.bits = b.wide_bits;
+        q.labels = nullptr;
+        q.label_counts = nullptr;
+        q.seed_xh = nullptr;
+        q.unit_mask = nullptr;
+        q.ub = nullptr;
+        KM_TRY(launch_pass(q, tmW, r));
+        if (ps)
+            KM_TRY(launch_wide_settle(PairRows{ps->xyz, reinterpret_cast<const int2 *>(ps->pairs), ps->n_atoms, d}, d,
+                                      C, k, b, p.bit_words, labels, r, fl));
+        else
+            KM_TRY(launch_wide_settle(DenseRows{X, d}, d, C, k, b, p.bit_words, labels, r, fl));
+        KM_TRY(launch_full_recheck(X, b.rc_frames, b.wide_counts + 1, n, d, C, k, b.rc_keys, labels, b.flipped, r, fl,
+                                   ps));
+        if (prof) prof->end(kProfFull, r);
+    } else if (n_chunks == 1) {
         if (prof) prof->begin(kProfFull, r);
         KM_TRY(launch_full_recheck(X, b.full_frames, b.counters + 1, n, d, C, k, b.full_keys, labels, b.flipped, r,
                                    fl, ps));

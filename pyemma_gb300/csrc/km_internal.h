@@ -217,6 +217,14 @@ struct TcBuffers {
     int32_t *counters = nullptr;  // [0] recheck entries, [1] full entries, [2] pairs, [3] unsettled entries
     unsigned long long *flipped = nullptr;
     uint32_t *err = nullptr;
+    // frames whose lists overflowed, taken a second time (wide_cap = 0: not)
+    void *wide_xh = nullptr;
+    float4 *wide_xnorm = nullptr;
+    float *wide_thr = nullptr;
+    int32_t *wide_frames = nullptr;
+    uint32_t *wide_bits = nullptr;
+    int32_t *wide_counts = nullptr;  // frames taken again (may exceed wide_cap), frames of the full re-check
+    int64_t wide_cap = 0;
     void *sch = nullptr;         // narrow frames (assign_small.cu): split FP16 operand rows of the centers
     float *scg = nullptr;        // narrow frames: the centers by groups of eight, [group][feature][8]
     float *chn = nullptr;        // FP8 only: -||c~_j||^2 / 2 per center (the norm is not folded into the GEMM)
