@@ -354,11 +354,15 @@ int km_pair_distances(const float *xyz, int64_t n, int32_t n_atoms, const int32_
  * atom pairs (device, d x 2 int32, every index in [0, n_atoms), checked on
  * the host after a read-back of the d x 2 table), and every kernel that
  * needs a float32 feature computes it where it reads it, with the
- * arithmetic of km_pair_distances, so no n x d feature matrix is ever
- * written.  Results equal km_assign / km_lloyd / km_kmpp on the output of
+ * arithmetic of km_pair_distances, so no n x d feature matrix has to be
+ * written.  (km_lloyd_pairs with max_iter >= 2 does write the float32
+ * features, once, where its workspace has the room that
+ * km_lloyd_pairs_workspace_size asks for: up to 2 GiB of them.  With the
+ * workspace of km_lloyd_workspace_size it computes them in every iteration.)
+ * Results equal km_assign / km_lloyd / km_kmpp on the output of
  * km_pair_distances, bit for bit (labels, kmeans++ draws) or to the
- * rounding of the float64 centroid sums (centers, inertia).  Workspaces are
- * those of the dense calls with the same n, d, k.  KM_PREC_FP8 is not built
+ * rounding of the float64 centroid sums (centers, inertia).  The other
+ * workspaces are those of the dense calls with the same n, d, k.  KM_PREC_FP8 is not built
  * for coordinate frames (KM_ERR_UNSUPPORTED). */
 size_t km_assign_pairs_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision);
 int km_assign_pairs(const float *xyz, int64_t n, int32_t n_atoms, const int32_t *pairs, int32_t d, const float *C,

@@ -725,7 +725,11 @@ def lloyd_pairs(xyz, pairs, C, max_iter, tolerance, precision="auto", callback=N
     n_iter = ctypes.c_int32(0)
     conv = ctypes.c_int32(0)
     ws_bytes = L.km_lloyd_pairs_workspace_size(n, d, k, p)
-    ws = _workspace(torch, ws_bytes, xyz.device)
+    try:
+        ws = _workspace(torch, ws_bytes, xyz.device)
+    except torch.OutOfMemoryError:  # without room for the features, which are then computed where they are read
+        ws_bytes = L.km_lloyd_workspace_size(n, d, k, p)
+        ws = _workspace(torch, ws_bytes, xyz.device)
     cb, keep = _callback(callback)
     check(L.km_lloyd_pairs(_ptr(xyz), n, n_atoms, _ptr(pairs), d, k, _ptr(C), int(max_iter), float(tolerance), p,
                            _ptr(labels), inertias.ctypes.data_as(ctypes.c_void_p), ctypes.byref(n_iter),

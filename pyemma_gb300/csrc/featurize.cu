@@ -46,6 +46,17 @@ __global__ void __launch_bounds__(256) pair_distances_kernel(const float *__rest
 
 }  // namespace
 
+int launch_pair_distances(const float *xyz, int64_t n, int n_atoms, const int32_t *pairs, int npairs, float *out,
+                          cudaStream_t s) {
+    int64_t g = (n * 32 + 255) / 256;  // a warp per frame
+    const int64_t cap = (int64_t)num_sms() * 16;
+    if (g > cap) g = cap;
+    pair_distances_kernel<<<(unsigned)g, 256, 0, s>>>(xyz, n, n_atoms, reinterpret_cast<const int2 *>(pairs), npairs,
+                                                      out);
+    KM_CUDA(cudaGetLastError());
+    return KM_OK;
+}
+
 // Atom pairs (device, npairs x 2) are read back (a few KB) and checked on the
 // host: an index outside [0, n_atoms) would make every kernel that computes
 // the features read outside the coordinates.
@@ -77,13 +88,7 @@ int km_pair_distances(const float *xyz, int64_t n, int32_t n_atoms, const int32_
     const int64_t total = n * (int64_t)npairs;
     if (total == 0) return KM_OK;
     KM_TRY(check_pairs(pairs, npairs, n_atoms, static_cast<cudaStream_t>(stream)));
-    int64_t g = (n * 32 + 255) / 256;  // a warp per frame
-    const int64_t cap = (int64_t)num_sms() * 16;
-    if (g > cap) g = cap;
-    pair_distances_kernel<<<(unsigned)g, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        xyz, n, n_atoms, reinterpret_cast<const int2 *>(pairs), npairs, out);
-    KM_CUDA(cudaGetLastError());
-    return KM_OK;
+    return launch_pair_distances(xyz, n, n_atoms, pairs, npairs, out, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -15,7 +15,8 @@ namespace km {
 // Frames given as atom coordinates: feature f of frame i is the distance
 // between atoms pairs[2f] and pairs[2f+1] of xyz[i] (device arrays).  The
 // launchers below take a nullable PairSrc; when it is set, X is ignored and
-// every float32 feature is computed from the coordinates where it is read.
+// every float32 feature is computed from the coordinates where it is read
+// (Lloyd runs write them once instead where they have the room: capi.cu).
 struct PairSrc {
     const float *xyz = nullptr;   // (n, n_atoms, 3)
     const int32_t *pairs = nullptr;  // (d, 2)
@@ -25,6 +26,9 @@ struct PairSrc {
 // featurize.cu: KM_ERR_BAD_SHAPE unless every atom index of the pairs (device,
 // npairs x 2) lies in [0, n_atoms); synchronises s.
 int check_pairs(const int32_t *pairs, int32_t npairs, int32_t n_atoms, cudaStream_t s);
+// The features of checked pairs, (n, npairs) at out.
+int launch_pair_distances(const float *xyz, int64_t n, int n_atoms, const int32_t *pairs, int npairs, float *out,
+                          cudaStream_t s);
 
 // ---- profiling (capi.cu) ------------------------------------------------------
 // Event pairs recorded around the main kernels of one pass when profiling is

@@ -51,7 +51,7 @@ def ca_distances(xyz, excluded_neighbors=2, pairs=None):
 
 
 class PairDistanceFrames(object):
-    """Atom-pair distance features that are never written out.
+    """Atom-pair distance features that need not be written out.
 
     Holds the coordinates (T, n_atoms, 3) and the atom pairs on the device.
     cluster_kmeans, KmeansClustering.estimate, assign_to_centers and the
@@ -59,7 +59,9 @@ class PairDistanceFrames(object):
     (T, n_pairs) feature array: the kernels compute every feature where they
     read it (km_assign_pairs, km_lloyd_pairs, km_kmpp_pairs), with the
     float32 arithmetic of ca_distances, so the results equal those on
-    ca_distances(xyz) and no T x n_pairs matrix is allocated.
+    ca_distances(xyz) and no T x n_pairs matrix is allocated (Lloyd runs of two
+    and more iterations hold one in their workspace up to 2 GiB, if there is
+    memory for it).
     """
 
     def __init__(self, xyz, pairs):
