@@ -128,6 +128,7 @@ struct TcParams {
     const int32_t *inv;
     const uint32_t *unit_mask;
     float *ub;
+    const float *drift;  // ub and the labels are of the last iteration, whose centers have moved by up to this
     float *tile_lo;
     // Frames whose lists overflowed, a second time: *n_dev of them, the
     // threshold each ended with, and instead of labels a bit per operand row
@@ -811,7 +812,10 @@ __device__ __forceinline__ float hi_bound(float v, float E, float R, float g_hi)
 // operands (128 elements per 128-byte chunk, kind::f8f6f4); the epilogue
 // turns the accumulator into a_j = acc_j / (s_i t) - ||c~_j||^2 / 2 with the
 // frame's scale s_i and the centers' t, in unscaled units.
-template <bool PAIR, int L, bool F8>
+// AUX: the pass fills tile_lo or bits (TcParams) instead of labels; a form of
+// its own, because a few more instructions per 32 columns cost the epilogue of
+// short rows 12% (2M x 64, k = 2000).
+template <bool PAIR, int L, bool F8, bool AUX>
 __global__ void __launch_bounds__(kThreadsTC, 1)
     tc_assign_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const TcParams p) {
@@ -846,11 +850,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     // Frame units: 128 frames per CTA; a pair takes 256 consecutive frames,
     // its rank-r CTA the r-th half.
     const int64_t unit = PAIR ? 2 * kBM : kBM;
-    const int64_t n_end = p.n_dev ? min((int64_t)*p.n_dev, p.n) : p.n;
+    const int64_t n_end = AUX && p.n_dev ? min((int64_t)*p.n_dev, p.n) : p.n;
     const int64_t n_units = (n_end - p.frame0 + unit - 1) / unit;
     const int64_t unit0 = PAIR ? blockIdx.x / 2 : blockIdx.x;
     const int64_t unit_stride = PAIR ? gridDim.x / 2 : gridDim.x;
-    if (unit0 >= n_units) return;  // both CTAs of a pair; only where the count is the device's
+    if (AUX && unit0 >= n_units) return;  // both CTAs of a pair; only where the count is the device's
     // The center tiles of a unit: all of them, or the set bits of its mask.
     const uint32_t *masks = p.unit_mask ? p.unit_mask + p.frame0 / unit : nullptr;
 
@@ -1141,16 +1145,27 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 la[m] = kNegInf;
                 lid[m] = -1;
             }
-            if (p.tile_lo) thr = kInf;  // no candidates
-            if (p.bits) {
-                best = kInf;  // the threshold stays
-                thr = i < n_end ? p.row_thr[i] : kInf;
+            if (!AUX && p.drift && i < n_end) {
+                // The frame's last center is still within u, so its
+                // accumulator is at least this, and the largest one too: a
+                // seed as above, without the rows.
+                const float u = __fadd_ru(__fadd_ru(p.ub[i], p.drift[p.labels[i]]), Rmax);
+                const float v = __fmul_ru(__fadd_ru(__fmul_ru(u, u), Emax), s2);
+                const float seed = __fmul_rd(0.5f, __fsub_rd(xn.x, v));
+                if (seed > best && seed < kInf) {
+                    best = seed;
+                    thr = window_threshold(best, xn.x, inv_s2, s2, Emax, Rmax, Rpad, p.g_ratio);
+                }
+            }
+            if (AUX) {
+                best = kInf;  // the threshold stays; in tile_lo's form none is reached
+                thr = p.bits && i < n_end ? p.row_thr[i] : kInf;
             }
             uint32_t todo = masks ? masks[ft] : 0u;
             const int n_ct = masks ? __popc(todo) : p.n_ctiles;
             for (int q = 0; q < n_ct; ++q, todo &= todo - 1u) {
                 const int ct = masks ? __ffs(todo) - 1 : q;
-                float top = kNegInf;  // the largest accumulator of the tile
+                [[maybe_unused]] float top = kNegInf;  // the largest accumulator of the tile
                 const uint32_t buf = accq & 1u;
                 const bool got = __all_sync(0xffffffffu, mbar_wait_timed(&acc_full[buf], (accq >> 1) & 1u, pw_acc));
                 if (!got) {
@@ -1202,8 +1217,8 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     const float m4c = max3f(m12[6], m12[7], m12[8]);
                     const float m4d = max3f(m12[9], m12[10], m12[11]);
                     const float mx = fmaxf(max3f(m4a, m4b, m4c), m4d);
-                    top = fmaxf(top, mx);
                     uint32_t reach = 0u;
+                    if (AUX) top = fmaxf(top, mx);
                     if (mx >= thr && mx > kNegInf) {
                         if (mx > best) {
                             best = mx;
@@ -1220,7 +1235,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         unsigned msk = (mk[0] | mk[1]) | (mk[2] | mk[3]);
                         const int nv = p.k - j0;
                         if (nv < 32) msk &= nv > 0 ? (1u << nv) - 1u : 0u;
-                        if (p.bits) {
+                        if (AUX) {
                             reach = msk;
                             msk = 0u;
                         }
@@ -1251,7 +1266,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                             lid[0] = j0 + c;
                         }
                     }
-                    if (p.bits && i < n_end) p.bits[i * p.bit_words + (j0 >> 5)] = reach;
+                    if (AUX && p.bits && i < n_end) p.bits[i * p.bit_words + (j0 >> 5)] = reach;
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -1262,7 +1277,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         mbar_arrive(&acc_empty[buf]);
                 }
                 ++accq;
-                if (p.tile_lo && i < n_end) {
+                if (AUX && p.tile_lo && i < n_end) {
                     // sqrt(v - E) - R of the nearest one; 0 (no bound) unless finite
                     const float v = fmaf(-2.0f, top, xn.x) * inv_s2;
                     const float lo = __fsub_rd(__fsqrt_rd(fmaxf(__fsub_rd(v, Emax), 0.0f)), Rmax);
@@ -1270,7 +1285,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 }
             }
             if (!ok) break;
-            if (p.tile_lo || p.bits) {
+            if (AUX) {
                 if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
                 continue;
             }
@@ -1724,6 +1739,8 @@ size_t carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
         b.wide_frames = c.take<int32_t>(b.wide_cap);
         b.wide_bits = c.take<uint32_t>((size_t)b.wide_cap * (k_pad_of(k) / 32 + 8));
         b.wide_counts = b.counters + kTcDiagWords;
+        b.rest_frames = c.take<int32_t>(nn);
+        b.rest_keys = c.take<unsigned long long>(nn);
     }
     return c.bytes();
 }
@@ -1913,9 +1930,10 @@ void set_lists(TcParams &p, const TcBuffers &v) {
 template <bool PAIR>
 cudaError_t launch_tc_variant(const cudaLaunchConfig_t &cfg, int list_len, bool fp8, const CUtensorMap &tmA,
                               const CUtensorMap &tmB, const TcParams &p) {
-    if (fp8) return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 16, true>, tmA, tmB, p);
-    if (list_len == 8) return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 8, false>, tmA, tmB, p);
-    return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 16, false>, tmA, tmB, p);
+    if (p.tile_lo || p.bits) return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 8, false, true>, tmA, tmB, p);
+    if (fp8) return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 16, true, false>, tmA, tmB, p);
+    if (list_len == 8) return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 8, false, false>, tmA, tmB, p);
+    return cudaLaunchKernelEx(&cfg, tc_assign_kernel<PAIR, 16, false, false>, tmA, tmB, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -2113,24 +2131,26 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         const int dev = current_device();
         std::lock_guard<std::mutex> lk(attr_mu);
         if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
-            const void *fns[6] = {(const void *)tc_assign_kernel<false, 16, false>,
-                                  (const void *)tc_assign_kernel<true, 16, false>,
-                                  (const void *)tc_assign_kernel<false, 8, false>,
-                                  (const void *)tc_assign_kernel<true, 8, false>,
-                                  (const void *)tc_assign_kernel<false, 16, true>,
-                                  (const void *)tc_assign_kernel<true, 16, true>};
+            const void *fns[8] = {(const void *)tc_assign_kernel<false, 8, false, true>,
+                                  (const void *)tc_assign_kernel<true, 8, false, true>,
+                                  (const void *)tc_assign_kernel<false, 16, false, false>,
+                                  (const void *)tc_assign_kernel<true, 16, false, false>,
+                                  (const void *)tc_assign_kernel<false, 8, false, false>,
+                                  (const void *)tc_assign_kernel<true, 8, false, false>,
+                                  (const void *)tc_assign_kernel<false, 16, true, false>,
+                                  (const void *)tc_assign_kernel<true, 16, true, false>};
             for (const void *f : fns)
                 KM_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
             if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
         }
     }
     // (the FP8 kernel keeps 16 candidates: make_plan set list_len)
-    const void *kfn = b.fp8 ? (pl.pair ? (const void *)tc_assign_kernel<true, 16, true>
-                                       : (const void *)tc_assign_kernel<false, 16, true>)
-                            : pl.pair ? (pl.list_len == 8 ? (const void *)tc_assign_kernel<true, 8, false>
-                                                          : (const void *)tc_assign_kernel<true, 16, false>)
-                                      : (pl.list_len == 8 ? (const void *)tc_assign_kernel<false, 8, false>
-                                                          : (const void *)tc_assign_kernel<false, 16, false>);
+    const void *kfn = b.fp8 ? (pl.pair ? (const void *)tc_assign_kernel<true, 16, true, false>
+                                       : (const void *)tc_assign_kernel<false, 16, true, false>)
+                            : pl.pair ? (pl.list_len == 8 ? (const void *)tc_assign_kernel<true, 8, false, false>
+                                                          : (const void *)tc_assign_kernel<true, 16, false, false>)
+                                      : (pl.list_len == 8 ? (const void *)tc_assign_kernel<false, 8, false, false>
+                                                          : (const void *)tc_assign_kernel<false, 16, false, false>);
 
     CUtensorMap tmA, tmB;
     KM_TRY(make_map(&tmA, b.xh, n, b.kp, kBM, b, CU_TENSOR_MAP_SWIZZLE_128B));
@@ -2191,7 +2211,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     // k = 1000, four tiles: no gain, and 2.5% slower at d = 10).
     // KM_TC_SEED=0 or 1 in the environment forces the choice for 16-bit
     // operands (both give the same labels).
-    bool seed = !b.fp8 && b.kp <= 128 && k >= 2048;
+    bool seed = !b.fp8 && b.kp <= 128 && k >= 2048 && !(b.ub && b.drift);
     if (const char *e = std::getenv("KM_TC_SEED")) seed = !b.fp8 && e[0] == '1';
     seed = seed && !tile_lo;
     p.seed_xh = seed ? b.xh : nullptr;
@@ -2205,6 +2225,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     p.inv = b.inv;
     p.unit_mask = b.unit_mask;
     p.ub = b.ub;
+    p.drift = b.ub ? b.drift : nullptr;
     p.tile_lo = tile_lo;
     p.n_dev = nullptr;
     p.row_thr = nullptr;
@@ -2308,6 +2329,44 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
 
     if (tile_lo) return launch_pass(p, tmA, s);
 
+    // The frames whose lists overflowed, of all chunks: gathered and passed a
+    // second time on s, before the caller's next work takes the SMs (beside
+    // the segment sums the pass would wait for their end: 2M x 64, k = 2000,
+    // 0.11 ms per iteration with nothing to do).
+    auto second_pass = [&]() -> int {
+        FullCounts fc = {};
+        fc.chunks = n_chunks;
+        int64_t f0 = 0;
+        for (int c = 0; c < n_chunks; ++c) {
+            TcBuffers v;
+            chunk_lists(b, f0, c, v);
+            fc.count[c] = v.counters + 1;
+            fc.first[c] = f0;
+            if (c + 1 < n_chunks) f0 = std::min(n, std::max(f0 + 256, chunk_first(n, n_chunks, c + 1, wave)));
+        }
+        wide_gather_kernel<<<(unsigned)num_sms() * 2, 256, 0, s>>>(
+            fc, n, b.full_frames, b.full_keys, static_cast<const uint4 *>(b.xh), b.xnorm, b.kp / 8, b.wide_cap,
+            static_cast<uint4 *>(b.wide_xh), b.wide_xnorm, b.wide_thr, b.wide_frames, b.rest_frames, b.rest_keys,
+            b.wide_counts);
+        KM_CUDA(cudaGetLastError());
+        CUtensorMap tmW;
+        KM_TRY(make_map(&tmW, b.wide_xh, b.wide_cap, b.kp, kBM, b, CU_TENSOR_MAP_SWIZZLE_128B));
+        TcParams w = p;
+        w.frame0 = 0;
+        w.n = b.wide_cap;
+        w.n_dev = b.wide_counts;
+        w.xnorm = b.wide_xnorm;
+        w.row_thr = b.wide_thr;
+        w.bits = b.wide_bits;
+        w.labels = nullptr;
+        w.label_counts = nullptr;
+        w.seed_xh = nullptr;
+        w.unit_mask = nullptr;
+        w.drift = nullptr;
+        w.ub = nullptr;
+        return launch_pass(w, tmW, s);
+    };
+
     // Each chunk: the tensor-core launch on s, then its exact re-checks on s,
     // or on `side` beside the next chunk (and, after the last chunk, beside
     // the caller's next work).  Beside the centroid update the re-check keeps
@@ -2328,6 +2387,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
         f_next = f1;
         set_lists(q, v);
         KM_TRY(launch_pass(q, tmA, s));
+        if (wide && c + 1 == n_chunks) KM_TRY(second_pass());
         if (prof && c + 1 == n_chunks) prof->end(kProfTc, s);
         if (side) {
             KM_CUDA(cudaEventRecord(ev_fork[c], s));
@@ -2347,44 +2407,13 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     if (prof) prof->end(kProfRecheck, r);
     if (wide) {
         if (prof) prof->begin(kProfFull, r);
-        FullCounts fc = {};
-        fc.chunks = n_chunks;
-        int64_t f0 = 0;
-        for (int c = 0; c < n_chunks; ++c) {
-            TcBuffers v;
-            chunk_lists(b, f0, c, v);
-            fc.count[c] = v.counters + 1;
-            fc.first[c] = f0;
-            if (c + 1 < n_chunks) f0 = std::min(n, std::max(f0 + 256, chunk_first(n, n_chunks, c + 1, wave)));
-        }
-        // (the candidate lists' frames and keys are free again)
-        wide_gather_kernel<<<(unsigned)num_sms() * 2, 256, 0, r>>>(
-            fc, n, b.full_frames, b.full_keys, static_cast<const uint4 *>(b.xh), b.xnorm, b.kp / 8, b.wide_cap,
-            static_cast<uint4 *>(b.wide_xh), b.wide_xnorm, b.wide_thr, b.wide_frames, b.rc_frames, b.rc_keys,
-            b.wide_counts);
-        KM_CUDA(cudaGetLastError());
-        CUtensorMap tmW;
-        KM_TRY(make_map(&tmW, b.wide_xh, b.wide_cap, b.kp, kBM, b, CU_TENSOR_MAP_SWIZZLE_128B));
-        TcParams q = p;
-        q.frame0 = 0;
-        q.n = b.wide_cap;
-        q.n_dev = b.wide_counts;
-        q.xnorm = b.wide_xnorm;
-        q.row_thr = b.wide_thr;
-        q.bits = b.wide_bits;
-        q.labels = nullptr;
-        q.label_counts = nullptr;
-        q.seed_xh = nullptr;
-        q.unit_mask = nullptr;
-        q.ub = nullptr;
-        KM_TRY(launch_pass(q, tmW, r));
         if (ps)
             KM_TRY(launch_wide_settle(PairRows{ps->xyz, reinterpret_cast<const int2 *>(ps->pairs), ps->n_atoms, d}, d,
                                       C, k, b, p.bit_words, labels, r, fl));
         else
             KM_TRY(launch_wide_settle(DenseRows{X, d}, d, C, k, b, p.bit_words, labels, r, fl));
-        KM_TRY(launch_full_recheck(X, b.rc_frames, b.wide_counts + 1, n, d, C, k, b.rc_keys, labels, b.flipped, r, fl,
-                                   ps));
+        KM_TRY(launch_full_recheck(X, b.rest_frames, b.wide_counts + 1, n, d, C, k, b.rest_keys, labels, b.flipped, r,
+                                   fl, ps));
         if (prof) prof->end(kProfFull, r);
     } else if (n_chunks == 1) {
         if (prof) prof->begin(kProfFull, r);
@@ -2523,6 +2552,19 @@ __global__ void __launch_bounds__(256) center_drift_kernel(const float *__restri
     if (lane == 0) drift[j] = __fadd_ru(__fsqrt_ru(__fmul_ru(acc, inflate)), 1e-30f);
 }
 
+// Distinct labels of 256 consecutive frames, summed over gridDim.x samples.
+__global__ void __launch_bounds__(256) distinct_labels_kernel(int64_t n, int k, const int32_t *__restrict__ labels,
+                                                              unsigned long long *__restrict__ sum) {
+    __shared__ uint32_t seen[kMaxMaskTiles * 256 / 32];
+    for (int w = threadIdx.x; w < (k + 31) / 32; w += 256) seen[w] = 0u;
+    __syncthreads();
+    const int64_t i = (n - 256) * blockIdx.x / gridDim.x + threadIdx.x;
+    const int a = labels[i];
+    const uint32_t bit = 1u << (a & 31);
+    const int found = __syncthreads_count((atomicOr(&seen[a >> 5], bit) & bit) == 0u);
+    if (threadIdx.x == 0) atomicAdd(sum, (unsigned long long)found);
+}
+
 // One CTA per frame unit, a thread per frame.
 __global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int n_ct, int bn,
                                                         const int32_t *__restrict__ labels,
@@ -2530,8 +2572,7 @@ __global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int
                                                         const float *__restrict__ drift,
                                                         const int32_t *__restrict__ inv,
                                                         const float *__restrict__ tile_lo, float factor,
-                                                        uint32_t *__restrict__ mask,
-                                                        unsigned long long *__restrict__ bits) {
+                                                        uint32_t *__restrict__ mask) {
     __shared__ uint32_t any;
     if (threadIdx.x == 0) any = 0u;
     __syncthreads();
@@ -2548,17 +2589,20 @@ __global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int
     m = __reduce_or_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0 && m) atomicOr(&any, m);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        mask[blockIdx.x] = any;
-        if (bits) atomicAdd(bits, (unsigned long long)__popc(any));
-    }
+    if (threadIdx.x == 0) mask[blockIdx.x] = any;
 }
 
 }  // namespace
 
-// Worth asking for from 4e11 flop per pass on (0.3 ms; the order and the first
-// masks cost about 0.15 ms once, and the masks are used only where they leave
-// out a quarter of the tiles).  KM_TC_BOUNDS=0 or 1 in the environment forces
+// Worth it from 4e11 flop per pass on (0.3 ms): the order costs about 0.1 ms
+// once and the masks 0.05 ms per iteration.  They are made where 256
+// neighbouring frames have at most half of the different labels that frames in
+// no order would have (tc_bounds_neighbours: 0.02-0.15 for trajectories, 0.87
+// and more for shuffled mixtures, whose masks leave nothing out); elsewhere
+// the bounds only seed the pass's thresholds.  Ten iterations, without ->
+// with: 2M x 64, k = 2000 21.8 -> 17.3 ms; 1M x 128, k = 4000 20.4 -> 13.4;
+// 400,000 x 528, k = 1000 7.5 -> 6.3; shuffled 500,000 x 300, k = 1500 9.9 ->
+// 9.6 (9.9 with masks).  KM_TC_BOUNDS=0 or 1 in the environment forces
 // the choice (the labels are the same).
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b) {
     Plan pl;
@@ -2567,6 +2611,18 @@ bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b)
     if (n_ct < 2 || n_ct > kMaxMaskTiles || max_iter < 2) return false;
     if (const char *e = std::getenv("KM_TC_BOUNDS")) return e[0] == '1';
     return max_iter >= 4 && 2.0 * (double)n * k * d >= 4e11;
+}
+
+// Labels of 256 neighbouring frames, the sum of distinct ones over samples to
+// t.bits; frames in no order would give about *random of them.
+int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, double *random, cudaStream_t s) {
+    const unsigned samples = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n / 256, 128));
+    *random = samples * (double)k * (1.0 - std::exp(-256.0 / k));
+    KM_CUDA(cudaMemsetAsync(t.bits, 0, sizeof(unsigned long long), s));
+    if (n < 256) return KM_OK;
+    distinct_labels_kernel<<<samples, 256, 0, s>>>(n, k, labels, t.bits);
+    KM_CUDA(cudaGetLastError());
+    return KM_OK;
 }
 
 bool tc_bounds_forced() {
@@ -2598,7 +2654,6 @@ int tc_bounds_order(const float *C, int d, int k, TcBuffers &b, const TcBounds &
     KM_CUDA(cudaGetLastError());
     b.perm = t.perm;
     b.inv = t.inv;
-    b.ub = t.ub;
     return KM_OK;
 }
 
@@ -2609,10 +2664,9 @@ int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBo
 }
 
 // The units' masks for centers C (whose operands are prepared), from the
-// labels, ub and drift of the last iteration; *bits (nullable, cleared here)
-// counts the tiles they hold.
+// labels, ub and drift of the last iteration.
 int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
-                    unsigned long long *bits, int64_t *units, int *tiles, cudaStream_t s) {
+                    cudaStream_t s) {
     Plan pl;
     if (!make_plan(d, k, pl, false, b.bf16 != 0)) return KM_ERR_UNSUPPORTED;
     TcBuffers v = b;
@@ -2631,12 +2685,9 @@ int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labe
     const double u = std::ldexp(1.0, -24), g = (d + 2) * u / (1.0 - (d + 2) * u) * 1.01;
     const float factor =
         std::nextafter((float)((1.0 + std::sqrt((1.0 + g) / (1.0 - g))) * (1.0 + std::ldexp(1.0, -19))), INFINITY);
-    if (bits) KM_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned long long), s));
     unit_mask_kernel<<<(unsigned)n_units, unit, 0, s>>>(n, unit, n_ct, pl.bn, labels, t.ub, t.drift, t.inv, t.tile_lo,
-                                                        factor, t.mask, bits);
+                                                        factor, t.mask);
     KM_CUDA(cudaGetLastError());
-    if (units) *units = n_units;
-    if (tiles) *tiles = n_ct;
     return KM_OK;
 }
 

@@ -1043,7 +1043,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
 
     TcBuffers b;
     TcBounds bounds;
-    bool with_bounds = false;  // the pass keeps the bounds; masked below once they are worth it
+    bool with_bounds = false;  // the pass keeps the frames' distance bounds
+    bool neighbours = false;   // neighbouring frames share centers: masks from the second iteration on
     if (tc) {
         // The shift and scale stay fixed for the whole run so that the 16-bit
         // frame copy is made once (narrow frames have none).
@@ -1057,7 +1058,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         if (is_tc(prec)) {
             tc_bounds_carve(cv.take<char>(tc_bounds_carve(nullptr, n, d, k, bounds)), n, d, k, bounds);
             with_bounds = tc_bounds_wanted(n, d, k, max_iter, b);
-            if (with_bounds) KM_TRY(tc_bounds_order(C, d, k, b, bounds, s));
+            if (with_bounds) b.ub = bounds.ub;
         }
         if (!hf && !small) KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
     }
@@ -1085,7 +1086,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         if (tc) {
             KM_TRY(small ? small_prepare_centers(C, d, k, b, st) : tc_prepare_centers(C, d, k, b, st));
             if (b.unit_mask) {
-                KM_TRY(tc_bounds_masks(C, n, d, k, labels, b, bounds, nullptr, nullptr, nullptr, st));
+                KM_TRY(tc_bounds_masks(C, n, d, k, labels, b, bounds, st));
                 b.keep_err = 1;  // cleared by the masks' pass
             }
             KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
@@ -1267,25 +1268,11 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             break;
         }
         if (it == 1 && with_bounds) {
-            // Masks on trial: kept where they leave out a quarter of the tiles.
-            unsigned long long set = 0;
-            int64_t units = 0;
-            int tiles = 0;
-            status = tc_prepare_centers(C, d, k, b, s);
-            if (status == KM_OK)
-                status = tc_bounds_masks(C, n, d, k, labels, b, bounds, bounds.bits, &units, &tiles, s);
-            if (status != KM_OK) break;
-            cudaError_t e = cudaMemcpyAsync(&set, bounds.bits, sizeof(set), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) {
-                status = cuda_fail(e, "center bounds");
-                break;
-            }
-            if (tc_bounds_forced() || (double)set <= 0.75 * (double)units * tiles)
+            b.drift = bounds.drift;
+            if (neighbours) {
+                status = tc_bounds_order(C, d, k, b, bounds, s);
+                if (status != KM_OK) break;
                 b.unit_mask = bounds.mask;
-            else {
-                with_bounds = false;
-                b.ub = nullptr;
             }
         }
         if (it == 1 && !cb && !prof.active) {
@@ -1323,8 +1310,14 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             }
         }
         if (status != KM_OK) break;
-        double h_cost = 0.0;
+        double h_cost = 0.0, random = 0.0;
         uint32_t h_err = 0, tc_err = 0;
+        unsigned long long distinct = 0;
+        if (it == 0 && with_bounds) {
+            status = tc_bounds_neighbours(n, k, labels, bounds, &random, s);
+            if (status != KM_OK) break;
+            KM_CUDA(cudaMemcpyAsync(&distinct, bounds.bits, sizeof(distinct), cudaMemcpyDeviceToHost, s));
+        }
         cudaError_t e = cudaMemcpyAsync(&h_cost, cost, sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && tc)
@@ -1335,6 +1328,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             break;
         }
         h_err |= tc_err;
+        if (it == 0) neighbours = tc_bounds_forced() || (double)distinct <= 0.5 * random;
         prof.collect();
         status = check_device_errors(h_err);
         if (status != KM_OK) break;

@@ -228,6 +228,8 @@ struct TcBuffers {
     int32_t *wide_frames = nullptr;
     uint32_t *wide_bits = nullptr;
     int32_t *wide_counts = nullptr;  // frames taken again (may exceed wide_cap), frames of the full re-check
+    int32_t *rest_frames = nullptr;  // those of the full re-check, and their keys
+    unsigned long long *rest_keys = nullptr;
     int64_t wide_cap = 0;
     void *sch = nullptr;         // narrow frames (assign_small.cu): split FP16 operand rows of the centers
     float *scg = nullptr;        // narrow frames: the centers by groups of eight, [group][feature][8]
@@ -237,6 +239,7 @@ struct TcBuffers {
     const int32_t *perm = nullptr;
     const int32_t *inv = nullptr;
     float *ub = nullptr;
+    const float *drift = nullptr;  // ub and labels of the last iteration, and what the centers have moved since
     const uint32_t *unit_mask = nullptr;
     int kp = 0;        // operand row length in elements
     int esize = 2;     // operand bytes per element: 2 (FP16, BF16) or 1 (FP8 e4m3)
@@ -275,10 +278,11 @@ struct TcBounds {
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b);
 bool tc_bounds_forced();
 size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t);  // its size with ws = nullptr
+int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, double *random, cudaStream_t s);
 int tc_bounds_order(const float *C, int d, int k, TcBuffers &b, const TcBounds &t, cudaStream_t s);
 int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBounds &t, cudaStream_t s);
 int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
-                    unsigned long long *bits, int64_t *units, int *tiles, cudaStream_t s);
+                    cudaStream_t s);
 
 // Sets the operand type of carved buffers from the precision (KM_PREC_FP16,
 // KM_PREC_BF16 or KM_PREC_FP8): element size and row length.
