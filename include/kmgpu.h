@@ -187,7 +187,9 @@ int km_update_noalloc(const float *X, int64_t n, int32_t d, const int32_t *label
 /* ---- kmeans++ initialisation: KMeans(init_strategy='kmeans++') -----------
  * kmeans.py:211-212,253; seed = fixed_seed (kmeans.py:146-164).  Writes k
  * centers into C0 (device, k*d floats) and, when idx is given (device, k
- * int64), the chosen frame indices.  cb (nullable) fires once per center. */
+ * int64), the chosen frame indices.  cb (nullable) fires once per center;
+ * without it up to 64 centers are drawn per launch.  Enqueues only: should a
+ * device-side wait run out, the centers not drawn are NaN and idx -1. */
 size_t km_kmpp_workspace_size(int64_t n, int32_t d, int32_t k);
 int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, float *C0, int64_t *idx,
             km_callback cb, void *cb_user, void *workspace, size_t workspace_bytes, void *stream);
@@ -197,7 +199,9 @@ int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, floa
  * k*d) holds the initial centers and receives the final ones.  labels
  * (device, n) receives the assignment of the last iteration.  inertias
  * (host, max_iter doubles, nullable), n_iter and converged (host) report the
- * run.  Each iteration is one CUDA-graph launch; cb fires after each. */
+ * run.  cb fires after each iteration; without it up to 64 iterations are one
+ * launch (a CUDA-graph loop, or one cooperative kernel for few, narrow
+ * centers). */
 size_t km_lloyd_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision);
 int km_lloyd(const float *X, int64_t n, int32_t d, int32_t k, float *C, int32_t max_iter,
              double tolerance, int32_t precision, int32_t *labels, double *inertias,
