@@ -1943,8 +1943,8 @@ cudaError_t launch_tc_variant(const cudaLaunchConfig_t &cfg, int list_len, bool 
 // 22 ms.  Their operand rows are gathered and go through the same kernel
 // again, with the threshold that the first pass ended with, which now writes
 // a bit per center that reaches it; each frame's exact distances to those
-// centers follow, 32 at a time.  There 21.96 -> 6.06 ms; 500,000 x 528 with 6%
-// such frames 8.26 -> 1.95 ms; 1M x 528, k = 1000, 1,772 frames 2.23 -> 2.02.
+// centers follow, 32 at a time.  There 21.96 -> 5.89 ms; 500,000 x 528 with 6%
+// such frames 8.26 -> 1.91 ms; 1M x 528, k = 1000, 1,772 frames 2.23 -> 2.02.
 // Lists of at most kWideFew frames, frames beyond the room for the copies
 // (n / 16) and frames that are not finite go to the full re-check.
 // ---------------------------------------------------------------------------
@@ -1999,6 +1999,9 @@ __global__ void __launch_bounds__(256) wide_gather_kernel(
 // 32 at a time (coalesced rows, squares transposed in shared memory, lane j
 // adds center j's in feature order: sqdist_exact, bit for bit), the smallest
 // (distance, center) and the label from it as in recheck_finalize_kernel.
+// What bounds it: the center rows from L2 and a wait per 32 features; the next
+// rows load beside the sums (2M x 528 with 4% such frames, the assignment: 5.95
+// -> 5.89 ms).
 constexpr int kSettleWarps = 8;
 template <class Src>
 __global__ void __launch_bounds__(kSettleWarps * 32) wide_settle_kernel(
@@ -2017,19 +2020,22 @@ __global__ void __launch_bounds__(kSettleWarps * 32) wide_settle_kernel(
         const uint32_t *row = bits + r * words;
         unsigned long long key = ~0ull;
         auto eval = [&](int m) {
-            float acc = 0.0f;
-            for (int f0 = 0; f0 < d; f0 += 32) {
+            float acc = 0.0f, v[32], x;
+            auto load = [&](int f0) {
                 const int f = f0 + lane;
-                float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = (j < m && f < d) ? __ldg(C + (int64_t)ids[j] * d + f) : 0.0f;
-                const float x = f < d ? src.get(i, f) : 0.0f;
+                x = f < d ? src.get(i, f) : 0.0f;
+            };
+            load(0);
+            for (int f0 = 0; f0 < d; f0 += 32) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) sq[lane][j] = sq_term(x, v[j]);
                 __syncwarp();
+                if (f0 + 32 < d) load(f0 + 32);  // on its way during the sums
                 const int run = min(32, d - f0);
                 if (run == 32) {
-#pragma unroll
+#pragma unroll 8
                     for (int q = 0; q < 32; ++q) acc = __fadd_rn(acc, sq[q][lane]);
                 } else {
                     for (int q = 0; q < run; ++q) acc = __fadd_rn(acc, sq[q][lane]);
