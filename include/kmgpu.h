@@ -109,8 +109,9 @@ int km_profile_enable(int on);
 int km_profile_read(int32_t kind, double *ms_total, int64_t *launches);
 
 /* ---- test hook (diagnostics; no reference counterpart) --------------------
- * The next km_update or km_update_noalloc call ORs `bits` into the device
- * error word it reads back, as if a kernel had set them (1, 2, 4: a
+ * The next km_update or km_update_noalloc call, or the next Lloyd iteration
+ * whose error word is read on its own (the first of a run, and every one with
+ * a callback), ORs `bits` into that word, as if a kernel had set them (1, 2, 4: a
  * device-side wait ran out; 8: a label out of range), and returns the
  * status that word maps to.  Lets tests check the mapping without making a
  * device wait run out. */

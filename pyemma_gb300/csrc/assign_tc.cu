@@ -2558,7 +2558,8 @@ __global__ void __launch_bounds__(256) center_drift_kernel(const float *__restri
     if (lane == 0) drift[j] = __fadd_ru(__fsqrt_ru(__fmul_ru(acc, inflate)), 1e-30f);
 }
 
-// Distinct labels of 256 consecutive frames, summed over gridDim.x samples.
+// Distinct labels of 256 consecutive frames, summed over gridDim.x samples
+// (labels outside [0, k) are not counted).
 __global__ void __launch_bounds__(256) distinct_labels_kernel(int64_t n, int k, const int32_t *__restrict__ labels,
                                                               unsigned long long *__restrict__ sum) {
     __shared__ uint32_t seen[kMaxMaskTiles * 256 / 32];
@@ -2567,7 +2568,8 @@ __global__ void __launch_bounds__(256) distinct_labels_kernel(int64_t n, int k, 
     const int64_t i = (n - 256) * blockIdx.x / gridDim.x + threadIdx.x;
     const int a = labels[i];
     const uint32_t bit = 1u << (a & 31);
-    const int found = __syncthreads_count((atomicOr(&seen[a >> 5], bit) & bit) == 0u);
+    const bool in = (unsigned)a < (unsigned)k;
+    const int found = __syncthreads_count(in && (atomicOr(&seen[a >> 5], bit) & bit) == 0u);
     if (threadIdx.x == 0) atomicAdd(sum, (unsigned long long)found);
 }
 
@@ -2619,21 +2621,23 @@ bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b)
     return max_iter >= 4 && 2.0 * (double)n * k * d >= 4e11;
 }
 
-// Labels of 256 neighbouring frames, the sum of distinct ones over samples to
-// t.bits; frames in no order would give about *random of them.
-int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, double *random, cudaStream_t s) {
-    const unsigned samples = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n / 256, 128));
-    *random = samples * (double)k * (1.0 - std::exp(-256.0 / k));
+// Whether neighbouring frames share centers: the distinct labels of 256
+// consecutive frames, over up to 128 samples, are at most half of what frames
+// in no order would give.  Synchronises s.
+int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, bool *neighbours,
+                         cudaStream_t s) {
+    *neighbours = true;
+    const char *e = std::getenv("KM_TC_BOUNDS");
+    if (n < 256 || (e && e[0] == '1')) return KM_OK;
+    const unsigned samples = (unsigned)std::min<int64_t>(n / 256, 128);
+    unsigned long long distinct = 0;
     KM_CUDA(cudaMemsetAsync(t.bits, 0, sizeof(unsigned long long), s));
-    if (n < 256) return KM_OK;
     distinct_labels_kernel<<<samples, 256, 0, s>>>(n, k, labels, t.bits);
     KM_CUDA(cudaGetLastError());
+    KM_CUDA(cudaMemcpyAsync(&distinct, t.bits, sizeof(distinct), cudaMemcpyDeviceToHost, s));
+    KM_CUDA(cudaStreamSynchronize(s));
+    *neighbours = (double)distinct <= 0.5 * samples * (double)k * (1.0 - std::exp(-256.0 / k));
     return KM_OK;
-}
-
-bool tc_bounds_forced() {
-    const char *e = std::getenv("KM_TC_BOUNDS");
-    return e && e[0] == '1';
 }
 
 size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t) {

@@ -466,8 +466,9 @@ int centers_d(const km_centers *h) { return h->d; }
 int centers_device(const km_centers *h) { return h->device; }
 int device_error_status(uint32_t e) { return check_device_errors(e); }
 
-// Test hook: bits that the next km_update / km_update_noalloc call adds to
-// the error word it reads back from the device, as if a kernel had set them.
+// Test hook: bits that the next km_update / km_update_noalloc call, or the
+// next Lloyd iteration checked on the host, adds to the error word it reads
+// back from the device, as if a kernel had set them.
 // It lets the tests check how each bit maps to a status without making a
 // device-side wait run out.
 static std::atomic<uint32_t> g_fake_device_error{0};
@@ -1044,7 +1045,6 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     TcBuffers b;
     TcBounds bounds;
     bool with_bounds = false;  // the pass keeps the frames' distance bounds
-    bool neighbours = false;   // neighbouring frames share centers: masks from the second iteration on
     if (tc) {
         // The shift and scale stay fixed for the whole run so that the 16-bit
         // frame copy is made once (narrow frames have none).
@@ -1269,6 +1269,11 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         }
         if (it == 1 && with_bounds) {
             b.drift = bounds.drift;
+            // Only now that the first iteration's error words are known to be
+            // clear: a pass that gave up leaves labels unwritten.
+            bool neighbours = false;  // neighbouring frames share centers
+            status = tc_bounds_neighbours(n, k, labels, bounds, &neighbours, s);
+            if (status != KM_OK) break;
             if (neighbours) {
                 status = tc_bounds_order(C, d, k, b, bounds, s);
                 if (status != KM_OK) break;
@@ -1310,14 +1315,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             }
         }
         if (status != KM_OK) break;
-        double h_cost = 0.0, random = 0.0;
+        double h_cost = 0.0;
         uint32_t h_err = 0, tc_err = 0;
-        unsigned long long distinct = 0;
-        if (it == 0 && with_bounds) {
-            status = tc_bounds_neighbours(n, k, labels, bounds, &random, s);
-            if (status != KM_OK) break;
-            KM_CUDA(cudaMemcpyAsync(&distinct, bounds.bits, sizeof(distinct), cudaMemcpyDeviceToHost, s));
-        }
         cudaError_t e = cudaMemcpyAsync(&h_cost, cost, sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && tc)
@@ -1327,8 +1326,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             status = cuda_fail(e, "Lloyd iteration");
             break;
         }
-        h_err |= tc_err;
-        if (it == 0) neighbours = tc_bounds_forced() || (double)distinct <= 0.5 * random;
+        h_err |= tc_err | take_fake_device_error();
         prof.collect();
         status = check_device_errors(h_err);
         if (status != KM_OK) break;

@@ -276,9 +276,9 @@ struct TcBounds {
     float4 *cxnorm;
 };
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b);
-bool tc_bounds_forced();
 size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t);  // its size with ws = nullptr
-int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, double *random, cudaStream_t s);
+int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, bool *neighbours,
+                         cudaStream_t s);
 int tc_bounds_order(const float *C, int d, int k, TcBuffers &b, const TcBounds &t, cudaStream_t s);
 int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBounds &t, cudaStream_t s);
 int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
