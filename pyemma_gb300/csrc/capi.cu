@@ -386,7 +386,10 @@ __global__ void lloyd_loop_step_kernel(LoopState *st, const double *cost, const 
     cudaGraphSetConditional(h, (conv || e != 0u || it + 1 >= st->max_it) ? 0u : 1u);
 }
 
-size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
+// The workspace of a Lloyd run; small: its assignment is the narrow-frame
+// kernel's, which has no center bounds.  bounds = false: what a run needs that
+// keeps none.
+size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small, bool bounds = true) {
     Carver c(nullptr);
     c.take<unsigned long long>(2);  // host copy counter pair
     c.take<LoopState>(1);
@@ -400,7 +403,7 @@ size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
         c.take<int32_t>(3 * (size_t)n);  // flip list
         c.take<int32_t>(1);              // its count
     }
-    if (is_tc(prec)) {
+    if (is_tc(prec) && !small && bounds) {
         TcBounds t;
         c.take<char>(tc_bounds_carve(nullptr, n, d, k, t));
     }
@@ -907,8 +910,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
                       (!narrow || (!small_forced() && small_lloyd_beats_narrow(n, d, k)));
     const bool small = narrow && !fits;
     const bool tc = is_tc(prec) || small;
-    const size_t need = lloyd_ws_bytes(n, d, k, prec, narrow);
-    KM_TRY(check_ws(workspace, workspace_bytes, need));
+    KM_TRY(check_ws(workspace, workspace_bytes, lloyd_ws_bytes(n, d, k, prec, narrow, false)));
+    const bool bounds_fit = workspace_bytes >= lloyd_ws_bytes(n, d, k, prec, narrow);
     if (max_iter == 0 && !hf) return KM_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     float *X = const_cast<float *>(X_in);  // written only by the host-frame copies
@@ -1055,10 +1058,11 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             carve_small(ws_assign, n, d, k, b);
         }
         KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
-        if (is_tc(prec)) {
+        // (not with the narrow-frame kernel, which takes FP16 runs too)
+        with_bounds = !small && bounds_fit && tc_bounds_wanted(n, d, k, max_iter, b);
+        if (with_bounds) {
             tc_bounds_carve(cv.take<char>(tc_bounds_carve(nullptr, n, d, k, bounds)), n, d, k, bounds);
-            with_bounds = tc_bounds_wanted(n, d, k, max_iter, b);
-            if (with_bounds) b.ub = bounds.ub;
+            b.ub = bounds.ub;
         }
         if (!hf && !small) KM_TRY(tc_prepare_frames(X, n, d, b, s, ps));
     }
