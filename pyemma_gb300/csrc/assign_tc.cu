@@ -1572,6 +1572,13 @@ bool make_plan(int d, int k, Plan &pl, bool fp8 = false, bool bf16 = false) {
     return build_plan(d, bn, false, 0, len, pl, fp8);
 }
 
+// The plan of a pass over b: the shape it keeps, or the one of now.
+bool plan_of(const TcBuffers &b, int d, int k, Plan &pl) {
+    if (b.plan.bn > 0)
+        return build_plan(d, b.plan.bn, b.plan.pair != 0, b.plan.stages, b.plan.list_len, pl, b.fp8 != 0);
+    return make_plan(d, k, pl, b.fp8 != 0, b.bf16 != 0);
+}
+
 float norm_inflate_of(int d) {
     // A compensated float32 sum of d squares is within a few u of the true value.
     return 1.0f + (float)(d + 8) * 5.9604645e-8f + 1e-6f;
@@ -1642,6 +1649,13 @@ bool tc_plan_set(int d, int k) {
     if (t_forced_plan) return true;
     std::lock_guard<std::mutex> lk(g_plans.m);
     return g_plans.choice.count(std::make_pair(d, k)) > 0;
+}
+
+bool tc_fix_plan(int d, int k, TcBuffers &b) {
+    Plan pl;
+    if (!make_plan(d, k, pl, b.fp8 != 0, b.bf16 != 0)) return false;
+    b.plan = TilePlan{pl.bn, pl.pair, pl.stages, pl.list_len};
+    return true;
 }
 
 bool tc_supported(int d, int k) {
@@ -2126,7 +2140,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
                    int32_t *label_counts, float *tile_lo = nullptr) {
     if (n == 0) return KM_OK;
     Plan pl;
-    if (!make_plan(d, k, pl, b.fp8 != 0, b.bf16 != 0) || !device_is_sm10x()) {
+    if (!plan_of(b, d, k, pl) || !device_is_sm10x()) {
         set_error("no tensor-core plan for d=%d k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
@@ -2614,7 +2628,7 @@ __global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int
 // the choice (the labels are the same).
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b) {
     Plan pl;
-    if (b.fp8 || !make_plan(d, k, pl, false, b.bf16 != 0)) return false;
+    if (b.fp8 || !plan_of(b, d, k, pl)) return false;
     const int n_ct = (k + pl.bn - 1) / pl.bn;
     if (n_ct < 2 || n_ct > kMaxMaskTiles || max_iter < 2) return false;
     if (const char *e = std::getenv("KM_TC_BOUNDS")) return e[0] == '1';
@@ -2678,7 +2692,7 @@ int tc_bounds_drift(const float *C, const float *C_new, int d, int k, const TcBo
 int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labels, TcBuffers &b, const TcBounds &t,
                     cudaStream_t s) {
     Plan pl;
-    if (!make_plan(d, k, pl, false, b.bf16 != 0)) return KM_ERR_UNSUPPORTED;
+    if (!plan_of(b, d, k, pl)) return KM_ERR_UNSUPPORTED;
     TcBuffers v = b;
     v.xh = t.cxh;
     v.xnorm = t.cxnorm;

@@ -904,6 +904,16 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
+    // One tile shape for the whole run: the tables and masks of the center
+    // bounds are laid out for it.
+    TcBuffers b;
+    if (is_tc(prec)) {
+        tc_set_operand(b, d, prec);
+        if (!tc_fix_plan(d, k, b)) {
+            set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
+            return KM_ERR_UNSUPPORTED;
+        }
+    }
     const bool narrow = !ps && small_route(precision, prec, n, d, k, true);
     // Few, narrow centers: whole iterations in one launch (lloyd_small.cu).
     const bool fits = !ps && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
@@ -1045,7 +1055,6 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         KM_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
     }
 
-    TcBuffers b;
     TcBounds bounds;
     bool with_bounds = false;  // the pass keeps the frames' distance bounds
     if (tc) {

@@ -167,6 +167,7 @@ int run_kmpp(const float *X, int64_t n, int d, int k, uint32_t seed, float *C0, 
 
 // ---- assign_tc.cu ------------------------------------------------------------
 // Tensor-core (tcgen05, FP16 operands) assignment with exact FP32 recheck.
+struct TcBuffers;
 bool tc_supported(int d, int k);   // a plan exists and the device is sm_10x
 bool tc_plan_exists(int d, int k); // shape check only (no device query)
 
@@ -187,6 +188,9 @@ void tc_clear_plans();
 bool tc_current_plan(int d, int k, TilePlan *out, bool *tuned);
 // A shape is forced on this thread or stored for (d, k).
 bool tc_plan_set(int d, int k);
+// Keeps the shape of now in b (operand type set): every pass over b takes it,
+// whatever is forced or stored later.  False: no shape for (d, k).
+bool tc_fix_plan(int d, int k, TcBuffers &b);
 size_t tc_frames_ws_size(int64_t n, int d);     // fp16 frame copy + norms
 size_t tc_centers_ws_size(int d, int k);        // fp16 centers + norms + shift + scalars
 size_t tc_assign_ws_size(int64_t n, int d, int k);  // candidate lists + counters
@@ -245,6 +249,7 @@ struct TcBuffers {
     int esize = 2;     // operand bytes per element: 2 (FP16, BF16) or 1 (FP8 e4m3)
     int bf16 = 0;      // operand type of xh / ch: 0 FP16, 1 BF16
     int fp8 = 0;       // 1: e4m3 operands (frames scaled per row), norms applied in the epilogue
+    TilePlan plan;     // bn > 0: the tile shape of every pass over these buffers (tc_fix_plan)
     int keep_err = 0;  // 1: tc_assign leaves err as it is (the caller clears it once for several calls)
 };
 
