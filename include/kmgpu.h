@@ -109,9 +109,9 @@ int km_profile_enable(int on);
 int km_profile_read(int32_t kind, double *ms_total, int64_t *launches);
 
 /* ---- test hook (diagnostics; no reference counterpart) --------------------
- * The next km_update or km_update_noalloc call, or the next Lloyd iteration
- * whose error word is read on its own (the first of a run, and every one with
- * a callback), ORs `bits` into that word, as if a kernel had set them (1, 2, 4: a
+ * The next km_update, km_update_noalloc, km_lloyd, km_lloyd_host,
+ * km_lloyd_pairs, km_kmpp or km_kmpp_pairs call finds `bits` in its device
+ * error word, as if a kernel had set them (1, 2, 4: a
  * device-side wait ran out; 8: a label out of range), and returns the
  * status that word maps to.  Lets tests check the mapping without making a
  * device wait run out. */
@@ -190,7 +190,9 @@ int km_update_noalloc(const float *X, int64_t n, int32_t d, const int32_t *label
  * centers into C0 (device, k*d floats) and, when idx is given (device, k
  * int64), the chosen frame indices.  cb (nullable) fires once per center;
  * without it up to 64 centers are drawn per launch.  Enqueues only: should a
- * device-side wait run out, the centers not drawn are NaN and idx -1. */
+ * device-side wait run out, the centers not drawn are NaN and their idx -1;
+ * idx[k - 1] is then -1, which a caller checks once the stream has run (the
+ * Python binding does, and raises KM_ERR_TIMEOUT). */
 size_t km_kmpp_workspace_size(int64_t n, int32_t d, int32_t k);
 int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, float *C0, int64_t *idx,
             km_callback cb, void *cb_user, void *workspace, size_t workspace_bytes, void *stream);

@@ -373,6 +373,14 @@ def _callback(fn):
     return cb, cb
 
 
+def _check_drawn(torch, idx):
+    """Raises when a device-side wait of kmeans++ ran out (the centers from
+    there on are NaN, their frames -1).  Not while the stream is captured,
+    when nothing has run yet."""
+    if not torch.cuda.is_current_stream_capturing() and int(idx[-1]) < 0:
+        raise KmError(KM_ERR_TIMEOUT, "libkmgpu: a device-side wait of kmeans++ timed out; its centers are incomplete")
+
+
 def kmpp(X, k, seed, callback=None):
     """kmeans++ initial centers (k, d) and chosen frame indices."""
     torch = _torch()
@@ -387,6 +395,7 @@ def kmpp(X, k, seed, callback=None):
     check(L.km_kmpp(_ptr(X), n, d, k, int(seed) & 0xFFFFFFFF, _ptr(C0), _ptr(idx), cb, None, _ptr(ws),
                     ws_bytes, _stream(torch, X.device)))
     del keep
+    _check_drawn(torch, idx)
     return C0, idx
 
 
@@ -753,6 +762,7 @@ def kmpp_pairs(xyz, pairs, k, seed, callback=None):
     check(L.km_kmpp_pairs(_ptr(xyz), n, n_atoms, _ptr(pairs), d, k, int(seed) & 0xFFFFFFFF, _ptr(C0), _ptr(idx), cb,
                           None, _ptr(ws), ws_bytes, _stream(torch, xyz.device)))
     del keep
+    _check_drawn(torch, idx)
     return C0, idx
 
 

@@ -469,9 +469,9 @@ int centers_d(const km_centers *h) { return h->d; }
 int centers_device(const km_centers *h) { return h->device; }
 int device_error_status(uint32_t e) { return check_device_errors(e); }
 
-// Test hook: bits that the next km_update / km_update_noalloc call, or the
-// next Lloyd iteration checked on the host, adds to the error word it reads
-// back from the device, as if a kernel had set them.
+// Test hook: bits that the next call with a device error word (km_update,
+// km_update_noalloc, Lloyd runs, km_kmpp) finds in it, as if a kernel had set
+// them.
 // It lets the tests check how each bit maps to a status without making a
 // device-side wait run out.
 static std::atomic<uint32_t> g_fake_device_error{0};
@@ -1232,7 +1232,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             it += hs.it;
             *n_iter = it;
             if (hs.it > 0) prev = hin[hs.it - 1];
-            status = check_device_errors(hs.err);
+            status = check_device_errors(hs.err | take_fake_device_error());
             if (status != KM_OK) break;
             if (hs.converged) {
                 *converged = 1;
@@ -1259,7 +1259,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             KM_CUDA(cudaMemcpyAsync(&hs, loop_st, sizeof(hs), cudaMemcpyDeviceToHost, s));
             KM_CUDA(cudaMemcpyAsync(hin, loop_inertias, sizeof(double) * hs.max_it, cudaMemcpyDeviceToHost, s));
             KM_CUDA(cudaStreamSynchronize(s));
-            KM_TRY(check_device_errors(hs.err));
+            KM_TRY(check_device_errors(hs.err | take_fake_device_error()));
             for (int32_t j = 0; j < hs.it; ++j)
                 if (inertias) inertias[it + j] = hin[j];
             it += hs.it;

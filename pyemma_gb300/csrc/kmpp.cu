@@ -764,7 +764,8 @@ int run_kmpp_src(const Src &src, int64_t n, int d, int k, uint32_t seed, float *
     p.seed = seed;
     KM_CUDA(cudaMemsetAsync(p.w.tile_sum, 0, 3 * p.ntiles * sizeof(unsigned long long), s));
     KM_CUDA(cudaMemsetAsync(p.w.maxbits, 0, sizeof(uint32_t), s));
-    KM_CUDA(cudaMemsetAsync(p.w.err, 0, sizeof(uint32_t), s));
+    // (the planted bits of the test hook: the launches then draw nothing)
+    KM_CUDA(cudaMemsetAsync(p.w.err, (int)(take_fake_device_error() & 0xffu), sizeof(uint32_t), s));
     // A pruned round pays a second barrier and the bounds, and saves rows of
     // d words less two.  us per round (unpruned, pruned), k = 300:
     //   d = 2:    n = 500,000 8.6, 10.5;  2M 16.2, 15.1;  10M 67, 39
