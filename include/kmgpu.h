@@ -124,7 +124,10 @@ int km_debug_fake_device_error(uint32_t bits);
  * before they write it: a value in [0, k) seeds the frame's search (a
  * previous labelling makes it faster where k >= 2048 and d <= 126); the
  * result does not depend on what the array held, and the array need not be
- * initialised. */
+ * initialised.  A KM_PREC_AUTO call on narrow frames (km_assign,
+ * km_assign_centers, km_lloyd*) asks for the narrow-frame kernel's lists, 4 or
+ * 16 bytes per frame (16 or 28 in Lloyd runs); with a workspace that holds
+ * only what KM_PREC_FP32 needs it takes the exact kernel instead. */
 size_t km_assign_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision);
 int km_assign(const float *X, int64_t n, int32_t d, const float *C, int32_t k, int32_t precision,
               int32_t *labels, void *workspace, size_t workspace_bytes, km_assign_stats *stats,

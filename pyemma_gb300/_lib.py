@@ -266,6 +266,21 @@ def _workspace(torch, nbytes, device):
     return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
+def _workspace_or_fp32(torch, size, p, device):
+    """(precision, workspace, bytes) of a call whose workspace takes size(p)
+    bytes.  The narrow frames that "auto" takes to the tensor cores need a
+    list that the exact kernel does not: without the memory for it, the call
+    is made in fp32 (the labels are the same)."""
+    n = size(p)
+    try:
+        return p, _workspace(torch, n, device), n
+    except torch.OutOfMemoryError:
+        least = size(PRECISIONS["fp32"])
+        if p != PRECISIONS["auto"] or least >= n:
+            raise
+        return PRECISIONS["fp32"], _workspace(torch, least, device), least
+
+
 def precision_code(precision):
     if isinstance(precision, str):
         try:
@@ -293,8 +308,7 @@ def assign(X, C, precision="auto", labels=None):
     p = precision_code(precision)
     if labels is None:
         labels = torch.empty(n, dtype=torch.int32, device=X.device)
-    ws_bytes = L.km_assign_workspace_size(n, d, k, p)
-    ws = _workspace(torch, ws_bytes, X.device)
+    p, ws, ws_bytes = _workspace_or_fp32(torch, lambda q: L.km_assign_workspace_size(n, d, k, q), p, X.device)
     stats = AssignStats()
     check(L.km_assign(_ptr(X), n, d, _ptr(C), k, p, _ptr(labels), _ptr(ws), ws_bytes, ctypes.byref(stats),
                       _stream(torch, X.device)))
@@ -340,8 +354,8 @@ def batch_assign(X_packed, offsets, C, precision="auto", labels=None):
     p = precision_code(precision)
     if labels is None:
         labels = torch.empty(n, dtype=torch.int32, device=X_packed.device)
-    ws_bytes = L.km_assign_workspace_size(n, d, k, p)
-    ws = _workspace(torch, ws_bytes, X_packed.device)
+    p, ws, ws_bytes = _workspace_or_fp32(torch, lambda q: L.km_assign_workspace_size(n, d, k, q), p,
+                                         X_packed.device)
     stats = AssignStats()
     check(L.km_batch_assign(_ptr(X_packed), offs.ctypes.data_as(ctypes.c_void_p), n_traj, d, _ptr(C), k, p,
                             _ptr(labels), _ptr(ws), ws_bytes, ctypes.byref(stats),
@@ -413,8 +427,7 @@ def lloyd(X, C, max_iter, tolerance, precision="auto", callback=None, labels=Non
     inertias = np.zeros(max(1, max_iter), dtype=np.float64)
     n_iter = ctypes.c_int32(0)
     conv = ctypes.c_int32(0)
-    ws_bytes = L.km_lloyd_workspace_size(n, d, k, p)
-    ws = _workspace(torch, ws_bytes, X.device)
+    p, ws, ws_bytes = _workspace_or_fp32(torch, lambda q: L.km_lloyd_workspace_size(n, d, k, q), p, X.device)
     cb, keep = _callback(callback)
     check(L.km_lloyd(_ptr(X), n, d, k, _ptr(C), int(max_iter), float(tolerance), p, _ptr(labels),
                      inertias.ctypes.data_as(ctypes.c_void_p), ctypes.byref(n_iter), ctypes.byref(conv), cb,
@@ -458,8 +471,7 @@ def lloyd_host(parts, C, max_iter, tolerance, precision="auto", callback=None, X
     inertias = np.zeros(max(1, max_iter), dtype=np.float64)
     n_iter = ctypes.c_int32(0)
     conv = ctypes.c_int32(0)
-    ws_bytes = L.km_lloyd_workspace_size(n, d, k, p)
-    ws = _workspace(torch, ws_bytes, C.device)
+    p, ws, ws_bytes = _workspace_or_fp32(torch, lambda q: L.km_lloyd_workspace_size(n, d, k, q), p, C.device)
     cb, keep = _callback(callback)
     check(L.km_lloyd_host(ptrs, rows.ctypes.data_as(ctypes.c_void_p), len(arrs), _ptr(X), n, d, k, _ptr(C),
                           int(max_iter), float(tolerance), p, _ptr(labels),
@@ -580,7 +592,12 @@ class Centers(object):
         if labels is None:
             labels = torch.empty(n, dtype=torch.int32, device=X.device)
         ws_bytes = self._L.km_assign_centers_workspace_size(n, self.handle)
-        ws = _workspace(torch, ws_bytes, X.device)
+        try:
+            ws = _workspace(torch, ws_bytes, X.device)
+        except torch.OutOfMemoryError:  # the exact kernel needs no workspace
+            if self.precision != "fp32":
+                raise
+            ws, ws_bytes = None, 0
         stats = AssignStats()
         check(self._L.km_assign_centers(_ptr(X), n, d, self.handle, _ptr(labels), _ptr(ws), ws_bytes,
                                         ctypes.byref(stats), _stream(torch, X.device)))

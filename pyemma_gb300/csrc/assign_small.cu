@@ -640,6 +640,35 @@ int small_prepare_centers(const float *C, int d, int k, TcBuffers &b, cudaStream
 
 namespace {
 
+// Launches over the centers.
+int sm_passes(int d, int k) {
+    const int tiles = sm_kpad(k) / kSmN, fit = sm_tiles_fit(sm_panels(d));
+    return (tiles + fit - 1) / fit;
+}
+
+size_t carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b) {
+    Carver c(ws);
+    const size_t nn = n > 0 ? n : 1;
+    b.counters = c.take<int32_t>(kTcStatusWords);
+    b.flipped = reinterpret_cast<unsigned long long *>(b.counters + 4);
+    b.err = reinterpret_cast<uint32_t *>(b.counters + 6);
+    b.full_frames = c.take<int32_t>(nn);
+    b.pair_lo = sm_passes(d, k) > 1 ? c.take<float>(3 * nn) : nullptr;
+    b.wide_cap = 0;
+    return c.bytes();
+}
+
+}  // namespace
+
+size_t small_lists_ws_size(int64_t n, int d, int k) {
+    TcBuffers b;
+    return carve_lists(nullptr, n, d, k, b);
+}
+
+void small_carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b) { carve_lists(ws, n, d, k, b); }
+
+namespace {
+
 template <int DP>
 int launch_small(const CUtensorMap &tmB, const SmParams &p, unsigned grid, size_t smem, cudaStream_t s) {
     static bool attr_done[kDeviceSlots] = {};
@@ -705,7 +734,7 @@ int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuf
     p.shift = b.shift;
     p.scal = b.scal;
     p.cg = b.scg;
-    p.state = b.pair_lo;  // 16 floats per frame, of which three are used here
+    p.state = b.pair_lo;  // three floats per frame
     p.labels = labels;
     p.label_counts = label_counts;
     p.full_frames = b.full_frames;
@@ -713,7 +742,7 @@ int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuf
     p.err = b.err;
 
     const int tiles = kpad / kSmN;
-    const int passes = (tiles + sm_tiles_fit(panels) - 1) / sm_tiles_fit(panels);
+    const int passes = sm_passes(d, k);
     const int per = (tiles + passes - 1) / passes;
     const int64_t n_tiles = (n + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(num_sms(), n_tiles);

@@ -1770,10 +1770,10 @@ void tc_carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
 }
 
 int tc_clear_status(const TcBuffers &b, cudaStream_t s) {
-    // err is the last of the words
     // err is the last of the words before the second pass's counts
-    KM_CUDA(cudaMemsetAsync(b.counters, 0, (b.keep_err ? 6 : kTcDiagWords + 2) * sizeof(int32_t), s));
-    if (b.keep_err) KM_CUDA(cudaMemsetAsync(b.counters + kTcDiagWords, 0, 2 * sizeof(int32_t), s));
+    KM_CUDA(cudaMemsetAsync(b.counters, 0, (b.keep_err ? 6 : kTcStatusWords) * sizeof(int32_t), s));
+    if (b.keep_err)
+        KM_CUDA(cudaMemsetAsync(b.counters + kTcDiagWords, 0, (kTcStatusWords - kTcDiagWords) * sizeof(int32_t), s));
     return KM_OK;
 }
 

@@ -161,9 +161,11 @@ bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_de
 }
 
 // The workspace of an assignment; small: the narrow-frame kernel may run
-// (its center half and lists; the FP16 form's workspace holds both).
+// (its center half and lists; the FP16 form's workspace holds both).  An
+// assignment that resolves to FP32 needs none of it: with less room it takes
+// the exact kernel (the labels are the same).
 size_t small_ws_bytes(int64_t n, int d, int k) {
-    return tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k) + 2 * 256;
+    return tc_centers_ws_size(d, k) + small_lists_ws_size(n, d, k) + 2 * 256;
 }
 
 size_t assign_ws_bytes(int64_t n, int d, int k, int prec, bool small = false) {
@@ -184,7 +186,7 @@ void carve_small(void *ws, int64_t n, int d, int k, TcBuffers &b) {
     char *p = static_cast<char *>(ws);
     tc_carve_centers(p, d, k, b);
     p += (tc_centers_ws_size(d, k) + 255) / 256 * 256;
-    tc_carve_assign(p, n, d, k, b);
+    small_carve_lists(p, n, d, k, b);
 }
 
 int check_device_errors(uint32_t e) {
@@ -270,7 +272,8 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
-    const bool small = !ps && small_route(precision, prec, n, d, k, true);
+    bool small = !ps && small_route(precision, prec, n, d, k, true);
+    if (small && !is_tc(prec)) small = ws && ws_bytes >= small_ws_bytes(n, d, k);
     KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec, small)));
     TcBuffers b;
     if (is_tc(prec) && n > 0) {
@@ -288,7 +291,7 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
 
 // Workspace of an assignment whose centers are prepared: frames + lists.
 size_t resident_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
-    if (!is_tc(prec)) return small ? tc_assign_ws_size(n, d, k) + 256 : 0;
+    if (!is_tc(prec)) return small ? small_lists_ws_size(n, d, k) + 256 : 0;
     return tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k) + 2 * 256;
 }
 
@@ -386,6 +389,19 @@ __global__ void lloyd_loop_step_kernel(LoopState *st, const double *cost, const 
     cudaGraphSetConditional(h, (conv || e != 0u || it + 1 >= st->max_it) ? 0u : 1u);
 }
 
+// How a Lloyd run assigns its frames: small = the narrow-frame kernel, fits =
+// whole iterations in one cooperative launch (few, narrow centers:
+// lloyd_small.cu), neither = the kernels of `prec`.
+struct LloydRoute {
+    bool small, fits;
+};
+LloydRoute lloyd_route(int64_t n, int d, int k, int precision, int prec, bool dense, bool check_device) {
+    const bool narrow = dense && small_route(precision, prec, n, d, k, check_device);
+    const bool fits = dense && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
+                      (!narrow || (!small_forced() && small_lloyd_beats_narrow(n, d, k)));
+    return LloydRoute{narrow && !fits, fits};
+}
+
 // The workspace of a Lloyd run; small: its assignment is the narrow-frame
 // kernel's, which has no center bounds.  bounds = false: what a run needs that
 // keeps none.
@@ -427,9 +443,15 @@ struct km_centers {
     TcBuffers tc;  // center half: ch, cnorm, shift, scal (tensor-core precisions)
     bool small = false;       // the narrow-frame form of the center half is prepared too
     int asked = KM_PREC_FP32; // the precision km_centers_create was given
-    // Whether n frames take the narrow-frame kernel.
+    // Whether n frames take the narrow-frame kernel (in a workspace of ws_bytes).
     bool small_for(int64_t n) const { return small && small_route(asked, prec, n, d, k, true); }
+    bool small_for(int64_t n, const void *ws, size_t ws_bytes) const;
 };
+
+bool km_centers::small_for(int64_t n, const void *ws, size_t ws_bytes) const {
+    if (!small_for(n)) return false;
+    return is_tc(prec) || (ws && ws_bytes >= resident_ws_bytes(n, d, k, prec, true));
+}
 
 namespace km {
 // Enqueues the assignment of n frames against a resident center set without
@@ -438,13 +460,13 @@ namespace km {
 int assign_centers_enqueue(const float *X, int64_t n, const km_centers *h, int32_t *labels, void *ws,
                            size_t ws_bytes, uint32_t *err_host, cudaStream_t s) {
     *err_host = 0;
-    const bool small = h->small_for(n);
+    const bool small = h->small_for(n, ws, ws_bytes);
     KM_TRY(check_ws(ws, ws_bytes, resident_ws_bytes(n, h->d, h->k, h->prec, small)));
     if (n == 0) return KM_OK;
     TcBuffers b = h->tc;
     char *p = static_cast<char *>(ws);
     if (small) {
-        tc_carve_assign(p, n, h->d, h->k, b);
+        small_carve_lists(p, n, h->d, h->k, b);
         KM_TRY(small_assign(X, n, h->d, h->k, labels, b, s));
         KM_CUDA(cudaMemcpyAsync(err_host, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         return KM_OK;
@@ -645,7 +667,7 @@ int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, floa
 size_t km_lloyd_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
     if (check_shape(n, d, k) != KM_OK) return 0;
     const int prec = resolve_precision(precision, d, k, false);
-    return lloyd_ws_bytes(n, d, k, prec, small_route(precision, prec, n, d, k, false));
+    return lloyd_ws_bytes(n, d, k, prec, lloyd_route(n, d, k, precision, prec, true, false).small);
 }
 
 }  // extern "C"
@@ -914,14 +936,16 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             return KM_ERR_UNSUPPORTED;
         }
     }
-    const bool narrow = !ps && small_route(precision, prec, n, d, k, true);
-    // Few, narrow centers: whole iterations in one launch (lloyd_small.cu).
-    const bool fits = !ps && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
-                      (!narrow || (!small_forced() && small_lloyd_beats_narrow(n, d, k)));
-    const bool small = narrow && !fits;
+    const LloydRoute route = lloyd_route(n, d, k, precision, prec, !ps, true);
+    bool small = route.small, fits = route.fits;
+    if (small && !is_tc(prec) && workspace_bytes < lloyd_ws_bytes(n, d, k, prec, true)) {
+        // the run needs no narrow-frame kernel: without its room, as FP32
+        small = false;
+        fits = small_lloyd_ok(n, d, k);
+    }
     const bool tc = is_tc(prec) || small;
-    KM_TRY(check_ws(workspace, workspace_bytes, lloyd_ws_bytes(n, d, k, prec, narrow, false)));
-    const bool bounds_fit = workspace_bytes >= lloyd_ws_bytes(n, d, k, prec, narrow);
+    KM_TRY(check_ws(workspace, workspace_bytes, lloyd_ws_bytes(n, d, k, prec, small, false)));
+    const bool bounds_fit = workspace_bytes >= lloyd_ws_bytes(n, d, k, prec, small);
     if (max_iter == 0 && !hf) return KM_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     float *X = const_cast<float *>(X_in);  // written only by the host-frame copies
@@ -1596,12 +1620,12 @@ int km_assign_centers(const float *X, int64_t n, int32_t d, const km_centers *h,
         set_error("X and labels must be non-NULL");
         return KM_ERR_BAD_SHAPE;
     }
-    const bool small = h->small_for(n);
+    const bool small = h->small_for(n, workspace, workspace_bytes);
     KM_TRY(check_ws(workspace, workspace_bytes, resident_ws_bytes(n, d, h->k, h->prec, small)));
     TcBuffers b;
     if (small && n > 0) {
         b = h->tc;  // no frame copy: the lists only
-        tc_carve_assign(workspace, n, d, h->k, b);
+        small_carve_lists(workspace, n, d, h->k, b);
     } else if (is_tc(h->prec) && n > 0) {
         b = h->tc;  // prepared center half; the carves below fill the frame and list fields
         char *p = static_cast<char *>(workspace);

@@ -197,6 +197,8 @@ size_t tc_assign_ws_size(int64_t n, int d, int k);  // candidate lists + counter
 
 // Word of counters at which the eight 64-bit diagnostic counters start.
 constexpr int kTcDiagWords = 8;
+// Words that tc_clear_status clears: the status and the second pass's counts.
+constexpr int kTcStatusWords = kTcDiagWords + 2;
 
 #define TC_CANDIDATES 16  // candidate centers kept per frame by the tensor-core pass
 
@@ -334,6 +336,11 @@ bool small_forced();
 size_t small_centers_elems(int d, int k);  // FP16 elements of sch
 size_t small_groups_floats(int d, int k);  // floats of scg
 int small_prepare_centers(const float *C, int d, int k, TcBuffers &b, cudaStream_t s);
+// The lists of n frames: status words, the frames to re-check and, with more
+// centers than one launch holds, three values per frame (4 or 16 bytes per
+// frame).  The room of tc_carve_assign holds them too.
+size_t small_lists_ws_size(int64_t n, int d, int k);
+void small_carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b);
 // The pass on s, then the exact re-check over all centers of the frames it
 // could not settle: on s, or with `side` on that stream (after `fork`,
 // recorded on s) with the changed labels in fl, as in tc_assign_deferred.
