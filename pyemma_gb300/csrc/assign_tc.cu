@@ -1722,11 +1722,28 @@ namespace {
 constexpr int kMaxTcChunks = kTcMaxChunks;
 constexpr int kChunkCounters0 = kTcDiagWords + 16;
 
-// One carving sequence for sizing (ws == nullptr) and for carving.
-// Frames that a pass takes a second time at most (0: none).
-int64_t wide_cap(int64_t n, int d) { return d >= 32 && n >= 4096 ? (n / 16 + 255) / 256 * 256 : 0; }
+// Frames that a pass takes a second time at most (0: none).  A sixteenth of
+// the frames, and no more than fit a bit table of kWideBitsMax: its rows have
+// a bit per center, so that without the limit it grows as n k / 128 bytes (8
+// GB at 1M frames and k = 2^20).  Frames beyond go to the full re-check.
+// None below 2e11 flop per pass: the launches of the second pass cost about
+// 10 us when no list overflows (250,007 x 1,023, k = 777 922 -> 933 us; 50,000
+// x 128, k = 500 168 -> 178, which keeps the full re-check).  KM_TC_WIDE=0 or
+// 1 in the environment forces the choice (the labels are the same).
+constexpr size_t kWideBitsMax = size_t(256) << 20;
+size_t wide_words(int k) { return (size_t)k_pad_of(k) / 32 + 8; }
+bool wide_wanted(int64_t n, int d, int k) {
+    if (const char *e = std::getenv("KM_TC_WIDE")) return e[0] == '1';
+    return 2.0 * (double)n * k * d >= 2e11;
+}
+int64_t wide_cap(int64_t n, int d, int k, int prec) {
+    if (prec == KM_PREC_FP8 || d < 32 || n < 4096 || !wide_wanted(n, d, k)) return 0;
+    const int64_t rows = (int64_t)(kWideBitsMax / (4 * wide_words(k))) / 256 * 256;
+    return std::min((n / 16 + 255) / 256 * 256, rows);
+}
 
-size_t carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
+// One carving sequence for sizing (ws == nullptr) and for carving.
+size_t carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b) {
     Carver c(ws);
     const size_t nn = n > 0 ? n : 1;
     b.rc_frames = c.take<int32_t>(nn);
@@ -1745,13 +1762,13 @@ size_t carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
     b.counters = c.take<int32_t>(kChunkCounters0 + 4 * (kMaxTcChunks - 1));
     b.flipped = reinterpret_cast<unsigned long long *>(b.counters + 4);
     b.err = reinterpret_cast<uint32_t *>(b.counters + 6);
-    b.wide_cap = wide_cap(n, d);
+    b.wide_cap = wide_cap(n, d, k, prec);
     if (b.wide_cap > 0) {
         b.wide_xh = c.take<uint16_t>((size_t)b.wide_cap * kp_of(d));
         b.wide_xnorm = c.take<float4>(b.wide_cap);
         b.wide_thr = c.take<float>(b.wide_cap);
         b.wide_frames = c.take<int32_t>(b.wide_cap);
-        b.wide_bits = c.take<uint32_t>((size_t)b.wide_cap * (k_pad_of(k) / 32 + 8));
+        b.wide_bits = c.take<uint32_t>((size_t)b.wide_cap * wide_words(k));
         b.wide_counts = b.counters + kTcDiagWords;
         b.rest_frames = c.take<int32_t>(nn);
         b.rest_keys = c.take<unsigned long long>(nn);
@@ -1760,13 +1777,13 @@ size_t carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
 }
 }  // namespace
 
-size_t tc_assign_ws_size(int64_t n, int d, int k) {
+size_t tc_assign_ws_size(int64_t n, int d, int k, int prec) {
     TcBuffers b;
-    return carve_assign(nullptr, n, d, k, b);
+    return carve_assign(nullptr, n, d, k, prec, b);
 }
 
-void tc_carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
-    carve_assign(ws, n, d, k, b);
+void tc_carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b) {
+    carve_assign(ws, n, d, k, prec, b);
 }
 
 int tc_clear_status(const TcBuffers &b, cudaStream_t s) {
@@ -2251,13 +2268,7 @@ int tc_assign_impl(const float *X, int64_t n, int d, const float *C, int k, int3
     p.row_thr = nullptr;
     p.bits = nullptr;
     p.bit_words = p.n_ctiles * p.bn / 32;
-    // The launches of the second pass cost about 10 us when no list overflows
-    // (250,007 x 1,023, k = 777 922 -> 933 us; 50,000 x 128, k = 500 168 ->
-    // 178, which keeps the full re-check).  KM_TC_WIDE=0 or 1 in the environment forces the choice (the
-    // labels are the same).
-    bool wide = 2.0 * (double)n * k * d >= 2e11;
-    if (const char *e = std::getenv("KM_TC_WIDE")) wide = e[0] == '1';
-    wide = wide && b.wide_cap > 0 && !b.fp8 && !dump && !wait_cycles && !tile_lo;
+    const bool wide = wide_wanted(n, d, k) && b.wide_cap > 0 && !b.fp8 && !dump && !wait_cycles && !tile_lo;
     p.full_thr = wide;
     set_lists(p, b);
     p.err = b.err;
@@ -2626,6 +2637,15 @@ __global__ void __launch_bounds__(256) unit_mask_kernel(int64_t n, int unit, int
 // 400,000 x 528, k = 1000 7.5 -> 6.3; shuffled 500,000 x 300, k = 1500 9.9 ->
 // 9.6 (9.9 with masks).  KM_TC_BOUNDS=0 or 1 in the environment forces
 // the choice (the labels are the same).
+// tc_bounds_room is the part of the rule that a workspace size can follow:
+// neither the iterations nor the tile shape of the run (at most 256 centers
+// per tile, at least 32).
+bool tc_bounds_room(int64_t n, int d, int k, int prec) {
+    if (prec == KM_PREC_FP8 || k <= 32 || k > 256 * kMaxMaskTiles) return false;
+    if (const char *e = std::getenv("KM_TC_BOUNDS")) return e[0] == '1';
+    return 2.0 * (double)n * k * d >= 4e11;
+}
+
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b) {
     Plan pl;
     if (b.fp8 || !plan_of(b, d, k, pl)) return false;

@@ -170,16 +170,16 @@ size_t small_ws_bytes(int64_t n, int d, int k) {
 
 size_t assign_ws_bytes(int64_t n, int d, int k, int prec, bool small = false) {
     if (!is_tc(prec)) return small ? small_ws_bytes(n, d, k) : 0;
-    return tc_frames_ws_size(n, d) + tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k) + 3 * 256;
+    return tc_frames_ws_size(n, d) + tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k, prec) + 3 * 256;
 }
 
-void carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b) {
+void carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b) {
     char *p = static_cast<char *>(ws);
     tc_carve_frames(p, n, d, b);
     p += (tc_frames_ws_size(n, d) + 255) / 256 * 256;
     tc_carve_centers(p, d, k, b);
     p += (tc_centers_ws_size(d, k) + 255) / 256 * 256;
-    tc_carve_assign(p, n, d, k, b);
+    tc_carve_assign(p, n, d, k, prec, b);
 }
 
 void carve_small(void *ws, int64_t n, int d, int k, TcBuffers &b) {
@@ -277,7 +277,7 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
     KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec, small)));
     TcBuffers b;
     if (is_tc(prec) && n > 0) {
-        carve_assign(ws, n, d, k, b);
+        carve_assign(ws, n, d, k, prec, b);
         tc_set_operand(b, d, prec);
     } else if (small && n > 0) {
         carve_small(ws, n, d, k, b);
@@ -292,7 +292,7 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
 // Workspace of an assignment whose centers are prepared: frames + lists.
 size_t resident_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
     if (!is_tc(prec)) return small ? small_lists_ws_size(n, d, k) + 256 : 0;
-    return tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k) + 2 * 256;
+    return tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k, prec) + 2 * 256;
 }
 
 // dst (device) <- src (host memory that the device reads in place, or any
@@ -419,7 +419,7 @@ size_t lloyd_ws_bytes(int64_t n, int d, int k, int prec, bool small, bool bounds
         c.take<int32_t>(3 * (size_t)n);  // flip list
         c.take<int32_t>(1);              // its count
     }
-    if (is_tc(prec) && !small && bounds) {
+    if (is_tc(prec) && !small && bounds && tc_bounds_room(n, d, k, prec)) {
         TcBounds t;
         c.take<char>(tc_bounds_carve(nullptr, n, d, k, t));
     }
@@ -475,7 +475,7 @@ int assign_centers_enqueue(const float *X, int64_t n, const km_centers *h, int32
         return launch_assign_fp32(X, nullptr, nullptr, n, h->d, h->C, h->k, labels, nullptr, nullptr, s);
     tc_carve_frames(p, n, h->d, b);
     p += (tc_frames_ws_size(n, h->d) + 255) / 256 * 256;
-    tc_carve_assign(p, n, h->d, h->k, b);
+    tc_carve_assign(p, n, h->d, h->k, h->prec, b);
     tc_set_operand(b, h->d, h->prec);
     KM_TRY(tc_prepare_frames(X, n, h->d, b, s));
     KM_TRY(tc_assign(X, n, h->d, h->C, h->k, labels, b, s, nullptr));
@@ -601,7 +601,7 @@ int km_debug_tc_distances(const float *X, int64_t n, int32_t d, const float *C, 
     if (n == 0) return KM_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     TcBuffers b;
-    carve_assign(workspace, n, d, k, b);
+    carve_assign(workspace, n, d, k, KM_PREC_FP16, b);
     tc_set_operand(b, d, precision);
     KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
     KM_TRY(tc_prepare_centers(C, d, k, b, s));
@@ -1085,14 +1085,15 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         // The shift and scale stay fixed for the whole run so that the 16-bit
         // frame copy is made once (narrow frames have none).
         if (is_tc(prec)) {
-            carve_assign(ws_assign, n, d, k, b);
+            carve_assign(ws_assign, n, d, k, prec, b);
             tc_set_operand(b, d, prec);
         } else {
             carve_small(ws_assign, n, d, k, b);
         }
         KM_TRY(tc_prepare_shift_from_centers(C, d, k, b, s));
         // (not with the narrow-frame kernel, which takes FP16 runs too)
-        with_bounds = !small && bounds_fit && tc_bounds_wanted(n, d, k, max_iter, b);
+        with_bounds = !small && bounds_fit && tc_bounds_room(n, d, k, prec) &&
+                      tc_bounds_wanted(n, d, k, max_iter, b);
         if (with_bounds) {
             tc_bounds_carve(cv.take<char>(tc_bounds_carve(nullptr, n, d, k, bounds)), n, d, k, bounds);
             b.ub = bounds.ub;
@@ -1631,7 +1632,7 @@ int km_assign_centers(const float *X, int64_t n, int32_t d, const km_centers *h,
         char *p = static_cast<char *>(workspace);
         tc_carve_frames(p, n, d, b);
         p += (tc_frames_ws_size(n, d) + 255) / 256 * 256;
-        tc_carve_assign(p, n, d, h->k, b);
+        tc_carve_assign(p, n, d, h->k, h->prec, b);
         tc_set_operand(b, d, h->prec);
     }
     return assign_core(X, n, d, h->C, h->k, h->prec, small, labels, b, true, stats, static_cast<cudaStream_t>(stream));

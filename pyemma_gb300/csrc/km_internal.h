@@ -193,7 +193,7 @@ bool tc_plan_set(int d, int k);
 bool tc_fix_plan(int d, int k, TcBuffers &b);
 size_t tc_frames_ws_size(int64_t n, int d);     // fp16 frame copy + norms
 size_t tc_centers_ws_size(int d, int k);        // fp16 centers + norms + shift + scalars
-size_t tc_assign_ws_size(int64_t n, int d, int k);  // candidate lists + counters
+size_t tc_assign_ws_size(int64_t n, int d, int k, int prec);  // candidate lists + counters
 
 // Word of counters at which the eight 64-bit diagnostic counters start.
 constexpr int kTcDiagWords = 8;
@@ -282,6 +282,7 @@ struct TcBounds {
     void *cxh;  // the centers as frames
     float4 *cxnorm;
 };
+bool tc_bounds_room(int64_t n, int d, int k, int prec);  // runs of this size may keep them
 bool tc_bounds_wanted(int64_t n, int d, int k, int max_iter, const TcBuffers &b);
 size_t tc_bounds_carve(void *ws, int64_t n, int d, int k, TcBounds &t);  // its size with ws = nullptr
 int tc_bounds_neighbours(int64_t n, int k, const int32_t *labels, const TcBounds &t, bool *neighbours,
@@ -296,7 +297,7 @@ int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labe
 void tc_set_operand(TcBuffers &b, int d, int prec);
 void tc_carve_frames(void *ws, int64_t n, int d, TcBuffers &b);
 void tc_carve_centers(void *ws, int d, int k, TcBuffers &b);
-void tc_carve_assign(void *ws, int64_t n, int d, int k, TcBuffers &b);
+void tc_carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b);
 
 // shift == nullptr: the shift is the mean of the centers (computed on device).
 int tc_prepare_shift_from_centers(const float *C, int d, int k, TcBuffers &b, cudaStream_t s);

@@ -9,7 +9,7 @@ import pytest
 
 
 def test_narrow_lloyd_reserves_no_bounds(kmlib, monkeypatch):
-    n, d, k, fp16 = 1_000_000, 24, 2000, 1
+    n, d, k, fp16 = 5_000_000, 24, 2000, 1
     monkeypatch.setenv("KM_TC_SMALL", "0")
     general = kmlib.km_lloyd_workspace_size(n, d, k, fp16)
     monkeypatch.setenv("KM_TC_SMALL", "1")
