@@ -384,8 +384,10 @@ __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumu
 // cp.async copies, kPairSlots - 1 frames ahead (a frame's 12 n_atoms bytes
 // are not a 16-byte multiple, so no bulk copy), and each lane's atom pairs
 // held in registers as offsets into a slot (two 16-bit halves).  The
-// features are those of PairRows (pair_feature).  Bound by issue: 608 us for
-// 500,000 frames of 33 atoms (694 with two compensated sums per feature).
+// features are those of PairRows (pair_feature).  Bound by issue: 694 us for
+// 500,000 frames of 33 atoms.  (A Kahan sum per feature and the squares in
+// plain chains take 608, at the cost of the sums' last bits: the inertia then
+// repeats to 3e-10 instead of 1e-15.)
 // ---------------------------------------------------------------------------
 constexpr int kPairSlots = 4;
 constexpr int kPairMaxAtoms = 128;  // slots of up to 384 floats: 48 KB per CTA at most
@@ -438,17 +440,14 @@ __global__ void __launch_bounds__(256) seg_accumulate_pairs_kernel(
             if (__shfl_sync(0xffffffffu, my_l[0], t) >= 0) fetch(__shfl_sync(0xffffffffu, my_i[0], t), t);
             cp_async_commit();
         }
-        // Per feature a Kahan sum (ks, kc: the sum is ks - kc); per row the
-        // squared deviations of the lane's features in two FMA chains, added
-        // to a compensated row total, as in seg_accumulate_bulk_kernel.
-        float ks[MW], kc[MW], cold[MW];
-        CSum qacc;
+        CSum acc[MW], qacc;
+        float cold[MW];
         int cur = -1;
         auto flush = [&]() {
 #pragma unroll
             for (int m = 0; m < MW; ++m) {
                 const int f = f_base + lane + 32 * m;
-                if (f < d) atomicAdd(&S[(int64_t)cur * d + f], (double)ks[m] - (double)kc[m]);
+                if (f < d) atomicAdd(&S[(int64_t)cur * d + f], acc[m].value());
             }
             double q = qacc.value();
             for (int off = 16; off > 0; off >>= 1) q += __shfl_xor_sync(0xffffffffu, q, off);
@@ -486,12 +485,10 @@ __global__ void __launch_bounds__(256) seg_accumulate_pairs_kernel(
 #pragma unroll
                     for (int m = 0; m < MW; ++m) {
                         const int f = f_base + lane + 32 * m;
-                        ks[m] = 0.0f;
-                        kc[m] = 0.0f;
+                        acc[m].reset();
                         cold[m] = f < d ? __ldg(C_old + (int64_t)l * d + f) : 0.0f;
                     }
                 }
-                float q0 = 0.0f, q1 = 0.0f;
 #pragma unroll
                 for (int m = 0; m < MW; ++m) {
                     const int f = f_base + lane + 32 * m;
@@ -499,18 +496,11 @@ __global__ void __launch_bounds__(256) seg_accumulate_pairs_kernel(
                         const float *a = xr + (ofs[m] & 0xFFFFu);
                         const float *b = xr + (ofs[m] >> 16);
                         const float x = pair_feature(a[0], a[1], a[2], b[0], b[1], b[2]);
-                        const float t2 = __fsub_rn(x, cold[m]);
-                        const float y = __fsub_rn(t2, kc[m]);
-                        const float sn = __fadd_rn(ks[m], y);
-                        kc[m] = __fsub_rn(__fsub_rn(sn, ks[m]), y);
-                        ks[m] = sn;
-                        if (m & 1)
-                            q1 = __fmaf_rn(t2, t2, q1);
-                        else
-                            q0 = __fmaf_rn(t2, t2, q0);
+                        const float t2 = x - cold[m];
+                        acc[m].add(t2);
+                        qacc.add(t2 * t2);
                     }
                 }
-                qacc.add(q0 + q1);
                 __syncwarp();
             }
         }
