@@ -395,9 +395,12 @@ __global__ void lloyd_loop_step_kernel(LoopState *st, const double *cost, const 
 struct LloydRoute {
     bool small, fits;
 };
-LloydRoute lloyd_route(int64_t n, int d, int k, int precision, int prec, bool dense, bool check_device) {
-    const bool narrow = dense && small_route(precision, prec, n, d, k, check_device);
-    const bool fits = dense && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
+// The frames of a run: rows, features of coordinate frames stored as rows
+// (whose sums the cooperative launch does not make), or coordinates.
+enum class LloydFrames { kRows, kPairRows, kPairs };
+LloydRoute lloyd_route(int64_t n, int d, int k, int precision, int prec, LloydFrames of, bool check_device) {
+    const bool narrow = of != LloydFrames::kPairs && small_route(precision, prec, n, d, k, check_device);
+    const bool fits = of == LloydFrames::kRows && !is_tc(prec) && small_lloyd_ok(n, d, k) &&
                       (!narrow || (!small_forced() && small_lloyd_beats_narrow(n, d, k)));
     return LloydRoute{narrow && !fits, fits};
 }
@@ -664,10 +667,14 @@ int km_kmpp(const float *X, int64_t n, int32_t d, int32_t k, uint32_t seed, floa
     return run_kmpp(X, n, d, k, seed, C0, idx, cb, cb_user, workspace, static_cast<cudaStream_t>(stream));
 }
 
-size_t km_lloyd_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
+static size_t lloyd_size(int64_t n, int32_t d, int32_t k, int32_t precision, LloydFrames of) {
     if (check_shape(n, d, k) != KM_OK) return 0;
     const int prec = resolve_precision(precision, d, k, false);
-    return lloyd_ws_bytes(n, d, k, prec, lloyd_route(n, d, k, precision, prec, true, false).small);
+    return lloyd_ws_bytes(n, d, k, prec, lloyd_route(n, d, k, precision, prec, of, false).small);
+}
+
+size_t km_lloyd_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
+    return lloyd_size(n, d, k, precision, LloydFrames::kRows);
 }
 
 }  // extern "C"
@@ -913,7 +920,7 @@ struct Stager {
 int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int32_t k, float *C, int32_t max_iter,
               double tolerance, int32_t precision, int32_t *labels, double *inertias, int32_t *n_iter,
               int32_t *converged, km_callback cb, void *cb_user, void *workspace, size_t workspace_bytes,
-              void *stream, const PairSrc *ps = nullptr) {
+              void *stream, const PairSrc *ps = nullptr, bool pair_rows = false) {
     KM_TRY(check_shape(n, d, k));
     if (n < 1 || (!X_in && !ps) || !C || !labels || !n_iter || !converged || max_iter < 0) {
         set_error("Lloyd needs n >= 1, max_iter >= 0 and non-NULL X, C, labels, n_iter, converged");
@@ -936,12 +943,13 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             return KM_ERR_UNSUPPORTED;
         }
     }
-    const LloydRoute route = lloyd_route(n, d, k, precision, prec, !ps, true);
+    const LloydFrames of = ps ? LloydFrames::kPairs : pair_rows ? LloydFrames::kPairRows : LloydFrames::kRows;
+    const LloydRoute route = lloyd_route(n, d, k, precision, prec, of, true);
     bool small = route.small, fits = route.fits;
     if (small && !is_tc(prec) && workspace_bytes < lloyd_ws_bytes(n, d, k, prec, true)) {
         // the run needs no narrow-frame kernel: without its room, as FP32
         small = false;
-        fits = small_lloyd_ok(n, d, k);
+        fits = of == LloydFrames::kRows && small_lloyd_ok(n, d, k);
     }
     const bool tc = is_tc(prec) || small;
     KM_TRY(check_ws(workspace, workspace_bytes, lloyd_ws_bytes(n, d, k, prec, small, false)));
@@ -1115,7 +1123,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     } closer{prof};
     auto enqueue_update = [&](cudaStream_t st) -> int {
         prof.begin(kProfUpdate, st);
-        KM_TRY(launch_update(X, n, d, labels, k, C, C_new, nullptr, cost, err, ws_update, st, ps));
+        KM_TRY(launch_update(X, n, d, labels, k, C, C_new, nullptr, cost, err, ws_update, st, ps, pair_rows));
         prof.end(kProfUpdate, st);
         KM_CUDA(cudaMemcpyAsync(C, C_new, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, st));
         return KM_OK;
@@ -1129,7 +1137,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
             }
             KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
             // the tensor-core pass counts the members as it writes the labels
-            int32_t *counts = update_counts_from_labels(d, k, ps) ? update_counts(ws_update, n, d, k) : nullptr;
+            int32_t *counts =
+                update_counts_from_labels(d, k, ps, pair_rows) ? update_counts(ws_update, n, d, k) : nullptr;
             if (counts) KM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * k, st));
             if (small)
                 KM_TRY(small_assign(X, n, d, k, labels, b, st, &prof, side.st, side.fork[0], &fl, counts));
@@ -1138,7 +1147,8 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
                                           ps, counts));
             prof.begin(kProfUpdate, st);
             // one segment-sum CTA per SM: room for the re-check beside it
-            KM_TRY(launch_update_accumulate(X, n, d, labels, k, C, err, ws_update, st, 1, ps, counts != nullptr));
+            KM_TRY(launch_update_accumulate(X, n, d, labels, k, C, err, ws_update, st, 1, ps, counts != nullptr,
+                                            pair_rows));
             KM_CUDA(cudaEventRecord(side.join, side.st));
             KM_CUDA(cudaStreamWaitEvent(st, side.join, 0));
             KM_TRY(launch_apply_flips(X, n, d, k, C, fl, labels, ws_update, st, ps));
@@ -1437,7 +1447,7 @@ int km_assign_pairs(const float *xyz, int64_t n, int32_t n_atoms, const int32_t 
 // Every iteration sums all features into the centers; computing them there
 // takes 0.6 ms at 500,000 x 528 and, as one long chain per cluster, no less at
 // 3,000, where the rows of 500,000 are 0.16 ms of memory traffic.  Ten
-// iterations, features computed -> stored: 500,000, k = 1000 13.5 -> 7.7 ms;
+// iterations, features computed -> stored: 500,000, k = 1000 13.5 -> 8.8 ms;
 // 100,000, k = 300 8.7 -> 3.1; 20,000, k = 100 6.9 -> 2.2.  One iteration
 // gains nothing (500,000: 2.2 ms either way).  A caller's workspace without
 // that room, and longer data, keep the features unwritten.
@@ -1450,7 +1460,7 @@ static size_t pair_rows_bytes(int64_t n, int32_t d) {
 }
 
 size_t km_lloyd_pairs_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
-    const size_t base = km_lloyd_workspace_size(n, d, k, precision);
+    const size_t base = lloyd_size(n, d, k, precision, LloydFrames::kPairRows);
     const size_t rows = pair_rows_bytes(n, d);
     return base == 0 || rows == 0 ? base : (base + 255) / 256 * 256 + rows;
 }
@@ -1466,13 +1476,13 @@ int km_lloyd_pairs(const float *xyz, int64_t n, int32_t n_atoms, const int32_t *
         set_error("FP8 operands are not built for coordinate frames");
         return KM_ERR_UNSUPPORTED;
     }
-    const size_t base = (km_lloyd_workspace_size(n, d, k, precision) + 255) / 256 * 256;
+    const size_t base = (lloyd_size(n, d, k, precision, LloydFrames::kPairRows) + 255) / 256 * 256;
     const size_t rows = pair_rows_bytes(n, d);
     if (n >= 1 && rows > 0 && max_iter >= kPairRowsIterations && workspace && workspace_bytes >= base + rows) {
         float *X = reinterpret_cast<float *>(static_cast<char *>(workspace) + base);
         KM_TRY(launch_pair_distances(xyz, n, n_atoms, pairs, d, X, s));
         return lloyd_run(X, nullptr, n, d, k, C, max_iter, tolerance, precision, labels, inertias, n_iter, converged,
-                         cb, cb_user, workspace, base, stream);
+                         cb, cb_user, workspace, base, stream, nullptr, true);
     }
     PairSrc ps;
     ps.xyz = xyz;

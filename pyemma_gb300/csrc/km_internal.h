@@ -97,21 +97,23 @@ size_t update_ws_size(int64_t n, int d, int k);
 // uint32) receives kDevBadLabel when a label is outside [0, k).
 int launch_update(const float *X, int64_t n, int d, const int32_t *labels, int k,
                   const float *C_old, float *C_new, int64_t *counts_out, double *cost,
-                  uint32_t *err, void *ws, cudaStream_t s, const PairSrc *ps = nullptr);
+                  uint32_t *err, void *ws, cudaStream_t s, const PairSrc *ps = nullptr, bool comp = false);
 // launch_update in two halves: the sums over the members (counting sort and
 // segment sums) and the new centers and inertia from those sums.
 // seg_per_sm > 0 caps the segment-sum CTAs per SM (room for a kernel beside it).
 // counted: the member counts of `labels` are already in the workspace (added
 // by the tensor-core pass into update_counts(), cleared before it); only
 // valid where update_counts_from_labels() holds.
+// comp: X holds the features of coordinate frames; every term of the sums is
+// compensated, as where the features are computed (ps).
 int launch_update_accumulate(const float *X, int64_t n, int d, const int32_t *labels, int k, const float *C_old,
                              uint32_t *err, void *ws, cudaStream_t s, int seg_per_sm = 0,
-                             const PairSrc *ps = nullptr, bool counted = false);
+                             const PairSrc *ps = nullptr, bool counted = false, bool comp = false);
 // The member-count array of an update workspace, and whether the update of
 // (d, k) counts its members from the labels in a pass of its own (the
 // counting-sort path; the one-pass small-shape path counts as it sums).
 int32_t *update_counts(void *ws, int64_t n, int d, int k);
-bool update_counts_from_labels(int d, int k, const PairSrc *ps);
+bool update_counts_from_labels(int d, int k, const PairSrc *ps, bool comp);
 int launch_update_finish(int64_t n, int d, int k, const float *C_old, float *C_new, int64_t *counts_out,
                          double *cost, void *ws, cudaStream_t s);
 // The update of frames that arrive in parts: begin clears the totals, each

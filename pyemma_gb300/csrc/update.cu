@@ -250,13 +250,26 @@ __device__ __forceinline__ void ring_fetch(void *dst, const void *src, uint32_t 
                  : "memory");
 }
 
+// s + c += v with the exact error of the leading sum in c: CSum::add without
+// its comparison.
+__device__ __forceinline__ void two_sum_add(float &s, float &c, float v) {
+    const float t = __fadd_rn(s, v);
+    const float b = __fsub_rn(t, s);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(v, b)));
+    s = t;
+}
+
 // Ring rows hold MW*32 floats (zero beyond d), so the inner loop needs no
 // bounds test.
 size_t bulk_smem_bytes(int mw, int ring) {
     return (size_t)kBulkWarps * ((size_t)ring * mw * 128 + 2 * kPiece * 4 + ring * 8);
 }
 
-template <int MW, int RING>
+// COMP: the sums of seg_accumulate_wide_kernel (every deviation and every
+// square added with its rounding error) instead of a Kahan sum per feature and
+// the squares in FMA chains; for the stored features of coordinate frames,
+// whose sums are those of the features computed where they are read.
+template <int MW, int RING, bool COMP>
 __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumulate_bulk_kernel(
     const float *__restrict__ X, int d, const int32_t *__restrict__ perm, const int32_t *__restrict__ slab,
     int64_t n_max, const int32_t *__restrict__ n_sorted, const float *__restrict__ C_old, double *__restrict__ S,
@@ -305,7 +318,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumu
 
         // Per feature a Kahan sum (ks, kc: the sum is ks - kc); per row the
         // squared deviations of the lane's features in two FMA chains, added
-        // to a compensated row total.
+        // to a compensated row total.  COMP: ks + kc, and every square for itself.
         float ks[MW], kc[MW], cold[MW];
         CSum qacc;
         int cur = -1;
@@ -313,7 +326,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumu
 #pragma unroll
             for (int m = 0; m < MW; ++m) {
                 const int f = lane + 32 * m;
-                if (f < d) atomicAdd(&S[(int64_t)cur * d + f], (double)ks[m] - (double)kc[m]);
+                if (f < d) atomicAdd(&S[(int64_t)cur * d + f], (double)ks[m] + (COMP ? (double)kc[m] : -(double)kc[m]));
             }
             double qq = qacc.value();
             for (int off = 16; off > 0; off >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, off);
@@ -343,6 +356,11 @@ __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumu
 #pragma unroll
             for (int m = 0; m < MW; ++m) {
                 const float t = __fsub_rn(row[lane + 32 * m], cold[m]);  // zero beyond d
+                if constexpr (COMP) {
+                    two_sum_add(ks[m], kc[m], t);
+                    two_sum_add(qacc.s, qacc.c, __fmul_rn(t, t));
+                    continue;
+                }
                 const float y = __fsub_rn(t, kc[m]);
                 const float sn = __fadd_rn(ks[m], y);
                 kc[m] = __fsub_rn(__fsub_rn(sn, ks[m]), y);
@@ -352,7 +370,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32, (MW > 17 ? 1 : 2)) seg_accumu
                 else
                     q0 = __fmaf_rn(t, t, q0);
             }
-            qacc.add(q0 + q1);
+            if constexpr (!COMP) qacc.add(q0 + q1);
             __syncwarp();
             if (q + RING < cnt) {
                 // The slot's shared-memory reads above come before the copy
@@ -775,7 +793,7 @@ bool try_wide(int mw, const Src &X, int64_t n, int d, const UpdateWs &u, int k, 
     return true;
 }
 
-template <int MW, int RING>
+template <int MW, int RING, bool COMP>
 int launch_bulk_ring(const float *X, int64_t n, int d, const UpdateWs &u, int k, const float *C_old, uint32_t *err,
                      cudaStream_t s, int seg_per_sm) {
     const size_t smem = bulk_smem_bytes(MW, RING);
@@ -785,10 +803,10 @@ int launch_bulk_ring(const float *X, int64_t n, int d, const UpdateWs &u, int k,
     const int dev = current_device();
     int per_sm = dev >= 0 && dev < kDeviceSlots ? per_sm_dev[dev] : 0;
     if (per_sm <= 0) {
-        KM_CUDA(cudaFuncSetAttribute(seg_accumulate_bulk_kernel<MW, RING>,
+        KM_CUDA(cudaFuncSetAttribute(seg_accumulate_bulk_kernel<MW, RING, COMP>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(232448)));
         int v = 0;
-        KM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, seg_accumulate_bulk_kernel<MW, RING>,
+        KM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, seg_accumulate_bulk_kernel<MW, RING, COMP>,
                                                               kBulkWarps * 32, smem));
         per_sm = v > 0 ? v : 1;
         if (dev >= 0 && dev < kDeviceSlots) per_sm_dev[dev] = per_sm;
@@ -797,7 +815,7 @@ int launch_bulk_ring(const float *X, int64_t n, int d, const UpdateWs &u, int k,
     int64_t g = (npieces + kBulkWarps - 1) / kBulkWarps;
     const int64_t cap = (int64_t)num_sms() * (seg_per_sm > 0 && seg_per_sm < per_sm ? seg_per_sm : per_sm);
     if (g > cap) g = cap;
-    seg_accumulate_bulk_kernel<MW, RING><<<(unsigned)(g < 1 ? 1 : g), kBulkWarps * 32, smem, s>>>(
+    seg_accumulate_bulk_kernel<MW, RING, COMP><<<(unsigned)(g < 1 ? 1 : g), kBulkWarps * 32, smem, s>>>(
         X, d, u.perm, u.slab, n, u.offsets + k, C_old, u.S, u.Q, err);
     KM_CUDA(cudaGetLastError());
     return KM_OK;
@@ -805,28 +823,35 @@ int launch_bulk_ring(const float *X, int64_t n, int d, const UpdateWs &u, int k,
 
 // One CTA per SM (room for another kernel beside it) keeps twice the rows in
 // flight per warp when they fit in shared memory.
-template <int MW>
-int launch_bulk(const float *X, int64_t n, int d, const UpdateWs &u, int k, const float *C_old, uint32_t *err,
+template <int MW, bool COMP>
+int launch_bulk_form(const float *X, int64_t n, int d, const UpdateWs &u, int k, const float *C_old, uint32_t *err,
                 cudaStream_t s, int seg_per_sm) {
     if (seg_per_sm == 1 && bulk_smem_bytes(MW, 2 * kRing) <= 227 * 1024)
-        return launch_bulk_ring<MW, 2 * kRing>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-    return launch_bulk_ring<MW, kRing>(X, n, d, u, k, C_old, err, s, seg_per_sm);
+        return launch_bulk_ring<MW, 2 * kRing, COMP>(X, n, d, u, k, C_old, err, s, seg_per_sm);
+    return launch_bulk_ring<MW, kRing, COMP>(X, n, d, u, k, C_old, err, s, seg_per_sm);
+}
+
+template <int MW>
+int launch_bulk(const float *X, int64_t n, int d, const UpdateWs &u, int k, const float *C_old, uint32_t *err,
+                cudaStream_t s, int seg_per_sm, bool comp) {
+    return comp ? launch_bulk_form<MW, true>(X, n, d, u, k, C_old, err, s, seg_per_sm)
+                : launch_bulk_form<MW, false>(X, n, d, u, k, C_old, err, s, seg_per_sm);
 }
 
 int launch_segments_bulk(const float *X, int64_t n, int d, const UpdateWs &u, int k, const float *C_old,
-                         uint32_t *err, cudaStream_t s, int seg_per_sm) {
+                         uint32_t *err, cudaStream_t s, int seg_per_sm, bool comp) {
     const int mw = (d + 31) / 32;
     switch (mw) {
-        case 1: return launch_bulk<1>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 2: return launch_bulk<2>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 3: return launch_bulk<3>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 4: return launch_bulk<4>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 5: case 6: return launch_bulk<6>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 7: case 8: return launch_bulk<8>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 9: case 10: case 11: case 12: return launch_bulk<12>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 13: case 14: case 15: case 16: case 17: return launch_bulk<17>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        case 18: case 19: case 20: case 21: case 22: case 23: case 24: return launch_bulk<24>(X, n, d, u, k, C_old, err, s, seg_per_sm);
-        default: return launch_bulk<32>(X, n, d, u, k, C_old, err, s, seg_per_sm);
+        case 1: return launch_bulk<1>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 2: return launch_bulk<2>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 3: return launch_bulk<3>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 4: return launch_bulk<4>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 5: case 6: return launch_bulk<6>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 7: case 8: return launch_bulk<8>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 9: case 10: case 11: case 12: return launch_bulk<12>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 13: case 14: case 15: case 16: case 17: return launch_bulk<17>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        case 18: case 19: case 20: case 21: case 22: case 23: case 24: return launch_bulk<24>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
+        default: return launch_bulk<32>(X, n, d, u, k, C_old, err, s, seg_per_sm, comp);
     }
 }
 
@@ -914,20 +939,20 @@ size_t update_ws_size(int64_t n, int d, int k) {
 
 int32_t *update_counts(void *ws, int64_t n, int d, int k) { return carve(ws, n, d, k, nullptr).counts; }
 
-bool update_counts_from_labels(int d, int k, const PairSrc *ps) { return ps || !small_ok(d, k); }
+bool update_counts_from_labels(int d, int k, const PairSrc *ps, bool comp) { return ps || comp || !small_ok(d, k); }
 
 int launch_update_accumulate(const float *X, int64_t n, int d, const int32_t *labels, int k, const float *C_old,
                              uint32_t *err, void *ws, cudaStream_t s, int seg_per_sm, const PairSrc *ps,
-                             bool counted) {
+                             bool counted, bool comp) {
     UpdateWs u = carve(ws, n, d, k, nullptr);
-    if (counted && !update_counts_from_labels(d, k, ps)) {
+    if (counted && !update_counts_from_labels(d, k, ps, comp)) {
         set_error("precounted members only on the counting-sort path of the update");
         return KM_ERR_UNSUPPORTED;
     }
     if (!counted) KM_CUDA(cudaMemsetAsync(u.counts, 0, sizeof(int32_t) * k, s));
     KM_CUDA(cudaMemsetAsync(u.S, 0, sizeof(double) * (size_t)k * d, s));
     KM_CUDA(cudaMemsetAsync(u.Q, 0, sizeof(double) * k, s));
-    if (n > 0 && !ps && small_ok(d, k)) {
+    if (n > 0 && !ps && !comp && small_ok(d, k)) {
         const int dp = d <= 1 ? 1 : d <= 2 ? 2 : d <= 4 ? 4 : d <= 8 ? 8 : 16;
         // one frame per thread while the frames fill 8 CTAs of every SM, runs
         // of up to kSmallMaxRun frames beyond that
@@ -966,7 +991,7 @@ int launch_update_accumulate(const float *X, int64_t n, int d, const int32_t *la
                 KM_TRY(launch_segments(pair_rows_of(*ps, d), n, d, u, k, C_old, g, s));
             }
         } else if (bulk_ok(X, d)) {
-            KM_TRY(launch_segments_bulk(X, n, d, u, k, C_old, err, s, seg_per_sm));
+            KM_TRY(launch_segments_bulk(X, n, d, u, k, C_old, err, s, seg_per_sm, comp));
         } else {
             const int64_t npieces = (n + kPiece - 1) / kPiece;
             const unsigned g = grid_for(npieces * 32, 256, 8);
@@ -1004,8 +1029,8 @@ int launch_apply_flips(const float *X, int64_t n, int d, int k, const float *C_o
 
 int launch_update(const float *X, int64_t n, int d, const int32_t *labels, int k,
                   const float *C_old, float *C_new, int64_t *counts_out, double *cost,
-                  uint32_t *err, void *ws, cudaStream_t s, const PairSrc *ps) {
-    KM_TRY(launch_update_accumulate(X, n, d, labels, k, C_old, err, ws, s, 0, ps));
+                  uint32_t *err, void *ws, cudaStream_t s, const PairSrc *ps, bool comp) {
+    KM_TRY(launch_update_accumulate(X, n, d, labels, k, C_old, err, ws, s, 0, ps, false, comp));
     return launch_update_finish(n, d, k, C_old, C_new, counts_out, cost, ws, s);
 }
 
@@ -1031,7 +1056,7 @@ int launch_update_part(const float *X, int64_t n, int d, const int32_t *labels, 
     scatter_kernel<<<grid_for(rows, 256, 8), 256, 0, s>>>(labels, rows, k, u.cursor, u.perm, u.slab);
     KM_CUDA(cudaGetLastError());
     if (bulk_ok(X, d)) {
-        KM_TRY(launch_segments_bulk(X, rows, d, u, k, C_old, err, s, 0));
+        KM_TRY(launch_segments_bulk(X, rows, d, u, k, C_old, err, s, 0, false));
     } else {
         const int64_t npieces = (rows + kPiece - 1) / kPiece;
         KM_TRY(launch_segments(DenseRows{X, d}, rows, d, u, k, C_old, grid_for(npieces * 32, 256, 8), s));

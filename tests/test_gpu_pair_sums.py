@@ -28,7 +28,7 @@ def _step(X, C, labels):
     return C2, inertia
 
 
-@pytest.mark.parametrize("iters", [1])  # features computed where they are read
+@pytest.mark.parametrize("iters", [1, 2])  # features computed where they are read, and stored once
 @pytest.mark.parametrize("prec", ["fp16", "fp32"])
 @pytest.mark.parametrize("n,n_atoms,k", [(4000, 33, 20), (3001, 9, 40), (5000, 6, 7), (2500, 20, 300)])
 def test_pair_sums_keep_their_bits(oracle, prec, iters, n, n_atoms, k):
