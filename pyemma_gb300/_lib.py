@@ -387,16 +387,23 @@ def _callback(fn):
     return cb, cb
 
 
-def _check_drawn(torch, idx):
+def check_drawn(idx, centers=None):
     """Raises when a device-side wait of kmeans++ ran out (the centers from
-    there on are NaN, their frames -1).  Not while the stream is captured,
-    when nothing has run yet."""
+    there on are NaN, their frames idx -1).  Not while the stream is captured,
+    when nothing has run yet.  centers: the host centers of the Lloyd run from
+    the drawn ones, if there was one; a center that was not drawn is still NaN
+    in them (no frame is nearest to it), so finite ones need no look at idx."""
+    if centers is not None and np.isfinite(centers).all():
+        return
+    torch = _torch()
     if not torch.cuda.is_current_stream_capturing() and int(idx[-1]) < 0:
         raise KmError(KM_ERR_TIMEOUT, "libkmgpu: a device-side wait of kmeans++ timed out; its centers are incomplete")
 
 
-def kmpp(X, k, seed, callback=None):
-    """kmeans++ initial centers (k, d) and chosen frame indices."""
+def kmpp(X, k, seed, callback=None, check_now=True):
+    """kmeans++ initial centers (k, d) and chosen frame indices.  With
+    check_now=False the caller passes the indices to check_drawn later (after
+    a Lloyd run, say, whose set-up then overlaps the draws)."""
     torch = _torch()
     L = load()
     _check_frames(torch, X)
@@ -409,7 +416,8 @@ def kmpp(X, k, seed, callback=None):
     check(L.km_kmpp(_ptr(X), n, d, k, int(seed) & 0xFFFFFFFF, _ptr(C0), _ptr(idx), cb, None, _ptr(ws),
                     ws_bytes, _stream(torch, X.device)))
     del keep
-    _check_drawn(torch, idx)
+    if check_now:
+        check_drawn(idx)
     return C0, idx
 
 
@@ -765,9 +773,9 @@ def lloyd_pairs(xyz, pairs, C, max_iter, tolerance, precision="auto", callback=N
                 converged=bool(conv.value))
 
 
-def kmpp_pairs(xyz, pairs, k, seed, callback=None):
+def kmpp_pairs(xyz, pairs, k, seed, callback=None, check_now=True):
     """kmeans++ initial centers (k, d) and chosen frame indices for the
-    pair-distance features of coordinate frames."""
+    pair-distance features of coordinate frames (check_now as in kmpp)."""
     torch = _torch()
     L = load()
     n, n_atoms, d = _pair_args(torch, xyz, pairs)
@@ -779,7 +787,8 @@ def kmpp_pairs(xyz, pairs, k, seed, callback=None):
     check(L.km_kmpp_pairs(_ptr(xyz), n, n_atoms, _ptr(pairs), d, k, int(seed) & 0xFFFFFFFF, _ptr(C0), _ptr(idx), cb,
                           None, _ptr(ws), ws_bytes, _stream(torch, xyz.device)))
     del keep
-    _check_drawn(torch, idx)
+    if check_now:
+        check_drawn(idx)
     return C0, idx
 
 

@@ -175,11 +175,15 @@ class KmeansClustering(AbstractClustering):
                 raise ValueError("initial centers have shape %s, data has dimension %d"
                                  % (self.clustercenters.shape, dim))
             C = _device.centers_to_device(self.clustercenters)
+            drawn = None
         else:
-            C, _ = _lib.kmpp_pairs(src.xyz, src.pairs, int(self.n_clusters), self.fixed_seed)
+            C, drawn = _lib.kmpp_pairs(src.xyz, src.pairs, int(self.n_clusters), self.fixed_seed, check_now=False)
         res = _lib.lloyd_pairs(src.xyz, src.pairs, C, int(self.max_iter), float(self.tolerance),
                                precision=self.precision)
-        self.clustercenters = C.cpu().numpy()
+        centers = C.cpu().numpy()
+        if drawn is not None:
+            _lib.check_drawn(drawn, centers)
+        self.clustercenters = centers
         self._converged = res["converged"]
         self.inertias = res["inertias"]
         self.n_iter = res["n_iter"]
@@ -229,6 +233,7 @@ class KmeansClustering(AbstractClustering):
                     len(self.clustercenters), self.n_clusters))
 
         try:
+            drawn = None
             if self._check_resume_iteration():
                 if self.clustercenters.ndim != 2 or self.clustercenters.shape[1] != dim:
                     raise ValueError("initial centers have shape %s, data has dimension %d"
@@ -237,7 +242,7 @@ class KmeansClustering(AbstractClustering):
             elif minrmsd:
                 C, _ = _lib.kmpp_minrmsd(self._in_memory_chunks, int(self.n_clusters), self.fixed_seed)
             else:
-                C, _ = _lib.kmpp(self._in_memory_chunks, int(self.n_clusters), self.fixed_seed)
+                C, drawn = _lib.kmpp(self._in_memory_chunks, int(self.n_clusters), self.fixed_seed, check_now=False)
             if minrmsd:
                 res = _lib.lloyd_minrmsd(self._in_memory_chunks, C, int(self.max_iter), float(self.tolerance))
             elif host_parts is not None:
@@ -247,7 +252,10 @@ class KmeansClustering(AbstractClustering):
             else:
                 res = _lib.lloyd(self._in_memory_chunks, C, int(self.max_iter), float(self.tolerance),
                                  precision=self.precision)
-            self.clustercenters = C.cpu().numpy()
+            centers = C.cpu().numpy()
+            if drawn is not None:
+                _lib.check_drawn(drawn, centers)
+            self.clustercenters = centers
             self._converged = res["converged"]
             self.inertias = res["inertias"]
             self.n_iter = res["n_iter"]

@@ -72,9 +72,10 @@ def _centers(centers):
 
 
 def _kmpp(X, k, seed, metric, callback=None):
-    fn = _lib.kmpp_minrmsd if metric == "minRMSD" else _lib.kmpp
-    C, _ = fn(X, int(k), seed, callback=callback)
-    return C
+    """kmeans++ centers and the drawn frames (for _lib.check_drawn)."""
+    if metric == "minRMSD":
+        return _lib.kmpp_minrmsd(X, int(k), seed, callback=callback)
+    return _lib.kmpp(X, int(k), seed, callback=callback, check_now=False)
 
 
 def _uniform(X, k, seed):
@@ -159,15 +160,16 @@ class KMeans(object):
         self._initial_centers = _centers(value)
 
     def _start(self, X, callback=None):
+        """The centers to start from, and the frames that kmeans++ drew (None: not drawn)."""
         if self.initial_centers is not None:
             c = self.initial_centers
             if c.shape[0] != self.n_clusters or c.shape[1] != X.shape[1]:
                 raise ValueError("initial centers have shape %s, expected (%d, %d)"
                                  % (c.shape, self.n_clusters, X.shape[1]))
-            return _device.centers_to_device(c)
+            return _device.centers_to_device(c), None
         if self.init_strategy == "kmeans++":
             return _kmpp(X, self.n_clusters, _seed(self.fixed_seed), self.metric, callback)
-        return _uniform(X, self.n_clusters, _seed(self.fixed_seed))
+        return _uniform(X, self.n_clusters, _seed(self.fixed_seed)), None
 
     def fit(self, data, callback_init_centers=None, callback_loop=None, n_jobs=None, **kwargs):
         """Initial centers (unless given), then Lloyd iterations until the
@@ -175,12 +177,15 @@ class KMeans(object):
         iterations ran.  callback_init_centers fires once per kmeans++ center,
         callback_loop once per iteration."""
         X = _frames(data, self.metric)
-        C = self._start(X, callback_init_centers)
+        C, drawn = self._start(X, callback_init_centers)
         if self.metric == "minRMSD":
             res = _lib.lloyd_minrmsd(X, C, self.max_iter, self.tolerance, callback=callback_loop)
         else:
             res = _lib.lloyd(X, C, self.max_iter, self.tolerance, precision=self.precision, callback=callback_loop)
-        self._model = KMeansModel(C.cpu().numpy(), metric=self.metric, tolerance=self.tolerance,
+        centers = C.cpu().numpy()
+        if drawn is not None:
+            _lib.check_drawn(drawn, centers)
+        self._model = KMeansModel(centers, metric=self.metric, tolerance=self.tolerance,
                                   inertias=res["inertias"], converged=res["converged"])
         return self
 
@@ -209,14 +214,17 @@ class MiniBatchKMeans(KMeans):
     def partial_fit(self, data, n_jobs=None):
         X = _frames(data, self.metric)
         if self._model is None:
-            C = self._start(X)
+            C, drawn = self._start(X)
         else:
-            C = _device.centers_to_device(self._model.cluster_centers)
+            C, drawn = _device.centers_to_device(self._model.cluster_centers), None
         if self.metric == "minRMSD":
             res = _lib.lloyd_minrmsd(X, C, 1, -1.0)
         else:
             res = _lib.lloyd(X, C, 1, -1.0, precision=self.precision)
-        self._model = KMeansModel(C.cpu().numpy(), metric=self.metric, tolerance=self.tolerance,
+        centers = C.cpu().numpy()
+        if drawn is not None:
+            _lib.check_drawn(drawn, centers)
+        self._model = KMeansModel(centers, metric=self.metric, tolerance=self.tolerance,
                                   inertias=res["inertias"][:1], converged=False)
         return self
 
@@ -288,7 +296,9 @@ class _KmppBinding(object):
         """kmeans++ centers (k, d) float32 of X (the binding test_kmeans.py:304
         calls); random_seed -1 draws a random seed."""
         Xd = _frames(X, self._metric)
-        return _kmpp(Xd, k, _seed(random_seed), self._metric, callback).cpu().numpy()
+        C, drawn = _kmpp(Xd, k, _seed(random_seed), self._metric, callback)
+        _lib.check_drawn(drawn)
+        return C.cpu().numpy()
 
 
 class _EuclideanImpl(object):
