@@ -24,8 +24,16 @@
 // threshold of the first, every possible argmin lies in the best group: the
 // thread computes the eight exact distances (feature order, every operation
 // rounded on its own) and takes the lowest index among the minima.
-// Otherwise, and where a value is not finite, the frame goes to the exact
-// re-check over all centers.
+// Otherwise, and where a value is not finite, the frame is listed with its
+// threshold.
+//
+// Listed frames (0.02-5% of continuous data at d >= 2, up to all of them on a
+// lattice or with duplicate centers) are compared with all centers, by a warp
+// each, or by a warp per eight where the list is long.  Large calls take long
+// lists through the same kernel again, which now leaves a bit per group of
+// eight centers that reaches the frame's threshold, and only those groups'
+// exact distances follow; frames that are not finite, and frames beyond the
+// room for the bits, are still compared with all centers.
 //
 // One persistent CTA per SM.  Warps 0-3 and 4-7 take the frame tiles (128
 // frames, one per thread) in turn and write their split operand rows to
@@ -72,6 +80,21 @@ constexpr int kSmConvWarps = 8;
 constexpr int kSmN = 128;                   // columns per MMA tile
 constexpr int kSmPanel = 128 * 128;         // bytes of 128 rows x 64 FP16 columns
 constexpr int kSmSmem = 232448;
+// Lists from which eight frames share a warp: the 4,864 warps then have about
+// eight each (10,000 frames beside the segment sums of 4.3M x 10, k = 1000: 8 us
+// per iteration more in eights).
+constexpr int kSmFew = 32768;
+// The second pass.  It is launched from n k (3 d + 2) = 2e10 on, where the 4 us
+// of an empty launch are at most 1.5% of the call (1M x 10, k = 1000 270 us),
+// and goes over lists whose comparison with all centers takes longer than it
+// does (list k (3 d + 2) = 1e9, about 50 us).  us per assignment with every
+// center twice, a warp per listed frame / eight / a second pass (and by the exact
+// kernel or the general pass): 1M x 2, k = 500 698 / 470 / 284 (370); 1M x 10, k
+// = 1000 3613 / 1436 / 599 (3908); 1M x 16, k = 2000 14,055 / 4231 / 2319 (4626).
+// Frames on a lattice of spacing 0.5: 1M x 16, k = 2000 2229 -> 1118 (1909).
+constexpr double kSmTwiceWork = 2e10, kSmTwiceList = 1e9;
+constexpr size_t kSmBitsMax = size_t(256) << 20;
+int sm_twice_few(int d, int k) { return std::max(kSmFew, (int)(kSmTwiceList / ((double)k * (3 * d + 2)))); }
 
 // 64-column panels per operand row: 4 columns per feature and 4 for the norm.
 __host__ __device__ constexpr int sm_panels(int d) { return 4 * (d + 1) > 64 ? 2 : 1; }
@@ -97,7 +120,12 @@ struct SmParams {
     float *state;        // (m1, m2, group) per frame between launches
     int32_t *labels;
     int32_t *label_counts;
-    int32_t *full_frames;
+    int32_t *full_frames;  // listed frames; the second pass goes over them
+    float *full_thr;       // the thresholds of the first `cap` of them (NaN: none)
+    int64_t cap;
+    int few;               // no second pass over lists of this many
+    uint8_t *bits;         // the second pass: bit q of byte t of a frame: group 8 t + q reaches its threshold
+    int bit_row;           // bytes per frame
     int32_t *counters;
     uint32_t *err;
 };
@@ -147,6 +175,24 @@ __device__ __forceinline__ void sm_scan(const uint32_t (&r)[32], int j0, int k, 
     }
 }
 
+// Bit q: group q of the 32 columns reaches thr (a NaN threshold: none does).
+template <bool MASK>
+__device__ __forceinline__ uint32_t sm_reach(const uint32_t (&r)[32], int j0, int k, float thr) {
+    uint32_t m = 0u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            w[c] = __uint_as_float(r[8 * q + c]);
+            if (MASK && j0 + 8 * q + c >= k) w[c] = __int_as_float(0xff800000);
+        }
+        const float g = max3f(max3f(w[0], w[1], w[2]), max3f(w[3], w[4], w[5]), fmaxf(w[6], w[7]));
+        if (g >= thr) m |= 1u << q;
+    }
+    return m;
+}
+
 __device__ __forceinline__ uint32_t half_bits(__half a, __half b) {
     const __half2 h = __halves2half2(a, b);
     uint32_t w;
@@ -154,8 +200,9 @@ __device__ __forceinline__ uint32_t half_bits(__half a, __half b) {
     return w;
 }
 
-// DP: features padded to 4, 8, 12, 16 or 32 (registers).
-template <int DP>
+// DP: features padded to 4, 8, 12, 16 or 32 (registers).  TWICE: the second
+// pass, over the first `cap` listed frames.
+template <int DP, bool TWICE>
 __global__ void __launch_bounds__(kSmThreads, 1)
     small_assign_kernel(const __grid_constant__ CUtensorMap tmB, const SmParams p) {
     constexpr int PANELS = DP > 16 ? 2 : 1;  // DP = 16 covers d <= 15
@@ -185,7 +232,15 @@ __global__ void __launch_bounds__(kSmThreads, 1)
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int64_t n_tiles = (p.n + 127) / 128;
+    int64_t rows = p.n;
+    if (TWICE) {
+        rows = p.counters[1];
+        // (a center that FP16 cannot encode, a NaN, leaves no thresholds)
+        if (rows <= p.few || !(__uint_as_float(p.scal[kSmallHcMax]) < __int_as_float(0x7f800000))) return;
+        rows = min(rows, p.cap);
+    }
+    const int64_t n_tiles = (rows + 127) / 128;
+    if (TWICE && blockIdx.x >= n_tiles) return;
     // This CTA's tiles are blockIdx.x + u gridDim.x, u < nt.
     const int nt = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
 
@@ -227,8 +282,10 @@ __global__ void __launch_bounds__(kSmThreads, 1)
         const uint32_t one1 = half_bits(__float2half_rn(1.0f), __float2half_rn(0.0f));
         float x[DP];
         auto load = [&](int u) {
-            const int64_t i = ((int64_t)blockIdx.x + (int64_t)u * gridDim.x) * 128 + r;
-            const float *src = p.X + (u < nt && i < p.n ? i : 0) * p.d;
+            int64_t i = ((int64_t)blockIdx.x + (int64_t)u * gridDim.x) * 128 + r;
+            if (u >= nt || i >= rows) i = 0;
+            if (TWICE) i = p.full_frames[i];
+            const float *src = p.X + i * p.d;
 #pragma unroll
             for (int f = 0; f < DP; ++f)
                 if (f < p.d) x[f] = ldg_pinned(src + f);
@@ -236,7 +293,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
         load(half);
         for (int u = half; u < nt; u += 2) {
             const int slot = u % NS;
-            const bool valid = ((int64_t)blockIdx.x + (int64_t)u * gridDim.x) * 128 + r < p.n;
+            const bool valid = ((int64_t)blockIdx.x + (int64_t)u * gridDim.x) * 128 + r < rows;
             // ||x||^2 of the split values by a Kahan sum (the distance bound
             // allows 8 u for it); the two norms of bounds by plain sums
             // inflated by norm_inflate.
@@ -372,6 +429,31 @@ __global__ void __launch_bounds__(kSmThreads, 1)
             const float4 fp = fpar[slot * 128 + row];
             __syncwarp();
             if (lane == 0) mbar_arrive(&a_empty[slot]);
+            if constexpr (TWICE) {
+                const float thr = i < rows ? p.full_thr[i] : kInf;
+                for (int t = 0; t < p.n_ct; ++t) {
+                    const uint32_t buf = accq % BUFS;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[BUFS * g + buf], (accq / BUFS) & 1u));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t base = tmem_base + lane_off + (BUFS * g + buf) * kSmN + 64 * half;
+                    const int j0 = (p.ct0 + t) * kSmN + 64 * half;
+                    uint32_t r[32];
+                    tmem_ld32(base, r);
+                    tmem_wait_ld32(r);
+                    uint32_t m = sm_reach<true>(r, j0, p.k, thr);
+                    tmem_ld32(base + 32, r);
+                    tmem_wait_ld32(r);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[BUFS * g + buf]);
+                    m |= sm_reach<true>(r, j0 + 32, p.k, thr) << 4;
+                    if (i < rows) p.bits[i * p.bit_row + 2 * (p.ct0 + t) + half] = (uint8_t)m;
+                    ++accq;
+                }
+                if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
+                continue;
+            }
             Best2 b{kNegInf, kNegInf, 0};
             if (!p.first && half == 0 && i < p.n) {
                 b.m1 = p.state[3 * i];
@@ -434,6 +516,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
                 continue;
             }
             bool need_full = false;
+            float thr = 0.0f;  // of a listed frame
             if (i < p.n) {
                 // The exact distances of the best group's centers.
                 float acc[8];
@@ -458,11 +541,11 @@ __global__ void __launch_bounds__(kSmThreads, 1)
                         best = acc[q];
                         label = b.group * 8 + q;
                     }
-                const float thr = window_threshold(b.m1, fp.x, inv_s2, s2, fp.z, fp.y, __fadd_ru(fp.y, 1e-18f),
-                                                   p.g_ratio);
-                const bool sure = b.m1 > kNegInf && b.m1 < kInf && fp.y < kInf && fp.z < kInf && fp.x < kInf &&
-                                  best < kInf && b.m2 < thr;
-                need_full = !sure;
+                thr = window_threshold(b.m1, fp.x, inv_s2, s2, fp.z, fp.y, __fadd_ru(fp.y, 1e-18f), p.g_ratio);
+                const bool finite = b.m1 > kNegInf && b.m1 < kInf && fp.y < kInf && fp.z < kInf && fp.x < kInf &&
+                                    best < kInf;
+                need_full = !finite || !(b.m2 < thr);
+                if (!finite) thr = __int_as_float(0x7fc00000);
                 p.labels[i] = label;  // provisional when the frame is re-checked
                 if (p.label_counts) atomicAdd(&p.label_counts[label], 1);
             }
@@ -472,7 +555,10 @@ __global__ void __launch_bounds__(kSmThreads, 1)
                 int at = 0;
                 if (lane == leader) at = atomicAdd(&p.counters[1], __popc(m_full));
                 at = __shfl_sync(0xffffffffu, at, leader) + __popc(m_full & ((1u << lane) - 1u));
-                if (need_full) p.full_frames[at] = (int32_t)i;
+                if (need_full) {
+                    p.full_frames[at] = (int32_t)i;
+                    if (at < p.cap) p.full_thr[at] = thr;
+                }
             }
             if (__any_sync(0xffffffffu, *abort_flag != 0)) ok = false;
         }
@@ -489,30 +575,60 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     }
 }
 
-// The exact re-check of the listed frames over all centers, a warp per frame:
-// lanes own centers (the grouped copy gives each eight of them 32 consecutive
-// bytes per feature), every distance in feature order with every operation
-// rounded on its own, then the lexicographic (distance, index) minimum; label
-// 0 when no distance is finite.  A changed label is written, or listed (flips
-// non-null).  One launch where the general re-check takes three; the lists
-// are short (0.02-5% of the frames at d >= 2).
+// The exact distances of the listed frames: every distance in feature order
+// with every operation rounded on its own, the lexicographic (distance, index)
+// minimum, label 0 when no distance is finite.  A changed label is written, or
+// listed (flips non-null).
+//   * A frame of a long list with bits: a thread, over its groups' eight
+//     centers at a time (ascending, so the first minimum has the lowest index).
+//   * Others are compared with all centers by a warp whose lanes own centers
+//     (the grouped copy gives each eight of them 32 consecutive bytes per
+//     feature): one at a time, or in a long list up to eight together, so that
+//     each center value read serves eight distances.
+// 1M x 2, k = 500: frames with bits, a warp each 523 us the call, a thread each
+// 284; a NaN center (no bits), a warp per frame 907, per eight 420.
+constexpr int kFullWarps = 8;
 template <int DP>
-__global__ void __launch_bounds__(256) small_full_kernel(
+__global__ void __launch_bounds__(kFullWarps * 32, DP > 16 ? 2 : 4) small_full_kernel(
     const float *__restrict__ X, int d, int k, const float *__restrict__ cg, const int32_t *__restrict__ frames,
-    const int32_t *__restrict__ n_dev, int64_t n_max, int32_t *__restrict__ labels, unsigned long long *flipped,
+    const int32_t *__restrict__ n_dev, int64_t n_max, const float *__restrict__ thr, const uint16_t *__restrict__ bits,
+    int bit_row, int64_t cap, int few, int32_t *__restrict__ labels, unsigned long long *flipped,
     int32_t *__restrict__ flips, int32_t *__restrict__ n_flips, int64_t max_flips) {
+    __shared__ __align__(16) float xs_s[kFullWarps][kSmMaxD * 8];  // [feature][frame]
+    __shared__ int32_t id_s[kFullWarps][32];                       // frames of a unit without bits
     int64_t n = *n_dev;
     if (n > n_max) n = n_max;
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n; e += nw) {
-        const int64_t i = frames[e];
-        float x[DP];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool lng = n > kSmFew;
+    if (n <= few) cap = 0;  // no second pass, no bits
+    const int unit = !lng ? 1 : cap > 0 ? 32 : 8;
+    const int64_t nw = (int64_t)gridDim.x * kFullWarps;
+    const float kInf = __int_as_float(0x7f800000);
+    auto settle = [&](int64_t i, int label) {
+        const int before = labels[i];
+        if (before == label) return;
+        if (flipped) atomicAdd(flipped, 1ull);
+        if (flips) {
+            const int slot = atomicAdd(n_flips, 1);
+            if (slot < max_flips) {
+                flips[3 * (int64_t)slot] = (int32_t)i;
+                flips[3 * (int64_t)slot + 1] = before;
+                flips[3 * (int64_t)slot + 2] = label;
+            }
+        } else {
+            labels[i] = label;
+        }
+    };
+    auto load = [&](int64_t i, float (&x)[DP]) {
 #pragma unroll
         for (int f = 0; f < DP; ++f) x[f] = f < d ? __ldg(X + i * d + f) : 0.0f;
-        float bd = __int_as_float(0x7f800000);
+    };
+    const float *c_lane = cg + (int64_t)(lane >> 3) * d * 8 + (lane & 7);  // the first 32 centers
+    auto one = [&](int64_t i) {
+        float x[DP], bd = kInf;
+        load(i, x);
         int bj = 0;
-        const float *c = cg + (int64_t)(lane >> 3) * d * 8 + (lane & 7);
+        const float *c = c_lane;
 #pragma unroll 2
         for (int j0 = 0; j0 < k; j0 += 32, c += 32 * d) {
             float acc = 0.0f;
@@ -525,22 +641,102 @@ __global__ void __launch_bounds__(256) small_full_kernel(
             }
         }
         warp_argmin(bd, bj);
-        if (lane == 0) {
-            const int before = labels[i];
-            if (before != bj) {
-                if (flipped) atomicAdd(flipped, 1ull);
-                if (flips) {
-                    const int slot = atomicAdd(n_flips, 1);
-                    if (slot < max_flips) {
-                        flips[3 * (int64_t)slot] = (int32_t)i;
-                        flips[3 * (int64_t)slot + 1] = before;
-                        flips[3 * (int64_t)slot + 2] = bj;
+        if (lane == 0) settle(i, bj);
+    };
+    float *xs = xs_s[warp];
+    auto eight = [&](const int32_t *ids, int m) {  // m frames, two to eight
+        for (int t = lane; t < 8 * d; t += 32) {
+            const int q = t / d, f = t - q * d;
+            xs[f * 8 + q] = q < m ? __ldg(X + (int64_t)ids[q] * d + f) : 0.0f;
+        }
+        __syncwarp();
+        float bd[8];
+        int bj[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) bd[q] = kInf, bj[q] = 0;
+        const float *c = c_lane;
+#pragma unroll 2
+        for (int j0 = 0; j0 < k; j0 += 32, c += 32 * d) {
+            float acc[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+#pragma unroll
+            for (int f = 0; f < DP; ++f) {
+                if (f >= d) break;
+                const float cf = __ldg(c + 8 * f);
+                const float4 a = *reinterpret_cast<const float4 *>(xs + 8 * f);
+                const float4 b = *reinterpret_cast<const float4 *>(xs + 8 * f + 4);
+                const float xq[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int q = 0; q < 8; ++q) acc[q] = __fadd_rn(acc[q], sq_term(xq[q], cf));
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (acc[q] < bd[q]) {
+                    bd[q] = acc[q];
+                    bj[q] = j0 + lane;
+                }
+        }
+        int label = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            warp_argmin(bd[q], bj[q]);
+            if (lane == q) label = bj[q];
+        }
+        if (lane < m) settle(ids[lane], label);
+        __syncwarp();  // xs is rewritten by the next eight
+    };
+    for (int64_t e0 = ((int64_t)blockIdx.x * kFullWarps + warp) * unit; e0 < n; e0 += nw * unit) {
+        if (!lng) {
+            one(frames[e0]);
+            continue;
+        }
+        const int64_t e = e0 + lane;
+        bool todo = lane < unit && e < n;
+        const int64_t i = todo ? frames[e] : 0;
+        if (todo && e < cap && thr[e] == thr[e]) {
+            float x[DP], bd = kInf;
+            load(i, x);
+            int bj = 0;
+            for (int t = 0; t < bit_row; ++t) {
+                for (uint32_t v = bits[e * bit_row + t]; v; v &= v - 1u) {
+                    todo = false;
+                    const int g = 16 * t + __ffs(v) - 1;
+                    const float *c = cg + (int64_t)g * d * 8;
+                    float acc[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+#pragma unroll
+                    for (int f = 0; f < DP; ++f) {
+                        if (f < d) {
+                            float w[8];
+                            ldg_f32x8(c + 8 * f, w);
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) acc[q] = __fadd_rn(acc[q], sq_term(x[f], w[q]));
+                        }
                     }
-                } else {
-                    labels[i] = bj;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (acc[q] < bd) {
+                            bd = acc[q];
+                            bj = 8 * g + q;
+                        }
                 }
             }
+            if (!todo) settle(i, bj);  // (the best center reaches its threshold; else all are compared)
         }
+        const unsigned rest = __ballot_sync(0xffffffffu, todo);
+        const int cnt = __popc(rest);
+        int32_t *ids = id_s[warp];
+        if (todo) ids[__popc(rest & ((1u << lane) - 1u))] = (int32_t)i;
+        __syncwarp();
+        for (int q = 0; q < cnt; q += 8) {
+            if (cnt - q > 1)
+                eight(ids + q, min(8, cnt - q));
+            else
+                one(ids[q]);
+        }
+        __syncwarp();  // ids are rewritten
     }
 }
 
@@ -640,10 +836,18 @@ int small_prepare_centers(const float *C, int d, int k, TcBuffers &b, cudaStream
 
 namespace {
 
+int sm_bit_row(int k) { return 2 * (sm_kpad(k) / kSmN); }
+
 // Launches over the centers.
 int sm_passes(int d, int k) {
     const int tiles = sm_kpad(k) / kSmN, fit = sm_tiles_fit(sm_panels(d));
     return (tiles + fit - 1) / fit;
+}
+
+// Frames that a second pass takes at most (0: none is made).
+int64_t sm_twice_cap(int64_t n, int d, int k) {
+    if (n <= sm_twice_few(d, k) || (double)n * k * (3 * d + 2) < kSmTwiceWork) return 0;
+    return std::min<int64_t>(n, (int64_t)(kSmBitsMax / (size_t)(sm_bit_row(k) + 4)));
 }
 
 size_t carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b) {
@@ -654,7 +858,9 @@ size_t carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b) {
     b.err = reinterpret_cast<uint32_t *>(b.counters + 6);
     b.full_frames = c.take<int32_t>(nn);
     b.pair_lo = sm_passes(d, k) > 1 ? c.take<float>(3 * nn) : nullptr;
-    b.wide_cap = 0;
+    b.wide_cap = sm_twice_cap(n, d, k);
+    b.wide_thr = b.wide_cap > 0 ? c.take<float>(b.wide_cap) : nullptr;
+    b.wide_bits = b.wide_cap > 0 ? c.take<uint32_t>(((size_t)b.wide_cap * sm_bit_row(k) + 3) / 4) : nullptr;
     return c.bytes();
 }
 
@@ -669,24 +875,51 @@ void small_carve_lists(void *ws, int64_t n, int d, int k, TcBuffers &b) { carve_
 
 namespace {
 
-template <int DP>
-int launch_small(const CUtensorMap &tmB, const SmParams &p, unsigned grid, size_t smem, cudaStream_t s) {
+template <int DP, bool TWICE>
+int launch_small_dp(const CUtensorMap &tmB, const SmParams &p, unsigned grid, size_t smem, cudaStream_t s) {
     static bool attr_done[kDeviceSlots] = {};
     const int dev = current_device();
     if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
-        KM_CUDA(cudaFuncSetAttribute(small_assign_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmSmem));
+        KM_CUDA(cudaFuncSetAttribute(small_assign_kernel<DP, TWICE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kSmSmem));
         if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
     }
-    small_assign_kernel<DP><<<grid, kSmThreads, smem, s>>>(tmB, p);
+    small_assign_kernel<DP, TWICE><<<grid, kSmThreads, smem, s>>>(tmB, p);
     KM_CUDA(cudaGetLastError());
     return KM_OK;
 }
 
+// A pass over all center tiles, `per` at a time.
+template <bool TWICE>
+int launch_small(const CUtensorMap &tmB, SmParams p, int tiles, int per, unsigned grid, cudaStream_t s) {
+    const int panels = sm_panels(p.d);
+    for (int t = 0; t < tiles; t += per) {
+        p.ct0 = t;
+        p.n_ct = std::min(per, tiles - t);
+        p.first = t == 0;
+        p.last = t + p.n_ct == tiles;
+        // at least 120 KB: one CTA per SM (it takes all of TMEM)
+        const size_t smem = std::max<size_t>(120 * 1024, sm_fixed_smem(panels) + (size_t)p.n_ct * panels * kSmPanel);
+        if (p.d <= 4)
+            KM_TRY((launch_small_dp<4, TWICE>(tmB, p, grid, smem, s)));
+        else if (p.d <= 8)
+            KM_TRY((launch_small_dp<8, TWICE>(tmB, p, grid, smem, s)));
+        else if (p.d <= 12)
+            KM_TRY((launch_small_dp<12, TWICE>(tmB, p, grid, smem, s)));
+        else if (p.d <= 15)
+            KM_TRY((launch_small_dp<16, TWICE>(tmB, p, grid, smem, s)));
+        else
+            KM_TRY((launch_small_dp<32, TWICE>(tmB, p, grid, smem, s)));
+    }
+    return KM_OK;
+}
+
 template <int DP>
-void launch_small_full(const float *X, int64_t n, int d, int k, const TcBuffers &b, int32_t *labels,
+void launch_small_full(const float *X, int64_t n, int d, int k, const TcBuffers &b, int64_t cap, int32_t *labels,
                        const FlipList *fl, unsigned grid, cudaStream_t s) {
-    small_full_kernel<DP><<<grid, 256, 0, s>>>(X, d, k, b.scg, b.full_frames, b.counters + 1, n, labels, b.flipped,
-                                               fl ? fl->rows : nullptr, fl ? fl->count : nullptr, fl ? fl->cap : 0);
+    small_full_kernel<DP><<<grid, kFullWarps * 32, 0, s>>>(
+        X, d, k, b.scg, b.full_frames, b.counters + 1, n, b.wide_thr, reinterpret_cast<const uint16_t *>(b.wide_bits),
+        sm_bit_row(k) / 2, cap, sm_twice_few(d, k), labels, b.flipped, fl ? fl->rows : nullptr, fl ? fl->count : nullptr, fl ? fl->cap : 0);
 }
 
 }  // namespace
@@ -738,6 +971,14 @@ int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuf
     p.labels = labels;
     p.label_counts = label_counts;
     p.full_frames = b.full_frames;
+    p.full_thr = b.wide_thr;
+    // (beside the caller's next work a list of up to a sixteenth of the frames
+    // costs nothing, and a second pass before it does: 4.3M x 10, k = 1000, with
+    // 1% listed 1.10 -> 1.12 ms per Lloyd iteration)
+    p.cap = side ? 0 : b.wide_cap;
+    p.bits = reinterpret_cast<uint8_t *>(b.wide_bits);
+    p.bit_row = sm_bit_row(k);
+    p.few = sm_twice_few(d, k);
     p.counters = b.counters;
     p.err = b.err;
 
@@ -747,24 +988,8 @@ int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuf
     const int64_t n_tiles = (n + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(num_sms(), n_tiles);
     if (prof) prof->begin(kProfTc, s);
-    for (int t = 0; t < tiles; t += per) {
-        p.ct0 = t;
-        p.n_ct = std::min(per, tiles - t);
-        p.first = t == 0;
-        p.last = t + p.n_ct == tiles;
-        // at least 120 KB: one CTA per SM (it takes all of TMEM)
-        const size_t smem = std::max<size_t>(120 * 1024, sm_fixed_smem(panels) + (size_t)p.n_ct * panels * kSmPanel);
-        if (d <= 4)
-            KM_TRY(launch_small<4>(tmB, p, grid, smem, s));
-        else if (d <= 8)
-            KM_TRY(launch_small<8>(tmB, p, grid, smem, s));
-        else if (d <= 12)
-            KM_TRY(launch_small<12>(tmB, p, grid, smem, s));
-        else if (d <= 15)
-            KM_TRY(launch_small<16>(tmB, p, grid, smem, s));
-        else
-            KM_TRY(launch_small<32>(tmB, p, grid, smem, s));
-    }
+    KM_TRY(launch_small<false>(tmB, p, tiles, per, grid, s));
+    if (p.cap > 0) KM_TRY(launch_small<true>(tmB, p, tiles, per, grid, s));
     if (prof) prof->end(kProfTc, s);
     cudaStream_t r = side ? side : s;
     if (side) {
@@ -774,13 +999,13 @@ int small_assign(const float *X, int64_t n, int d, int k, int32_t *labels, TcBuf
     if (prof) prof->begin(kProfFull, r);
     const unsigned fgrid = (unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)num_sms() * 4);
     if (d <= 4)
-        launch_small_full<4>(X, n, d, k, b, labels, fl, fgrid, r);
+        launch_small_full<4>(X, n, d, k, b, p.cap, labels, fl, fgrid, r);
     else if (d <= 8)
-        launch_small_full<8>(X, n, d, k, b, labels, fl, fgrid, r);
+        launch_small_full<8>(X, n, d, k, b, p.cap, labels, fl, fgrid, r);
     else if (d <= 16)
-        launch_small_full<16>(X, n, d, k, b, labels, fl, fgrid, r);
+        launch_small_full<16>(X, n, d, k, b, p.cap, labels, fl, fgrid, r);
     else
-        launch_small_full<32>(X, n, d, k, b, labels, fl, fgrid, r);
+        launch_small_full<32>(X, n, d, k, b, p.cap, labels, fl, fgrid, r);
     KM_CUDA(cudaGetLastError());
     if (prof) prof->end(kProfFull, r);
     return KM_OK;

@@ -141,8 +141,7 @@ int resolve_precision(int precision, int d, int k, bool check_device) {
 //     kernel's instructions, on.  Above: 200k x 2, k = 250 72 -> 67; 200k x 5, k
 //     = 100 76 -> 68; 2M x 4, k = 500 964 -> 230.  Below: 200k x 2, k = 100 58
 //     -> 61; 60k x 5, k = 250 53 -> 59.  Not for d = 1: there the centers lie
-//     so densely that 5-89% of the frames are re-checked over all of them (1M,
-//     k = 1000 506 -> 1024).
+//     so densely that 5-89% of the frames are taken a second time.
 constexpr double kSmallMinWork = 3.5e8;
 bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_device) {
     // The cheap tests first: small calls are host-bound, and the plan lookups
@@ -160,17 +159,18 @@ bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_de
     return g_tune.choice.count(std::make_pair(d, k)) == 0;
 }
 
-// The workspace of an assignment; small: the narrow-frame kernel may run
-// (its center half and lists; the FP16 form's workspace holds both).  An
-// assignment that resolves to FP32 needs none of it: with less room it takes
-// the exact kernel (the labels are the same).
+// The workspace of an assignment; small: the narrow-frame kernel may run (its
+// center half and lists).  With less room than that the kernels of `prec` run
+// instead, which need none under FP32 (the labels are the same).
 size_t small_ws_bytes(int64_t n, int d, int k) {
     return tc_centers_ws_size(d, k) + small_lists_ws_size(n, d, k) + 2 * 256;
 }
 
 size_t assign_ws_bytes(int64_t n, int d, int k, int prec, bool small = false) {
-    if (!is_tc(prec)) return small ? small_ws_bytes(n, d, k) : 0;
-    return tc_frames_ws_size(n, d) + tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k, prec) + 3 * 256;
+    const size_t narrow = small ? small_ws_bytes(n, d, k) : 0;
+    if (!is_tc(prec)) return narrow;
+    return std::max(narrow, tc_frames_ws_size(n, d) + tc_centers_ws_size(d, k) + tc_assign_ws_size(n, d, k, prec) +
+                                3 * 256);
 }
 
 void carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b) {
@@ -273,14 +273,14 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
         return KM_ERR_UNSUPPORTED;
     }
     bool small = !ps && small_route(precision, prec, n, d, k, true);
-    if (small && !is_tc(prec)) small = ws && ws_bytes >= small_ws_bytes(n, d, k);
+    small = small && ws && ws_bytes >= small_ws_bytes(n, d, k);
     KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec, small)));
     TcBuffers b;
-    if (is_tc(prec) && n > 0) {
+    if (small && n > 0) {
+        carve_small(ws, n, d, k, b);
+    } else if (is_tc(prec) && n > 0) {
         carve_assign(ws, n, d, k, prec, b);
         tc_set_operand(b, d, prec);
-    } else if (small && n > 0) {
-        carve_small(ws, n, d, k, b);
     }
     if (ps && prec == KM_PREC_FP8) {
         set_error("FP8 operands are not built for coordinate frames");
@@ -291,8 +291,9 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
 
 // Workspace of an assignment whose centers are prepared: frames + lists.
 size_t resident_ws_bytes(int64_t n, int d, int k, int prec, bool small) {
-    if (!is_tc(prec)) return small ? small_lists_ws_size(n, d, k) + 256 : 0;
-    return tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k, prec) + 2 * 256;
+    const size_t narrow = small ? small_lists_ws_size(n, d, k) + 256 : 0;
+    if (!is_tc(prec)) return narrow;
+    return std::max(narrow, tc_frames_ws_size(n, d) + tc_assign_ws_size(n, d, k, prec) + 2 * 256);
 }
 
 // dst (device) <- src (host memory that the device reads in place, or any
@@ -452,8 +453,7 @@ struct km_centers {
 };
 
 bool km_centers::small_for(int64_t n, const void *ws, size_t ws_bytes) const {
-    if (!small_for(n)) return false;
-    return is_tc(prec) || (ws && ws_bytes >= resident_ws_bytes(n, d, k, prec, true));
+    return small_for(n) && ws && ws_bytes >= small_lists_ws_size(n, d, k);
 }
 
 namespace km {
@@ -946,10 +946,10 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     const LloydFrames of = ps ? LloydFrames::kPairs : pair_rows ? LloydFrames::kPairRows : LloydFrames::kRows;
     const LloydRoute route = lloyd_route(n, d, k, precision, prec, of, true);
     bool small = route.small, fits = route.fits;
-    if (small && !is_tc(prec) && workspace_bytes < lloyd_ws_bytes(n, d, k, prec, true)) {
-        // the run needs no narrow-frame kernel: without its room, as FP32
+    if (small && workspace_bytes < lloyd_ws_bytes(n, d, k, prec, true, false)) {
+        // without its room, by the kernels of `prec`
         small = false;
-        fits = of == LloydFrames::kRows && small_lloyd_ok(n, d, k);
+        fits = of == LloydFrames::kRows && !is_tc(prec) && small_lloyd_ok(n, d, k);
     }
     const bool tc = is_tc(prec) || small;
     KM_TRY(check_ws(workspace, workspace_bytes, lloyd_ws_bytes(n, d, k, prec, small, false)));
@@ -1092,7 +1092,7 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
     if (tc) {
         // The shift and scale stay fixed for the whole run so that the 16-bit
         // frame copy is made once (narrow frames have none).
-        if (is_tc(prec)) {
+        if (!small) {
             carve_assign(ws_assign, n, d, k, prec, b);
             tc_set_operand(b, d, prec);
         } else {
@@ -1128,6 +1128,12 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         KM_CUDA(cudaMemcpyAsync(C, C_new, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, st));
         return KM_OK;
     };
+    // Narrow frames: the listed frames are settled before the sums (the first
+    // iteration, and all of a run whose first one listed more than a
+    // sixteenth), or beside them, with the changed labels moved afterwards: a
+    // move is 2 d float64 atomics, and frames on a lattice change by the
+    // hundred thousand (1M x 2, k = 500, five iterations: 3.3 -> 2.0 ms).
+    bool settle_first = small;
     auto enqueue = [&](cudaStream_t st) -> int {
         if (tc) {
             KM_TRY(small ? small_prepare_centers(C, d, k, b, st) : tc_prepare_centers(C, d, k, b, st));
@@ -1135,11 +1141,16 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
                 KM_TRY(tc_bounds_masks(C, n, d, k, labels, b, bounds, st));
                 b.keep_err = 1;  // cleared by the masks' pass
             }
-            KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
+            if (!settle_first) KM_CUDA(cudaMemsetAsync(fl.count, 0, sizeof(int32_t), st));
             // the tensor-core pass counts the members as it writes the labels
-            int32_t *counts =
-                update_counts_from_labels(d, k, ps, pair_rows) ? update_counts(ws_update, n, d, k) : nullptr;
+            int32_t *counts = !settle_first && update_counts_from_labels(d, k, ps, pair_rows)
+                                  ? update_counts(ws_update, n, d, k)
+                                  : nullptr;
             if (counts) KM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * k, st));
+            if (settle_first) {
+                KM_TRY(small_assign(X, n, d, k, labels, b, st, &prof));
+                return enqueue_update(st);
+            }
             if (small)
                 KM_TRY(small_assign(X, n, d, k, labels, b, st, &prof, side.st, side.fork[0], &fl, counts));
             else
@@ -1364,17 +1375,23 @@ int lloyd_run(const float *X_in, const HostFrames *hf, int64_t n, int32_t d, int
         }
         if (status != KM_OK) break;
         double h_cost = 0.0;
-        uint32_t h_err = 0, tc_err = 0;
+        uint32_t h_err = 0;
+        TcStatus tc_st = {};
         cudaError_t e = cudaMemcpyAsync(&h_cost, cost, sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && tc)
-            e = cudaMemcpyAsync(&tc_err, b.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            e = cudaMemcpyAsync(&tc_st, b.counters, sizeof(tc_st), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             status = cuda_fail(e, "Lloyd iteration");
             break;
         }
-        h_err |= tc_err | take_fake_device_error();
+        h_err |= tc_st.err | take_fake_device_error();
+        if (it == 0 && small) {
+            // (with host frames the counts are those of the last chunk)
+            const int64_t seen = hf ? n - sm.begin[sm.begin.size() - 2] : n;
+            settle_first = tc_st.counters[1] > seen / 16;
+        }
         prof.collect();
         status = check_device_errors(h_err);
         if (status != KM_OK) break;
