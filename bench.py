@@ -206,6 +206,24 @@ def tc_chunks(n):
     return max(1, min(want, n >> 18))
 
 
+def lloyd_launches(n, steps):
+    """Kernels of one km_lloyd call of `steps` iterations on n frames of the
+    headline workload (16-bit operands, features of a trajectory).  Each:
+    the centers' operands; per chunk of the tensor-core pass its launch (which
+    also counts the members) and 3 candidate re-checks; the second pass for
+    overflowing lists (gather, launch, settle) and 3 full re-checks (short
+    list, tiled, finalize); 6 of the update (scan, scatter, segment sums,
+    flips, finalize, cost).  Once: shift, center norms, scale, frame copy.
+    From the second iteration on: the loop's step.  From 4 iterations on a run
+    keeps center bounds: the centers' moves each, once the neighbour test and
+    the center groups and order, from the second iteration on the centers as
+    frames, their tile bounds and the masks."""
+    once, each, later = 4, 1 + 4 * tc_chunks(n) + 6 + 6, 1
+    if steps >= 4:
+        once, each, later = once + 3, each + 1, later + 3
+    return each * steps + later * (steps - 1) + once
+
+
 def tc_roofline(n, tc_ms, tc_n, timed_ms, k=K, d=D):
     """Roofline record of the tensor-core distance kernel: 2 n k d flops per
     launch over its mean CUDA-event launch time, against the measured bf16
@@ -641,354 +659,12 @@ def run_ours(args):
         dist.destroy_process_group()
     if rank != 0:
         return
-    # Per iteration: prep_centers; per chunk of the tensor-core pass the
-    # tensor-core launch (which also counts the members) and 3 candidate
-    # re-check kernels; the second pass for overflowing lists (gather,
-    # tensor-core launch, settle) and 3 full re-check kernels (short list,
-    # tiled, finalize); 6 centroid-update kernels (scan, scatter, segment sums,
-    # flips, finalize, cost) and the centers' moves.  From the second iteration
-    # of a call on: the centers as frames, their tile bounds, the masks, and
-    # the loop step.  Once per km_lloyd call: shift, center norms, scale, FP16
-    # frame copy, the neighbour test, center groups and order.
-    launches_per_step = 1 + 4 * tc_chunks(n) + 6 + 7
-    line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": args.gpus, "steps": steps,
-            "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f32 distances, f64 sums", "data": "synthetic (seeded C-alpha distances)",
-            "config": config(args, {"precision": "fp32 (CPU)"}), "impl": "reference",
-            "cpu_baseline": {"value": value, "unit": UNIT, "cores": threads, "kind": "port", "sample": sample},
-            "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
-
-
-# ---------------------------------------------------------------------------
-# GPU arm
-# ---------------------------------------------------------------------------
-def run_ours(args):
-    import torch
-    from pyemma_gb300 import _lib, datasets
-    from pyemma_gb300.coordinates import KmeansClustering
-
-    world = int(os.environ.get("WORLD_SIZE", "1"))
-    rank = int(os.environ.get("RANK", "0"))
-    local = int(os.environ.get("LOCAL_RANK", "0"))
-    torch.cuda.set_device(local)
-    dist = None
-    if world > 1:
-        import torch.distributed as dist
-        dist.init_process_group(backend="nccl", device_id=torch.device("cuda", local))
-
-    def barrier():
-        if dist is not None:
-            dist.barrier()
-        torch.cuda.synchronize()
-
-    _lib.load()
-    n = args.frames
-    X = datasets.calpha_distances(n_frames=n, seed=rank_seed(rank), device="cuda")
-    rng = np.random.default_rng(rank_seed(rank))
-    C0 = X[torch.from_numpy(rng.choice(n, K, replace=False)).cuda()].contiguous()
-    torch.cuda.synchronize()
-
-    sampler = ClockSampler(gpu_id_for_smi(torch)) if rank == 0 else None
-    if sampler:
-        sampler.start()
-
-    # warm-up (also builds the one-time state of the library)
-    C = C0.clone()
-    _lib.lloyd(X, C, max(3, args.warmup), -1.0, precision="fp16")
-
-    # ---- timed region: K Lloyd iterations, graph-launched ----
-    C = C0.clone()
-    _lib.profile_enable(True)
-    barrier()
-    t_wall0 = time.time()
-    ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    ev0.record()
-    res = _lib.lloyd(X, C, args.steps, -1.0, precision="fp16")
-    ev1.record()
-    torch.cuda.synchronize()
-    barrier()
-    t_wall1 = time.time()
-    ms = ev0.elapsed_time(ev1)
-    prof = _lib.profile_read()
-    _lib.profile_enable(False)
-    assert res["n_iter"] == args.steps
-    ms_max = max_over_ranks(ms, dist, "cuda")
-    ms_per_step = ms_max / args.steps
-    value = whole_job_rate(world, n, args.steps, ms_max)
-
-    clocks = sampler.summary(t_wall0, t_wall1) if sampler else None
-    if sampler:
-        # nvidia-smi's queries take driver locks: keep them out of the
-        # end-to-end copies measured below
-        sampler.stop()
-        sampler = None
-
-    # ---- roofline of the tensor-core distance kernel ----
-    # In the step, one iteration's pass is tc_chunks(n) launches with the
-    # exact re-check of each chunk beside the next: ms_per_launch is the span
-    # from the first launch's start to the last one's end.  The same kernel
-    # alone (one launch over all frames, the re-check after it) is timed
-    # below as "isolated".
-    # Both compare every frame with every center (KM_TC_BOUNDS=0); the timed
-    # steps skip the center tiles the triangle inequality rules out, so their
-    # pass has no 2 n k d flops to divide.
-    def full_pass(steps, **env):
-        old = {key: os.environ.get(key) for key in env}
-        os.environ.update(env)
-        try:
-            Ci = C0.clone()
-            _lib.lloyd(X, Ci, 2, -1.0, precision="fp16")
-            Ci = C0.clone()
-            _lib.profile_enable(True)
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            _lib.lloyd(X, Ci, steps, -1.0, precision="fp16")
-            e1.record()
-            torch.cuda.synchronize()
-            iprof = _lib.profile_read()
-            _lib.profile_enable(False)
-            r = tc_roofline(n, iprof["tc"][0], iprof["tc"][1], e0.elapsed_time(e1))
-            r["ms_per_step"] = e0.elapsed_time(e1) / steps
-            return r
-        finally:
-            for key, value in old.items():
-                if value is None:
-                    del os.environ[key]
-                else:
-                    os.environ[key] = value
-
-    full_steps = 20
-    roofline = full_pass(full_steps, KM_TC_BOUNDS="0")
-    roofline["step_breakdown_ms"] = {k: (v[0] / v[1] if v[1] else None) for k, v in prof.items()}
-    roofline["chunks_per_iteration"] = tc_chunks(n)
-    roofline["span"] = ("ms_per_launch: one full iteration's tensor-core pass (KM_TC_BOUNDS=0, %d iterations), %d "
-                        "launches over consecutive frame ranges, from the first start to the last end, each chunk's "
-                        "exact re-check running beside the next launch; step_breakdown_ms: the timed steps"
-                        % (full_steps, tc_chunks(n)))
-    if rank == 0:
-        iso = full_pass(full_steps, KM_TC_BOUNDS="0", KM_TC_CHUNKS="1")
-        roofline["isolated"] = {key: iso[key] for key in ("achieved", "frac", "issued_tflops", "frac_issued",
-                                                           "ms_per_launch", "launches", "peak_source", "ms_per_step")}
-        roofline["isolated"]["how"] = ("the same kernel as one launch over all %d frames per iteration "
-                                       "(KM_TC_CHUNKS=1), %d iterations" % (n, full_steps))
-
-    extra = {}
-    if rank == 0:
-        # assignment statistics and exactness against the plain FP32 kernel
-        lab16, st = _lib.assign(X, C, precision="fp16")
-        extra["recheck_fraction"] = (st["n_recheck"] + st["n_full"]) / float(n)
-        extra["full_recheck_frames"] = st["n_full"]
-        extra["flipped_ties"] = st["n_flipped"]
-        if not args.no_fp32:
-            lab32, _ = _lib.assign(X, C, precision="fp32")
-            extra["dtrajs_identical_to_fp32"] = bool(torch.equal(lab16, lab32))
-            del lab32
-            # plain FP32 Lloyd iteration for the mixed-vs-FP32 ratio
-            Cf = C0.clone()
-            _lib.lloyd(X, Cf, 1, -1.0, precision="fp32")
-            Cf = C0.clone()
-            steps32 = 2
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            _lib.lloyd(X, Cf, steps32, -1.0, precision="fp32")
-            e1.record()
-            torch.cuda.synchronize()
-            fp32_value = n * steps32 / (e0.elapsed_time(e1) / 1e3)
-            extra["plain_fp32"] = {"value": fp32_value, "unit": UNIT, "steps": steps32}
-            extra["mixed_vs_plain_fp32"] = (value / world) / fp32_value
-        del lab16
-    if rank == 0 and not args.no_kmpp:
-        # kmeans++ (k rounds of D^2 sampling) on the same frames
-        _lib.kmpp(X[:65536].contiguous(), 8, 42)
-        torch.cuda.synchronize()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        _, kidx = _lib.kmpp(X, K, 42)
-        e1.record()
-        torch.cuda.synchronize()
-        kmpp_ms = e0.elapsed_time(e1)
-        unpruned = float(K) * n * (4 * D + 8)
-        extra["kmeans++"] = {"ms": kmpp_ms, "rounds": K, "ms_per_round": kmpp_ms / K,
-                             "unpruned_bytes": unpruned,
-                             "unpruned_bytes_per_s": unpruned / (kmpp_ms / 1e3),
-                             "note": "km_kmpp, k=%d on all %d frames (seed 42); unpruned_bytes = k N (4d + 8), "
-                                     "the bytes a pass without distance bounds would read" % (K, n)}
-        del kidx
-
-    # ---- e2e through the public API from pinned host frames ----
-    e2e = None
-    if rank == 0 and not args.no_e2e:
-        Xh = torch.empty((n, D), dtype=torch.float32, pin_memory=True)
-        Xh.copy_(X)
-        Xh_np = Xh.numpy()
-        C0h = C0.cpu().numpy()
-        if not args.no_fp64:
-            # centers and inertia of one more iteration (from the timed run's
-            # centers) against the float64 reference on the same labels
-            C_prev = C.clone()
-            r1 = _lib.lloyd(X, C, 1, -1.0, precision="fp16")
-            extra.update(fp64_reference_check(Xh_np, r1["labels"].cpu().numpy(), C_prev.cpu().numpy(),
-                                              C.cpu().numpy(), float(r1["inertias"][0])))
-            del r1, C_prev
-        # the bare pinned host-to-device rate of this machine, for reading e2e
-        # (the best of three copies: a single one has read low on a busy host)
-        ec0, ec1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        X.copy_(Xh, non_blocking=True)
-        copy_ms = []
-        for _ in range(3):
-            ec0.record()
-            X.copy_(Xh, non_blocking=True)
-            ec1.record()
-            torch.cuda.synchronize()
-            copy_ms.append(ec0.elapsed_time(ec1))
-        link_gbs_engine = n * D * 4 / (min(copy_ms) / 1e3) / 1e9
-        # the same bytes through the library's own host copy (km_lloyd_host
-        # with no iteration: the copy kernel alone), best of three
-        kernel_ms = []
-        Cq = C0.clone()
-        for _ in range(4):
-            torch.cuda.synchronize()
-            tk = time.perf_counter()
-            _lib.lloyd_host([Xh_np], Cq, 0, -1.0, precision="fp16", X=X)
-            torch.cuda.synchronize()
-            kernel_ms.append((time.perf_counter() - tk) * 1e3)
-        link_gbs_kernel = n * D * 4 / (min(kernel_ms[1:]) / 1e3) / 1e9
-        link_gbs = max(link_gbs_engine, link_gbs_kernel)
-        del X, Cq  # the API makes its own device copy
-        torch.cuda.empty_cache()
-        # Warm-up: the first passes over a freshly allocated multi-GB pinned
-        # buffer run slower (32 against 21 ms per call here) while its pages
-        # are first mapped for the device; W >= 3 calls precede the timing.
-        e2e_warm = max(3, args.warmup)
-        for _ in range(e2e_warm):
-            KmeansClustering(n_clusters=K, max_iter=1, tolerance=-1.0, clustercenters=C0h,
-                             precision="fp16").estimate(Xh_np)
-        e2e_steps = max(1, min(args.steps, 8))
-        copy_ms_best = n * D * 4 / (link_gbs * 1e9) * 1e3
-
-        def e2e_round(frames):
-            # e2e_steps calls, each with its own clock; the mean is the rate.
-            # A call that took more than twice the bare copy of its frames met
-            # a disturbed host link (other users' traffic on the shared host):
-            # such a round is kept in the line as rejected and taken once more.
-            rounds = []
-            for _ in range(2):
-                step = []
-                torch.cuda.synchronize()
-                t0 = time.perf_counter()
-                for _ in range(e2e_steps):
-                    ts = time.perf_counter()
-                    km = KmeansClustering(n_clusters=K, max_iter=1, tolerance=-1.0, clustercenters=C0h,
-                                          precision="fp16")
-                    km.estimate(frames)
-                    _ = km.clustercenters  # host result (already copied back by estimate)
-                    step.append((time.perf_counter() - ts) * 1e3)
-                rounds.append(((time.perf_counter() - t0) / e2e_steps, step))
-                if max(step) <= 2.0 * copy_ms_best:
-                    break
-            rejected = [{"step_ms": st, "reason": "a call took more than twice the bare copy (%.1f ms)"
-                         % copy_ms_best} for _, st in rounds[:-1]]
-            return rounds[-1][0], rounds[-1][1], rejected
-
-        dt, step_ms, rejected = e2e_round(Xh_np)
-        e2e = {"value": n / dt, "unit": UNIT, "h2d_bytes_per_step": n * D * 4, "d2h_bytes_per_step": K * D * 4 + 8,
-               "api": "KmeansClustering(n_clusters=2000, max_iter=1, clustercenters=C).estimate(pinned host X)",
-               "steps": e2e_steps, "warmup": e2e_warm, "step_ms": step_ms, "rejected_rounds": rejected,
-               "h2d_link_gbs": link_gbs,
-               "h2d_link_gbs_copy_engine": link_gbs_engine, "h2d_link_gbs_copy_kernel": link_gbs_kernel,
-               "copy_bound_frames_per_s": link_gbs * 1e9 / (D * 4),
-               "overlap": "frames copied in chunks on a side stream while the first iteration assigns "
-                          "the chunks already copied (km_lloyd_host)"}
-        # The same call with the frames in an ordinary (pageable) numpy
-        # array, as PyEMMA callers hold them: where the GPU reads host memory
-        # in place (Grace), a device kernel copies the chunks; elsewhere the
-        # library stages them through page-locked buffers on worker threads.
-        Xpg = np.empty_like(Xh_np)
-        Xpg[...] = Xh_np
-        del Xh, Xh_np
-        for _ in range(e2e_warm):
-            KmeansClustering(n_clusters=K, max_iter=1, tolerance=-1.0, clustercenters=C0h,
-                             precision="fp16").estimate(Xpg)
-        dtp, step_ms_pg, rejected_pg = e2e_round(Xpg)
-        e2e["pageable"] = {"value": n / dtp, "unit": UNIT, "h2d_bytes_per_step": n * D * 4,
-                           "d2h_bytes_per_step": K * D * 4 + 8, "vs_pinned": (n / dtp) / e2e["value"],
-                           "step_ms": step_ms_pg, "rejected_rounds": rejected_pg,
-                           "api": "KmeansClustering(max_iter=1, clustercenters=C).estimate(pageable numpy X)"}
-        del Xpg
-        # The same iteration from pinned host C-alpha coordinates: the 528
-        # pair distances are never written out; every kernel that reads a
-        # feature computes it from the coordinates (km_lloyd_pairs), so 396
-        # bytes per frame cross the host link and no n x 528 matrix exists.
-        from pyemma_gb300 import featurize
-        xyz_d = datasets.calpha_coordinates(n_frames=n, seed=SEED + rank)
-        xyz_h = torch.empty(tuple(xyz_d.shape), dtype=torch.float32, pin_memory=True)
-        xyz_h.copy_(xyz_d)
-        src = featurize.pair_distance_frames(xyz_d, excluded_neighbors=0)
-        # Lloyd iterations on device-resident coordinates, for the step time
-        Cp = C0.clone()
-        _lib.lloyd_pairs(src.xyz, src.pairs, Cp, 2, -1.0, precision="fp16")
-        Cp = C0.clone()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        _lib.lloyd_pairs(src.xyz, src.pairs, Cp, 5, -1.0, precision="fp16")
-        e1.record()
-        torch.cuda.synchronize()
-        pair_ms = e0.elapsed_time(e1) / 5
-        del src, xyz_d, Cp
-        torch.cuda.empty_cache()
-        for _ in range(e2e_warm):
-            km = KmeansClustering(n_clusters=K, max_iter=1, tolerance=-1.0, clustercenters=C0h, precision="fp16")
-            km.estimate(featurize.pair_distance_frames(xyz_h, excluded_neighbors=0))
-        torch.cuda.synchronize()
-        t0 = time.perf_counter()
-        for _ in range(e2e_steps):
-            km = KmeansClustering(n_clusters=K, max_iter=1, tolerance=-1.0, clustercenters=C0h, precision="fp16")
-            km.estimate(featurize.pair_distance_frames(xyz_h, excluded_neighbors=0))
-            _ = km.clustercenters
-        dtc = (time.perf_counter() - t0) / e2e_steps
-        kp = 64 * (-(-(D + 2) // 64))
-        e2e["from_coordinates"] = {
-            "value": n / dtc, "unit": UNIT, "h2d_bytes_per_step": n * 33 * 3 * 4, "d2h_bytes_per_step": K * D * 4 + 8,
-            "api": "KmeansClustering(max_iter=1).estimate(featurize.pair_distance_frames(pinned host xyz (n, 33, 3)))",
-            "feature_matrix_bytes": 0,
-            "device_lloyd_ms_per_iter": pair_ms,
-            "hbm_bytes_per_iter": {"fp16_copy": n * kp * 2, "coordinates": n * 33 * 3 * 4,
-                                   "dense_path_float32_features": n * D * 4},
-            "workload": "same chain model, coordinates instead of precomputed distances; the features are computed "
-                        "where they are read (km_lloyd_pairs)"}
-        del xyz_h
-
-    # ---- CPU baseline (rank 0, N=1) ----
-    cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu:
-        threads = len(os.sched_getaffinity(0))
-        Xc = datasets.calpha_distances(n_frames=40000, seed=SEED)
-        rate, S, dt = cpu_lloyd_rate(Xc, C0.cpu().numpy(), 12.0, threads)
-        cpu = {"value": rate, "unit": UNIT, "cores": threads, "kind": "port",
-               "sample": "%d C-alpha frames (d=%d) x k=%d centers, one oracle Lloyd iteration, %.1f s"
-                         % (S, D, K, dt)}
-
-    if sampler:
-        sampler.stop()
-    if dist is not None:
-        dist.barrier()
-        dist.destroy_process_group()
-    if rank != 0:
-        return
-    # Per iteration: prep_centers; per chunk of the tensor-core pass the
-    # tensor-core launch (which also counts the members), 3 candidate
-    # re-check kernels and 3 full re-check kernels (short list, tiled,
-    # finalize); 6 centroid-update kernels (scan, scatter, segment sums,
-    # flips, finalize, cost).  Once per km_lloyd call: shift, center norms,
-    # scale, FP16 frame copy.
-    launches_per_step = 1 + 7 * tc_chunks(n) + 6
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "fp16 distances (fp32 accumulate), fp32 recheck, f64 sums",
             "data": "synthetic (seeded C-alpha distances, generated on device)",
             "config": config(args), "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks,
-            "gpu_launches": launches_per_step * args.steps + 4 * (args.steps - 1) + 7}
+            "gpu_launches": lloyd_launches(n, args.steps)}
     line.update(extra)
     print(json.dumps(line), flush=True)
 
@@ -1100,8 +776,8 @@ def run_c2(args):
     X = torch.from_numpy(np.concatenate(trajs)).cuda()
     rng = np.random.default_rng(SEED)
     C0 = X[torch.from_numpy(rng.choice(n, 1000, replace=False)).cuda()].contiguous()
-    # the library's own choice (precision "auto": FP16 tensor cores with the
-    # exact re-check at d = 10, k = 1000) and the plain exact FP32 kernel
+    # the library's own choice (precision "auto": the narrow-frame tensor-core
+    # kernel at d = 10, k = 1000) and the plain exact FP32 kernel
     ms, prof = _lloyd_rate(torch, _lib, X, C0, args.steps, "auto")
     ms32, prof32 = _lloyd_rate(torch, _lib, X, C0, args.steps, "fp32")
     lab_a, st_a = _lib.assign(X, C0, precision="auto")
@@ -1149,14 +825,14 @@ def run_c2(args):
            "unit": "frames/s", "n_gpus": 1, "steps": args.steps, "ms_per_step": ms, "higher_is_better": True,
            "dtype": "fp16 distances (fp32 accumulate) + exact fp32 recheck, f64 sums (precision auto)",
            "config": {"workload": "c2: 20 AR(1) metastable trajectories, lengths log-uniform [50k, 500k] "
-                                  "(%d frames), d=10, k=1000, one CUDA graph per Lloyd iteration" % n,
+                                  "(%d frames), d=10, k=1000, Lloyd iterations as one device-side loop" % n,
                       "lengths": [len(t) for t in trajs]},
-           "labels_identical_to_fp32": same, "recheck_fraction": st_a["n_recheck"] / float(n),
+           "labels_identical_to_fp32": same, "recheck_fraction": (st_a["n_recheck"] + st_a["n_full"]) / float(n),
            "tile_tuning": tiles,
            "roofline": {"bound": "tensor-core epilogue: 1,000 accumulator columns per frame through tcgen05.ld and the "
-                                 "candidate test; the MMA issues one 16-wide K step (10 features and 2 norm "
-                                 "columns) per center tile",
-                        "kernel": "tc_assign_kernel", "achieved": flops / (tc_ms / 1e3) / 1e12 if tc_ms else None,
+                                 "scan for the best group of eight; the MMA issues three 16-wide K steps (four "
+                                 "columns per feature and for the norm) per center tile",
+                        "kernel": "small_assign_kernel", "achieved": flops / (tc_ms / 1e3) / 1e12 if tc_ms else None,
                         "peak": tpeak, "unit": "TFLOP/s",
                         "frac": (flops / (tc_ms / 1e3) / 1e12) / tpeak if tc_ms else None,
                         "step_breakdown_ms": {k: (v[0] / v[1] if v[1] else None) for k, v in prof.items()}},
