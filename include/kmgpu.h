@@ -68,7 +68,8 @@ typedef enum {
  * KM_PREC_FP16, and under KM_PREC_AUTO where it resolves to KM_PREC_FP32 and
  * the call is large: operands split into two FP16 parts single out eight
  * centers per frame, whose exact float32 distances give the label; frames it
- * cannot settle (counted in n_full) are evaluated over all centers.  Same
+ * cannot settle (counted in n_full) are evaluated over all centers, or, in
+ * long lists of large calls, over those a second pass finds near enough.  Same
  * labels; the reported precision is the one AUTO resolved to. */
 typedef enum {
     KM_PREC_FP32 = 0,
@@ -86,7 +87,7 @@ typedef void (*km_callback)(void *user);
 typedef struct {
     int64_t n_frames;   /* frames assigned */
     int64_t n_recheck;  /* frames re-evaluated exactly over their candidate list */
-    int64_t n_full;     /* frames re-evaluated exactly over all k centers */
+    int64_t n_full;     /* frames whose list could not hold or settle them: exact over all k centers (or a second pass) */
     int64_t n_flipped;  /* frames whose exact label differs from the tensor-core argmin */
     int32_t precision;  /* precision actually used (km_precision) */
     int32_t reserved;
@@ -324,7 +325,8 @@ int km_debug_force_tile_plan(const km_tile_plan *plan);
  * (device, max_centers*d floats) receives them, *n_centers (host) their
  * number.  When a (max_centers+1)-th center would be added the walk stops
  * and *converged (host) is 0 (the reference's MaxCentersReached case).
- * Synchronises `stream` once per 65,536 frames. */
+ * Synchronises `stream`: at the end and, for d <= 32, every 16 chunks of up
+ * to 262,144 frames; for d > 32 after each chunk of up to 65,536. */
 size_t km_regspace_workspace_size(int32_t d);
 int km_regspace(const float *X, int64_t n, int32_t d, double dmin, int32_t max_centers, float *centers,
                 int32_t *n_centers, int32_t *converged, void *workspace, size_t workspace_bytes, void *stream);

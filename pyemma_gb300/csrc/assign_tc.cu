@@ -1580,7 +1580,9 @@ bool plan_of(const TcBuffers &b, int d, int k, Plan &pl) {
 }
 
 float norm_inflate_of(int d) {
-    // A compensated float32 sum of d squares is within a few u of the true value.
+    // Bounds of norms are sums of d squares inflated by this: plain float32
+    // sums per lane of a warp (d / 32 and a few roundings) or compensated ones,
+    // both within (d + 8) u.
     return 1.0f + (float)(d + 8) * 5.9604645e-8f + 1e-6f;
 }
 
@@ -1756,9 +1758,10 @@ size_t carve_assign(void *ws, int64_t n, int d, int k, int prec, TcBuffers &b) {
     b.amb_mask = c.take<int32_t>(nn);
     b.full_frames = c.take<int32_t>(nn);
     b.full_keys = c.take<unsigned long long>(nn);
-    // [0] recheck entries, [1] full entries, [2] pairs, [3] entries left to the exact pass, then flipped (two words),
-    // err and a spare word; [kTcDiagWords..kChunkCounters0) diagnostics, or the second pass's two counts; then the first four again for chunks 1.. of
-    // a chunked pass
+    // [0] recheck entries, [1] full entries, [2] pairs, [3] entries left to
+    // the exact pass, then flipped (two words), err and a spare word;
+    // [kTcDiagWords..kChunkCounters0) diagnostics, or the second pass's two
+    // counts; then the first four again for chunks 1.. of a chunked pass
     b.counters = c.take<int32_t>(kChunkCounters0 + 4 * (kMaxTcChunks - 1));
     b.flipped = reinterpret_cast<unsigned long long *>(b.counters + 4);
     b.err = reinterpret_cast<uint32_t *>(b.counters + 6);
@@ -2734,9 +2737,6 @@ int tc_bounds_masks(const float *C, int64_t n, int d, int k, const int32_t *labe
     KM_CUDA(cudaGetLastError());
     return KM_OK;
 }
-
-namespace {
-}  // namespace
 
 int tc_assign(const float *X, int64_t n, int d, const float *C, int k, int32_t *labels, TcBuffers &b,
               cudaStream_t s, ProfEvents *prof, float *dump, unsigned long long *wait_cycles, const PairSrc *ps) {

@@ -474,7 +474,7 @@ struct RmsdWarpSmem {
 
 // Brackets one frame's pairs with the warp's 32 centers, lists the ones that
 // the smallest upper bound (returned) does not rule out.  Out of line: few
-// groups of centers need it, and eight copies of it would not stay in the
+// groups of centers need it, and a copy per frame would not stay in the
 // instruction cache.
 template <int F>
 __device__ __noinline__ float rmsd_candidates(RmsdWarpSmem<F> &sm, int f, const float (&S)[9], QcpQuartic qu,
