@@ -38,7 +38,7 @@ namespace {
 constexpr int kRmsdWarps = 8;  // warps per CTA
 
 // Every row of an (n, d) array centered into Xc, traces into G: a warp per
-// row.  For rows too long for rmsd_center_tile_kernel.
+// row.  For rows that rmsd_center_tile_kernel does not take.
 __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_center_kernel(const float *__restrict__ X, int64_t n, int d,
                                                                       float *__restrict__ Xc, double *__restrict__ G) {
     const int lane = threadIdx.x & 31;
@@ -67,15 +67,12 @@ __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_center_kernel(const floa
 // Rows outside these conditions take the float64 form.  1,000,000 rows of 58
 // atoms: 1.5 ms (FP64 pipe 40% busy); 5.9 ms with a warp per row, which
 // repeats the divisions and the tree in every lane.
-constexpr int kCenterMaxSmem = 200 * 1024;
 constexpr int kCenterSlicedAtoms = 128;  // a slice's sum of this many values is exact
+constexpr int kCenterMaxAtoms = 150;
+constexpr int kCenterWarps = 2;          // per CTA: 115 KB of rows at most
 
 int center_stride(int d) { return d | 1; }
-int center_warps(int d) {  // warps per CTA; 0: the rows do not fit
-    const int64_t per = (int64_t)32 * center_stride(d) * 4;
-    const int64_t w = kCenterMaxSmem / per;
-    return w >= 4 ? 2 : (int)std::min<int64_t>(w, 1);
-}
+size_t center_smem(int d) { return (size_t)kCenterWarps * 32 * center_stride(d) * sizeof(float); }
 
 // The tree of rmsd_center_row_warp (offsets 16, 8, 4, 2, 1) over the 32
 // partial sums leaf(l): leaves in bit-reversed order, equal subtrees added as
@@ -159,17 +156,16 @@ __device__ __forceinline__ double rmsd_widen(float v) {
     return __hiloint2double((int)((b & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(b << 29));
 }
 
-__global__ void __launch_bounds__(64) rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, int d,
+__global__ void __launch_bounds__(kCenterWarps * 32) rmsd_center_tile_kernel(const float *__restrict__ X, int64_t n, int d,
                                                               int stride, float *__restrict__ Xc,
                                                               double *__restrict__ G) {
-    extern __shared__ float center_smem[];
+    extern __shared__ float center_rows_s[];
     const int lane = threadIdx.x & 31;
-    const int warps = blockDim.x >> 5;
-    float *rows = center_smem + (size_t)(threadIdx.x >> 5) * 32 * stride;
+    float *rows = center_rows_s + (size_t)(threadIdx.x >> 5) * 32 * stride;
     const int n_atoms = d / 3;
     const int64_t tiles = (n + 31) / 32;
-    for (int64_t tile = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); tile < tiles;
-         tile += (int64_t)gridDim.x * warps) {
+    for (int64_t tile = (int64_t)blockIdx.x * kCenterWarps + (threadIdx.x >> 5); tile < tiles;
+         tile += (int64_t)gridDim.x * kCenterWarps) {
         const int64_t r0 = tile * 32;
         const int m = (int)(n - r0 < 32 ? n - r0 : 32);
         // the tile's rows are consecutive floats; eight loads in flight per lane
@@ -741,22 +737,26 @@ int check_rmsd_shape(int64_t n, int d, int k) {
 
 int center_rows(const float *X, int64_t n, int d, float *Xc, double *G, cudaStream_t s) {
     if (n == 0) return KM_OK;
-    const int warps = center_warps(d);
-    // a warp per row while the rows (centers, short calls) give every SM no
-    // more than a few tiles: the thread-per-row form takes 0.18 ms for one tile
-    if (warps > 0 && n >= (int64_t)num_sms() * 128) {
+    // A warp per row while the rows (centers, short calls) give every SM no
+    // more than a few tiles: the thread-per-row form takes 0.18 ms for one
+    // tile.  And for long rows, of which few fit beside each other (us for twice n
+    // rows and their distances, thread per row, warp per row: n = 100,000, 58
+    // atoms 422, 1291; 100 1101, 2696; 140 1874, 2152; 200 4419, 2808; 400
+    // 15,661, 4877; n = 20,000, 100 atoms 331, 587; 140 603, 485).
+    const int64_t tiles_from = (int64_t)num_sms() * (d <= 3 * kCenterSlicedAtoms ? 128 : 512);
+    if (d <= 3 * kCenterMaxAtoms && n >= tiles_from) {
         static bool attr_done[kDeviceSlots] = {};
         const int dev = current_device();
         if (dev < 0 || dev >= kDeviceSlots || !attr_done[dev]) {
             KM_CUDA(cudaFuncSetAttribute(rmsd_center_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kCenterMaxSmem));
+                                         (int)center_smem(3 * kCenterMaxAtoms)));
             if (dev >= 0 && dev < kDeviceSlots) attr_done[dev] = true;
         }
-        const size_t smem = (size_t)warps * 32 * center_stride(d) * sizeof(float);
-        int64_t g = ((n + 31) / 32 + warps - 1) / warps;
+        int64_t g = ((n + 31) / 32 + kCenterWarps - 1) / kCenterWarps;
         const int64_t cap = (int64_t)num_sms() * 16;
         if (g > cap) g = cap;
-        rmsd_center_tile_kernel<<<(unsigned)g, warps * 32, smem, s>>>(X, n, d, center_stride(d), Xc, G);
+        rmsd_center_tile_kernel<<<(unsigned)g, kCenterWarps * 32, center_smem(d), s>>>(X, n, d, center_stride(d), Xc,
+                                                                                        G);
     } else {
         rmsd_center_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(X, n, d, Xc, G);
     }
