@@ -303,9 +303,9 @@ __device__ __forceinline__ void rmsd_store(int64_t r, double bm, int bj, int32_t
     if (rmsd) rmsd[r] = bj < 0 ? __int_as_float(0x7fc00000) : __double2float_rn(sqrt(bm));
 }
 
-// One warp per frame, every pair solved in double.  For one or two atoms,
-// whose correlation matrices have rank at most one: the largest root is then
-// a double root, and qcp_bracket never holds.
+// One warp per frame, every pair solved in double.  Always for one or two
+// atoms, whose correlation matrices have rank at most one: the largest root is
+// then a double root, and qcp_bracket never holds.
 __global__ void __launch_bounds__(kRmsdWarps * 32) rmsd_assign_full_kernel(
     const float *__restrict__ Xc, const double *__restrict__ G, int64_t n, int d, const float *__restrict__ Ct,
     const double *__restrict__ H, int k, int32_t *__restrict__ labels, float *__restrict__ rmsd) {
@@ -442,9 +442,11 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &
 // from L1/L2, serves all F frames (9 F multiply-adds per 3 loads).
 // Per frame a list of the centers whose lower bound does not exceed the
 // smallest upper bound so far, with their correlation sums; at the end the
-// lists of all F frames are solved in double, one entry per lane.  A frame
-// whose list runs over (near-ties, or pairs without a bracket) has all its
-// pairs solved in double.
+// lists of all F frames are solved in double, one entry per lane.  Pairs
+// without a bracket (1%) fill the lists of large center sets: there a list more
+// than half full is solved after a group of centers (k = 1000, 58 atoms: 64,000
+// frames 5.2 -> 2.6 ms, 1,000 frames 1.38 -> 0.46).  A frame with many near-ties
+// has all its pairs solved in double.
 // Bound by the FP32 pipe: 9 n_atoms multiply-adds and about 140 operations of
 // the bracket per pair, with three warps in four waiting (ncu, 200,000 frames:
 // issue slots 40% busy, FP32 pipe 34%, FP64 pipe 33%).  1,000,000 frames of
@@ -455,6 +457,7 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &
 constexpr int kRmsdFrames = 4;
 constexpr int kRmsdAtoms = 96;  // atoms staged at a time
 constexpr int kRmsdList = 8;    // candidates kept per frame
+constexpr int kRmsdMany = 128;  // centers from which lists are solved on the way
 
 template <int F>
 struct RmsdWarpSmem {
@@ -464,9 +467,48 @@ struct RmsdWarpSmem {
     float lb[F][kRmsdList];
     int32_t j[F][kRmsdList];
     double ga[F];
+    double bm[F];     // the best of the entries solved so far
+    int32_t bj[F];    // (-1: none)
     int32_t cnt[F];   // entries listed
-    int32_t full[F];  // the list ran over
+    int32_t room[F];  // times that a full list may still be solved in between
+    int32_t full[F];  // every pair is solved
 };
+
+// Solves the entries of frame f's list, one per lane, into its best so far, and
+// empties the list.
+template <int F>
+__device__ __noinline__ void rmsd_solve_list(RmsdWarpSmem<F> &sm, int f, const double *__restrict__ H, int n_atoms) {
+    const int lane = threadIdx.x & 31;
+    const int cnt = sm.cnt[f];
+    double m = 0.0;
+    int j = -1;
+    if (lane < cnt) {
+        float S[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) S[e] = sm.S[f][lane][e];
+        j = sm.j[f][lane];
+        m = qcp_msd(S, sm.ga[f], H[j], n_atoms);
+    }
+#pragma unroll
+    for (int off = kRmsdList / 2; off > 0; off >>= 1) {
+        const double om = __shfl_xor_sync(0xffffffffu, m, off);
+        const int oj = __shfl_xor_sync(0xffffffffu, j, off);
+        if (rmsd_better(om, oj, m, j)) {
+            m = om;
+            j = oj;
+        }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        if (rmsd_better(m, j, sm.bm[f], sm.bj[f])) {
+            sm.bm[f] = m;
+            sm.bj[f] = j;
+        }
+        sm.cnt[f] = 0;
+        --sm.room[f];
+    }
+    __syncwarp();
+}
 
 // Brackets one frame's pairs with the warp's 32 centers, lists the ones that
 // the smallest upper bound (returned) does not rule out.  Out of line: few
@@ -554,7 +596,9 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 3) rmsd_assign_kernel(
         if (n_atoms <= kRmsdAtoms) stage(r0, 0, n_atoms);
         if (lane < F) {
             sm.ga[lane] = G[r0 + lane < n ? r0 + lane : r0];
+            sm.bj[lane] = -1;
             sm.cnt[lane] = 0;
+            sm.room[lane] = 1 + k / 64;  // half of what solving every pair takes
             sm.full[lane] = 0;
         }
         __syncwarp();
@@ -612,6 +656,12 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 3) rmsd_assign_kernel(
                     best[f] = rmsd_candidates<F>(sm, f, Sp[h], qu, tot, best[f], j, k);
                 }
             }
+            // here, where no sums are held, and not inside rmsd_candidates,
+            // whose calls would then spill them (4% of 1M x 58, k = 100)
+            if (k > kRmsdMany)
+                for (int f = 0; f < F; ++f)
+                    if (sm.cnt[f] > kRmsdList / 2 && sm.room[f] > 0 && !sm.full[f])
+                        rmsd_solve_list<F>(sm, f, H, n_atoms);
         }
         // Lane f < F keeps frame f's best; lane e solves entry e of the
         // frames' lists laid end to end.
@@ -628,8 +678,8 @@ __global__ void __launch_bounds__(kRmsdWarps * 32, 3) rmsd_assign_kernel(
             if (lane >= off) end += y;
         }
         const int total = __shfl_sync(0xffffffffu, end, 31);
-        double bm = 0.0;
-        int bj = -1;
+        double bm = lane < F ? sm.bm[lane] : 0.0;  // read where bj >= 0
+        int bj = lane < F ? sm.bj[lane] : -1;
         for (int e0 = 0; e0 < total; e0 += 32) {
             const int e = e0 + lane;
             // the frame whose range holds e
@@ -793,10 +843,23 @@ int launch_rmsd_assign_f(const float *Xc, const double *G, int64_t n, int d, con
     return KM_OK;
 }
 
+// Every pair in double by a warp per frame: for one or two atoms (see the
+// kernel), and for so few frames that each SM has no more than eight of these
+// warps, where the four frames of a bracket warp would wait for each other: with
+// one group of centers, or with rows that are staged again for every group; up to
+// sixteen warps per SM with long rows.  us, here and bracketed: k = 10, 1,000
+// frames of 58 atoms 67, 72, 2,000 95, 83; k = 100, 1,000 frames of 97 atoms 175,
+// 158, of 200 214, 232, 2,000 of 200 300, 247, of 400 400, 421, 4,000 of 400 694,
+// 475.
+bool rmsd_full_route(int64_t n, int d, int k) {
+    const int64_t sms = num_sms();
+    return d < 9 || (n <= 8 * sms && (k <= 32 || d >= 3 * 192)) || (n <= 16 * sms && d >= 3 * 384);
+}
+
 int launch_rmsd_assign(const float *Xc, const double *G, int64_t n, int d, const RmsdCenters &rc, int k,
                        int32_t *labels, float *rmsd, cudaStream_t s) {
     if (n == 0) return KM_OK;
-    if (d < 9) {
+    if (rmsd_full_route(n, d, k)) {
         rmsd_assign_full_kernel<<<rmsd_grid(n), kRmsdWarps * 32, 0, s>>>(Xc, G, n, d, rc.Ct, rc.H, k, labels,
                                                                         rmsd);
         KM_CUDA(cudaGetLastError());
