@@ -118,13 +118,33 @@ __global__ void __launch_bounds__(kRsFilterThreads) regspace_filter_kernel(
     }
 }
 
-// d > 32: the bits from the smallest squared distances (launch_assign_fp32).
-__global__ void __launch_bounds__(256) regspace_bits_kernel(const float *__restrict__ dist2, int64_t m, float t2,
+// d > 32: the bits from the smallest squared distances (launch_assign_fp32)
+// to the nc centers so far.  A minimum passes over distances that are NaN,
+// which stop a frame (not at least dmin).  Such a frame has no finite distance:
+// it is not finite itself, or center 0 has a NaN and is the only one.  So the
+// frames whose smallest distance is infinite meet every center again, a warp
+// for each; finite data has none.
+__global__ void __launch_bounds__(256) regspace_bits_kernel(const float *__restrict__ X, int64_t m, int d,
+                                                            const float *__restrict__ centers, int nc,
+                                                            const float *__restrict__ dist2, float t2,
                                                             uint32_t *__restrict__ bits) {
+    const int lane = threadIdx.x & 31;
+    const DenseRows rows{X, d};
     for (int64_t base = (int64_t)blockIdx.x * 256; base < m; base += (int64_t)gridDim.x * 256) {
         const int64_t i = base + threadIdx.x;
-        const unsigned word = __ballot_sync(0xffffffffu, i < m && (dist2 == nullptr || dist2[i] >= t2));
-        if ((threadIdx.x & 31) == 0 && i < m) bits[i >> 5] = word;
+        const float v = i < m && nc > 0 ? dist2[i] : 0.0f;
+        unsigned word = __ballot_sync(0xffffffffu, i < m && (nc == 0 || v >= t2));
+        for (unsigned look = word & __ballot_sync(0xffffffffu, v == __int_as_float(0x7f800000)); look;
+             look &= look - 1u) {
+            const int q = __ffs(look) - 1;
+            for (int j = 0; j < nc; ++j) {
+                if (!(warp_sqdist_exact(rows, i - lane + q, centers + (int64_t)j * d, d, lane) >= t2)) {
+                    word &= ~(1u << q);
+                    break;
+                }
+            }
+        }
+        if (lane == 0 && i < m) bits[i >> 5] = word;
     }
 }
 
@@ -432,7 +452,8 @@ int km_regspace(const float *X, int64_t n, int32_t d, double dmin, int32_t max_c
             int64_t g = (b - a + 255) / 256;
             const int64_t cap = (int64_t)num_sms() * 8;
             if (g > cap) g = cap;
-            regspace_bits_kernel<<<(unsigned)g, 256, 0, s>>>(any ? w.dist : nullptr, b - a, t2, w.bits);
+            regspace_bits_kernel<<<(unsigned)g, 256, 0, s>>>(X + a * d, b - a, d, centers, h_state[kRsCount],
+                                                             w.dist, t2, w.bits);
             KM_CUDA(cudaGetLastError());
             regspace_walk_wide_kernel<<<1, kRsWideThreads, 0, s>>>(X, a, b, d, w.bits, t2, max_centers, centers,
                                                                    w.list, w.added, w.state);
