@@ -66,6 +66,10 @@ size_t fu_smem(int d, int k) {
 // Doubles of one buffer of global sums: S (k x d), Q (k), and the counts.
 __host__ __device__ inline size_t fu_buf_doubles(int d, int k) { return (size_t)k * d + k + (k + 1) / 2; }
 
+// Sums of finite terms may leave the range of float32 (squares of 1e18 and
+// more); they are then made in float64.  Terms that are not finite leave a NaN.
+__device__ __forceinline__ bool fu_finite(double v) { return fabs(v) <= 1.7976931348623157e308; }
+
 // Sum over the CTA in a fixed order (warp shuffles, then warp 0), in every thread.
 __device__ __forceinline__ double fu_block_sum(double v, double *red) {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -190,7 +194,14 @@ __global__ void __launch_bounds__(kFuThreads, 2) small_lloyd_kernel(
                             s = t;
                             c = __fadd_rn(__fadd_rn(c, c2), e);
                         }
-                        if (lane == 0) atomicAdd(to, (double)s + (double)c);
+                        double w = (double)s + (double)c;
+                        if (__any_sync(0xffffffffu, !fu_finite(w))) {
+                            double a = (double)v;
+#pragma unroll 1
+                            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                            if (fu_finite(a)) w = a;
+                        }
+                        if (lane == 0) atomicAdd(to, w);
                     };
 #pragma unroll
                     for (int f = 0; f < DP; ++f)
@@ -220,6 +231,11 @@ __global__ void __launch_bounds__(kFuThreads, 2) small_lloyd_kernel(
                 CSum sum;
                 for (int e = h; e < m; e += lanes) sum.add(dev[order[off[j] + e] * stride + f]);
                 double v = sum.value();
+                if (!fu_finite(v)) {
+                    double a = 0.0;
+                    for (int e = h; e < m; e += lanes) a += (double)dev[order[off[j] + e] * stride + f];
+                    if (fu_finite(a)) v = a;
+                }
                 if (lanes == 4) {
                     v += __shfl_xor_sync(0xffffffffu, v, 1);
                     v += __shfl_xor_sync(0xffffffffu, v, 2);
