@@ -16,7 +16,8 @@
 //      32 lanes that meet on one center serialise them; so the 512 frames are
 //      sorted by label in shared memory (native integer counts) and four
 //      lanes per center and feature (one, where the centers outnumber a
-//      quarter of the frames) walk its members with compensated sums.
+//      quarter of the frames) walk its members with compensated float32 sums
+//      (in float64 where those leave the range of float32).
 //      A warp whose frames all have one label (consecutive frames often do)
 //      adds them by shuffles and stays out of the sort;
 //   2. adds its sums to the iteration's global sums and meets the other CTAs
