@@ -137,20 +137,29 @@ int resolve_precision(int precision, int d, int k, bool check_device) {
 //     d = 16..31, whose centers take more launches, up to k = 2048 (1M x 24: k
 //     = 1000 881 -> 545, k = 2000 1169 -> 945, and the gap closes by 300 per
 //     1,000 centers).
-//   * AUTO where the rule says FP32: from n k (3 d + 2) = 3.5e8, the exact
-//     kernel's instructions, on.  Above: 200k x 2, k = 250 72 -> 67; 200k x 5, k
-//     = 100 76 -> 68; 2M x 4, k = 500 964 -> 230.  Below: 200k x 2, k = 100 58
-//     -> 61; 60k x 5, k = 250 53 -> 59.  Not for d = 1: there the centers lie
-//     so densely that 5-89% of the frames are taken a second time.
-constexpr double kSmallMinWork = 3.5e8;
-bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_device) {
+//   * AUTO where the rule says FP32: from a line of n k (3 d + 2), the exact
+//     kernel's instructions, on.  With prepared centers 3.5e8, and 5e8 below
+//     65,536 frames, whose tiles leave SMs idle, 9e8 with two operand panels.
+//     Above: 200k x 5, k = 100 76 -> 68; 2M x 4, k = 500 964 -> 230; 20,000 x
+//     15, k = 980 108 -> 80; 20,000 x 19, k = 980 123 -> 106.  Below: 60k x 5, k =
+//     250 53 -> 59; 40,000 x 3, k = 980 68 -> 79; 7,000 x 19, k = 980 76 -> 97.
+//     A call that prepares its centers itself (once) takes 40 us more: from 1.5e9
+//     (75,000 x 5, k = 980 112 -> 125; 14,000 x 30, k = 980 126 -> 158; no slower at
+//     75,000 x 5, k = 1300 and 20,000 x 30, k = 980).  Not for d = 1: there the centers
+//     lie so densely that 5-89% of the frames are taken a second time.
+double small_min_work(int64_t n, int d, bool once) {
+    if (once) return 1.5e9;
+    if (d > 15) return 9e8;
+    return n < 65536 ? 5e8 : 3.5e8;
+}
+bool small_route(int precision, int prec, int64_t n, int d, int k, bool check_device, bool once = false) {
     // The cheap tests first: small calls are host-bound, and the plan lookups
     // took 2 of their 37 us.
     if (!small_shape_ok(d, k) || (d > 15 && k > 2048)) return false;
     const bool fp16 = prec == KM_PREC_FP16;
     if (!fp16) {
         if (precision != KM_PREC_AUTO || prec != KM_PREC_FP32) return false;
-        const bool enough = d >= 2 && (n < 0 || (double)n * k * (3 * d + 2) >= kSmallMinWork);
+        const bool enough = d >= 2 && (n < 0 || (double)n * k * (3 * d + 2) >= small_min_work(n, d, once));
         if (!enough && !small_forced()) return false;
     }
     if (!small_allowed() || (check_device && !tc_supported(d, k)) || tc_plan_set(d, k)) return false;
@@ -272,7 +281,7 @@ int assign_impl(const float *X, int64_t n, int32_t d, const float *C, int32_t k,
         set_error("no tensor-core kernel for d=%d, k=%d on this device", d, k);
         return KM_ERR_UNSUPPORTED;
     }
-    bool small = !ps && small_route(precision, prec, n, d, k, true);
+    bool small = !ps && small_route(precision, prec, n, d, k, true, true);
     small = small && ws && ws_bytes >= small_ws_bytes(n, d, k);
     KM_TRY(check_ws(ws, ws_bytes, assign_ws_bytes(n, d, k, prec, small)));
     TcBuffers b;
@@ -552,7 +561,7 @@ int km_profile_read(int32_t kind, double *ms_total, int64_t *launches) {
 size_t km_assign_workspace_size(int64_t n, int32_t d, int32_t k, int32_t precision) {
     if (check_shape(n, d, k) != KM_OK) return 0;
     const int prec = resolve_precision(precision, d, k, false);
-    return assign_ws_bytes(n, d, k, prec, small_route(precision, prec, n, d, k, false));
+    return assign_ws_bytes(n, d, k, prec, small_route(precision, prec, n, d, k, false, true));
 }
 
 int km_assign(const float *X, int64_t n, int32_t d, const float *C, int32_t k, int32_t precision,
