@@ -846,14 +846,16 @@ int launch_rmsd_assign_f(const float *Xc, const double *G, int64_t n, int d, con
 // Every pair in double by a warp per frame: for one or two atoms (see the
 // kernel), and for so few frames that each SM has no more than eight of these
 // warps, where the four frames of a bracket warp would wait for each other: with
-// one group of centers, or with rows that are staged again for every group; up to
-// sixteen warps per SM with long rows.  us, here and bracketed: k = 10, 1,000
-// frames of 58 atoms 67, 72, 2,000 95, 83; k = 100, 1,000 frames of 97 atoms 175,
-// 158, of 200 214, 232, 2,000 of 200 300, 247, of 400 400, 421, 4,000 of 400 694,
-// 475.
+// one group of centers, with 6 to 24 atoms, whose many near-ties fill the lists,
+// or with rows that are staged again for every group; up to sixteen warps per SM
+// with long rows.  us, here and bracketed: k = 10, 1,000 frames of 58 atoms 67,
+// 72, 2,000 95, 83; k = 100, 1,216 of 6 atoms 133, 168, of 8 134, 238; k = 500, 957
+// of 20 391, 1013, 1,216 of 4 388, 185; k = 100, 1,000 frames of 97 atoms 175, 158,
+// of 200 214, 232, 2,000 of 200 300, 247, of 400 400, 421, 4,000 of 400 694, 475.
 bool rmsd_full_route(int64_t n, int d, int k) {
     const int64_t sms = num_sms();
-    return d < 9 || (n <= 8 * sms && (k <= 32 || d >= 3 * 192)) || (n <= 16 * sms && d >= 3 * 384);
+    return d < 9 || (n <= 8 * sms && (k <= 32 || (d >= 18 && d <= 72) || d >= 3 * 192)) ||
+           (n <= 16 * sms && d >= 3 * 384);
 }
 
 int launch_rmsd_assign(const float *Xc, const double *G, int64_t n, int d, const RmsdCenters &rc, int k,
